@@ -60,6 +60,7 @@ RL_DEFINE_ERROR_TEXT()
 #define RED_BYTES (2 * CONSUMER_WARPS * 32 * 16)
 #define SMALL_BYTES 1024
 #define SMEM_BYTES (STAGES * STAGE_BYTES + RED_BYTES + SMALL_BYTES)
+static_assert(MAX_M < 256 && KB_PER_WARP == 2, "the arrival's address depends on both of a stage's loads and on M >> 8 being 0");
 static_assert(SMEM_BYTES <= 227 * 1024, "more shared memory than a block can have");
 
 struct StreamBarriers {
@@ -329,6 +330,7 @@ gemv_stream_kernel(const bf16* __restrict__ x, int ldx, const __grid_constant__ 
     // abort flag to the wait that has to wait: every instruction here is paid by every product warp for every
     // stage, and at 16 KB a stage the SM has 640 cycles for all of them together.
     const uint32_t full0 = smem_u32(&bars.full[0]), empty0 = smem_u32(&bars.empty[0]);
+    const uint32_t zero_bits = (uint32_t)M >> 8;  // (see below; M is at most MAX_M)
     uint32_t st = 0, parity = 0, st_off = 0;  // the stage to consume next, the parity of its `full` barrier, its offset in the ring
     int slice = first_item / units, unit = first_item - slice * units;
     for (int item = first_item; item < end_item && ok; ++item, ++done_items) {
@@ -370,7 +372,11 @@ gemv_stream_kernel(const bf16* __restrict__ x, int ldx, const __grid_constant__ 
               mma_bf16_16x8x16(acc[2 * j + 1], lo.z, hi.z, lo.w, hi.w, b[j].z, b[j].w);
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive_s(empty0 + 8 * st);
+            // The stage may be handed back once its pieces are in registers, not once they were asked for: the arrival goes
+            // another way than the loads, which wait behind the activations' loads of warps that have already gone on to the
+            // next slice of k, and the ring's next copy then overtook them (one product in four of a 2048 x 14336 matrix with
+            // 8 rows).  So its address is made from what was loaded; `zero_bits` is 0, which the compiler does not know.
+            if (lane == 0) mbar_arrive_s(empty0 + 8 * st + ((b[0].x ^ b[KB_PER_WARP - 1].w) & zero_bits));
             if (warp == 0 && lane == 0 && item == first_item && s == 0) rl_trace_event(5);  // first stage consumed
             st_off += STAGE_BYTES;
             if (++st == STAGES) {
