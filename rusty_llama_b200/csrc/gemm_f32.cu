@@ -1,16 +1,26 @@
-// The matrix product of the true 32-bit path: out[M, N] = x[M, K] . w[N, K]^T
+// The matrix products of the true 32-bit path: out[M, N] = x[M, K] . w[N, K]^T
 // with 32-bit inputs, FMA on the CUDA cores and no tensor-core instruction, so
 // nothing is rounded to a shorter type on the way (the reference's oracle is its
 // CPU backend, a 32-bit dot product per output: src/backend/cpu.rs:107-136).
 //
-// Each output element is one running sum over k = 0 .. K-1 in ascending order,
-// held by one thread; it depends neither on M nor on where the element lies in
-// its tile.  A row's result is therefore the same bits whether it is computed
+// The order of every output's sum is fixed: k is cut into consecutive chunks of
+// KCHUNK, counted from 0; a chunk is one running sum in ascending order, started
+// at zero; the chunks' sums are added up in ascending order.  It depends neither
+// on M nor on where the element lies in its tile nor on which of the two kernels
+// below runs.  A row's result is therefore the same bits whether it is computed
 // alone, inside a prompt or inside a batch.
 //
-// The same kernel with bfloat16 operands (widened on load, the same 32-bit sums, the result rounded
-// once, optionally through silu(gate) * up of neighbouring columns) takes the bfloat16 products whose
-// k is no multiple of 8: the streaming and tensor-core kernels move rows in 16-byte pieces and refuse
+// Why chunks: with one running sum over all of k, a product with few rows had a
+// chain of K dependent FMAs per output and one thread for it (N / 64 blocks of a
+// tile kernel: 32 of them for the 2048 features of an output projection).  A chunk
+// per thread gives K / 128 times the threads and chains of 128.
+//
+//   gemv_f32_kernel  up to GEMV_ROWS rows: bound by reading the weights.
+//   gemm_f32_kernel  more rows, and operands that cannot be moved 16 bytes at a time: bound by the FMA pipe.
+//
+// gemm_fma_kernel with bfloat16 operands (widened on load, 32-bit sums over k in ascending order, the
+// result rounded once, optionally through silu(gate) * up of neighbouring columns) takes the bfloat16
+// products whose k is no multiple of 8: the streaming and tensor-core kernels move rows in 16-byte pieces and refuse
 // those.  It is slow and only there so that every size a configuration allows runs.
 #include "common.cuh"
 
@@ -82,15 +92,277 @@ gemm_fma_kernel(const TA* __restrict__ x, int ldx, const TA* __restrict__ w, int
   }
 }
 
-RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K,
-                       cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0) RL_REFUSE(1, "gemm_f32: M=%d N=%d K=%d", M, N, K);
-  if (ldx < K || ldw < K || ldo < N) RL_REFUSE(2, "gemm_f32: leading sizes %d/%d/%d too small", ldx, ldw, ldo);
-  const int gy = (M + TM - 1) / TM;
-  if (gy > 65535) RL_REFUSE(3, "gemm_f32: %d rows exceed %d", M, 65535 * TM);
-  dim3 grid((N + TN - 1) / TN, gy);
-  gemm_fma_kernel<float, float, false><<<grid, 256, 0, stream>>>(x, ldx, w, ldw, out, ldo, M, N, K, 1.f, 0.f);
+// ------------------------------------------------------------------ 32-bit, few rows
+#define KCHUNK 128        // the summation order's chunk of k: part of the result, not a tuning knob
+#define GEMV_ROWS 16      // rows up to which the weights are streamed; above, a tile's reuse of them wins
+#define GEMV_THREADS 128  // one (feature, chunk) pair each
+#define GEMV_STAGES 4
+#define GEMV_SUB 32       // k of a chunk that a stage of the ring holds
+#define GEMV_ITEM (GEMV_SUB + 4)      // floats per item in a stage: 144 bytes, so that eight lanes' 16-byte reads meet all banks
+#define GEMV_XCHUNK (KCHUNK + 4)      // the same for the rows of x, per chunk
+#define GEMV_MAX_ITEMS 1024           // items of a block, whose sums wait in shared memory
+#define GEMV_RING_BYTES (GEMV_STAGES * GEMV_THREADS * GEMV_ITEM * 4)
+
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// MB rows of x (blockIdx.y names which) against R features a block.  A thread owns a (feature, chunk) pair at a time and walks
+// its 128 k's; 128 such pairs go through the ring side by side, 32 k's a stage, copied so that eight lanes take a 128-byte line.
+// The ring's first stages are asked for before the kernel before this one has ended: no kernel writes weights.
+// Bound: the weights' bytes.  Two blocks an SM keep 128 KB in flight; every block has R = ceil(N / (2 SMs)) features, so the
+// grid is one wave.
+template <int MB>
+__global__ void __launch_bounds__(GEMV_THREADS)
+gemv_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int ldw, float* __restrict__ out, int ldo,
+                int M, int N, int K, int R) {
+  extern __shared__ __align__(16) float sm[];
+  const int nch = (K + KCHUNK - 1) / KCHUNK;
+  float* ring = sm;
+  float* xs = ring + GEMV_STAGES * GEMV_THREADS * GEMV_ITEM;  // [MB][nch][GEMV_XCHUNK]
+  float* part = xs + MB * nch * GEMV_XCHUNK;                  // [MB][R * nch]
+  const int tid = threadIdx.x;
+  const int n0 = blockIdx.x * R, rows = min(R, N - n0);
+  const int m0 = blockIdx.y * MB, mb = min(MB, M - m0);
+  const int items = rows * nch, most = R * nch;
+  const int steps = (items + GEMV_THREADS - 1) / GEMV_THREADS * (KCHUNK / GEMV_SUB);
+  pdl_trigger();
+
+  // eight 16-byte pieces a thread and stage: piece tid % 8 of items tid / 8 + 16 j
+  const int piece = (tid & 7) * 4;
+  const float* src[8];
+  int k_at[8];
+  auto load = [&](int step) {
+    const int sub = step % (KCHUNK / GEMV_SUB);
+    float* dst = ring + (size_t)(step % GEMV_STAGES) * GEMV_THREADS * GEMV_ITEM;
+    if (sub == 0) {
+      const int base = step / (KCHUNK / GEMV_SUB) * GEMV_THREADS + tid / 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int item = base + 16 * j;
+        const int r = item / nch, c = item - r * nch;
+        k_at[j] = item < items ? c * KCHUNK + piece : K;
+        src[j] = w + (size_t)(n0 + min(r, rows - 1)) * ldw + c * KCHUNK + piece;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (k_at[j] + sub * GEMV_SUB < K) cp_async16(dst + (tid / 8 + 16 * j) * GEMV_ITEM + piece, src[j] + sub * GEMV_SUB);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < GEMV_STAGES - 1; ++i) {
+    if (i < steps) load(i);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  pdl_wait();
+  for (int i = tid; i < MB * (K / 4); i += GEMV_THREADS) {
+    const int m = i / (K / 4), k = (i - m * (K / 4)) * 4;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (m < mb) load4_g(x + (size_t)(m0 + m) * ldx + k, v);
+    store4(xs + (m * nch + k / KCHUNK) * GEMV_XCHUNK + k % KCHUNK, v);
+  }
+
+  float acc[MB];
+#pragma unroll
+  for (int m = 0; m < MB; ++m) acc[m] = 0.f;
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GEMV_STAGES - 2) : "memory");
+    __syncthreads();  // everyone's pieces of this stage (and, first, x) are there, and the stage before it is free
+    if (step + GEMV_STAGES - 1 < steps) load(step + GEMV_STAGES - 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    const int sub = step % (KCHUNK / GEMV_SUB);
+    const int item = step / (KCHUNK / GEMV_SUB) * GEMV_THREADS + tid;
+    const int c = item % nch;
+    const float* wr = ring + (size_t)(step % GEMV_STAGES) * GEMV_THREADS * GEMV_ITEM + tid * GEMV_ITEM;
+    const float* xr = xs + c * GEMV_XCHUNK + sub * GEMV_SUB;
+    const int left = item < items ? (K - c * KCHUNK - sub * GEMV_SUB) : 0;  // k's of this stage that exist (a multiple of 4)
+#pragma unroll
+    for (int i = 0; i < GEMV_SUB; i += 4) {
+      if (i < left) {
+        const float4 a = *reinterpret_cast<const float4*>(wr + i);
+#pragma unroll
+        for (int m = 0; m < MB; ++m) {
+          const float4 b = *reinterpret_cast<const float4*>(xr + m * nch * GEMV_XCHUNK + i);
+          acc[m] = fmaf(b.x, a.x, acc[m]);
+          acc[m] = fmaf(b.y, a.y, acc[m]);
+          acc[m] = fmaf(b.z, a.z, acc[m]);
+          acc[m] = fmaf(b.w, a.w, acc[m]);
+        }
+      }
+    }
+    if (sub == KCHUNK / GEMV_SUB - 1) {
+#pragma unroll
+      for (int m = 0; m < MB; ++m) {
+        if (item < items) part[m * most + item] = acc[m];
+        acc[m] = 0.f;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < rows * mb; i += GEMV_THREADS) {
+    const int m = i / rows, r = i - m * rows;
+    float total = 0.f;
+    for (int c = 0; c < nch; ++c) total += part[m * most + r * nch + c];
+    out[(size_t)(m0 + m) * ldo + n0 + r] = total;
+  }
+}
+
+// ------------------------------------------------------------------ 32-bit, many rows
+#define GEMM_TK 16
+static_assert(KCHUNK % GEMM_TK == 0 && KCHUNK % GEMV_SUB == 0, "stages must not straddle the chunks of the summation order");
+
+// A tile of BM x BN outputs by THREADS threads, RM x RN of them each (rows ty * RM .., columns tx * RN ..); the next 16 k's are
+// on their way into registers while the present ones are multiplied.  VEC: rows start on 16 bytes and K is a multiple of 4.
+template <int BM, int BN, int RM, int RN, bool VEC>
+__global__ void __launch_bounds__(BM * BN / (RM * RN))
+gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int ldw, float* __restrict__ out, int ldo,
+                int M, int N, int K) {
+  constexpr int THREADS = BM * BN / (RM * RN), LX = BM * GEMM_TK / 4 / THREADS, LW = BN * GEMM_TK / 4 / THREADS;
+  static_assert(LX * THREADS * 4 == BM * GEMM_TK && LW * THREADS * 4 == BN * GEMM_TK, "a stage must be whole loads of every thread");
+  __shared__ __align__(16) float xs[2][GEMM_TK][BM + 4];
+  __shared__ __align__(16) float ws[2][GEMM_TK][BN + 4];
+  const int tid = threadIdx.x, ty = tid / (BN / RN), tx = tid % (BN / RN);
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  float px[LX][4], pw[LW][4];
+  auto fetch4 = [&](const float* base, int ld, int row, int limit, int k, float* v) {
+    v[0] = v[1] = v[2] = v[3] = 0.f;
+    if (row >= limit) return;
+    const float* p = base + (size_t)row * ld + k;
+    if (VEC) {
+      if (k < K) load4(p, v);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (k + e < K) v[e] = p[e];
+    }
+  };
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int j = 0; j < LX; ++j) {
+      const int i = tid + j * THREADS;
+      fetch4(x, ldx, m0 + i % BM, M, k0 + i / BM * 4, px[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < LW; ++j) {
+      const int i = tid + j * THREADS;
+      fetch4(w, ldw, n0 + i % BN, N, k0 + i / BN * 4, pw[j]);
+    }
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int j = 0; j < LX; ++j) {
+      const int i = tid + j * THREADS;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) xs[buf][i / BM * 4 + e][i % BM] = px[j][e];
+    }
+#pragma unroll
+    for (int j = 0; j < LW; ++j) {
+      const int i = tid + j * THREADS;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ws[buf][i / BN * 4 + e][i % BN] = pw[j][e];
+    }
+  };
+  float acc[RM][RN], total[RM][RN];
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < RN; ++j) acc[i][j] = total[i][j] = 0.f;
+  fetch(0);
+  put(0);
+  __syncthreads();
+  const int tiles = (K + GEMM_TK - 1) / GEMM_TK;
+  for (int t = 0; t < tiles; ++t) {
+    if (t + 1 < tiles) fetch((t + 1) * GEMM_TK);
+    const int buf = t & 1;
+#pragma unroll
+    for (int c = 0; c < GEMM_TK; ++c) {
+      float a[RM], b[RN];
+#pragma unroll
+      for (int i = 0; i < RM; i += 4) load4(&xs[buf][c][ty * RM + i], a + i);
+#pragma unroll
+      for (int j = 0; j < RN; j += 2) {
+        const float2 v = *reinterpret_cast<const float2*>(&ws[buf][c][tx * RN + j]);
+        b[j] = v.x;
+        b[j + 1] = v.y;
+      }
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+    }
+    if ((t + 1) % (KCHUNK / GEMM_TK) == 0 || t + 1 == tiles) {
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) {
+          total[i][j] += acc[i][j];
+          acc[i][j] = 0.f;
+        }
+    }
+    if (t + 1 < tiles) put(buf ^ 1);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int m = m0 + ty * RM + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < RN; ++j) {
+      const int n = n0 + tx * RN + j;
+      if (n < N) out[(size_t)m * ldo + n] = total[i][j];
+    }
+  }
+}
+
+template <int MB>
+static int launch_gemv_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K, int R,
+                           size_t smem, cudaStream_t stream) {
+  if (cudaFuncSetAttribute(gemv_f32_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    RL_REFUSE(4, "gemm_f32: cannot get %zu bytes of shared memory", smem);
+  dim3 grid((N + R - 1) / R, (M + MB - 1) / MB);
+  RL_LAUNCH_CHECK(rl_launch(gemv_f32_kernel<MB>, grid, GEMV_THREADS, smem, stream, x, ldx, w, ldw, out, ldo, M, N, K, R));
+  return 0;
+}
+
+template <int BM, int BN, int RM, int RN>
+static int launch_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K, bool vec,
+                           cudaStream_t stream) {
+  const int gy = (M + BM - 1) / BM;
+  if (gy > 65535) RL_REFUSE(3, "gemm_f32: %d rows exceed %d", M, 65535 * BM);
+  dim3 grid((N + BN - 1) / BN, gy);
+  if (vec) gemm_f32_kernel<BM, BN, RM, RN, true><<<grid, BM * BN / (RM * RN), 0, stream>>>(x, ldx, w, ldw, out, ldo, M, N, K);
+  else gemm_f32_kernel<BM, BN, RM, RN, false><<<grid, BM * BN / (RM * RN), 0, stream>>>(x, ldx, w, ldw, out, ldo, M, N, K);
   RL_LAUNCH_RESULT();
+}
+
+static size_t gemv_f32_smem(int mb, int nch, int R) { return GEMV_RING_BYTES + (size_t)mb * nch * (GEMV_XCHUNK + R) * sizeof(float); }
+
+RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K, int sms,
+                       cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) RL_REFUSE(1, "gemm_f32: M=%d N=%d K=%d on %d SMs", M, N, K, sms);
+  if (ldx < K || ldw < K || ldo < N) RL_REFUSE(2, "gemm_f32: leading sizes %d/%d/%d too small", ldx, ldw, ldo);
+  const bool vec = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+  const int nch = (K + KCHUNK - 1) / KCHUNK;
+  if (M <= GEMV_ROWS && vec && nch <= GEMV_MAX_ITEMS) {
+    int R = (N + 2 * sms - 1) / (2 * sms);
+    if (R > GEMV_MAX_ITEMS / nch) R = GEMV_MAX_ITEMS / nch;
+    // as many rows of x a block as there are, up to four, while two blocks fit an SM; else one row (up to K of about 34000)
+    int mb = M == 1 ? 1 : M == 2 ? 2 : 4;
+    while (mb > 1 && gemv_f32_smem(mb, nch, R) > 112 * 1024) mb /= 2;
+    const size_t smem = gemv_f32_smem(mb, nch, R);
+    if (smem <= 224 * 1024) {
+      if (mb == 1) return launch_gemv_f32<1>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
+      if (mb == 2) return launch_gemv_f32<2>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
+      return launch_gemv_f32<4>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
+    }
+  }
+  // the largest tile that still gives every SM a block of its own
+  auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+  if (blocks(128, 64) >= 2 * sms) return launch_gemm_f32<128, 64, 8, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  if (blocks(64, 64) >= sms) return launch_gemm_f32<64, 64, 4, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  if (blocks(32, 64) >= sms) return launch_gemm_f32<32, 64, 4, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  return launch_gemm_f32<32, 32, 4, 2>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
 }
 
 // bfloat16 operands of any k and any alignment; out_dtype bfloat16 or float32.

@@ -17,6 +17,7 @@ import torch
 
 from ..errors import KernelError
 from . import build
+from .device import sm_count
 
 PAGE_SIZE = 64  # tokens per cache page; the attention kernels' key tile
 
@@ -298,7 +299,7 @@ def attn_generic(
     rc = lib.rl_attn_generic(
         _p(q), c_int(_dt(q, "attn_generic")), c_int(qs), _p(k_pages), _p(v_pages), _p(block_table),
         c_int(block_table.shape[1]), _p(tok_seq), _p(tok_pos), _p(out), c_int(out.stride(0)), c_int(T),
-        c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(PAGE_SIZE), c_int(window), c_float(scale), _stream(),
+        c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(PAGE_SIZE), c_int(window), c_float(scale), c_int(sm_count(q.device)), _stream(),
     )
     _check(lib, rc, "attn_generic")
     return out
@@ -546,7 +547,8 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     _cuda(out, "gemm_f32 out", torch.float32, contiguous=False)
     _need(tuple(out.shape) == (M, N), "gemm_f32: out has the wrong shape")
     lib = build.load("gemm_f32")
-    rc = lib.rl_gemm_f32(_p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_rows(out, "gemm_f32 out")), c_int(M), c_int(N), c_int(K), _stream())
+    rc = lib.rl_gemm_f32(_p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_rows(out, "gemm_f32 out")), c_int(M), c_int(N), c_int(K),
+                         c_int(sm_count(x.device)), _stream())
     _check(lib, rc, "gemm_f32")
     return out
 

@@ -1,0 +1,82 @@
+"""The 32-bit products and the 32-bit attention: each launch form (few rows or many, tiles of every size, rows that cannot be moved
+16 bytes at a time; heads of a kv head together or alone) against 64 bits, and against the other forms bit for bit."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from rusty_llama_b200.kernels import ops
+
+    return ops
+
+
+def product_bound(x, w):
+    """A sum of K products in chunks of 128: each result is off by at most (128 + K / 128 + 1) roundings of what is added up so far,
+    which is never more than sum |x w|."""
+    K = x.shape[1]
+    return (130 + K / 128) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+
+
+@pytest.mark.parametrize("K", [4, 124, 128, 132, 516, 2048, 5632])
+@pytest.mark.parametrize("N", [1, 37, 296, 700])
+@pytest.mark.parametrize("M", [1, 2, 3, 7, 16, 17, 70])
+def test_product_in_every_form(ops, M, N, K):
+    g = torch.Generator().manual_seed(M * 7919 + N * 31 + K)
+    x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    xd, wd = x.to(DEV), w.to(DEV)
+    out = ops.gemm_f32(xd, wd)
+    assert bool(((out.cpu().double() - x.double() @ w.double().T).abs() <= product_bound(x, w)).all())
+    # rows that start off a 16-byte boundary take the tile kernel's scalar loads: the same bits
+    wide = torch.zeros(M, K + 1, device=DEV)
+    wide[:, 1:] = xd
+    assert torch.equal(ops.gemm_f32(wide[:, 1:], wd), out)
+    # among many rows (larger tiles), and alone
+    many = torch.cat([xd, torch.randn(4000, K, generator=g).to(DEV)])
+    for rows in (400, 1000, 4000):
+        assert torch.equal(ops.gemm_f32(many[: M + rows], wd)[:M], out)
+    assert torch.equal(ops.gemm_f32(xd[M - 1 :], wd)[0], out[M - 1])
+
+
+def test_product_of_a_very_long_k(ops):
+    """Rows too long for the few-row kernel's shared memory (K above 34000) go to the tile kernel."""
+    g = torch.Generator().manual_seed(5)
+    x, w = torch.randn(3, 40000, generator=g), torch.randn(9, 40000, generator=g)
+    out = ops.gemm_f32(x.to(DEV), w.to(DEV))
+    assert bool(((out.cpu().double() - x.double() @ w.double().T).abs() <= product_bound(x, w)).all())
+    assert torch.equal(ops.gemm_f32(x[:, :20000].to(DEV), w[:, :20000].to(DEV))[1], ops.gemm_f32(x[1:2, :20000].to(DEV), w[:, :20000].to(DEV))[0])
+
+
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("H, K, hd", [(8, 1, 64), (6, 2, 40), (16, 2, 128), (5, 5, 30), (6, 1, 256), (12, 4, 18)])
+def test_attention_of_few_and_of_many_tokens(ops, H, K, hd, window):
+    g = torch.Generator().manual_seed(H * 100 + hd + window)
+    L = 600
+    pages = (L + 63) // 64
+    k, v = torch.randn(L, K, hd, generator=g), torch.randn(L, K, hd, generator=g)
+    order = torch.randperm(pages, generator=g)
+    k_pages, v_pages = torch.zeros(pages, K, 64, hd), torch.zeros(pages, K, 64, hd)
+    for i in range(L):
+        k_pages[order[i // 64], :, i % 64], v_pages[order[i // 64], :, i % 64] = k[i], v[i]
+    table = order.to(torch.int32)[None].to(DEV)
+    pos = torch.cat([torch.arange(0, 100), torch.arange(250, 330), torch.arange(L - 120, L)]).to(torch.int32)
+    q = torch.randn(len(pos), H * hd, generator=g)
+    seq = torch.zeros(len(pos), dtype=torch.int32)
+    args = (k_pages.to(DEV), v_pages.to(DEV), table)
+    many = ops.attn_generic(q.to(DEV), *args, seq.to(DEV), pos.to(DEV), H, K, hd, window=window)
+    n = len(pos)
+    scores = torch.einsum("thd,khd->htk", q.view(n, H, hd).double(), k.repeat_interleave(H // K, 1).double()) / hd ** 0.5
+    back = pos[:, None] - torch.arange(L)[None]
+    scores = scores.masked_fill((back < 0) | ((back >= window) if window else (back < 0)), float("-inf"))
+    ref = torch.einsum("htk,khd->thd", torch.softmax(scores, -1), v.repeat_interleave(H // K, 1).double()).reshape(n, H * hd)
+    # a weight is off by the rounding of its score (hd terms of at most 6 in all) and of exp (2 ulp) and of the sums (32 terms, then groups, then
+    # warps): relative 2^-24 times (6 hd + 70), and no result exceeds the largest value
+    bound = 2.0 ** -24 * (hd * 6.0 + 70) * float(v.abs().max())
+    assert float((many.cpu().double() - ref).abs().max()) <= bound
+    for i in (0, 1, 31, 32, 99, 100, n - 1):  # one token: other heads per block, the same bits
+        one = ops.attn_generic(q[i : i + 1].to(DEV), *args, seq[i : i + 1].to(DEV), pos[i : i + 1].to(DEV), H, K, hd, window=window)
+        assert torch.equal(one[0], many[i])
