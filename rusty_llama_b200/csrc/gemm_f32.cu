@@ -15,8 +15,11 @@
 // tile kernel: 32 of them for the 2048 features of an output projection).  A chunk
 // per thread gives K / 128 times the threads and chains of 128.
 //
-//   gemv_f32_kernel  up to GEMV_ROWS rows: bound by reading the weights.
-//   gemm_f32_kernel  more rows, and operands that cannot be moved 16 bytes at a time: bound by the FMA pipe.
+//   gemv_f32_kernel  up to GEMV_ROWS rows: bound by reading the weights.  One row of 11264 x 2048: 17.4 us, 5.3 TB/s; 2048 x 5632: 12 us, 3.9 TB/s.
+//   gemm_f32_kernel  more rows, and operands that cannot be moved 16 bytes at a time: bound by the FMA pipe.  283 rows of
+//                    11264 x 2048: 344 us, 38 TFLOP/s; of 2048 x 2048, where the tiles are few: 84 us, 28 TFLOP/s.
+// Prompts of 219 and 64 tokens and twelve decode steps of both on three layers of d 2048 and ff 5632: 60.9 ms in one kernel that
+// held 64 x 64 tiles in registers whatever the rows, 6.1 ms in these two.
 //
 // gemm_fma_kernel with bfloat16 operands (widened on load, 32-bit sums over k in ascending order, the
 // result rounded once, optionally through silu(gate) * up of neighbouring columns) takes the bfloat16
@@ -94,13 +97,13 @@ gemm_fma_kernel(const TA* __restrict__ x, int ldx, const TA* __restrict__ w, int
 
 // ------------------------------------------------------------------ 32-bit, few rows
 #define KCHUNK 128        // the summation order's chunk of k: part of the result, not a tuning knob
-#define GEMV_ROWS 16      // rows up to which the weights are streamed; above, a tile's reuse of them wins
+#define GEMV_ROWS 8       // rows up to which the weights are streamed (measured, gate/up of 11264 x 2048: 8 rows 65 us, 16 rows 109 us; 17 rows in tiles 71 us)
 #define GEMV_THREADS 128  // one (feature, chunk) pair each
-#define GEMV_STAGES 4
+#define GEMV_STAGES 3
 #define GEMV_SUB 32       // k of a chunk that a stage of the ring holds
 #define GEMV_ITEM (GEMV_SUB + 4)      // floats per item in a stage: 144 bytes, so that eight lanes' 16-byte reads meet all banks
 #define GEMV_XCHUNK (KCHUNK + 4)      // the same for the rows of x, per chunk
-#define GEMV_MAX_ITEMS 1024           // items of a block, whose sums wait in shared memory
+#define GEMV_MAX_ITEMS 512            // items of a block, whose sums wait in shared memory
 #define GEMV_RING_BYTES (GEMV_STAGES * GEMV_THREADS * GEMV_ITEM * 4)
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
@@ -110,8 +113,8 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 // MB rows of x (blockIdx.y names which) against R features a block.  A thread owns a (feature, chunk) pair at a time and walks
 // its 128 k's; 128 such pairs go through the ring side by side, 32 k's a stage, copied so that eight lanes take a 128-byte line.
 // The ring's first stages are asked for before the kernel before this one has ended: no kernel writes weights.
-// Bound: the weights' bytes.  Two blocks an SM keep 128 KB in flight; every block has R = ceil(N / (2 SMs)) features, so the
-// grid is one wave.
+// Bound: the weights' bytes.  Two blocks an SM keep 64 KB in flight; every block has R = ceil(N / (2 SMs)) features (a grid of
+// one wave) until their sums take more shared memory than that leaves.
 template <int MB>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int ldw, float* __restrict__ out, int ldo,
@@ -209,87 +212,79 @@ gemv_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
 }
 
 // ------------------------------------------------------------------ 32-bit, many rows
-#define GEMM_TK 16
+#define GEMM_TK 32
+#define GEMM_ROW (GEMM_TK + 4)  // floats per row of a stage: 144 bytes, so that rows next to each other start four banks apart
+#define GEMM_STAGES 4
+#define GEMM_THREADS 128
 static_assert(KCHUNK % GEMM_TK == 0 && KCHUNK % GEMV_SUB == 0, "stages must not straddle the chunks of the summation order");
 
-// A tile of BM x BN outputs by THREADS threads, RM x RN of them each (rows ty * RM .., columns tx * RN ..); the next 16 k's are
-// on their way into registers while the present ones are multiplied.  VEC: rows start on 16 bytes and K is a multiple of 4.
+// A tile of BM x BN outputs by 128 threads, RM x RN of them each: thread (ty, tx) has rows ty + (128 RN / BN) i and columns
+// tx + (BN / RN) j, so that a warp's 16-byte reads along k meet all banks.  Three stages of 32 k's are on their way while one is
+// multiplied (with one stage ahead in registers, the loads' latency was three quarters of the time).  VEC: rows start on 16
+// bytes and K is a multiple of 4; otherwise a stage is put into shared memory number by number.
 template <int BM, int BN, int RM, int RN, bool VEC>
-__global__ void __launch_bounds__(BM * BN / (RM * RN))
+__global__ void __launch_bounds__(GEMM_THREADS)
 gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int ldw, float* __restrict__ out, int ldo,
                 int M, int N, int K) {
-  constexpr int THREADS = BM * BN / (RM * RN), LX = BM * GEMM_TK / 4 / THREADS, LW = BN * GEMM_TK / 4 / THREADS;
-  static_assert(LX * THREADS * 4 == BM * GEMM_TK && LW * THREADS * 4 == BN * GEMM_TK, "a stage must be whole loads of every thread");
-  __shared__ __align__(16) float xs[2][GEMM_TK][BM + 4];
-  __shared__ __align__(16) float ws[2][GEMM_TK][BN + 4];
-  const int tid = threadIdx.x, ty = tid / (BN / RN), tx = tid % (BN / RN);
+  constexpr int TX = BN / RN, TY = BM / RM, PIECES = GEMM_TK / 4;
+  static_assert(TX * TY == GEMM_THREADS && (BM + BN) * PIECES % GEMM_THREADS == 0, "a stage must be whole loads of every thread");
+  extern __shared__ __align__(16) float sm[];  // [STAGES][BM + BN][GEMM_ROW]
+  const int tid = threadIdx.x, ty = tid / TX, tx = tid % TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float px[LX][4], pw[LW][4];
-  auto fetch4 = [&](const float* base, int ld, int row, int limit, int k, float* v) {
-    v[0] = v[1] = v[2] = v[3] = 0.f;
-    if (row >= limit) return;
-    const float* p = base + (size_t)row * ld + k;
-    if (VEC) {
-      if (k < K) load4(p, v);
-    } else {
+  auto load = [&](int t) {
+    float* stage = sm + (size_t)(t % GEMM_STAGES) * (BM + BN) * GEMM_ROW;
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (k + e < K) v[e] = p[e];
+    for (int j = 0; j < (BM + BN) * PIECES / GEMM_THREADS; ++j) {
+      const int i = tid + j * GEMM_THREADS, row = i / PIECES, k = t * GEMM_TK + i % PIECES * 4;
+      const bool is_x = row < BM;
+      const int r = is_x ? m0 + row : n0 + row - BM;
+      const bool here = r < (is_x ? M : N);
+      const float* src = is_x ? x + (size_t)(here ? r : 0) * ldx + k : w + (size_t)(here ? r : 0) * ldw + k;
+      float* dst = stage + row * GEMM_ROW + i % PIECES * 4;
+      if (VEC) {  // zeros for what does not exist
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                     "l"(here && k < K ? src : (is_x ? x : w)), "r"(here && k < K ? 16 : 0) : "memory");
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) dst[e] = (here && k + e < K) ? src[e] : 0.f;
+      }
     }
-  };
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int j = 0; j < LX; ++j) {
-      const int i = tid + j * THREADS;
-      fetch4(x, ldx, m0 + i % BM, M, k0 + i / BM * 4, px[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < LW; ++j) {
-      const int i = tid + j * THREADS;
-      fetch4(w, ldw, n0 + i % BN, N, k0 + i / BN * 4, pw[j]);
-    }
-  };
-  auto put = [&](int buf) {
-#pragma unroll
-    for (int j = 0; j < LX; ++j) {
-      const int i = tid + j * THREADS;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) xs[buf][i / BM * 4 + e][i % BM] = px[j][e];
-    }
-#pragma unroll
-    for (int j = 0; j < LW; ++j) {
-      const int i = tid + j * THREADS;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) ws[buf][i / BN * 4 + e][i % BN] = pw[j][e];
-    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   float acc[RM][RN], total[RM][RN];
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
     for (int j = 0; j < RN; ++j) acc[i][j] = total[i][j] = 0.f;
-  fetch(0);
-  put(0);
-  __syncthreads();
   const int tiles = (K + GEMM_TK - 1) / GEMM_TK;
+#pragma unroll
+  for (int t = 0; t < GEMM_STAGES - 1; ++t) {
+    if (t < tiles) load(t);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   for (int t = 0; t < tiles; ++t) {
-    if (t + 1 < tiles) fetch((t + 1) * GEMM_TK);
-    const int buf = t & 1;
+    asm volatile("cp.async.wait_group %0;" ::"n"(GEMM_STAGES - 2) : "memory");
+    __syncthreads();  // this stage is there for everyone, and everyone has left the one that is loaded next
+    if (t + GEMM_STAGES - 1 < tiles) load(t + GEMM_STAGES - 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* xs = sm + (size_t)(t % GEMM_STAGES) * (BM + BN) * GEMM_ROW;
+    const float* ws = xs + BM * GEMM_ROW;
 #pragma unroll
-    for (int c = 0; c < GEMM_TK; ++c) {
-      float a[RM], b[RN];
+    for (int k = 0; k < GEMM_TK; k += 4) {
+      float4 a[RM], b[RN];
 #pragma unroll
-      for (int i = 0; i < RM; i += 4) load4(&xs[buf][c][ty * RM + i], a + i);
+      for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + (ty + TY * i) * GEMM_ROW + k);
 #pragma unroll
-      for (int j = 0; j < RN; j += 2) {
-        const float2 v = *reinterpret_cast<const float2*>(&ws[buf][c][tx * RN + j]);
-        b[j] = v.x;
-        b[j + 1] = v.y;
-      }
+      for (int j = 0; j < RN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + (tx + TX * j) * GEMM_ROW + k);
 #pragma unroll
       for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < RN; ++j) {
+          acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+          acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+          acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+          acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        }
     }
     if ((t + 1) % (KCHUNK / GEMM_TK) == 0 || t + 1 == tiles) {
 #pragma unroll
@@ -300,16 +295,14 @@ gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
           acc[i][j] = 0.f;
         }
     }
-    if (t + 1 < tiles) put(buf ^ 1);
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
-    const int m = m0 + ty * RM + i;
+    const int m = m0 + ty + TY * i;
     if (m >= M) continue;
 #pragma unroll
     for (int j = 0; j < RN; ++j) {
-      const int n = n0 + tx * RN + j;
+      const int n = n0 + tx + TX * j;
       if (n < N) out[(size_t)m * ldo + n] = total[i][j];
     }
   }
@@ -330,9 +323,12 @@ static int launch_gemm_f32(const float* x, int ldx, const float* w, int ldw, flo
                            cudaStream_t stream) {
   const int gy = (M + BM - 1) / BM;
   if (gy > 65535) RL_REFUSE(3, "gemm_f32: %d rows exceed %d", M, 65535 * BM);
+  constexpr int smem = GEMM_STAGES * (BM + BN) * GEMM_ROW * 4;
   dim3 grid((N + BN - 1) / BN, gy);
-  if (vec) gemm_f32_kernel<BM, BN, RM, RN, true><<<grid, BM * BN / (RM * RN), 0, stream>>>(x, ldx, w, ldw, out, ldo, M, N, K);
-  else gemm_f32_kernel<BM, BN, RM, RN, false><<<grid, BM * BN / (RM * RN), 0, stream>>>(x, ldx, w, ldw, out, ldo, M, N, K);
+  auto kern = vec ? gemm_f32_kernel<BM, BN, RM, RN, true> : gemm_f32_kernel<BM, BN, RM, RN, false>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    RL_REFUSE(5, "gemm_f32: cannot get %d bytes of shared memory", smem);
+  kern<<<grid, GEMM_THREADS, smem, stream>>>(x, ldx, w, ldw, out, ldo, M, N, K);
   RL_LAUNCH_RESULT();
 }
 
@@ -357,12 +353,21 @@ RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* 
       return launch_gemv_f32<4>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
     }
   }
-  // the largest tile that still gives every SM a block of its own
-  auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
-  if (blocks(128, 64) >= 2 * sms) return launch_gemm_f32<128, 64, 8, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
-  if (blocks(64, 64) >= sms) return launch_gemm_f32<64, 64, 4, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
-  if (blocks(32, 64) >= sms) return launch_gemm_f32<32, 64, 4, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
-  return launch_gemm_f32<32, 32, 4, 2>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  // the tile with the least work on the busiest SM: its blocks there, times the tile's outputs, times what an output costs with
+  // that many outputs a thread (shared-memory reads per FMA)
+  const int tile[4][2] = {{64, 64}, {64, 32}, {32, 32}, {128, 64}};
+  const float cost[4] = {1.05f, 1.2f, 1.5f, 1.0f};
+  int best = 0;
+  float least = INFINITY;
+  for (int i = 0; i < 4; ++i) {
+    const long long blocks = (long long)((M + tile[i][0] - 1) / tile[i][0]) * ((N + tile[i][1] - 1) / tile[i][1]);
+    const float c = (float)((blocks + sms - 1) / sms) * tile[i][0] * tile[i][1] * cost[i];
+    if (c < least) least = c, best = i;
+  }
+  if (best == 0) return launch_gemm_f32<64, 64, 8, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  if (best == 1) return launch_gemm_f32<64, 32, 4, 4>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  if (best == 2) return launch_gemm_f32<32, 32, 4, 2>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
+  return launch_gemm_f32<128, 64, 8, 8>(x, ldx, w, ldw, out, ldo, M, N, K, vec, stream);
 }
 
 // bfloat16 operands of any k and any alignment; out_dtype bfloat16 or float32.
