@@ -250,12 +250,17 @@ moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* __restrict__ ord
       place[i] = r;
       ++r;
     }
-  const int c = cnt[e];
-  for (int k = tid; k * tile_rows < c; k += PLAN_THREADS) {
+  // As few tiles as hold the expert's rows.  Where the products take tiles of any multiple of 16 rows (the heights from 128 on) they
+  // are equally high: 300 rows in two tiles of 160 and 140 instead of 256 and 44 (no last tile is empty: the others hold at most
+  // tile_rows each).
+  const int c = cnt[e], n_tiles = (c + tile_rows - 1) / tile_rows;
+  int high = tile_rows;
+  if (tile_rows >= 128 && n_tiles > 0) high = min(tile_rows, ((c + n_tiles - 1) / n_tiles + 15) & ~15);
+  for (int k = tid; k < n_tiles; k += PLAN_THREADS) {
     int* t = tiles + 1 + 3 * (first_tile + k);
     t[0] = e;
-    t[1] = first_row + k * tile_rows;
-    t[2] = min(tile_rows, c - k * tile_rows);
+    t[1] = first_row + k * high;
+    t[2] = min(high, c - k * high);
   }
 }
 

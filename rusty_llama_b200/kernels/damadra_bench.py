@@ -136,7 +136,7 @@ def kernel_table(z: dict, T: int, batch: int, ctx: int, peaks: dict) -> Dict[str
         us = timed(lambda: ops.moe_choose(linear(x, wr16, out_dtype=torch.float32), corr, E + I, top))
         us_like = timed(lambda: ops.moe_router(x, wr[:E], corr[:E], E, top))
         note(f"{tag}_router", us, (E + I) * d * 2 + rows * d * 2, 0, ("moe_router (32-bit rows)", us_like, E * d * 4 + rows * d * 2, 0))
-        tile_rows = 128 if rows * top >= 64 * E else 32
+        tile_rows = ops.moe_mma_tile_rows(rows * top, E)
         ids, wts, _ = ops.moe_router(x, wr, corr, E + I, top)
         ids_l, wts_l, _ = ops.moe_router(x, wr[:E], corr[:E], E, top)
         us, us_like = timed(lambda: ops.moe_plan(ids, E, tile_rows)), timed(lambda: ops.moe_plan(ids_l, E, tile_rows))

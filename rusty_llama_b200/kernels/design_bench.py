@@ -200,9 +200,9 @@ def kernel_table(z: dict, T: int, batch: int, ctx: int, peaks: dict) -> Dict[str
         us = mb._time(lambda i: ops.moe_router(x, wr, bias, E, top), 1, **it)
         note(f"{tag}_router", us, (E + 1) * d * 4 + rows * d * 2, 0)
         ids, wts, gate = ops.moe_router(x, wr, bias, E, top)
-        us = mb._time(lambda i: ops.moe_plan(ids, E, 128 if rows * top >= 64 * E else 32), 1, **it)
+        us = mb._time(lambda i: ops.moe_plan(ids, E, ops.moe_mma_tile_rows(rows * top, E)), 1, **it)
         note(f"{tag}_plan", us, rows * top * 12, 0)
-        tile_rows = 128 if rows * top >= 64 * E else 32  # as `RoutedExperts.forward` chooses
+        tile_rows = ops.moe_mma_tile_rows(rows * top, E)  # as `RoutedExperts.forward` chooses
         order, place, tiles, max_tiles = ops.moe_plan(ids, E, tile_rows)
         used = int(torch.unique(ids).numel())
         us = mb._time(lambda i: ops.moe_gemm(x, wg, tiles, max_tiles, rows * top, order=order, gather_div=top, w2=wu, tile_rows=tile_rows), 1, **it)

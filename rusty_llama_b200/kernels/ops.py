@@ -787,6 +787,9 @@ _STATUS_NAMES = {
     32: "gemv_stream: the copying lane (for a free stage)", 34: "gemv_stream: a product warp (for a stage's weights)",
     35: "gemv_stream: a storing warp (for an item's sums)", 36: "gemv_stream: shared memory not aligned",
     37: "gemv_stream: a product warp (for a free sum buffer)",
+    61: "grouped_gemm_tc: the copying lane (for a free stage)", 62: "grouped_gemm_tc: the tensor-core issuer (for a stage's data)",
+    63: "grouped_gemm_tc: a result warp (for a finished accumulator)", 64: "grouped_gemm_tc: the tensor-core issuer (for a free accumulator)",
+    65: "grouped_gemm_tc: a gathering warp (for a free stage)",
     51: "attn_decode_tma: the copying lane (for a free stage)", 52: "attn_decode_tma: a product warp (for a page)",
     56: "attn_decode_tma: shared memory not aligned",
 }
@@ -1135,6 +1138,9 @@ def latent_prep(
     return ql_out
 
 
+HEAD_LINEAR_MMA_MAX_ROWS = 32  # rows up to which head products go to mma.sync tiles of 32 rows (a decode step); above, to tcgen05
+
+
 def head_linear(
     x: torch.Tensor, x_head_stride: int, w: torch.Tensor, out: torch.Tensor, out_head_stride: int,
     gate: Optional[torch.Tensor] = None, gate_head_stride: int = 0,
@@ -1157,6 +1163,14 @@ def head_linear(
         ldg = _rows(gate, "head_linear gate")
         _need(gate.shape[0] == M and (H - 1) * gate_head_stride + N <= gate.shape[1], "head_linear: gate rows do not fit")
     if x.dtype == torch.bfloat16 and grouped_gemm_takes(K, ldx, x_head_stride) and x.data_ptr() % 16 == 0:
+        if M > HEAD_LINEAR_MMA_MAX_ROWS and w.data_ptr() % 16 == 0:
+            lib = build.load("grouped_gemm_tc")
+            rc = lib.rl_head_linear_tc(
+                _p(x), c_int(ldx), c_int(x_head_stride), _p(w), _p(out), c_int(ldo), c_int(out_head_stride), _p(gate), c_int(ldg),
+                c_int(gate_head_stride), c_int(M), c_int(H), c_int(N), c_int(K), _p(_tc_status_word(x.device)), *_wt(), _stream(),
+            )
+            _check(lib, rc, "head_linear_tc")
+            return out
         lib = build.load("grouped_gemm")
         rc = lib.rl_head_linear_mma(
             _p(x), c_int(ldx), c_int(x_head_stride), _p(w), _p(out), c_int(ldo), c_int(out_head_stride), _p(gate), c_int(ldg),
@@ -1278,7 +1292,21 @@ def moe_table_lookup(tokens: torch.Tensor, table: torch.Tensor, n_experts: int):
     return ids, weights
 
 
-MOE_MMA_TILE_ROWS = (32, 128)  # tile heights the tensor-core products are built for
+MOE_MMA_TILE_ROWS = (32, 128, 256)  # tile heights the tensor-core products are built for
+
+
+# Rows per expert from which they are put next to each other before the product instead of being gathered by its copies, which
+# every block of features repeats (gate and up of experts of 1408 x 2048: 37 rows each 129 us before, 123 by copies; 192 rows each
+# 181 before, 297 by copies).
+MOE_GATHER_ROWS_PER_EXPERT = 64
+
+
+def moe_mma_tile_rows(n_pairs: int, n_experts: int) -> int:
+    """The tile height for n_pairs (token, choice) pairs: one tile should hold all rows of nearly every expert, since each tile of an
+    expert reads its matrices again; beyond that a lower tile leaves more shared memory for weights on their way.  With rows spread
+    evenly an expert seldom gets more than twice the average (gate and up of 64 experts of 1408 x 2048, tiles of 32 / 128 / 256: 12 rows
+    each 118 / 118 / 129 us, 37 rows 177 / 123 / 137, 192 rows 604 / 225 / 181)."""
+    return 32 if n_pairs <= 16 * n_experts else 128 if n_pairs <= 64 * n_experts else 256
 
 
 def moe_max_tiles(n_pairs: int, n_experts: int, tile_rows: int = 0) -> int:
@@ -1326,13 +1354,18 @@ def moe_gemm(
     tile_rows = tile_rows or moe_tile_rows()
     _need(act is None or (act == "relu2") == (w2 is None), "moe_gemm: an activation of one argument goes with one matrix, a gate's with two")
     alpha, limit = _act(act)
-    if x.dtype == torch.bfloat16 and tile_rows in MOE_MMA_TILE_ROWS and grouped_gemm_takes(K, x.stride(0), 0) and x.data_ptr() % 16 == 0:
-        lib = build.load("grouped_gemm")
-        rc = lib.rl_moe_gemm_mma(
-            _p(x), c_int(x.stride(0)), _p(order), c_int(gather_div), _p(w), _p(w2), _p(out), c_int(_dt(out, "moe_gemm out")), c_int(N),
-            _p(tiles), c_int(max_tiles), c_int(tile_rows), c_int(N), c_int(K), alpha, limit, _stream(),
+    if x.dtype == torch.bfloat16 and tile_rows in MOE_MMA_TILE_ROWS and grouped_gemm_takes(K, x.stride(0), 0) and (x.data_ptr() | w.data_ptr()) % 16 == 0:
+        lib = build.load("grouped_gemm_tc")
+        if order is not None and n_rows >= MOE_GATHER_ROWS_PER_EXPERT * E:
+            rows = torch.empty((n_rows, K), dtype=x.dtype, device=x.device)
+            rc = lib.rl_moe_gather_rows(_p(x), c_int(x.stride(0)), c_int(x.shape[0]), _p(order), c_int(gather_div), _p(rows), c_int(n_rows), c_int(K), _stream())
+            _check(lib, rc, "moe_gather_rows")
+            x, order = rows, None
+        rc = lib.rl_moe_gemm_tc(
+            _p(x), c_int(x.stride(0)), c_int(x.shape[0]), _p(order), c_int(gather_div), _p(w), _p(w2), _p(out), c_int(_dt(out, "moe_gemm out")), c_int(N),
+            _p(tiles), c_int(max_tiles), c_int(tile_rows), c_int(E), c_int(N), c_int(K), alpha, limit, _p(_tc_status_word(x.device)), *_wt(), _stream(),
         )
-        _check(lib, rc, "moe_gemm_mma")
+        _check(lib, rc, "moe_gemm_tc")
         return out
     _need(tile_rows == moe_tile_rows(), f"moe_gemm: the plain kernel wants tiles of {moe_tile_rows()} rows, the plan has {tile_rows}")
     lib = build.load("moe")

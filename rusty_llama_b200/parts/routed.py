@@ -149,11 +149,10 @@ class RoutedExperts(FeedForward):
                 ids, weights, gate = ops.moe_choose(linear(xn, self.w_router16, out_dtype=torch.float32), self.bias, self.choices, self.top, **how)
             else:
                 ids, weights, gate = ops.moe_router(xn, self.w_router, self.bias, self.choices, self.top, **how)
-        # the height of a row tile: 128 once the experts get that many rows on average (a prompt step), else 32; the plain
-        # kernels of a 32-bit run have their own
+        # the height of a row tile; the plain kernels (32-bit runs, sizes that break 16-byte rows) have their own
         tile_rows = 0
-        if xn.dtype == torch.bfloat16 and self.d % 8 == 0 and self.ff % 8 == 0:  # (else the plain products, 16-byte rows or not)
-            tile_rows = 128 if T * self.top >= 64 * self.E else 32
+        if xn.dtype == torch.bfloat16 and self.d % 8 == 0 and self.ff % 8 == 0:
+            tile_rows = ops.moe_mma_tile_rows(T * self.top, self.E)
         order, place, tiles, max_tiles = ops.moe_plan(ids, self.E, tile_rows)
         if self.gated:
             h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, T * self.top, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act)
