@@ -40,18 +40,23 @@ def _need(cond: bool, msg: str) -> None:
 
 
 def _cuda(t: torch.Tensor, what: str, dtype=None, contiguous=True) -> torch.Tensor:
-    _need(isinstance(t, torch.Tensor), f"{what}: not a tensor")
-    _need(t.is_cuda, f"{what}: tensor is on {t.device}, the kernels run on CUDA only")
-    if dtype is not None:
-        _need(t.dtype == dtype, f"{what}: dtype {t.dtype}, expected {dtype}")
-    if contiguous:
-        _need(t.is_contiguous(), f"{what}: tensor is not contiguous")
+    # (a message is made only when it is raised, here and below: a launch asks several such questions of every tensor, and
+    # formatting sizes and devices for nobody took as long as the launch itself)
+    if not isinstance(t, torch.Tensor):
+        raise KernelError(f"{what}: not a tensor")
+    if not t.is_cuda:
+        raise KernelError(f"{what}: tensor is on {t.device}, the kernels run on CUDA only")
+    if dtype is not None and t.dtype != dtype:
+        raise KernelError(f"{what}: dtype {t.dtype}, expected {dtype}")
+    if contiguous and not t.is_contiguous():
+        raise KernelError(f"{what}: tensor is not contiguous")
     return t
 
 
 def _rows(t: torch.Tensor, what: str) -> int:
     """Row stride of a 2-D tensor whose rows are dense."""
-    _need(t.dim() == 2 and t.stride(1) == 1, f"{what}: expected a 2-D tensor with dense rows")
+    if t.dim() != 2 or t.stride(1) != 1:
+        raise KernelError(f"{what}: expected a 2-D tensor with dense rows")
     return t.stride(0)
 
 
@@ -60,7 +65,7 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))  # (without making a Stream object)
 
 
 _launches = 0
@@ -127,13 +132,16 @@ def add_rmsnorm(
     delta_dt = _DT[act_dtype]
     if delta is not None:
         _cuda(delta, "add_rmsnorm delta")
-        _need(delta.dtype in (act_dtype, torch.float32), f"add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
+        if not (delta.dtype in (act_dtype, torch.float32)):
+            raise KernelError(f"add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
         delta_dt = _DT[delta.dtype]
         if delta.dim() == 2:
-            _need(tuple(delta.shape) == (T, d), f"add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
+            if not (tuple(delta.shape) == (T, d)):
+                raise KernelError(f"add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
             n_parts = 1
         else:
-            _need(delta.dim() == 3 and tuple(delta.shape[1:]) == (T, d), f"add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
+            if not (delta.dim() == 3 and tuple(delta.shape[1:]) == (T, d)):
+                raise KernelError(f"add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
             n_parts, part_stride = delta.shape[0], T * d
     n_rows = T
     if rows is not None:
@@ -142,7 +150,8 @@ def add_rmsnorm(
     w_dt = _F32
     if weight is not None:
         _cuda(weight, "add_rmsnorm weight")
-        _need(tuple(weight.shape) == (d,), f"add_rmsnorm: weight {tuple(weight.shape)} does not match d={d}")
+        if not (tuple(weight.shape) == (d,)):
+            raise KernelError(f"add_rmsnorm: weight {tuple(weight.shape)} does not match d={d}")
         w_dt = _dt(weight, "add_rmsnorm weight")
         if out is None:
             out = torch.empty((n_rows, d), dtype=act_dtype, device=x.device)
@@ -156,7 +165,8 @@ def add_rmsnorm(
     if n_rows == 0:
         return out
     for name, t in (("x", x), ("delta", delta), ("weight", weight), ("out", out)):
-        _need(t is None or t.data_ptr() % 16 == 0, f"add_rmsnorm: {name} is not 16-byte aligned")
+        if not (t is None or t.data_ptr() % 16 == 0):
+            raise KernelError(f"add_rmsnorm: {name} is not 16-byte aligned")
     lib = build.load("elementwise")
     rc = lib.rl_add_rmsnorm(
         _p(x), _p(delta), c_int(delta_dt), c_int(n_parts), c_ll(part_stride), _p(weight), c_int(w_dt), _p(out),
@@ -190,11 +200,13 @@ def seq_begin_decode(state: torch.Tensor, slot_ids: torch.Tensor, tok_pos: torch
     """A decode step's positions from the records on the device (int32 [slots, 4]): row i of the batch, which belongs
     to slot slot_ids[i], stands at position record.len; the record moves on by one position and one decoded token."""
     _cuda(state, "seq_begin_decode state", torch.int32)
-    _need(state.dim() == 2 and state.shape[1] == SEQ_FIELDS, f"seq_begin_decode: records must be [slots, {SEQ_FIELDS}]")
+    if not (state.dim() == 2 and state.shape[1] == SEQ_FIELDS):
+        raise KernelError(f"seq_begin_decode: records must be [slots, {SEQ_FIELDS}]")
     S = slot_ids.numel()
     for name, t in (("slot_ids", slot_ids), ("tok_pos", tok_pos), ("seq_pos0", seq_pos0), ("seq_len", seq_len)):
         _cuda(t, f"seq_begin_decode {name}", torch.int32)
-        _need(t.numel() == S, f"seq_begin_decode: {name} has {t.numel()} entries for {S} sequences")
+        if not (t.numel() == S):
+            raise KernelError(f"seq_begin_decode: {name} has {t.numel()} entries for {S} sequences")
     lib = build.load("elementwise")
     rc = lib.rl_seq_begin_decode(_p(state), _p(slot_ids), c_int(S), _p(tok_pos), _p(seq_pos0), _p(seq_len), _stream())
     _check(lib, rc, "seq_begin_decode")
@@ -203,7 +215,8 @@ def seq_begin_decode(state: torch.Tensor, slot_ids: torch.Tensor, tok_pos: torch
 def seq_set_len(state: torch.Tensor, slot_ids: torch.Tensor, seq_len: torch.Tensor) -> None:
     """record.len = seq_len[i] for the sequences of a step whose positions the host gave."""
     _cuda(state, "seq_set_len state", torch.int32)
-    _need(state.dim() == 2 and state.shape[1] == SEQ_FIELDS, f"seq_set_len: records must be [slots, {SEQ_FIELDS}]")
+    if not (state.dim() == 2 and state.shape[1] == SEQ_FIELDS):
+        raise KernelError(f"seq_set_len: records must be [slots, {SEQ_FIELDS}]")
     _cuda(slot_ids, "seq_set_len slot_ids", torch.int32)
     _cuda(seq_len, "seq_set_len seq_len", torch.int32)
     _need(slot_ids.numel() == seq_len.numel(), "seq_set_len: one length per sequence")
@@ -246,10 +259,8 @@ def rope_kv_write(
         width = block_table.shape[1]
         for name, pages in (("k_pages", k_pages), ("v_pages", v_pages)):
             _cuda(pages, f"rope_kv_write {name}", qkv.dtype)
-            _need(
-                pages.dim() == 4 and tuple(pages.shape[1:]) == (num_kv_heads, PAGE_SIZE, head_dim),
-                f"rope_kv_write: {name} {tuple(pages.shape)} is not [pages, {num_kv_heads}, {PAGE_SIZE}, {head_dim}]",
-            )
+            if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (num_kv_heads, PAGE_SIZE, head_dim)):
+                raise KernelError(f"rope_kv_write: {name} {tuple(pages.shape)} is not [pages, {num_kv_heads}, {PAGE_SIZE}, {head_dim}]")
         _need(qkv.shape[1] >= (num_heads + 2 * num_kv_heads) * head_dim, "rope_kv_write: qkv rows too short")
     _need(qkv.data_ptr() % 16 == 0, "rope_kv_write: qkv is not 16-byte aligned")
     if rotary_dim:
@@ -268,10 +279,8 @@ def rope_kv_write(
 def _check_pages(k_pages, v_pages, dtype, K, hd, what):
     for name, pages in (("k_pages", k_pages), ("v_pages", v_pages)):
         _cuda(pages, f"{what} {name}", dtype)
-        _need(
-            pages.dim() == 4 and tuple(pages.shape[1:]) == (K, PAGE_SIZE, hd),
-            f"{what}: {name} {tuple(pages.shape)} is not [pages, {K}, {PAGE_SIZE}, {hd}]",
-        )
+        if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (K, PAGE_SIZE, hd)):
+            raise KernelError(f"{what}: {name} {tuple(pages.shape)} is not [pages, {K}, {PAGE_SIZE}, {hd}]")
 
 
 def attn_generic(
@@ -316,7 +325,8 @@ def attn_tma_takes(kdim: int, vdim: int) -> bool:
 def _check_sink(sink, num_heads: int, what: str) -> None:
     if sink is not None:
         _cuda(sink, f"{what} sink", torch.float32)
-        _need(sink.numel() == num_heads, f"{what}: one sink per head")
+        if not (sink.numel() == num_heads):
+            raise KernelError(f"{what}: one sink per head")
 
 
 def _bias_args(bias, num_heads: int, what: str):
@@ -325,7 +335,8 @@ def _bias_args(bias, num_heads: int, what: str):
     if bias is None:
         return c_void_p(0), c_int(0)
     _cuda(bias, f"{what} bias", torch.float32)
-    _need(bias.dim() == 2 and bias.shape[0] == num_heads and bias.shape[1] > 0, f"{what}: bias {tuple(bias.shape)} for {num_heads} heads")
+    if not (bias.dim() == 2 and bias.shape[0] == num_heads and bias.shape[1] > 0):
+        raise KernelError(f"{what}: bias {tuple(bias.shape)} for {num_heads} heads")
     return _p(bias), c_int(bias.shape[1])
 
 
@@ -392,7 +403,8 @@ def attn_decode(
     _need(block_table.dim() == 2 and block_table.shape[0] >= S and seq_len.numel() == S, "attn_decode: metadata sizes")
     _cuda(scratch, "attn_decode scratch", torch.float32)
     need = attn_decode_scratch_floats(S, num_heads, vdim, n_splits)
-    _need(scratch.numel() >= need, f"attn_decode: scratch holds {scratch.numel()} floats, {need} needed")
+    if not (scratch.numel() >= need):
+        raise KernelError(f"attn_decode: scratch holds {scratch.numel()} floats, {need} needed")
     if out is None:
         out = torch.empty((S, num_heads // maps * vdim), dtype=act, device=q.device)
     _cuda(out, "attn_decode out", act, contiguous=False)
@@ -402,10 +414,12 @@ def attn_decode(
     n_o = S * num_heads * n_splits * vdim
     part_o = c_void_p(scratch.data_ptr())
     part_ml = c_void_p(scratch.data_ptr() + 4 * n_o)
-    _need(impl in ("auto", "warp", "tma"), f"attn_decode: unknown impl {impl!r}")
+    if not (impl in ("auto", "warp", "tma")):
+        raise KernelError(f"attn_decode: unknown impl {impl!r}")
     if impl == "auto":
         impl = "tma" if (act == torch.bfloat16 and (head_dim in ATTN_DECODE_TMA_HEAD_DIMS or vdim != head_dim)) else "warp"
-    _need(fuse in (0, 1, 2), f"attn_decode: fuse={fuse}")
+    if not (fuse in (0, 1, 2)):
+        raise KernelError(f"attn_decode: fuse={fuse}")
     if fuse:
         _need(impl == "tma", "attn_decode: only the TMA kernel fuses the position encoding")
         if rotary_dim:
@@ -417,7 +431,8 @@ def attn_decode(
         _need(impl == "tma", "attn_decode: only the TMA kernel adds the splits up itself")
         _cuda(counters, "attn_decode counters", torch.int32)
         groups = num_kv_heads * ((num_heads // num_kv_heads + 7) // 8)
-        _need(counters.numel() >= S * groups, f"attn_decode: {counters.numel()} counters, {S * groups} needed")
+        if not (counters.numel() >= S * groups):
+            raise KernelError(f"attn_decode: {counters.numel()} counters, {S * groups} needed")
     _need(q_parts is None or impl == "tma", "attn_decode: only the TMA kernel takes partial sums")
     _check_sink(sink, num_heads, "attn_decode")
     if impl == "tma":
@@ -497,9 +512,11 @@ def flash_prefill_tc(
     cap c of s <- c tanh(s / c) on the scaled scores.
     maps: 1, or 2: query heads 2h and 2h + 1 are the two halves of row h's head_dim numbers, against the same halves of the keys.
     bias: None, or float32 [H, L], a learned bias of the scores by head and distance (`_bias_args`; one map only)."""
-    _need(maps in (1, 2) and num_heads % maps == 0, f"flash_prefill_tc: {maps} maps in {num_heads} heads")
+    if not (maps in (1, 2) and num_heads % maps == 0):
+        raise KernelError(f"flash_prefill_tc: {maps} maps in {num_heads} heads")
     vdim = value_dim or head_dim
-    _need(attn_tma_takes(head_dim, vdim), f"flash_prefill_tc: key and value sizes {head_dim} / {vdim}, this kernel is built for multiples of 8 up to 128")
+    if not (attn_tma_takes(head_dim, vdim)):
+        raise KernelError(f"flash_prefill_tc: key and value sizes {head_dim} / {vdim}, this kernel is built for multiples of 8 up to 128")
     _cuda(q, "flash_prefill_tc q", torch.bfloat16, contiguous=False)
     qs = _rows(q, "flash_prefill_tc q")
     T = q.shape[0]
@@ -541,7 +558,8 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     ldx, ldw = _rows(x, "gemm_f32 x"), _rows(w, "gemm_f32 w")
     M, K = x.shape
     N = w.shape[0]
-    _need(w.shape[1] == K, f"gemm_f32: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
+    if not (w.shape[1] == K):
+        raise KernelError(f"gemm_f32: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     _cuda(out, "gemm_f32 out", torch.float32, contiguous=False)
@@ -566,7 +584,8 @@ def _act(act):
     if act == "gelu_tanh":  # gelu(gate) * up, the tanh form (RL_GATED_GELU_TANH of csrc/common.cuh)
         return c_float(0.0), c_float(-3.0)
     alpha, limit = act
-    _need(limit > 0, f"a gated activation with limits needs a positive limit, got {limit}")
+    if not (limit > 0):
+        raise KernelError(f"a gated activation with limits needs a positive limit, got {limit}")
     return c_float(alpha), c_float(limit)
 
 
@@ -582,7 +601,8 @@ def gemm_bf16_any(
     ldx, ldw = _rows(x, "gemm_bf16_any x"), _rows(w, "gemm_bf16_any w")
     M, K = x.shape
     N = w.shape[0]
-    _need(w.shape[1] == K, f"gemm_bf16_any: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
+    if not (w.shape[1] == K):
+        raise KernelError(f"gemm_bf16_any: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     out = torch.empty((M, N // 2 if swiglu else N), dtype=out_dtype, device=x.device)
     lib = build.load("gemm_f32")
     rc = lib.rl_gemm_bf16_any(
@@ -609,7 +629,8 @@ def gemv_bf16(
     ldx, ldw = _rows(x, "gemv_bf16 x"), _rows(w, "gemv_bf16 w")
     M, K = x.shape
     N = w.shape[0]
-    _need(w.shape[1] == K, f"gemv_bf16: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
+    if not (w.shape[1] == K):
+        raise KernelError(f"gemv_bf16: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     _need(x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0, "gemv_bf16: operands must be 16-byte aligned")
     n_out = N // 2 if swiglu else N
     if k_splits > 1:
@@ -659,11 +680,12 @@ def gemv_stream_into_stream(
     _cuda(next_w, "gemv_stream_into_stream next_w")
     M, K = x.shape
     N = w.shape[0]
-    _need(w.shape[1] == K and tuple(resid.shape) == (M, N) and tuple(next_w.shape) == (N,),
-          f"gemv_stream_into_stream: x{tuple(x.shape)} w{tuple(w.shape)} resid{tuple(resid.shape)} next_w{tuple(next_w.shape)} do not fit")
+    if not (w.shape[1] == K and tuple(resid.shape) == (M, N) and tuple(next_w.shape) == (N,)):
+        raise KernelError(f"gemv_stream_into_stream: x{tuple(x.shape)} w{tuple(w.shape)} resid{tuple(resid.shape)} next_w{tuple(next_w.shape)} do not fit")
     lib = build.load("gemv_stream")
     blocks = int(lib.rl_gemv_stream_blocks(c_int(N), c_int(K)))
-    _need(blocks > 0, f"gemv_stream_into_stream: the kernel does not take N={N}, K={K}")
+    if not (blocks > 0):
+        raise KernelError(f"gemv_stream_into_stream: the kernel does not take N={N}, K={K}")
     if xw is None:
         xw = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
     if sumsq is None:
@@ -679,7 +701,8 @@ def gemv_stream_into_stream(
         c_int(_rows(xw, "gemv_stream_into_stream xw")), _p(sumsq), c_int(M), c_int(N), c_int(K), ctypes.byref(used), _p(status), *_wt(), _stream(),
     )
     _check(lib, rc, "gemv_stream_into_stream")
-    _need(used.value == blocks, f"gemv_stream_into_stream: the kernel ran {used.value} blocks, the wrapper planned {blocks}")
+    if not (used.value == blocks):
+        raise KernelError(f"gemv_stream_into_stream: the kernel ran {used.value} blocks, the wrapper planned {blocks}")
     return xw, sumsq, blocks
 
 
@@ -701,14 +724,16 @@ def gemv_stream(
     ldx, ldw = _rows(x, "gemv_stream x"), _rows(w, "gemv_stream w")
     M, K = x.shape
     N = w.shape[0]
-    _need(w.shape[1] == K, f"gemv_stream: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
+    if not (w.shape[1] == K):
+        raise KernelError(f"gemv_stream: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     n_out = N // 2 if swiglu else N
     used = c_int(1)
     _need(act in GATED_ACTS or not isinstance(act, str) or (not swiglu and k_splits == 1 and row_scale is None),
           "gemv_stream: an activation of one argument goes with a plain product and whole sums")
     _need(act not in GATED_ACTS or swiglu, "gemv_stream: a gate's activation goes with a gate/up product")
     slices = max(1, gemv_stream_slices(M, K, k_splits))  # (0: the launcher says what it does not take)
-    _need(k_splits > 1 or slices == 1, f"gemv_stream: k = {K} comes in {slices} slices, whose float32 partial sums have to be asked for (k_splits > 1)")
+    if not (k_splits > 1 or slices == 1):
+        raise KernelError(f"gemv_stream: k = {K} comes in {slices} slices, whose float32 partial sums have to be asked for (k_splits > 1)")
     if k_splits > 1 and slices > 1:
         _need(out is None and out_dtype == torch.float32 and not swiglu, "gemv_stream: partial sums over k slices are float32, without activation")
         out = torch.empty((slices, M, n_out), dtype=torch.float32, device=x.device)
@@ -736,7 +761,8 @@ def gemv_stream(
         c_int(M), c_int(N), c_int(K), c_int(1 if swiglu else 0), *_act(act), c_int(k_splits), ctypes.byref(used), _p(status), *_wt(), _stream(),
     )
     _check(lib, rc, "gemv_stream")
-    _need(used.value == slices, f"gemv_stream: kernel used {used.value} slices, the wrapper planned {slices}")
+    if not (used.value == slices):
+        raise KernelError(f"gemv_stream: kernel used {used.value} slices, the wrapper planned {slices}")
     return out
 
 
@@ -822,7 +848,8 @@ def gemm_tc(
     ldx, ldw = _rows(x, "gemm_tc x"), _rows(w, "gemm_tc w")
     M, K = x.shape
     N = w.shape[0]
-    _need(w.shape[1] == K, f"gemm_tc: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
+    if not (w.shape[1] == K):
+        raise KernelError(f"gemm_tc: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     n_out = N // 2 if swiglu else N
     used = c_int(1)
     if k_splits > 1:
@@ -846,7 +873,8 @@ def gemm_tc(
     )
     _check(lib, rc, "gemm_tc")
     if k_splits > 1:
-        _need(used.value == k_splits, f"gemm_tc: kernel used {used.value} slices, the wrapper planned {k_splits}")
+        if not (used.value == k_splits):
+            raise KernelError(f"gemm_tc: kernel used {used.value} slices, the wrapper planned {k_splits}")
     return out
 
 
@@ -880,7 +908,8 @@ def sample(
     _cuda(rng_index, "sample rng_index", torch.int32)
     _need(rng_index.numel() == R, "sample: one random-state index per row")
     _cuda(scratch, "sample scratch", torch.float32)
-    _need(scratch.numel() >= R * n, f"sample: scratch holds {scratch.numel()} floats, {R * n} needed")
+    if not (scratch.numel() >= R * n):
+        raise KernelError(f"sample: scratch holds {scratch.numel()} floats, {R * n} needed")
     if out is None:
         out = torch.empty((R,), dtype=torch.int32, device=logits.device)
     _cuda(out, "sample out", torch.int32)
@@ -924,11 +953,12 @@ def sample_chain(
     _need(slot_of_row.numel() == R, "sample_chain: one slot per row")
     _cuda(history, "sample_chain history", torch.int32)
     _cuda(history_count, "sample_chain history_count", torch.int32)
-    _need(history.dim() == 2 and history.shape[1] == SAMPLE_HISTORY_MAX and history.shape[0] == history_count.numel(),
-          f"sample_chain: history must be [slots, {SAMPLE_HISTORY_MAX}] with one count per slot")
+    if not (history.dim() == 2 and history.shape[1] == SAMPLE_HISTORY_MAX and history.shape[0] == history_count.numel()):
+        raise KernelError(f"sample_chain: history must be [slots, {SAMPLE_HISTORY_MAX}] with one count per slot")
     _cuda(work, "sample_chain work", torch.float32)
     need = R * 2 * ((n + 3) // 4 * 4)
-    _need(work.numel() >= need, f"sample_chain: work holds {work.numel()} floats, {need} needed")
+    if not (work.numel() >= need):
+        raise KernelError(f"sample_chain: work holds {work.numel()} floats, {need} needed")
     _need(work.data_ptr() % 16 == 0, "sample_chain: work must be 16-byte aligned")
     if out is None:
         out = torch.empty((R,), dtype=torch.int32, device=logits.device)
@@ -968,12 +998,15 @@ def normed_add_rmsnorm(
     _cuda(x, "normed_add_rmsnorm x", torch.float32)
     T, d = x.shape
     _cuda(delta, "normed_add_rmsnorm delta")
-    _need(delta.dtype in (act_dtype, torch.float32), f"normed_add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
+    if not (delta.dtype in (act_dtype, torch.float32)):
+        raise KernelError(f"normed_add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
     if delta.dim() == 2:
-        _need(tuple(delta.shape) == (T, d), f"normed_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
+        if not (tuple(delta.shape) == (T, d)):
+            raise KernelError(f"normed_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
         n_parts, part_stride = 1, 0
     else:
-        _need(delta.dim() == 3 and tuple(delta.shape[1:]) == (T, d), f"normed_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
+        if not (delta.dim() == 3 and tuple(delta.shape[1:]) == (T, d)):
+            raise KernelError(f"normed_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
         n_parts, part_stride = delta.shape[0], T * d
     _cuda(delta_weight, "normed_add_rmsnorm delta_weight")
     _need(tuple(delta_weight.shape) == (d,), "normed_add_rmsnorm: delta_weight does not match d")
@@ -1011,13 +1044,16 @@ def gated_add_rmsnorm(
     _cuda(x, "gated_add_rmsnorm x", torch.float32)
     _need(x.dim() == 2, "gated_add_rmsnorm: x must be [T, d]")
     T, d = x.shape
-    _need(groups >= 1 and d % groups == 0, f"gated_add_rmsnorm: {groups} groups do not divide a row of {d}")
+    if not (groups >= 1 and d % groups == 0):
+        raise KernelError(f"gated_add_rmsnorm: {groups} groups do not divide a row of {d}")
     n_parts, part_stride, delta_dt = 0, 0, _DT[act_dtype]
     if delta is not None:
         _cuda(delta, "gated_add_rmsnorm delta")
-        _need(delta.dtype in (act_dtype, torch.float32), f"gated_add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
+        if not (delta.dtype in (act_dtype, torch.float32)):
+            raise KernelError(f"gated_add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
         delta_dt = _DT[delta.dtype]
-        _need(tuple(delta.shape[-2:]) == (T, d) and delta.dim() in (2, 3), f"gated_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
+        if not (tuple(delta.shape[-2:]) == (T, d) and delta.dim() in (2, 3)):
+            raise KernelError(f"gated_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
         n_parts, part_stride = (1, 0) if delta.dim() == 2 else (delta.shape[0], T * d)
     z = bias = None
     zs = 0
@@ -1026,7 +1062,8 @@ def gated_add_rmsnorm(
         _need(delta is not None, "gated_add_rmsnorm: a gate but nothing to gate")
         _cuda(z, "gated_add_rmsnorm gate", act_dtype, contiguous=False)
         zs = _rows(z, "gated_add_rmsnorm gate")
-        _need(tuple(z.shape) == (T, d), f"gated_add_rmsnorm: gate {tuple(z.shape)} does not match x {(T, d)}")
+        if not (tuple(z.shape) == (T, d)):
+            raise KernelError(f"gated_add_rmsnorm: gate {tuple(z.shape)} does not match x {(T, d)}")
         _cuda(bias, "gated_add_rmsnorm bias", torch.float32)
         _need(tuple(bias.shape) == (d,), "gated_add_rmsnorm: bias does not match d")
     n_rows = T if rows is None else rows.numel()
@@ -1111,7 +1148,8 @@ def latent_prep(
         ldkv = _rows(kv, "latent_prep kv")
         _need(kv.shape[0] == T and kv.shape[1] >= rank + rot, "latent_prep: kv rows do not fit")
         _cuda(pages, "latent_prep pages", dt)
-        _need(pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot), f"latent_prep: pages {tuple(pages.shape)}")
+        if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot)):
+            raise KernelError(f"latent_prep: pages {tuple(pages.shape)}")
         _cuda(block_table, "latent_prep block_table", torch.int32)
         _need(block_table.dim() == 2, "latent_prep: block_table must be [S, width]")
         width = block_table.shape[1]
@@ -1198,7 +1236,8 @@ def latent_attn(
     _need(q_cat.dim() == 3 and q_cat.shape[2] == rank + rot, "latent_attn: q_cat must be [T, H, rank + rot]")
     T, H = q_cat.shape[0], q_cat.shape[1]
     _cuda(pages, "latent_attn pages", q_cat.dtype)
-    _need(pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot), f"latent_attn: pages {tuple(pages.shape)}")
+    if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot)):
+        raise KernelError(f"latent_attn: pages {tuple(pages.shape)}")
     _cuda(block_table, "latent_attn block_table", torch.int32)
     _cuda(tok_seq, "latent_attn tok_seq", torch.int32)
     _cuda(tok_pos, "latent_attn tok_pos", torch.int32)
@@ -1240,7 +1279,8 @@ def moe_router(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], n
     _cuda(w, "moe_router w", torch.float32)
     T, d = x.shape
     has_gate = w.shape[0] == n_experts + 1
-    _need(w.dim() == 2 and w.shape[1] == d and w.shape[0] in (n_experts, n_experts + 1), f"moe_router: w {tuple(w.shape)} for {n_experts} experts of width {d}")
+    if not (w.dim() == 2 and w.shape[1] == d and w.shape[0] in (n_experts, n_experts + 1)):
+        raise KernelError(f"moe_router: w {tuple(w.shape)} for {n_experts} experts of width {d}")
     if bias is not None:
         _cuda(bias, "moe_router bias", torch.float32)
         _need(bias.numel() == n_experts, "moe_router: one bias per expert")
@@ -1262,7 +1302,8 @@ def moe_choose(logits: torch.Tensor, bias: Optional[torch.Tensor], n_experts: in
                logistic: bool = False, renorm_eps: float = 0.0, weight_scale: float = 1.0):
     """`moe_router` behind its product: logits float32 [T, E (+1)] that another product made."""
     _cuda(logits, "moe_choose logits", torch.float32)
-    _need(logits.dim() == 2 and logits.shape[1] in (n_experts, n_experts + 1), f"moe_choose: logits {tuple(logits.shape)} for {n_experts} experts")
+    if not (logits.dim() == 2 and logits.shape[1] in (n_experts, n_experts + 1)):
+        raise KernelError(f"moe_choose: logits {tuple(logits.shape)} for {n_experts} experts")
     T = logits.shape[0]
     has_gate = logits.shape[1] == n_experts + 1
     if bias is not None:
@@ -1344,7 +1385,8 @@ def moe_gemm(
     tensor cores if it is one of MOE_MMA_TILE_ROWS, everything else to the plain kernel (which wants its own height)."""
     _cuda(x, "moe_gemm x", contiguous=False)
     _cuda(w, "moe_gemm w", x.dtype)
-    _need(w.dim() == 3 and w.shape[2] == x.shape[1], f"moe_gemm: w {tuple(w.shape)} against x {tuple(x.shape)}")
+    if not (w.dim() == 3 and w.shape[2] == x.shape[1]):
+        raise KernelError(f"moe_gemm: w {tuple(w.shape)} against x {tuple(x.shape)}")
     E, N, K = w.shape
     if w2 is not None:
         _cuda(w2, "moe_gemm w2", x.dtype)
@@ -1367,7 +1409,8 @@ def moe_gemm(
         )
         _check(lib, rc, "moe_gemm_tc")
         return out
-    _need(tile_rows == moe_tile_rows(), f"moe_gemm: the plain kernel wants tiles of {moe_tile_rows()} rows, the plan has {tile_rows}")
+    if not (tile_rows == moe_tile_rows()):
+        raise KernelError(f"moe_gemm: the plain kernel wants tiles of {moe_tile_rows()} rows, the plan has {tile_rows}")
     lib = build.load("moe")
     rc = lib.rl_moe_gemm(
         _p(x), c_int(_rows(x, "moe_gemm x")), c_int(_dt(x, "moe_gemm")), _p(order), c_int(gather_div), _p(w), _p(w2), _p(out),
@@ -1433,7 +1476,8 @@ def latent_attn_mma(
     _need(q_cat.dim() == 3 and q_cat.shape[2] == rank + rot, "latent_attn_mma: q_cat must be [T, H, rank + rot]")
     T, H = q_cat.shape[0], q_cat.shape[1]
     _cuda(pages, "latent_attn_mma pages", torch.bfloat16)
-    _need(pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot), f"latent_attn_mma: pages {tuple(pages.shape)}")
+    if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot)):
+        raise KernelError(f"latent_attn_mma: pages {tuple(pages.shape)}")
     _need(q_cat.data_ptr() % 16 == 0 and pages.data_ptr() % 16 == 0, "latent_attn_mma: tensors must be 16-byte aligned")
     _cuda(block_table, "latent_attn_mma block_table", torch.int32)
     _cuda(seq_start, "latent_attn_mma seq_start", torch.int32)
@@ -1446,7 +1490,8 @@ def latent_attn_mma(
     if n_splits > 1:
         _cuda(scratch, "latent_attn_mma scratch", torch.float32)
         need = latent_attn_mma_scratch_floats(T * H, rank, n_splits)
-        _need(scratch.numel() >= need, f"latent_attn_mma: scratch holds {scratch.numel()} floats, {need} needed")
+        if not (scratch.numel() >= need):
+            raise KernelError(f"latent_attn_mma: scratch holds {scratch.numel()} floats, {need} needed")
     if out is None:
         out = torch.empty((T, H, rank), dtype=torch.bfloat16, device=q_cat.device)
     _cuda(out, "latent_attn_mma out", torch.bfloat16)
@@ -1465,10 +1510,8 @@ def latent_attn_mma(
 def _check_kv_pages(k_pages, v_pages, dtype, K, kdim, vdim, what):
     for name, pages, size in (("k_pages", k_pages, kdim), ("v_pages", v_pages, vdim)):
         _cuda(pages, f"{what} {name}", dtype)
-        _need(
-            pages.dim() == 4 and tuple(pages.shape[1:]) == (K, PAGE_SIZE, size),
-            f"{what}: {name} {tuple(pages.shape)} is not [pages, {K}, {PAGE_SIZE}, {size}]",
-        )
+        if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (K, PAGE_SIZE, size)):
+            raise KernelError(f"{what}: {name} {tuple(pages.shape)} is not [pages, {K}, {PAGE_SIZE}, {size}]")
 
 
 def qkv_prep(
@@ -1503,10 +1546,12 @@ def qkv_prep(
     else:
         block_table = k_pages = v_pages = None
     coef, every = temperature or (0.0, 0)
-    _need(temperature is None or int(every) > 0, f"qkv_prep: a temperature that grows every {every} positions")
+    if not (temperature is None or int(every) > 0):
+        raise KernelError(f"qkv_prep: a temperature that grows every {every} positions")
     if bias is not None:
         _cuda(bias, "qkv_prep bias", torch.float32)
-        _need(bias.numel() == cols, f"qkv_prep: bias has {bias.numel()} numbers for {cols} columns")
+        if not (bias.numel() == cols):
+            raise KernelError(f"qkv_prep: bias has {bias.numel()} numbers for {cols} columns")
     if rotary_dim:
         _cuda(inv_freq, "qkv_prep inv_freq", torch.float32)
         _need(inv_freq.numel() == rotary_dim // 2, "qkv_prep: inv_freq must hold rotary_dim/2 values")
@@ -1514,12 +1559,14 @@ def qkv_prep(
         if w is not None:
             _cuda(w, f"qkv_prep {name}", torch.float32)
             want = heads * kdim if norm_whole else kdim
-            _need(w.numel() == want, f"qkv_prep: {name} must hold one weight per number of {'all heads' if norm_whole else 'a head'} ({want})")
+            if not (w.numel() == want):
+                raise KernelError(f"qkv_prep: {name} must hold one weight per number of {'all heads' if norm_whole else 'a head'} ({want})")
     vs_stride = 0
     if v_src is not None:
         _cuda(v_src, "qkv_prep v_src", qkv.dtype, contiguous=False)
         vs_stride = _rows(v_src, "qkv_prep v_src")
-        _need(tuple(v_src.shape) == (T, num_kv_heads * vdim), f"qkv_prep: v_src {tuple(v_src.shape)} is not [T, {num_kv_heads * vdim}]")
+        if not (tuple(v_src.shape) == (T, num_kv_heads * vdim)):
+            raise KernelError(f"qkv_prep: v_src {tuple(v_src.shape)} is not [T, {num_kv_heads * vdim}]")
         _cuda(v_lambda, "qkv_prep v_lambda", torch.float32)
         _need(v_lambda.numel() == 1, "qkv_prep: v_lambda is one number")
     lib = build.load("attention_ext")
@@ -1554,7 +1601,8 @@ def attn_ext(
     _cuda(q, "attn_ext q", contiguous=False)
     qs = _rows(q, "attn_ext q")
     T = q.shape[0]
-    _need(maps in (1, 2) and num_heads % maps == 0 and kdim % maps == 0, f"attn_ext: {maps} maps in {num_heads} heads of {kdim}")
+    if not (maps in (1, 2) and num_heads % maps == 0 and kdim % maps == 0):
+        raise KernelError(f"attn_ext: {maps} maps in {num_heads} heads of {kdim}")
     _need(q.shape[1] >= num_heads // maps * kdim, "attn_ext: q rows too short")
     _check_kv_pages(k_pages, v_pages, q.dtype, num_kv_heads, kdim, vdim, "attn_ext")
     _cuda(block_table, "attn_ext block_table", torch.int32)
@@ -1673,7 +1721,8 @@ def sigmoid_attn_mma(
     qs = _rows(q, "sigmoid_attn_mma q")
     T = q.shape[0]
     _need(q.shape[1] >= num_heads * kdim, "sigmoid_attn_mma: q rows too short")
-    _need(sigmoid_attn_mma_takes(kdim, vdim, num_heads), f"sigmoid_attn_mma: sizes {kdim}, {vdim} with {num_heads} heads are not built")
+    if not (sigmoid_attn_mma_takes(kdim, vdim, num_heads)):
+        raise KernelError(f"sigmoid_attn_mma: sizes {kdim}, {vdim} with {num_heads} heads are not built")
     _check_kv_pages(k_pages, v_pages, q.dtype, num_kv_heads, kdim, vdim, "sigmoid_attn_mma")
     _cuda(block_table, "sigmoid_attn_mma block_table", torch.int32)
     _cuda(seq_start, "sigmoid_attn_mma seq_start", torch.int32)
@@ -1733,12 +1782,14 @@ def decay_attn(
     silu: the activation is applied to q, k and v as they are read.  Returns float32 [T, H vdim]."""
     for name, t, n in (("q", q, num_heads * dim), ("k", k, num_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"decay_attn {name}", q.dtype, contiguous=False)
-        _need(_rows(t, f"decay_attn {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0], f"decay_attn: {name} has the wrong shape or stride")
+        if not (_rows(t, f"decay_attn {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0]):
+            raise KernelError(f"decay_attn: {name} has the wrong shape or stride")
     T = q.shape[0]
     _cuda(decay, "decay_attn decay", torch.float32)
     _need(decay.numel() == num_heads, "decay_attn: one decay per head")
     _cuda(state, "decay_attn state", torch.float32)
-    _need(state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vdim), f"decay_attn: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vdim}]")
+    if not (state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vdim)):
+        raise KernelError(f"decay_attn: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vdim}]")
     _cuda(slot_ids, "decay_attn slot_ids", torch.int32)
     _cuda(seq_start, "decay_attn seq_start", torch.int32)
     S = slot_ids.numel()
@@ -1750,7 +1801,8 @@ def decay_attn(
     lib = build.load("recurrent")
     if max_q_len > 0 and scratch is not None:
         _cuda(scratch, "decay_attn scratch", torch.float32)
-        _need(dim <= DECAY_CHUNKED_MAX_DIM, f"decay_attn: the chunked kernels take key sizes up to {DECAY_CHUNKED_MAX_DIM}")
+        if not (dim <= DECAY_CHUNKED_MAX_DIM):
+            raise KernelError(f"decay_attn: the chunked kernels take key sizes up to {DECAY_CHUNKED_MAX_DIM}")
         _need(scratch.numel() >= decay_attn_chunked_scratch_floats(S, max_q_len, num_heads, dim, vdim), "decay_attn: scratch too small")
         rc = lib.rl_decay_attn_chunked(
             _p(q), _p(k), _p(v), c_int(_dt(q, "decay_attn")), c_int(q.stride(0)), _p(decay), _p(state), _p(slot_ids), _p(seq_start), _p(scratch),
@@ -1809,13 +1861,16 @@ def min_gru(
     T, width = z.shape
     for name, t in (("z", z), ("x", x), ("g", g)):
         _cuda(t, f"min_gru {name}", z.dtype, contiguous=False)
-        _need(_rows(t, f"min_gru {name}") == z.stride(0) and tuple(t.shape) == (T, width), f"min_gru: {name} has the wrong shape or stride")
+        if not (_rows(t, f"min_gru {name}") == z.stride(0) and tuple(t.shape) == (T, width)):
+            raise KernelError(f"min_gru: {name} has the wrong shape or stride")
     for name, b in (("z_bias", z_bias), ("x_bias", x_bias)):
         if b is not None:
             _cuda(b, f"min_gru {name}", torch.float32)
-            _need(b.numel() == width, f"min_gru: {name} does not match the width")
+            if not (b.numel() == width):
+                raise KernelError(f"min_gru: {name} does not match the width")
     _cuda(state, "min_gru state", torch.float32)
-    _need(state.dim() == 2 and state.shape[1] == width, f"min_gru: state {tuple(state.shape)} is not [slots, {width}]")
+    if not (state.dim() == 2 and state.shape[1] == width):
+        raise KernelError(f"min_gru: state {tuple(state.shape)} is not [slots, {width}]")
     _cuda(slot_ids, "min_gru slot_ids", torch.int32)
     _cuda(seq_start, "min_gru seq_start", torch.int32)
     S = slot_ids.numel()
@@ -1868,7 +1923,8 @@ def mlstm_gates(
             _cuda(b, f"mlstm_gates {name}", torch.float32)
             _need(b.numel() == H, "mlstm_gates: one bias per head")
     _cuda(m_state, "mlstm_gates m_state", torch.float32)
-    _need(m_state.dim() == 2 and m_state.shape[1] == H, f"mlstm_gates: m_state {tuple(m_state.shape)} is not [slots, {H}]")
+    if not (m_state.dim() == 2 and m_state.shape[1] == H):
+        raise KernelError(f"mlstm_gates: m_state {tuple(m_state.shape)} is not [slots, {H}]")
     _cuda(slot_ids, "mlstm_gates slot_ids", torch.int32)
     _cuda(seq_start, "mlstm_gates seq_start", torch.int32)
     S = slot_ids.numel()
@@ -1896,20 +1952,24 @@ def gated_attn(
     (a per head), a = exp(log_decay).  in_scale: float32 [T, H] (b) or None (1).  ext: the state has one more column, fed with
     v = 1, and so has the result.  state: float32 [slots, H, dim, vdim (+1)].  Returns float32 [T, H (vdim (+1))]."""
     qk_heads = qk_heads or num_heads
-    _need(num_heads % qk_heads == 0, f"gated_attn: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
+    if not (num_heads % qk_heads == 0):
+        raise KernelError(f"gated_attn: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
     for name, t, n in (("q", q, qk_heads * dim), ("k", k, qk_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"gated_attn {name}", q.dtype, contiguous=False)
-        _need(_rows(t, f"gated_attn {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0], f"gated_attn: {name} has the wrong shape or stride")
+        if not (_rows(t, f"gated_attn {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0]):
+            raise KernelError(f"gated_attn: {name} has the wrong shape or stride")
     T = q.shape[0]
     vcols = vdim + (1 if ext else 0)
     _cuda(log_decay, "gated_attn log_decay", torch.float32)
     per_channel = log_decay.numel() == T * num_heads * dim
-    _need(per_channel or log_decay.numel() == T * num_heads, f"gated_attn: log_decay {tuple(log_decay.shape)} is neither [T, H dim] nor [T, H]")
+    if not (per_channel or log_decay.numel() == T * num_heads):
+        raise KernelError(f"gated_attn: log_decay {tuple(log_decay.shape)} is neither [T, H dim] nor [T, H]")
     if in_scale is not None:
         _cuda(in_scale, "gated_attn in_scale", torch.float32)
         _need(in_scale.numel() == T * num_heads, "gated_attn: in_scale must be [T, H]")
     _cuda(state, "gated_attn state", torch.float32)
-    _need(state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vcols), f"gated_attn: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vcols}]")
+    if not (state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vcols)):
+        raise KernelError(f"gated_attn: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vcols}]")
     _cuda(slot_ids, "gated_attn slot_ids", torch.int32)
     _cuda(seq_start, "gated_attn seq_start", torch.int32)
     S = slot_ids.numel()
@@ -1947,21 +2007,26 @@ def gated_attn_chunked(
     """`gated_attn` chunk by chunk (64 tokens, all chunks side by side, 32-bit arithmetic): equal within rounding, for prompts.
     max_q_len: the most tokens a sequence of the step brings; scratch: float32, at least `gated_attn_chunked_scratch_floats(...)`."""
     qk_heads = qk_heads or num_heads
-    _need(num_heads % qk_heads == 0, f"gated_attn_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
+    if not (num_heads % qk_heads == 0):
+        raise KernelError(f"gated_attn_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
     for name, t, n in (("q", q, qk_heads * dim), ("k", k, qk_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"gated_attn_chunked {name}", q.dtype, contiguous=False)
-        _need(_rows(t, f"gated_attn_chunked {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0], f"gated_attn_chunked: {name} has the wrong shape or stride")
+        if not (_rows(t, f"gated_attn_chunked {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0]):
+            raise KernelError(f"gated_attn_chunked: {name} has the wrong shape or stride")
     T = q.shape[0]
     vcols = vdim + (1 if ext else 0)
-    _need(gated_attn_chunked_takes(dim, vcols), f"gated_attn_chunked: key size {dim} is too large for the chunked kernels")
+    if not (gated_attn_chunked_takes(dim, vcols)):
+        raise KernelError(f"gated_attn_chunked: key size {dim} is too large for the chunked kernels")
     _cuda(log_decay, "gated_attn_chunked log_decay", torch.float32)
     per_channel = log_decay.numel() == T * num_heads * dim
-    _need(per_channel or log_decay.numel() == T * num_heads, f"gated_attn_chunked: log_decay {tuple(log_decay.shape)} is neither [T, H dim] nor [T, H]")
+    if not (per_channel or log_decay.numel() == T * num_heads):
+        raise KernelError(f"gated_attn_chunked: log_decay {tuple(log_decay.shape)} is neither [T, H dim] nor [T, H]")
     if in_scale is not None:
         _cuda(in_scale, "gated_attn_chunked in_scale", torch.float32)
         _need(in_scale.numel() == T * num_heads, "gated_attn_chunked: in_scale must be [T, H]")
     _cuda(state, "gated_attn_chunked state", torch.float32)
-    _need(state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vcols), f"gated_attn_chunked: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vcols}]")
+    if not (state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vcols)):
+        raise KernelError(f"gated_attn_chunked: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vcols}]")
     _cuda(slot_ids, "gated_attn_chunked slot_ids", torch.int32)
     _cuda(seq_start, "gated_attn_chunked seq_start", torch.int32)
     S = slot_ids.numel()
@@ -1995,7 +2060,8 @@ def head_norm_gate(
     xs = _rows(x, "head_norm_gate x")
     T = x.shape[0]
     xh = n + (1 if m is not None else 0)
-    _need(x.shape[1] == num_heads * xh, f"head_norm_gate: x {tuple(x.shape)} is not [T, {num_heads} * {xh}]")
+    if not (x.shape[1] == num_heads * xh):
+        raise KernelError(f"head_norm_gate: x {tuple(x.shape)} is not [T, {num_heads} * {xh}]")
     per_head = 0
     if weight is not None:
         _cuda(weight, "head_norm_gate weight", torch.float32)
@@ -2044,9 +2110,11 @@ def short_conv(
     xs = _rows(x, "short_conv x")
     T, C = x.shape
     _cuda(w, "short_conv w", torch.float32)
-    _need(w.dim() == 2 and w.shape[1] == C, f"short_conv: w {tuple(w.shape)} does not have {C} columns")
+    if not (w.dim() == 2 and w.shape[1] == C):
+        raise KernelError(f"short_conv: w {tuple(w.shape)} does not have {C} columns")
     taps = w.shape[0]
-    _need(1 <= taps <= SHORT_CONV_MAX_TAPS, f"short_conv: {taps} taps (1 to {SHORT_CONV_MAX_TAPS})")
+    if not (1 <= taps <= SHORT_CONV_MAX_TAPS):
+        raise KernelError(f"short_conv: {taps} taps (1 to {SHORT_CONV_MAX_TAPS})")
     _cuda(slot_ids, "short_conv slot_ids", torch.int32)
     _cuda(seq_start, "short_conv seq_start", torch.int32)
     _cuda(tok_seq, "short_conv tok_seq", torch.int32)
@@ -2054,11 +2122,13 @@ def short_conv(
     _need(seq_start.numel() == S + 1 and tok_seq.numel() == T, "short_conv: metadata sizes")
     if taps > 1:
         _cuda(state, "short_conv state", torch.float32)
-        _need(state.dim() == 3 and tuple(state.shape[1:]) == (taps - 1, C), f"short_conv: state {tuple(state.shape)} is not [slots, {taps - 1}, {C}]")
+        if not (state.dim() == 3 and tuple(state.shape[1:]) == (taps - 1, C)):
+            raise KernelError(f"short_conv: state {tuple(state.shape)} is not [slots, {taps - 1}, {C}]")
     if bias is not None:
         _cuda(bias, "short_conv bias", torch.float32)
         _need(bias.numel() == C, "short_conv: one bias per channel")
-    _need(not single or T == S, f"short_conv: {T} tokens of {S} sequences are not one each")
+    if not (not single or T == S):
+        raise KernelError(f"short_conv: {T} tokens of {S} sequences are not one each")
     out = torch.empty((T, C), dtype=x.dtype, device=x.device)
     lib = build.load("delta_rule")
     rc = lib.rl_short_conv(
@@ -2107,12 +2177,15 @@ def delta_rule(
     H, G = num_heads, num_qk_heads
     for name, t, n in (("qn", qn, G * dim), ("kn", kn, G * dim), ("kq", kq, G), ("beta", beta, H), ("decay", decay, H)):
         _cuda(t, f"delta_rule {name}", torch.float32)
-        _need(tuple(t.shape) == (T, n), f"delta_rule: {name} {tuple(t.shape)} is not [{T}, {n}]")
+        if not (tuple(t.shape) == (T, n)):
+            raise KernelError(f"delta_rule: {name} {tuple(t.shape)} is not [{T}, {n}]")
     _cuda(v, "delta_rule v", contiguous=False)
     _need(tuple(v.shape) == (T, H * vdim), "delta_rule: v must be [T, H vdim]")
-    _need(dim <= DELTA_RULE_MAX_DIM, f"delta_rule: key size {dim} exceeds {DELTA_RULE_MAX_DIM}")
+    if not (dim <= DELTA_RULE_MAX_DIM):
+        raise KernelError(f"delta_rule: key size {dim} exceeds {DELTA_RULE_MAX_DIM}")
     _cuda(state, "delta_rule state", torch.float32)
-    _need(state.dim() == 4 and tuple(state.shape[1:]) == (H, dim, vdim), f"delta_rule: state {tuple(state.shape)} is not [slots, {H}, {dim}, {vdim}]")
+    if not (state.dim() == 4 and tuple(state.shape[1:]) == (H, dim, vdim)):
+        raise KernelError(f"delta_rule: state {tuple(state.shape)} is not [slots, {H}, {dim}, {vdim}]")
     _cuda(slot_ids, "delta_rule slot_ids", torch.int32)
     _cuda(seq_start, "delta_rule seq_start", torch.int32)
     S = slot_ids.numel()
@@ -2134,7 +2207,8 @@ def ssm_gates(raw: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor):
     T, H = raw.shape
     for name, t in (("a_log", a_log), ("dt_bias", dt_bias)):
         _cuda(t, f"ssm_gates {name}", torch.float32)
-        _need(t.numel() == H, f"ssm_gates: one {name} per head")
+        if not (t.numel() == H):
+            raise KernelError(f"ssm_gates: one {name} per head")
     log_a, dt = (torch.empty((T, H), dtype=torch.float32, device=raw.device) for _ in range(2))
     lib = build.load("state_space")
     rc = lib.rl_ssm_gates(_p(raw), c_int(_dt(raw, "ssm_gates")), c_int(_rows(raw, "ssm_gates raw")), _p(a_log), _p(dt_bias), _p(log_a), _p(dt), c_int(T), c_int(H), _stream())
@@ -2152,11 +2226,13 @@ def ssm_gate_norm(
     T, n = y.shape
     for name, t in (("x", x), ("z", z)):
         _cuda(t, f"ssm_gate_norm {name}", act_dtype, contiguous=False)
-        _need(tuple(t.shape) == (T, n), f"ssm_gate_norm: {name} {tuple(t.shape)} does not match y {(T, n)}")
+        if not (tuple(t.shape) == (T, n)):
+            raise KernelError(f"ssm_gate_norm: {name} {tuple(t.shape)} does not match y {(T, n)}")
     _cuda(skip, "ssm_gate_norm skip", torch.float32)
     _cuda(weight, "ssm_gate_norm weight", torch.float32)
     H = skip.numel()
-    _need(n % H == 0 and n % groups == 0 and weight.numel() == n, f"ssm_gate_norm: {H} heads, {groups} parts and {weight.numel()} weights for a row of {n}")
+    if not (n % H == 0 and n % groups == 0 and weight.numel() == n):
+        raise KernelError(f"ssm_gate_norm: {H} heads, {groups} parts and {weight.numel()} weights for a row of {n}")
     if out is None:
         out = torch.empty((T, n), dtype=act_dtype, device=y.device)
     _cuda(out, "ssm_gate_norm out", act_dtype, contiguous=False)
@@ -2192,19 +2268,24 @@ def scalar_decay_chunked(
     value sizes up to 128: equal within rounding, for prompts.  max_q_len: the most tokens a sequence of the step brings; scratch:
     float32, `scalar_decay_chunked_scratch_floats(...)` numbers.  Returns float32 [T, H vdim]."""
     qk_heads = qk_heads or num_heads
-    _need(num_heads % qk_heads == 0, f"scalar_decay_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
+    if not (num_heads % qk_heads == 0):
+        raise KernelError(f"scalar_decay_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
     for name, t, n in (("q", q, qk_heads * dim), ("k", k, qk_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"scalar_decay_chunked {name}", torch.bfloat16, contiguous=False)
-        _need(_rows(t, f"scalar_decay_chunked {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0], f"scalar_decay_chunked: {name} has the wrong shape or stride")
+        if not (_rows(t, f"scalar_decay_chunked {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0]):
+            raise KernelError(f"scalar_decay_chunked: {name} has the wrong shape or stride")
     T = q.shape[0]
-    _need(scalar_decay_chunked_takes(dim, vdim), f"scalar_decay_chunked: sizes {dim} x {vdim} are not built")
+    if not (scalar_decay_chunked_takes(dim, vdim)):
+        raise KernelError(f"scalar_decay_chunked: sizes {dim} x {vdim} are not built")
     _cuda(log_decay, "scalar_decay_chunked log_decay", torch.float32)
-    _need(log_decay.numel() == T * num_heads, f"scalar_decay_chunked: log_decay {tuple(log_decay.shape)} is not [T, H]")
+    if not (log_decay.numel() == T * num_heads):
+        raise KernelError(f"scalar_decay_chunked: log_decay {tuple(log_decay.shape)} is not [T, H]")
     if in_scale is not None:
         _cuda(in_scale, "scalar_decay_chunked in_scale", torch.float32)
         _need(in_scale.numel() == T * num_heads, "scalar_decay_chunked: in_scale must be [T, H]")
     _cuda(state, "scalar_decay_chunked state", torch.float32)
-    _need(state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vdim), f"scalar_decay_chunked: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vdim}]")
+    if not (state.dim() == 4 and tuple(state.shape[1:]) == (num_heads, dim, vdim)):
+        raise KernelError(f"scalar_decay_chunked: state {tuple(state.shape)} is not [slots, {num_heads}, {dim}, {vdim}]")
     _cuda(slot_ids, "scalar_decay_chunked slot_ids", torch.int32)
     _cuda(seq_start, "scalar_decay_chunked seq_start", torch.int32)
     S = slot_ids.numel()
@@ -2281,9 +2362,11 @@ def flash_mix(
     qs = _rows(q, "flash_mix q")
     T = q.shape[0]
     parts = num_kv_heads if folded else 1
-    _need(maps in (1, 2) and num_heads % maps == 0 and kdim % (8 * maps) == 0, f"flash_mix: {maps} maps in {num_heads} heads of {kdim}")
+    if not (maps in (1, 2) and num_heads % maps == 0 and kdim % (8 * maps) == 0):
+        raise KernelError(f"flash_mix: {maps} maps in {num_heads} heads of {kdim}")
     _need(q.shape[1] >= num_heads // maps * parts * kdim, "flash_mix: q rows too short")
-    _need(flash_mix_takes(kdim, vdim, parts), f"flash_mix: sizes {kdim} / {vdim} with {parts} query parts are not built")
+    if not (flash_mix_takes(kdim, vdim, parts)):
+        raise KernelError(f"flash_mix: sizes {kdim} / {vdim} with {parts} query parts are not built")
     _check_kv_pages(k_pages, v_pages, torch.bfloat16, num_kv_heads, kdim, vdim, "flash_mix")
     _cuda(block_table, "flash_mix block_table", torch.int32)
     _cuda(seq_start, "flash_mix seq_start", torch.int32)
@@ -2337,12 +2420,14 @@ def flash_mix_decode(
     _cuda(qf, "flash_mix_decode qf", torch.bfloat16)
     S = qf.shape[0]
     _need(qf.dim() == 2 and qf.shape[1] == num_heads * num_kv_heads * kdim, "flash_mix_decode: qf must be [S, H K kdim]")
-    _need(flash_mix_decode_takes(num_heads, num_kv_heads, kdim, vdim), f"flash_mix_decode: sizes {num_heads} / {num_kv_heads} / {kdim} / {vdim} are not built")
+    if not (flash_mix_decode_takes(num_heads, num_kv_heads, kdim, vdim)):
+        raise KernelError(f"flash_mix_decode: sizes {num_heads} / {num_kv_heads} / {kdim} / {vdim} are not built")
     _check_kv_pages(k_pages, v_pages, torch.bfloat16, num_kv_heads, kdim, vdim, "flash_mix_decode")
     _cuda(block_table, "flash_mix_decode block_table", torch.int32)
     _cuda(seq_pos0, "flash_mix_decode seq_pos0", torch.int32)
     _need(seq_pos0.numel() == S and block_table.dim() == 2 and block_table.shape[0] >= S, "flash_mix_decode: metadata sizes")
-    _need(1 <= n_splits <= 256, f"flash_mix_decode: {n_splits} splits")
+    if not (1 <= n_splits <= 256):
+        raise KernelError(f"flash_mix_decode: {n_splits} splits")
     _check_sink(sink, num_heads, "flash_mix_decode")
     _cuda(scratch, "flash_mix_decode scratch", torch.float32)
     _need(scratch.numel() >= flash_mix_decode_scratch_floats(S, num_heads, vdim, n_splits), "flash_mix_decode: scratch too small")
