@@ -58,6 +58,10 @@
 // tile that lies wholly beyond the last distance with a number of its own adds one number to every score, which goes into the
 // exponent's constant.
 //
+// Keys of up to 192 beside values of up to 128 (latent attention whose keys and values were expanded for the call, with its output gate in
+// the way out): two blocks still fit an SM with one value stage, whose next tile is asked for behind the next key tile.  16 heads, 2048
+// tokens: 63 us, 21.5 GFLOP at 340 TFLOP/s; the same layer on its latents with mma.sync 468 us.
+//
 // Every mbarrier wait is bounded; on expiry a code goes to status[0] and the block drains.
 #include "tc_common.cuh"
 
@@ -83,7 +87,9 @@ RL_DEFINE_ERROR_TEXT()
 #define BIAS_GLOBAL 2
 // Q is KD / 64 sub-tiles of 16 KB; a K tile KD / 64 sub-tiles of 8 KB, a V tile VD / 64.  Two blocks must fit an SM and
 // no more (a third would wait for tensor memory): at small head sizes the request is padded to that end.
-#define SMEM_NEEDED(KD, VD) ((KD) / 64 * SUBQ_BYTES + KV_STAGES * ((KD) / 64 + (VD) / 64) * SUBK_BYTES + SMALL_BYTES)
+// With keys of 192 that leaves room for one value tile instead of two.
+#define V_STAGES(KD) ((KD) > 128 ? 1 : KV_STAGES)
+#define SMEM_NEEDED(KD, VD) ((KD) / 64 * SUBQ_BYTES + (KV_STAGES * ((KD) / 64) + V_STAGES(KD) * ((VD) / 64)) * SUBK_BYTES + SMALL_BYTES)
 #define SMEM_BYTES_OF(KD, VD) (SMEM_NEEDED(KD, VD) > 80 * 1024 ? SMEM_NEEDED(KD, VD) : 80 * 1024)
 
 struct SmallItems {
@@ -96,7 +102,7 @@ struct SmallItems {
 static_assert(sizeof(SmallItems) <= SMALL_BYTES, "the small items must fit behind the tiles");
 static_assert(KV_STAGES == 2, "tile j's key / value stage and its S buffer / product barrier share the index j & 1");
 static_assert(SOFTMAX_WARPS * ROW_STAGE_BYTES <= SUBQ_BYTES, "the output's way out uses the queries' buffer");
-static_assert(2 * (SMEM_BYTES_OF(128, 128) + 1024) <= 228 * 1024, "two blocks must fit an SM's shared memory");
+static_assert(2 * (SMEM_BYTES_OF(128, 128) + 1024) <= 228 * 1024 && 2 * (SMEM_BYTES_OF(192, 128) + 1024) <= 228 * 1024, "two blocks must fit an SM's shared memory");
 
 // 2^x for x <= 8 or so; -inf gives 0
 __device__ __forceinline__ float exp2_fast(float x) {
@@ -113,7 +119,55 @@ template <int KD>
 __device__ __forceinline__ uint32_t qk_block(uint32_t tmem_s, uint64_t q_desc, uint64_t k_desc, uint32_t idesc, uint32_t commit_bar,
                                              uint32_t peek_bar, uint32_t peek_parity) {
   uint32_t ready;
-  if (KD == 128) {
+  if (KD == 192) {
+    asm volatile(
+        "{\n"
+        ".reg .pred t, f, q;\n"
+        ".reg .b64 a1, a2, a3, a4, a5, a6, a7, a8, a9, a10, a11, b1, b2, b3, b4, b5, b6, b7, b8, b9, b10, b11;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 q, [%6], %7;\n"
+        "setp.eq.b32 t, 0, 0;\n"
+        "setp.ne.b32 f, 0, 0;\n"
+        "add.u64 a1, %2, 2;\n"
+        "add.u64 b1, %3, 2;\n"
+        "add.u64 a2, %2, 4;\n"
+        "add.u64 b2, %3, 4;\n"
+        "add.u64 a3, %2, 6;\n"
+        "add.u64 b3, %3, 6;\n"
+        "add.u64 a4, %2, 1024;\n"
+        "add.u64 b4, %3, 512;\n"
+        "add.u64 a5, %2, 1026;\n"
+        "add.u64 b5, %3, 514;\n"
+        "add.u64 a6, %2, 1028;\n"
+        "add.u64 b6, %3, 516;\n"
+        "add.u64 a7, %2, 1030;\n"
+        "add.u64 b7, %3, 518;\n"
+        "add.u64 a8, %2, 2048;\n"
+        "add.u64 b8, %3, 1024;\n"
+        "add.u64 a9, %2, 2050;\n"
+        "add.u64 b9, %3, 1026;\n"
+        "add.u64 a10, %2, 2052;\n"
+        "add.u64 b10, %3, 1028;\n"
+        "add.u64 a11, %2, 2054;\n"
+        "add.u64 b11, %3, 1030;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, f;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a1, b1, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a2, b2, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a3, b3, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a4, b4, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a5, b5, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a6, b6, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a7, b7, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a8, b8, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a9, b9, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a10, b10, %4, t;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%1], a11, b11, %4, t;\n"
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n"
+        "selp.u32 %0, 1, 0, q;\n"
+        "}\n"
+        : "=r"(ready)
+        : "r"(tmem_s), "l"(q_desc), "l"(k_desc), "r"(idesc), "r"(commit_bar), "r"(peek_bar), "r"(peek_parity)
+        : "memory");
+  } else if (KD == 128) {
     asm volatile(
         "{\n"
         ".reg .pred t, f, q;\n"
@@ -229,22 +283,23 @@ __device__ __forceinline__ uint32_t pv_block(uint32_t tmem_o, uint32_t tmem_p, u
 // KD, VD: the padded sizes of a key and a value; kdim, vdim: the sizes themselves.
 // MAPS 2: query heads 2h and 2h + 1 are the two halves of the KD numbers of row h (the values are the same for both); the row's
 // tile is loaded whole and a block's scores use its half of it and of the keys (kdim is then KD).
-template <int KD, int VD, int MAPS, int BIAS>
+// EXPANDED: keys and values as rows of their own for this call (no page table), and the result may go through an output gate.
+template <int KD, int VD, int MAPS, int BIAS, bool EXPANDED>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table, int table_width,
                         const int* __restrict__ seq_start, const int* __restrict__ seq_pos0, bf16* __restrict__ out,
                         int out_stride, int H, int K, int window, float scale_log2, int* __restrict__ status,
                         int test_role, uint32_t test_ns, const float* __restrict__ sink, int chunk, float softcap,
-                        const float* __restrict__ bias, int bias_len, int kdim, int vdim) {
+                        const float* __restrict__ bias, int bias_len, int kdim, int vdim, const bf16* __restrict__ gate, int gate_stride) {
   // All shared memory is dynamic, so that the tiles start at the block's first byte (1024-byte
   // aligned, as the 128-byte swizzle needs) and the small items fit behind them.
-  constexpr int K_SUBS = KD / 64, V_SUBS = VD / 64, Q_BYTES = K_SUBS * SUBQ_BYTES, K_BYTES = K_SUBS * SUBK_BYTES, V_BYTES = V_SUBS * SUBK_BYTES;
+  constexpr int K_SUBS = KD / 64, V_SUBS = VD / 64, VS = V_STAGES(KD), Q_BYTES = K_SUBS * SUBQ_BYTES, K_BYTES = K_SUBS * SUBK_BYTES, V_BYTES = V_SUBS * SUBK_BYTES;
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   unsigned char* q_s = smem_dyn;                          // 128 rows x KD
   unsigned char* k_s = q_s + Q_BYTES;                     // KV_STAGES x (64 keys x KD)
-  unsigned char* v_s = k_s + KV_STAGES * K_BYTES;         // KV_STAGES x (64 keys x VD)
-  SmallItems& sm = *reinterpret_cast<SmallItems*>(v_s + KV_STAGES * V_BYTES);
+  unsigned char* v_s = k_s + KV_STAGES * K_BYTES;         // VS x (64 keys x VD)
+  SmallItems& sm = *reinterpret_cast<SmallItems*>(v_s + VS * V_BYTES);
   uint64_t& q_full = sm.q_full;
   uint64_t(&k_full)[KV_STAGES] = sm.k_full;
   uint64_t(&v_full)[KV_STAGES] = sm.v_full;
@@ -318,34 +373,49 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
       for (int b = 0; b < K_SUBS; ++b) tma_load_2d(q_s + b * SUBQ_BYTES, &map_q, &q_full, (h / MAPS) * kdim + 64 * b, tok0 + row0);
       const int* table = block_table + (size_t)s * table_width;
-      for (int j = 0; j < n_tiles; ++j) {
-        const int st = j % KV_STAGES;
-        const uint32_t round = j / KV_STAGES;
+      // a page past the sequence's end is never attended to; without a table a sequence has `table_width` pages of its own
+      auto page_of = [&](int j) {
         const int tile = tile_lo + j;
-        const int page = tile < table_width ? table[tile] : 0;  // a page past the sequence's end is never attended to
-        // K
+        return EXPANDED ? s * table_width + tile : tile < table_width ? table[tile] : 0;
+      };
+      auto load_k = [&](int j) -> bool {
+        const int st = j % KV_STAGES;
         // (a key stage is free when the S it fed is complete, a value stage when its P V is: with two stages and two S
         // buffers, tile j's stage and its S buffer have the same index, and one commit serves both waiters)
-        if (round > 0 && !mbar_wait_role(&s_full[st], (round - 1) & 1, ctl, 11)) {
+        if (j >= KV_STAGES && !mbar_wait_role(&s_full[st], (j / KV_STAGES - 1) & 1, ctl, 11)) {
           give_up_code(status, 11);
           abort_flag = 1;
-          break;
+          return false;
         }
-        if (*(volatile int*)&abort_flag) break;
+        if (*(volatile int*)&abort_flag) return false;
+        const int page = page_of(j);
         mbar_expect_tx(&k_full[st], K_BYTES);
 #pragma unroll
         for (int b = 0; b < K_SUBS; ++b) tma_load_4d(k_s + (size_t)st * K_BYTES + b * SUBK_BYTES, &map_k, &k_full[st], 64 * b, 0, kh, page);
         issued_k = j + 1;
-        // V
-        if (round > 0 && !mbar_wait_role(&pv_done[st], (round - 1) & 1, ctl, 12)) {
+        return true;
+      };
+      auto load_v = [&](int j) -> bool {
+        const int st = j % VS, before = j - VS;  // the tile whose product must be done with the stage
+        if (before >= 0 && !mbar_wait_role(&pv_done[before & 1], (before >> 1) & 1, ctl, 12)) {
           give_up_code(status, 12);
           abort_flag = 1;
-          break;
+          return false;
         }
+        const int page = page_of(j);
         mbar_expect_tx(&v_full[st], V_BYTES);
 #pragma unroll
         for (int b = 0; b < V_SUBS; ++b) tma_load_4d(v_s + (size_t)st * V_BYTES + b * SUBK_BYTES, &map_v, &v_full[st], 64 * b, 0, kh, page);
         issued_v = j + 1;
+        return true;
+      };
+      if (VS == KV_STAGES) {
+        for (int j = 0; j < n_tiles; ++j)
+          if (!load_k(j) || !load_v(j)) break;
+      } else if (load_k(0)) {
+        // with one value stage, value tile j waits for the product before it: the next key tile is asked for first
+        for (int j = 0; j < n_tiles; ++j)
+          if ((j + 1 < n_tiles && !load_k(j + 1)) || !load_v(j)) break;
       }
     }
   } else if (warp == SOFTMAX_WARPS + 1) {
@@ -382,7 +452,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int st = j % KV_STAGES;
         tc_fence_after();
         v_ready = qk_block<KD / MAPS>(tmem_base + (uint32_t)((j & 1) * BNK), q_desc, make_smem_desc(smem_u32(k_s + (size_t)st * K_BYTES)) + k_half, idesc_qk,
-                               smem_u32(&s_full[j & 1]), smem_u32(&v_full[jv % KV_STAGES]), (uint32_t)((jv / KV_STAGES) & 1));
+                               smem_u32(&s_full[j & 1]), smem_u32(&v_full[jv % VS]), (uint32_t)((jv / VS) & 1));
       };
       if (ok) ok = wait_for(&k_full[0], 0, 14);
       if (ok) issue_qk(0, 0);
@@ -396,8 +466,8 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // (P has a barrier per S buffer: the softmax warps may finish tile j + 1 before this thread looks for tile j, and a wait
         // on the parity of ONE barrier that had completed both phases by then would never return)
         if (!(ok = wait_for(&p_ready[j & 1], (j >> 1) & 1, 15))) break;
-        const int st = j % KV_STAGES;
-        if (!(ok = wait_for(&v_full[st], (j / KV_STAGES) & 1, 16))) break;
+        const int st = j % VS;
+        if (!(ok = wait_for(&v_full[st], (j / VS) & 1, 16))) break;
         tc_fence_after();
         // O += P(j) V(j); asks for key tile j + 2
         const int jk = j + 2;
@@ -564,6 +634,21 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           v0[i] = __float_as_uint(__uint_as_float(v0[i]) * inv);
           v1[i] = __float_as_uint(__uint_as_float(v1[i]) * inv);
         }
+        if (EXPANDED && gate != nullptr && r < rows_here) {  // every number times the logistic function of its gate's
+          const bf16* g = gate + (size_t)(tok0 + row0 + r) * gate_stride + (size_t)h * vdim + c * 64;
+          const int cols = min(64, vdim - c * 64);  // (a multiple of 8)
+#pragma unroll
+          for (int i = 0; i < 64; i += 8) {
+            if (i >= cols) break;
+            float f[8];
+            bf16x8_to_f32(__ldcg(reinterpret_cast<const uint4*>(g + i)), f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              uint32_t& x = i < 32 ? v0[(i + e) & 31] : v1[(i + e) & 31];
+              x = __float_as_uint(__uint_as_float(x) / (1.0f + expf(-f[e])));
+            }
+          }
+        }
         store_rows64_bf16(o + c * 64, out_stride, rows_valid, v0, v1, stage, lane, vdim - c * 64);
       }
     }
@@ -578,7 +663,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   if (threadIdx.x == SOFTMAX_WARPS * 32 && *(volatile int*)&abort_flag) {
     mbar_wait(&q_full, 0);
     for (int j = max(0, issued_k - KV_STAGES); j < issued_k; ++j) mbar_wait(&k_full[j % KV_STAGES], (j / KV_STAGES) & 1);
-    for (int j = max(0, issued_v - KV_STAGES); j < issued_v; ++j) mbar_wait(&v_full[j % KV_STAGES], (j / KV_STAGES) & 1);
+    for (int j = max(0, issued_v - VS); j < issued_v; ++j) mbar_wait(&v_full[j % VS], (j / VS) & 1);
   }
 }
 
@@ -586,26 +671,42 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 // Key and value sizes this kernel is built for (1 if it takes them): multiples of 8 up to 128.
 RL_API int rl_flash_prefill_tc_takes(int kdim, int vdim) { return kdim > 0 && vdim > 0 && kdim <= 128 && vdim <= 128 && kdim % 8 == 0 && vdim % 8 == 0; }
 
-template <int KD, int VD, int MAPS, int BIAS>
+// Keys or values as rows of K heads side by side, `head_stride` numbers apart: [page][position][head][dim] seen as pages of 64 positions of
+// one head, boxes and swizzle as make_page_map's.  0 on success.
+static int make_rows_map(CUtensorMap* map, const void* base, int n_pages, int heads, int dim, int head_stride) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return 1;
+  cuuint64_t dims[4] = {(cuuint64_t)dim, PAGE, (cuuint64_t)heads, (cuuint64_t)n_pages};
+  cuuint64_t strides[3] = {(cuuint64_t)heads * head_stride * 2, (cuuint64_t)head_stride * 2, (cuuint64_t)PAGE * heads * head_stride * 2};
+  cuuint32_t box[4] = {64, PAGE, 1, 1}, estr[4] = {1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
+}
+
+template <int KD, int VD, int MAPS, int BIAS, bool EXPANDED = false>
 static int launch_flash_tc(const void* q, int q_stride, int n_tokens, const void* k_pages, const void* v_pages, int n_pages,
                            const int* block_table, int table_width, const int* seq_start, const int* seq_pos0, void* out,
                            int out_stride, int n_seqs, int max_q_len, int H, int K, int kdim, int vdim, int window, float scale, int* status,
-                           int wait_test_role, unsigned int wait_test_ns, const float* sink, int chunk, float softcap, const float* bias, int bias_len, cudaStream_t stream) {
+                           int wait_test_role, unsigned int wait_test_ns, const float* sink, int chunk, float softcap, const float* bias, int bias_len, cudaStream_t stream,
+                           int head_stride = 0, const bf16* gate = nullptr, int gate_stride = 0) {
   CUtensorMap map_q, map_k, map_v;
   if (make_matrix_map(&map_q, q, n_tokens, q_stride, q_stride, BMQ))
     RL_REFUSE(10, "flash_prefill_tc: cannot describe the query tensor to TMA");
-  if (make_page_map(&map_k, k_pages, n_pages, K, PAGE, kdim, PAGE) || make_page_map(&map_v, v_pages, n_pages, K, PAGE, vdim, PAGE))
+  if (EXPANDED) {
+    if (make_rows_map(&map_k, k_pages, n_pages, K, kdim, head_stride) || make_rows_map(&map_v, v_pages, n_pages, K, vdim, head_stride))
+      RL_REFUSE(11, "flash_prefill_tc: cannot describe the keys and values to TMA");
+  } else if (make_page_map(&map_k, k_pages, n_pages, K, PAGE, kdim, PAGE) || make_page_map(&map_v, v_pages, n_pages, K, PAGE, vdim, PAGE))
     RL_REFUSE(11, "flash_prefill_tc: cannot describe the cache pages to TMA");
   size_t smem = SMEM_BYTES_OF(KD, VD);
   const size_t with_bias = SMEM_NEEDED(KD, VD) + (size_t)(bias_len + 2 * BIAS_PAD) * 4;
   if (BIAS == BIAS_SMEM && with_bias > smem) smem = with_bias;
-  auto kern = flash_prefill_tc_kernel<KD, VD, MAPS, BIAS>;
+  auto kern = flash_prefill_tc_kernel<KD, VD, MAPS, BIAS, EXPANDED>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     RL_REFUSE(12, "flash_prefill_tc: cannot get %zu bytes of shared memory", smem);
   dim3 grid(H * n_seqs, (max_q_len + BMQ - 1) / BMQ);
   RL_LAUNCH_CHECK(rl_launch(kern, grid, NUM_THREADS, smem, stream, map_q, map_k, map_v, block_table, table_width, seq_start, seq_pos0,
                             (bf16*)out, out_stride, H, K, window, scale * 1.4426950408889634f, status, wait_test_role,
-                            (uint32_t)wait_test_ns, sink, chunk, softcap, bias, bias_len, kdim, vdim));
+                            (uint32_t)wait_test_ns, sink, chunk, softcap, bias, bias_len, kdim, vdim, gate, gate_stride));
   return 0;
 }
 
@@ -653,4 +754,35 @@ RL_API int rl_flash_prefill_tc(const void* q, int q_stride, int n_tokens, const 
   RL_FTC_BIAS(128, 128);
 #undef RL_FTC_BIAS
 #undef RL_FTC
+}
+
+// The same over keys and values that were expanded for this call, every head its own: rows [n_seqs][pages_per_seq * 64][H][head_stride]
+// of bfloat16, a head's value at its start (vdim numbers) and its key behind (kdim numbers).  Key sizes up to 192, value sizes up to
+// 128, multiples of 8.  gate: null, or rows of >= H vdim numbers, one row a token: the result is multiplied by their logistic function.
+RL_API int rl_flash_prefill_tc_expanded_takes(int kdim, int vdim) { return kdim > 0 && vdim > 0 && kdim <= 192 && vdim <= 128 && kdim % 8 == 0 && vdim % 8 == 0; }
+
+RL_API int rl_flash_prefill_tc_expanded(const void* q, int q_stride, int n_tokens, const void* kv, int pages_per_seq, int head_stride,
+                                        const int* seq_start, const int* seq_pos0, void* out, int out_stride, int n_seqs, int max_q_len, int H,
+                                        int kdim, int vdim, int window, float scale, const float* sink, const void* gate, int gate_stride,
+                                        int* status, int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
+  if (n_seqs <= 0 || max_q_len <= 0 || H <= 0 || n_tokens <= 0 || pages_per_seq <= 0)
+    RL_REFUSE(1, "flash_prefill_tc_expanded: S=%d max_q=%d H=%d T=%d pages=%d", n_seqs, max_q_len, H, n_tokens, pages_per_seq);
+  if (!rl_flash_prefill_tc_expanded_takes(kdim, vdim)) RL_REFUSE(2, "flash_prefill_tc_expanded: key and value sizes %d / %d (multiples of 8 up to 192 / 128)", kdim, vdim);
+  if (head_stride % 8 || head_stride < kdim + vdim) RL_REFUSE(3, "flash_prefill_tc_expanded: heads %d apart hold no value of %d and key of %d", head_stride, vdim, kdim);
+  if (q_stride % 8 || out_stride % 8 || (gate != nullptr && gate_stride % 8)) RL_REFUSE(5, "flash_prefill_tc_expanded: strides %d/%d/%d break 16-byte alignment", q_stride, out_stride, gate_stride);
+  if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out | (uintptr_t)gate) & 15) RL_REFUSE(6, "flash_prefill_tc_expanded: operands must be 16-byte aligned");
+  if ((long long)H * n_seqs > 0x7fffffffLL || (max_q_len + BMQ - 1) / BMQ > 65535 || (long long)n_seqs * pages_per_seq > 0x7fffffffLL)
+    RL_REFUSE(7, "flash_prefill_tc_expanded: H=%d x S=%d blocks or %d query rows exceed the grid", H, n_seqs, max_q_len);
+  if (window < 0 || status == nullptr || !(scale > 0.f)) RL_REFUSE(8, "flash_prefill_tc_expanded: bad window or scale, or no status word");
+#define RL_FTX(KDV, VDV)                                                                                                                     \
+  return launch_flash_tc<KDV, VDV, 1, BIAS_NONE, true>(q, q_stride, n_tokens, (const bf16*)kv + vdim, kv, n_seqs * pages_per_seq, nullptr, pages_per_seq, \
+                                                 seq_start, seq_pos0, out, out_stride, n_seqs, max_q_len, H, H, kdim, vdim, window, scale, status,  \
+                                                 wait_test_role, wait_test_ns, sink, 0, 0.f, nullptr, 0, stream, head_stride, (const bf16*)gate, gate_stride)
+  if (kdim <= 64 && vdim <= 64) RL_FTX(64, 64);
+  if (kdim <= 64) RL_FTX(64, 128);
+  if (kdim <= 128 && vdim <= 64) RL_FTX(128, 64);
+  if (kdim <= 128) RL_FTX(128, 128);
+  if (vdim <= 64) RL_FTX(192, 64);
+  RL_FTX(192, 128);
+#undef RL_FTX
 }

@@ -83,6 +83,8 @@ struct Groups {
   int gather_div;
   const int* tiles;    // the plan: [0] groups, then (expert, first row, rows) of each; null: heads
   int heads, M;        // heads: groups of up to NT of M tokens, head after head
+  const int* held;     // heads: null, or how many rows each of M / seq_rows runs of `seq_rows` rows holds (rounded up to 64; the rest is left out)
+  int seq_rows;
   long long ldo, oh;
   const bf16* gate;    // SIGMOID
   long long ldg, gh;
@@ -125,7 +127,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   tc_fence_before();
   pdl_trigger();
   pdl_wait();  // the plan, the rows: other kernels' output
-  const int blocks_n = (g.N + UNIT_N - 1) / UNIT_N, per_head = (g.M + NT - 1) / NT;
+  const int blocks_n = (g.N + UNIT_N - 1) / UNIT_N, per_run = g.held != nullptr ? (g.seq_rows + NT - 1) / NT : 0;
+  const int per_head = g.held != nullptr ? g.M / g.seq_rows * per_run : (g.M + NT - 1) / NT;
   const int n_groups = g.tiles != nullptr ? __ldcg(g.tiles) : g.heads * per_head;
   if (g.tiles != nullptr)
     for (int i = threadIdx.x; i < 3 * min(n_groups, LISTED_TILES); i += NUM_THREADS) listed[i] = __ldcg(g.tiles + 1 + i);
@@ -133,13 +136,19 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   const int n_units = n_groups * blocks_n, n_k = (g.K + BK - 1) / BK;
-  // the group of a unit: its matrix, its first row and how many
+  // the group of a unit: its matrix, its first row and how many (none, of a run that holds fewer: every role passes over the unit)
   auto group = [&](int unit, int& e, int& r0, int& rows) {
     const int t = unit / blocks_n;
     if (g.tiles == nullptr) {
       e = t / per_head;
-      r0 = (t - e * per_head) * NT;
-      rows = min(NT, g.M - r0);
+      if (g.held == nullptr) {
+        r0 = (t - e * per_head) * NT;
+        rows = min(NT, g.M - r0);
+      } else {
+        const int run = (t - e * per_head) / per_run, at = (t - e * per_head - run * per_run) * NT;
+        r0 = run * g.seq_rows + at;
+        rows = min(NT, min(g.seq_rows, (__ldcg(g.held + run) + 63) & ~63) - at);
+      }
     } else if (t < LISTED_TILES) {
       e = listed[3 * t];
       r0 = listed[3 * t + 1];
@@ -160,6 +169,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
         int e, r0, rows;
         group(unit, e, r0, rows);
+        if (rows <= 0) continue;
         const int w_row = e * g.N + (unit % blocks_n) * UNIT_N;
         const int w_row2 = EPI == GATED ? w_row : w_row + FEATURES / 2;
         for (int kb = 0; kb < n_k; ++kb, ++it) {
@@ -190,9 +200,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       uint32_t s = 0, phase = 0, ready = 0;
       bool ok = true;
       int local = 0;
-      for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++local) {
+      for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
         int e, r0, rows;
         group(unit, e, r0, rows);
+        if (rows <= 0) continue;
         const uint32_t idesc = make_idesc(FEATURES, (rows + 15) & ~15);
         const int acc = local & 1;
         const uint32_t use = local >> 1;
@@ -222,6 +233,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           ready = umma_bf16_x4_commit_peek(tmem_d, a_desc0 + off, b_desc0 + off, idesc, kb > 0 ? 1u : 0u, empty0 + 8 * here, full0 + 8 * s, phase);
         }
         if (ok) umma_commit(&acc_full[acc]);
+        ++local;
       }
       if (!ok) {  // neither tensor memory nor the block may go before what was issued is done
         umma_commit(&drain_bar);
@@ -244,9 +256,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     bool ok = true;
     const bool gathered = g.order != nullptr;
     if (gathered) ask(blockIdx.x);
-    for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, base += n_k) {
+    for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
       int e, r0, rows;
       group(unit, e, r0, rows);
+      if (rows <= 0) continue;
       const int n16 = (rows + 15) & ~15;
       if (gathered) {
         __syncwarp();
@@ -273,11 +286,12 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const int boxes = (rows + SH::BOX_ROWS - 1) / SH::BOX_ROWS;
             mbar_expect_tx_s(bar, boxes * SH::BOX_ROWS * BK * 2);
             for (int i = 0; i < boxes; ++i)
-              tma_load_3d_s(dst + i * SH::BOX_ROWS * BK * 2, &map_x, bar, k, g.tiles == nullptr ? e : 0, r0 + i * SH::BOX_ROWS);
+              tma_load_3d_s(dst + i * SH::BOX_ROWS * BK * 2, &map_x, bar, k, g.tiles == nullptr && g.xh != 0 ? e : 0, r0 + i * SH::BOX_ROWS);
           }
         }
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      base += n_k;
     }
     if (lane == 0) rows_asked[w] = mine;
   } else {
@@ -288,9 +302,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     float* traded = trade + (half * 2 + pair) * (2 * 2 * 8 * 32);
     const bool relu2 = EPI == PLAIN && g.act_limit == RL_UNARY_RELU2;
     int local = 0;
-    for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x, ++local) {
+    for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
       int e, r0, rows;
       group(unit, e, r0, rows);
+      if (rows <= 0) continue;
       const int acc = local & 1;
       // one warp polls and decides for all; the others wait at a hardware barrier, off the issue slots
       if (warp == 2) {
@@ -355,6 +370,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      ++local;
     }
   }
   tc_fence_before();
@@ -382,7 +398,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 static int make_rows_map(CUtensorMap* map, const Groups& g, int box_rows) {
   EncodeTiledFn enc = encode_tiled();
   if (!enc) return 1;
-  const int heads = g.tiles == nullptr ? g.heads : 1;
+  const int heads = g.tiles == nullptr && g.xh != 0 ? g.heads : 1;  // (without a step from head to head all read the same rows)
   cuuint64_t dims[3] = {(cuuint64_t)g.K, (cuuint64_t)heads, (cuuint64_t)g.x_rows};
   cuuint64_t strides[2] = {(cuuint64_t)(heads > 1 ? g.xh : g.ldx) * 2, (cuuint64_t)g.ldx * 2};
   cuuint32_t box[3] = {64, 1, (cuuint32_t)box_rows}, estr[3] = {1, 1, 1};
@@ -490,10 +506,12 @@ RL_API int rl_moe_gemm_tc(const void* x, int ldx, int x_rows, const int* order, 
   RL_REFUSE(6, "moe_gemm_tc: unsupported output type %d (activation %d)", out_dtype, (int)(w2 != nullptr));
 }
 
-// x, out, gate: element (t, h, i) at base + t * ld + h * head stride + i.  w: [H, N, K] dense.
+// x, out, gate: element (t, h, i) at base + t * ld + h * head stride + i.  w: [H, N, K] dense.  held: null, or for each run of seq_rows
+// rows how many of them exist: only those, rounded up to 64, are computed.
 RL_API int rl_head_linear_tc(const void* x, int ldx, int xh, const void* w, void* out, int ldo, int oh, const void* gate, int ldg, int gh,
-                             int M, int H, int N, int K, int* status, int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
+                             int M, int H, int N, int K, const int* held, int seq_rows, int* status, int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
   if (M <= 0 || H <= 0 || N <= 0 || K <= 0) RL_REFUSE(1, "head_linear_tc: M=%d H=%d N=%d K=%d", M, H, N, K);
+  if (held != nullptr && (seq_rows <= 0 || M % seq_rows)) RL_REFUSE(4, "head_linear_tc: %d rows are no runs of %d", M, seq_rows);
   if (status == nullptr) RL_REFUSE(2, "head_linear_tc: no status word");
   if (int rc = refuse_operands("head_linear_tc", x, ldx, xh, w, nullptr, H, N, K)) return rc;
   Groups g = {};
@@ -511,7 +529,9 @@ RL_API int rl_head_linear_tc(const void* x, int ldx, int xh, const void* w, void
   g.gh = gh;
   g.N = N;
   g.K = K;
-  const long long groups = (long long)H * ((M + 255) / 256);
+  g.held = held;
+  g.seq_rows = seq_rows;
+  const long long groups = (long long)H * (held != nullptr ? M / seq_rows * ((seq_rows + 255) / 256) : (M + 255) / 256);
   if (gate != nullptr) return launch_grouped<bf16, SIGMOID, 256>(w, nullptr, H, out, g, groups, status, wait_test_role, wait_test_ns, stream);
   return launch_grouped<bf16, PLAIN, 256>(w, nullptr, H, out, g, groups, status, wait_test_role, wait_test_ns, stream);
 }

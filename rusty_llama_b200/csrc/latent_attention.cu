@@ -48,14 +48,15 @@ __device__ __forceinline__ void turn_pair(const T* __restrict__ src, T* __restri
   dst[d1] = from_f32<T>(v);
 }
 
+// (q may be q_cat: a pair is read before it is written, by one thread)
 template <typename T>
-__global__ void latent_prep_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ kv, int ldkv,
+__global__ void latent_prep_kernel(const T* q, int ldq, const T* __restrict__ kv, int ldkv,
                                    const float* __restrict__ norm_w, float eps, const float* __restrict__ freq,
                                    int n_pairs, int interleaved, float mag, const int* __restrict__ tok_pos,
                                    const int* __restrict__ tok_seq, const int* __restrict__ block_table,
-                                   int table_width, T* __restrict__ pages, int page_size, T* __restrict__ q_cat,
+                                   int table_width, T* __restrict__ pages, int page_size, T* q_cat,
                                    int H, int dim, int rot, int rank, const T* __restrict__ ql, int ldql, int q_rank,
-                                   const float* __restrict__ q_norm_w, T* __restrict__ ql_out) {
+                                   const float* __restrict__ q_norm_w, T* __restrict__ ql_out, long long cat_ld, int cat_head, int cat_at) {
   __shared__ float red[32];
   pdl_trigger();
   pdl_wait();
@@ -90,11 +91,11 @@ __global__ void latent_prep_kernel(const T* __restrict__ q, int ldq, const T* __
   const int half = rot / 2;
   for (int idx = threadIdx.x; idx < H * half; idx += blockDim.x) {
     const int h = idx / half, i = idx % half;
-    turn_pair(q + (size_t)t * ldq + (size_t)h * (dim + rot) + dim, q_cat + ((size_t)t * H + h) * Dk + rank, i, n_pairs, interleaved, pos, freq, mag);
+    turn_pair(q + (size_t)t * ldq + (size_t)h * (dim + rot) + dim, q_cat + t * cat_ld + (size_t)h * cat_head + cat_at, i, n_pairs, interleaved, pos, freq, mag);
   }
   if (rot & 1)
     for (int h = threadIdx.x; h < H; h += blockDim.x)
-      q_cat[((size_t)t * H + h) * Dk + rank + rot - 1] = q[(size_t)t * ldq + (size_t)h * (dim + rot) + dim + rot - 1];
+      q_cat[t * cat_ld + (size_t)h * cat_head + cat_at + rot - 1] = q[(size_t)t * ldq + (size_t)h * (dim + rot) + dim + rot - 1];
 }
 
 // q, kv, ql: each may be null, its part of the work is then left out.  ql: [T, >= q_rank] rows, the queries' latent; ql_out: [T, q_rank].
@@ -102,7 +103,7 @@ RL_API int rl_latent_prep(const void* q, int ldq, const void* kv, int ldkv, int 
                           const float* freq, int n_pairs, int interleaved, float mag, const int* tok_pos, const int* tok_seq,
                           const int* block_table, int table_width, void* pages, int page_size, void* q_cat,
                           int n_tokens, int H, int dim, int rot, int rank, const void* ql, int ldql, int q_rank, const float* q_norm_w,
-                          void* ql_out, cudaStream_t stream) {
+                          void* ql_out, int in_place, cudaStream_t stream) {
   if (n_tokens <= 0 || H <= 0 || dim < 0 || rot < 0 || rank <= 0 || page_size <= 0)
     RL_REFUSE(1, "latent_prep: T=%d H=%d dim=%d rot=%d rank=%d page=%d", n_tokens, H, dim, rot, rank, page_size);
   if (2 * n_pairs > rot) RL_REFUSE(2, "latent_prep: %d rotated pairs do not fit %d dimensions", n_pairs, rot);
@@ -110,17 +111,59 @@ RL_API int rl_latent_prep(const void* q, int ldq, const void* kv, int ldkv, int 
     RL_REFUSE(3, "latent_prep: a latent row to store, but no pages, page table or norm weight");
   if (ql != nullptr && (q_rank <= 0 || ldql < q_rank || q_norm_w == nullptr || ql_out == nullptr))
     RL_REFUSE(5, "latent_prep: a query latent of %d in rows of %d needs a norm weight and an output", q_rank, ldql);
-  if (q != nullptr && q_cat == nullptr) RL_REFUSE(6, "latent_prep: queries to turn, but nowhere to put them");
+  if (q != nullptr && q_cat == nullptr && !in_place) RL_REFUSE(6, "latent_prep: queries to turn, but nowhere to put them");
+  // in place: the turned parts go back into q's own rows
+  if (in_place) q_cat = const_cast<void*>(q);
+  const long long cat_ld = in_place ? ldq : (long long)H * (rank + rot);
+  const int cat_head = in_place ? dim + rot : rank + rot, cat_at = in_place ? dim : rank;
   if (dtype == RL_BF16)
     RL_LAUNCH_CHECK(rl_launch<false>(latent_prep_kernel<bf16>, n_tokens, 128, 0, stream, (const bf16*)q, ldq, (const bf16*)kv, ldkv,
                               norm_w, eps, freq, n_pairs, interleaved, mag, tok_pos, tok_seq, block_table, table_width, (bf16*)pages,
-                              page_size, (bf16*)q_cat, H, dim, rot, rank, (const bf16*)ql, ldql, q_rank, q_norm_w, (bf16*)ql_out));
+                              page_size, (bf16*)q_cat, H, dim, rot, rank, (const bf16*)ql, ldql, q_rank, q_norm_w, (bf16*)ql_out, cat_ld, cat_head, cat_at));
   else if (dtype == RL_F32)
     RL_LAUNCH_CHECK(rl_launch<false>(latent_prep_kernel<float>, n_tokens, 128, 0, stream, (const float*)q, ldq, (const float*)kv,
                               ldkv, norm_w, eps, freq, n_pairs, interleaved, mag, tok_pos, tok_seq, block_table, table_width,
-                              (float*)pages, page_size, (float*)q_cat, H, dim, rot, rank, (const float*)ql, ldql, q_rank, q_norm_w, (float*)ql_out));
+                              (float*)pages, page_size, (float*)q_cat, H, dim, rot, rank, (const float*)ql, ldql, q_rank, q_norm_w, (float*)ql_out, cat_ld, cat_head, cat_at));
   else
     RL_REFUSE(4, "latent_prep: unknown dtype %d", dtype);
+  return 0;
+}
+
+// ---------------------------------------------------------------- the rows whose keys and values are expanded per head
+// Row (s, j) of the call's [S, seq_rows] rows is position j of sequence s: its latent goes to latents[row][rank], its turned key part
+// behind the place of every head's plain key part, kv[row][h][key_at .. key_at + rot).  Positions that a sequence does not hold are
+// zeros up to its last page's end (the attention multiplies them by zero), and left alone behind it.  A warp a row, 16 bytes a lane.
+__global__ void __launch_bounds__(256)
+latent_rows_kernel(const bf16* __restrict__ pages, const int* __restrict__ block_table, int table_width, const int* __restrict__ seq_len,
+                   int seq_rows, bf16* __restrict__ latents, bf16* __restrict__ kv, int H, int head_stride, int key_at, int rot, int rank) {
+  pdl_trigger();
+  pdl_wait();
+  const int s = blockIdx.y, j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int len = __ldcg(seq_len + s);
+  if (j >= min(seq_rows, (len + 63) & ~63)) return;
+  const bool held = j < len;
+  const int page = held ? __ldcg(block_table + (size_t)s * table_width + j / 64) : 0;
+  const uint4* src = reinterpret_cast<const uint4*>(pages + ((size_t)page * 64 + j % 64) * (rank + rot));
+  const size_t row = (size_t)s * seq_rows + j;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4* dst = reinterpret_cast<uint4*>(latents + row * rank);
+  for (int i = lane; i < rank / 8; i += 32) dst[i] = held ? __ldcg(src + i) : zero;
+  const int pieces = rot / 8;
+  for (int i = lane; i < H * pieces; i += 32) {
+    const int h = i / pieces, c = i - h * pieces;
+    *reinterpret_cast<uint4*>(kv + (row * H + h) * head_stride + key_at + c * 8) = held ? __ldcg(src + rank / 8 + c) : zero;
+  }
+}
+
+RL_API int rl_latent_rows(const void* pages, const int* block_table, int table_width, const int* seq_len, int n_seqs, int seq_rows,
+                          void* latents, void* kv, int H, int head_stride, int key_at, int rot, int rank, cudaStream_t stream) {
+  if (n_seqs <= 0 || seq_rows <= 0 || H <= 0 || rank <= 0 || rot < 0 || n_seqs > 65535)
+    RL_REFUSE(1, "latent_rows: S=%d rows=%d H=%d rank=%d rot=%d", n_seqs, seq_rows, H, rank, rot);
+  if (seq_rows % 64 || seq_rows / 64 > table_width) RL_REFUSE(2, "latent_rows: %d rows a sequence from tables of %d pages", seq_rows, table_width);
+  if (rank % 8 || rot % 8 || head_stride % 8 || key_at % 8 || key_at + rot > head_stride || (((uintptr_t)pages | (uintptr_t)latents | (uintptr_t)kv) & 15))
+    RL_REFUSE(3, "latent_rows: sizes %d / %d at %d of %d break 16-byte rows", rank, rot, key_at, head_stride);
+  RL_LAUNCH_CHECK(rl_launch(latent_rows_kernel, dim3(seq_rows / 8, n_seqs), 256, 0, stream, (const bf16*)pages, block_table, table_width, seq_len, seq_rows,
+                            (bf16*)latents, (bf16*)kv, H, head_stride, key_at, rot, rank));
   return 0;
 }
 

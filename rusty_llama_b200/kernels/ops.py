@@ -1122,13 +1122,13 @@ def latent_prep(
     q: Optional[torch.Tensor], kv: Optional[torch.Tensor], norm_w: Optional[torch.Tensor], eps: float, freq: Optional[torch.Tensor], n_pairs: int,
     magnitude: float, tok_pos: torch.Tensor, tok_seq: torch.Tensor, block_table: Optional[torch.Tensor], pages: Optional[torch.Tensor],
     q_cat: Optional[torch.Tensor], num_heads: int, dim: int, rot: int, rank: int, interleaved: bool = True,
-    q_latent: Optional[torch.Tensor] = None, q_norm: Optional[torch.Tensor] = None,
+    q_latent: Optional[torch.Tensor] = None, q_norm: Optional[torch.Tensor] = None, in_place: bool = False,
 ) -> Optional[torch.Tensor]:
     """Per token: kv's first `rank` values RMS-normed (weight norm_w) and its last `rot` values rotated go into the token's
     place in `pages` [pages, 1, PAGE_SIZE, rank + rot] (kv None: nothing is stored); the rotated part of every head of
     q [T, >= H (dim + rot)] is rotated into q_cat[T, H, rank:] (q None: left out); the rows q_latent [T, q_rank] are RMS-normed
     (weight q_norm float32 [q_rank], the same eps) and returned (q_latent None: nothing is returned).
-    interleaved: whether a rotated pair is (2i, 2i + 1) or (i, i + n_pairs)."""
+    interleaved: whether a rotated pair is (2i, 2i + 1) or (i, i + n_pairs).  in_place: the rotated parts go back into q instead."""
     some = q if q is not None else (kv if kv is not None else q_latent)
     _need(some is not None, "latent_prep: nothing to do")
     T, dt = some.shape[0], some.dtype
@@ -1137,8 +1137,9 @@ def latent_prep(
         _cuda(q, "latent_prep q", contiguous=False)
         ldq = _rows(q, "latent_prep q")
         _need(q.shape[1] >= num_heads * (dim + rot), "latent_prep: q rows too short")
-        _cuda(q_cat, "latent_prep q_cat", dt)
-        _need(tuple(q_cat.shape) == (T, num_heads, rank + rot), "latent_prep: q_cat has the wrong shape")
+        if not in_place:
+            _cuda(q_cat, "latent_prep q_cat", dt)
+            _need(tuple(q_cat.shape) == (T, num_heads, rank + rot), "latent_prep: q_cat has the wrong shape")
     _cuda(tok_pos, "latent_prep tok_pos", torch.int32)
     _cuda(tok_seq, "latent_prep tok_seq", torch.int32)
     _need(tok_pos.numel() == T and tok_seq.numel() == T, "latent_prep: one position and one sequence index per token")
@@ -1170,7 +1171,7 @@ def latent_prep(
         _p(q), c_int(ldq), _p(kv), c_int(ldkv), c_int(_dt(some, "latent_prep")), _p(norm_w), c_float(eps), _p(freq), c_int(n_pairs),
         c_int(1 if interleaved else 0), c_float(magnitude), _p(tok_pos), _p(tok_seq), _p(block_table) if kv is not None else c_void_p(0), c_int(width),
         _p(pages) if kv is not None else c_void_p(0), c_int(PAGE_SIZE), _p(q_cat) if q is not None else c_void_p(0), c_int(T), c_int(num_heads),
-        c_int(dim), c_int(rot), c_int(rank), _p(q_latent), c_int(ldql), c_int(q_rank), _p(q_norm), _p(ql_out), _stream(),
+        c_int(dim), c_int(rot), c_int(rank), _p(q_latent), c_int(ldql), c_int(q_rank), _p(q_norm), _p(ql_out), c_int(1 if in_place and q is not None else 0), _stream(),
     )
     _check(lib, rc, "latent_prep")
     return ql_out
@@ -1181,11 +1182,13 @@ HEAD_LINEAR_MMA_MAX_ROWS = 32  # rows up to which head products go to mma.sync t
 
 def head_linear(
     x: torch.Tensor, x_head_stride: int, w: torch.Tensor, out: torch.Tensor, out_head_stride: int,
-    gate: Optional[torch.Tensor] = None, gate_head_stride: int = 0,
+    gate: Optional[torch.Tensor] = None, gate_head_stride: int = 0, held: Optional[torch.Tensor] = None, seq_rows: int = 0,
 ) -> torch.Tensor:
     """out[t, h, n] = sum_k x[t, h, k] * w[h, n, k] (optionally times sigmoid(gate[t, h, n])), one small product per head.
 
-    x, out, gate: 2-D [T, row] tensors with dense rows; head h's values start `*_head_stride` * h into a row.  w: [H, N, K]."""
+    x, out, gate: 2-D [T, row] tensors with dense rows; head h's values start `*_head_stride` * h into a row.  w: [H, N, K].
+    held: None, or int32 [T / seq_rows]: how many rows of every run of seq_rows exist; the tcgen05 kernel computes those (up to the next
+    multiple of 64) and leaves the others' outputs as they are."""
     _cuda(x, "head_linear x", contiguous=False)
     _cuda(w, "head_linear w", x.dtype)
     _cuda(out, "head_linear out", x.dtype, contiguous=False)
@@ -1205,7 +1208,7 @@ def head_linear(
             lib = build.load("grouped_gemm_tc")
             rc = lib.rl_head_linear_tc(
                 _p(x), c_int(ldx), c_int(x_head_stride), _p(w), _p(out), c_int(ldo), c_int(out_head_stride), _p(gate), c_int(ldg),
-                c_int(gate_head_stride), c_int(M), c_int(H), c_int(N), c_int(K), _p(_tc_status_word(x.device)), *_wt(), _stream(),
+                c_int(gate_head_stride), c_int(M), c_int(H), c_int(N), c_int(K), _p(held), c_int(seq_rows), _p(_tc_status_word(x.device)), *_wt(), _stream(),
             )
             _check(lib, rc, "head_linear_tc")
             return out
@@ -1222,6 +1225,70 @@ def head_linear(
         _p(gate), c_int(ldg), c_int(gate_head_stride), c_int(_dt(x, "head_linear")), c_int(M), c_int(H), c_int(N), c_int(K), _stream(),
     )
     _check(lib, rc, "head_linear")
+    return out
+
+
+def latent_expand(pages: torch.Tensor, block_table: torch.Tensor, seq_len: torch.Tensor, seq_rows: int, w_vk: torch.Tensor, rot: int) -> torch.Tensor:
+    """Keys and values of every head for the positions that the sequences hold, bfloat16 [S * seq_rows, H, vdim + dim + rot]: row
+    (s, j) holds position j of sequence s, a head's value and plain key part = w_vk[h] (rows: vdim, then dim) . latent, then the turned
+    key part that all heads share.  Rows a sequence does not hold are zeros up to a multiple of 64 and undefined behind it.
+    pages [pages, 1, PAGE_SIZE, rank + rot]; seq_rows: a multiple of 64, at least every sequence's length."""
+    _cuda(pages, "latent_expand pages", torch.bfloat16)
+    _cuda(block_table, "latent_expand block_table", torch.int32)
+    _cuda(seq_len, "latent_expand seq_len", torch.int32)
+    _cuda(w_vk, "latent_expand w_vk", torch.bfloat16)
+    H, n, rank = w_vk.shape
+    S, width = block_table.shape
+    if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot) and seq_len.numel() == S):
+        raise KernelError(f"latent_expand: pages {tuple(pages.shape)} and {seq_len.numel()} lengths for {S} sequences of latents of {rank} + {rot}")
+    rows = S * seq_rows
+    latents = torch.empty((rows, rank), dtype=pages.dtype, device=pages.device)
+    kv = torch.empty((rows, H, n + rot), dtype=pages.dtype, device=pages.device)
+    lib = build.load("latent_attention")
+    rc = lib.rl_latent_rows(
+        _p(pages), _p(block_table), c_int(width), _p(seq_len), c_int(S), c_int(seq_rows), _p(latents), _p(kv), c_int(H), c_int(n + rot), c_int(n),
+        c_int(rot), c_int(rank), _stream(),
+    )
+    _check(lib, rc, "latent_rows")
+    head_linear(latents, 0, w_vk, kv.view(rows, H * (n + rot)), n + rot, held=seq_len, seq_rows=seq_rows)
+    return kv
+
+
+def flash_expanded_takes(kdim: int, vdim: int) -> bool:
+    """Key and value sizes that `flash_expanded` is built for."""
+    return 0 < kdim <= 192 and 0 < vdim <= 128 and kdim % 8 == 0 and vdim % 8 == 0
+
+
+def flash_expanded(
+    q: torch.Tensor, kv: torch.Tensor, seq_rows: int, seq_start: torch.Tensor, seq_pos0: torch.Tensor, max_q_len: int, vdim: int, window: int,
+    scale: float, sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
+) -> torch.Tensor:
+    """`flash_prefill_tc` over keys and values expanded for this call (`latent_expand`), every head its own: q [T, >= H kdim] rows, kv
+    [S * seq_rows, H, vdim + kdim]; the result [T, H vdim] is multiplied by sigmoid(gate [T, >= H vdim]) if a gate is given."""
+    _cuda(q, "flash_expanded q", torch.bfloat16, contiguous=False)
+    _cuda(kv, "flash_expanded kv", torch.bfloat16)
+    T, S = q.shape[0], seq_pos0.numel()
+    H, stride = kv.shape[1], kv.shape[2]
+    kdim = stride - vdim
+    if not (flash_expanded_takes(kdim, vdim) and q.shape[1] >= H * kdim and kv.shape[0] == S * seq_rows and seq_rows % PAGE_SIZE == 0):
+        raise KernelError(f"flash_expanded: q {tuple(q.shape)} against keys and values {tuple(kv.shape)} of {S} sequences")
+    _cuda(seq_start, "flash_expanded seq_start", torch.int32)
+    _cuda(seq_pos0, "flash_expanded seq_pos0", torch.int32)
+    _need(seq_start.numel() == S + 1, "flash_expanded: metadata sizes")
+    _check_sink(sink, H, "flash_expanded")
+    ldg = 0
+    if gate is not None:
+        _cuda(gate, "flash_expanded gate", torch.bfloat16, contiguous=False)
+        ldg = _rows(gate, "flash_expanded gate")
+        _need(gate.shape[0] == T and gate.shape[1] >= H * vdim, "flash_expanded: gate rows do not fit")
+    out = torch.empty((T, H * vdim), dtype=torch.bfloat16, device=q.device)
+    lib = build.load("attention_prefill_tc")
+    rc = lib.rl_flash_prefill_tc_expanded(
+        _p(q), c_int(_rows(q, "flash_expanded q")), c_int(T), _p(kv), c_int(seq_rows // PAGE_SIZE), c_int(stride), _p(seq_start), _p(seq_pos0), _p(out),
+        c_int(H * vdim), c_int(S), c_int(max_q_len), c_int(H), c_int(kdim), c_int(vdim), c_int(window), c_float(scale), _p(sink), _p(gate), c_int(ldg),
+        _p(_tc_status_word(q.device)), *_wt(), _stream(),
+    )
+    _check(lib, rc, "flash_prefill_tc_expanded")
     return out
 
 

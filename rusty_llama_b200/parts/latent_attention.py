@@ -13,6 +13,14 @@ from ..kernels.linear import linear, linear_to_stream
 from ..spec import PartSpec
 from .base import MIXERS, POSITIONS, KVNeed, Mixer, ParamInfo
 
+# A step expands keys and values per head from so many tokens on (above the head products' few-row form), while there are at most so many
+# rows to expand for each of them: a row costs 0.26 million operations a head at the sizes below, a pair on the latents 1.5 thousand more
+# at about a quarter of the rate, so that 43 rows a query break even where every row is seen once; a chunk of a prompt sees each of them
+# from every query.  And they have to fit so many bytes for the call.
+_EXPAND_MIN_TOKENS = 33
+_EXPAND_MAX_ROWS_PER_TOKEN = 64
+_EXPAND_MAX_BYTES = 1 << 30
+
 _NAMES = {"q": "q", "q_down": "dq", "q_norm": "dq.norm", "q_up": "uq", "kv": "dkv", "kv_norm": "dkv.norm", "k_up": "uk", "v_up": "uv", "sink": "sink", "gate": "g", "out": "o"}
 
 
@@ -27,9 +35,11 @@ class LatentAttention(Mixer):
         score = (q_plain . W_uk[h] c_j + q_rot . kr_j) * scale,  softmax whose denominator also holds exp(sink[h])
         result = W_o ( concat_h(sum_j p_j W_uv[h] c_j) * sigmoid(W_g xn[t]) )
 
-    The kernels never expand the cache into per-head keys and values: W_uk[h]^T is applied to the query
+    A decode step never expands the cache into per-head keys and values: W_uk[h]^T is applied to the query
     (q_lat = W_uk[h]^T q_plain, so that the score is [q_lat | q_rot] . [c_j | kr_j]) and W_uv[h] to the
-    probability-weighted sum of the latents, which is the same arithmetic in another order.
+    probability-weighted sum of the latents, which is the same arithmetic in another order.  A prompt step of a bfloat16
+    run expands them for the call (`_expands`): with dim = vdim = 128, rot 64 and rank 512 a (query, key) pair then costs 640 operations a
+    head instead of 2176, and the tcgen05 prompt attention takes the sizes.
 
     With `q_rank` the queries come from a latent of their own, q[t] = W_uq (rmsnorm(W_dq xn[t]) * w_qnorm), in the place of W_q xn[t].
 
@@ -77,7 +87,7 @@ class LatentAttention(Mixer):
         self.n_pairs = rotary_dim // 2
         self.magnitude = float(getattr(self.position, "magnitude", 1.0))
         self.qd, self.vd, self.kvd = self.H * (self.dim + self.rot), self.H * self.vdim, self.rank + self.rot
-        self.w_in = self.w_o = self.w_ukT = self.w_uv = self.w_norm = self.sink = self.w_uq = self.w_q_norm = None
+        self.w_in = self.w_o = self.w_ukT = self.w_uv = self.w_vk = self.w_norm = self.sink = self.w_uq = self.w_q_norm = None
 
     def cache_need(self):
         return KVNeed(1, self.kvd, self.window, values=False) if self.own_kv else None
@@ -124,12 +134,34 @@ class LatentAttention(Mixer):
         # W_uk[h] as [rank, dim]: the map from a head's plain query part to the latent space
         self.w_ukT = tensors[p + n["k_up"]].view(self.H, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[p + n["v_up"]].view(self.H, self.vdim, self.rank).contiguous()
+        # the maps from a latent to a head's value and plain key part, one behind the other, for steps that expand them
+        self.w_vk = None
+        if self.rt.dtype == torch.bfloat16:
+            self.w_vk = torch.cat([self.w_uv, tensors[p + n["k_up"]].view(self.H, self.dim, self.rank)], dim=1).contiguous()
         self.w_o = tensors[p + n["out"]].contiguous()
         self.sink = tensors[p + n["sink"]].contiguous() if self.has_sink else None
 
     def forward(self, xn: torch.Tensor, step, cache, shared_cache: bool = False) -> torch.Tensor:
         a, w_o = self.forward_unprojected(xn, step, cache, shared_cache)
         return linear_to_stream(a, w_o)
+
+    def _expands(self, step, q: torch.Tensor, gate) -> int:
+        """How many rows a sequence's keys and values are expanded to (a multiple of the page size), or 0: the step works on the latents.
+
+        Expanding costs 2 rank (dim + vdim) operations a head and cached position; working on the latents costs 2 (2 rank - dim - vdim)
+        more a head and (query, key) pair and 2 rank (dim + vdim) a head and token, on mma.sync.  Measured, 16 heads of 128 + 64 / 128, rank
+        512, one prompt of 2048: 468 us on the latents and 25 us for the two products around it; expanded, 16 us for the products, 5 for the
+        rows, 63 for the attention."""
+        if step.decode_only or self.w_vk is None or step.n_tokens < _EXPAND_MIN_TOKENS or not q.is_cuda:
+            return 0
+        if not ops.flash_expanded_takes(self.dim + self.rot, self.vdim) or self.dim % 8 or self.rot % 8 or self.rank % 8 or self.dim == 0:
+            return 0
+        if q.stride(0) % 8 or q.data_ptr() % 16 or (gate is not None and (gate.stride(0) % 8 or gate.data_ptr() % 16)):
+            return 0
+        seq_rows = (step.max_kv_len + ops.PAGE_SIZE - 1) // ops.PAGE_SIZE * ops.PAGE_SIZE
+        rows = step.n_seqs * seq_rows
+        small = rows * self.H * (self.vdim + self.dim + self.rot) * 2 <= _EXPAND_MAX_BYTES
+        return seq_rows if small and rows <= _EXPAND_MAX_ROWS_PER_TOKEN * step.n_tokens else 0
 
     def forward_unprojected(self, xn: torch.Tensor, step, cache, shared_cache: bool = False):
         if shared_cache == self.own_kv:
@@ -140,13 +172,20 @@ class LatentAttention(Mixer):
         q = proj[:, :first]
         g = proj[:, first : first + self.vd] if self.has_gate else None
         kv = proj[:, proj.shape[1] - self.kvd :] if self.own_kv else None
-        q_cat = torch.empty((T, self.H, self.kvd), dtype=xn.dtype, device=xn.device)
         turn = (self.freq, self.n_pairs, self.magnitude, step.tok_pos, step.tok_seq, cache.block_table, cache.k_pages)
         sizes = (self.H, self.dim, self.rot, self.rank, self.interleaved)
         if self.q_rank:
             # the queries' latent is normed beside the row that is cached; the queries exist after the product with it
             c_q = ops.latent_prep(None, kv, self.w_norm, self.eps, *turn, None, *sizes, q_latent=q, q_norm=self.w_q_norm)
             q, kv = linear(c_q, self.w_uq), None
+        seq_rows = self._expands(step, q, g)
+        if seq_rows:
+            ops.latent_prep(q, kv, self.w_norm, self.eps, *turn, None, *sizes, in_place=True)
+            expanded = ops.latent_expand(cache.k_pages, cache.block_table, step.seq_len, seq_rows, self.w_vk, self.rot)
+            a = ops.flash_expanded(q, expanded, seq_rows, step.seq_start, step.seq_pos0, step.max_q_len, self.vdim, self.window, self.scale,
+                                   sink=self.sink, gate=g)
+            return a, self.w_o
+        q_cat = torch.empty((T, self.H, self.kvd), dtype=xn.dtype, device=xn.device)
         ops.latent_prep(q, kv, self.w_norm, self.eps, *turn, q_cat, *sizes)
         if self.dim:
             ops.head_linear(q, self.dim + self.rot, self.w_ukT, q_cat.view(T, self.H * self.kvd), self.kvd)
