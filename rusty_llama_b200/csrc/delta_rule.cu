@@ -17,7 +17,8 @@
 //                     meet; the partial sums of a column's row slices (lanes of one warp) are added by shuffles in a fixed
 //                     order, and u_t is folded into the read-out: o_t = (g S)^T q + u (k . q).  Prompts, parts of
 //                     prompts and single tokens run the same code, so a result's bits depend neither on how a sequence
-//                     was cut into steps nor on what else is in the batch.
+//                     was cut into steps nor on what else is in the batch.  (The prompts of a bfloat16 run go chunk by chunk
+//                     through delta_chunk.cu instead, equal within rounding.)
 #include "common.cuh"
 
 RL_DEFINE_ERROR_TEXT()
@@ -189,7 +190,7 @@ template <typename T>
 __global__ void delta_prep_kernel(const T* __restrict__ qk, int qk_stride, const T* __restrict__ ba, int ba_stride,
                                   const float* __restrict__ a_log, const float* __restrict__ dt_bias, float unit_eps, float q_scale,
                                   float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ kq, float* __restrict__ beta,
-                                  float* __restrict__ decay, int G, int H, int dim) {
+                                  float* __restrict__ decay, int G, int H, int dim, int log_decay) {
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const T* row = qk + (size_t)t * qk_stride;
@@ -220,23 +221,24 @@ __global__ void delta_prep_kernel(const T* __restrict__ qk, int qk_stride, const
     beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-to_f32(bar[h])));
     const float z = to_f32(bar[H + h]) + dt_bias[h];
     const float sp = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
-    decay[(size_t)t * H + h] = expf(-expf(a_log[h]) * sp);
+    const float l = -expf(a_log[h]) * sp;
+    decay[(size_t)t * H + h] = log_decay ? l : expf(l);
   }
 }
 
 RL_API int rl_delta_prep(const void* qk, int dtype, int qk_stride, const void* ba, int ba_stride, const float* a_log, const float* dt_bias,
                          float unit_eps, float q_scale, float* qn, float* kn, float* kq, float* beta, float* decay, int n_tokens, int G, int H,
-                         int dim, cudaStream_t stream) {
+                         int dim, int log_decay, cudaStream_t stream) {
   if (n_tokens <= 0 || G <= 0 || H <= 0 || dim <= 0) RL_REFUSE(1, "delta_prep: T=%d G=%d H=%d dim=%d", n_tokens, G, H, dim);
   if (qk_stride < 2 * G * dim || ba_stride < 2 * H) RL_REFUSE(2, "delta_prep: rows too short");
   int threads = 32 * (G < 8 ? G : 8);
   if (threads < 64) threads = 64;
   if (dtype == RL_BF16)
     delta_prep_kernel<bf16><<<n_tokens, threads, 0, stream>>>((const bf16*)qk, qk_stride, (const bf16*)ba, ba_stride, a_log, dt_bias, unit_eps,
-                                                              q_scale, qn, kn, kq, beta, decay, G, H, dim);
+                                                              q_scale, qn, kn, kq, beta, decay, G, H, dim, log_decay);
   else if (dtype == RL_F32)
     delta_prep_kernel<float><<<n_tokens, threads, 0, stream>>>((const float*)qk, qk_stride, (const float*)ba, ba_stride, a_log, dt_bias, unit_eps,
-                                                               q_scale, qn, kn, kq, beta, decay, G, H, dim);
+                                                               q_scale, qn, kn, kq, beta, decay, G, H, dim, log_decay);
   else
     RL_REFUSE(3, "delta_prep: unknown dtype %d", dtype);
   RL_LAUNCH_RESULT();

@@ -2208,11 +2208,11 @@ def short_conv(
 
 def delta_prep(
     qk: torch.Tensor, ba: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor, num_qk_heads: int, num_heads: int, dim: int,
-    unit_eps: float, q_scale: float,
+    unit_eps: float, q_scale: float, log_decay: bool = False,
 ):
     """What the gated delta rule's recurrence takes, all float32: qk [T, 2 G dim] rows (G q heads, then G k heads) -> unit vectors
     qn (times q_scale) and kn [T, G dim], their products kq [T, G]; ba [T, >= 2 H] rows (b, then a) -> beta = logistic(b) and
-    decay = exp(-exp(a_log) softplus(a + dt_bias)), both [T, H]."""
+    decay = exp(-exp(a_log) softplus(a + dt_bias)) (log_decay: its logarithm), both [T, H]."""
     _cuda(qk, "delta_prep qk", contiguous=False)
     _cuda(ba, "delta_prep ba", qk.dtype, contiguous=False)
     T = qk.shape[0]
@@ -2227,7 +2227,8 @@ def delta_prep(
     lib = build.load("delta_rule")
     rc = lib.rl_delta_prep(
         _p(qk), c_int(_dt(qk, "delta_prep")), c_int(_rows(qk, "delta_prep qk")), _p(ba), c_int(_rows(ba, "delta_prep ba")), _p(a_log), _p(dt_bias),
-        c_float(unit_eps), c_float(q_scale), _p(qn), _p(kn), _p(kq), _p(beta), _p(decay), c_int(T), c_int(G), c_int(H), c_int(dim), _stream(),
+        c_float(unit_eps), c_float(q_scale), _p(qn), _p(kn), _p(kq), _p(beta), _p(decay), c_int(T), c_int(G), c_int(H), c_int(dim),
+        c_int(1 if log_decay else 0), _stream(),
     )
     _check(lib, rc, "delta_prep")
     return qn, kn, kq, beta, decay
@@ -2264,6 +2265,49 @@ def delta_rule(
         _p(seq_start), _p(out), c_int(out.stride(0)), c_int(S), c_int(H), c_int(G), c_int(dim), c_int(vdim), _stream(),
     )
     _check(lib, rc, "delta_rule")
+    return out
+
+
+def delta_chunked_takes(dim: int, vdim: int) -> bool:
+    """Whether `delta_chunked` is built for these sizes."""
+    return 0 < dim <= 128 and dim % 4 == 0 and 0 < vdim and vdim % 4 == 0
+
+
+def delta_chunked_scratch_floats(n_tokens: int, n_seqs: int, num_heads: int, dim: int, vdim: int) -> int:
+    lib = build.load("delta_chunk")
+    lib.rl_delta_chunked_scratch.restype = c_ll
+    return int(lib.rl_delta_chunked_scratch(c_int(n_tokens), c_int(n_seqs), c_int(num_heads), c_int(dim), c_int(vdim)))
+
+
+def delta_chunked(
+    qn: torch.Tensor, kn: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log_decay: torch.Tensor, state: torch.Tensor, slot_ids: torch.Tensor,
+    seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int, max_q_len: int, scratch: torch.Tensor,
+) -> torch.Tensor:
+    """`delta_rule` chunk by chunk, for prompts of bfloat16 runs: the same result within 32-bit rounding.  log_decay: float32 [T, H], the
+    logarithms of the decays; v: bfloat16 rows; scratch: float32, `delta_chunked_scratch_floats` numbers."""
+    T, H, G = qn.shape[0], num_heads, num_qk_heads
+    for name, t, n in (("qn", qn, G * dim), ("kn", kn, G * dim), ("beta", beta, H), ("log_decay", log_decay, H)):
+        _cuda(t, "delta_chunked rows", torch.float32)
+        if tuple(t.shape) != (T, n):
+            raise KernelError(f"delta_chunked: {name} {tuple(t.shape)} is not [{T}, {n}]")
+    _cuda(v, "delta_chunked v", torch.bfloat16, contiguous=False)
+    _need(tuple(v.shape) == (T, H * vdim), "delta_chunked: v must be [T, H vdim]")
+    _cuda(state, "delta_chunked state", torch.float32)
+    if not (state.dim() == 4 and tuple(state.shape[1:]) == (H, dim, vdim)):
+        raise KernelError(f"delta_chunked: state {tuple(state.shape)} is not [slots, {H}, {dim}, {vdim}]")
+    _cuda(slot_ids, "delta_chunked slot_ids", torch.int32)
+    _cuda(seq_start, "delta_chunked seq_start", torch.int32)
+    S = slot_ids.numel()
+    _need(seq_start.numel() == S + 1, "delta_chunked: seq_start must hold one more entry than there are sequences")
+    _cuda(scratch, "delta_chunked scratch", torch.float32)
+    _need(scratch.numel() >= delta_chunked_scratch_floats(T, S, H, dim, vdim), "delta_chunked: scratch too small")
+    out = torch.empty((T, H * vdim), dtype=torch.float32, device=qn.device)
+    lib = build.load("delta_chunk")
+    rc = lib.rl_delta_chunked(
+        _p(qn), _p(kn), _p(v), c_int(_rows(v, "delta_chunked v")), _p(beta), _p(log_decay), _p(state), _p(slot_ids), _p(seq_start), _p(out), c_int(out.stride(0)),
+        c_int(T), c_int(S), c_int(max_q_len), c_int(H), c_int(G), c_int(dim), c_int(vdim), _p(scratch), _stream(),
+    )
+    _check(lib, rc, "delta_chunked", kernels=3)
     return out
 
 

@@ -5,7 +5,7 @@ delta rule (a decay per head, and a write that corrects what the state already h
 
 All keep their state in 32-bit in the cache's state records, one record per sequence slot, zero when the sequence starts;
 the first three run on the same recurrence kernel (csrc/gated_recurrent.cu; for the state-space layer's prompts also
-csrc/state_space.cu), the delta rule on its own (csrc/delta_rule.cu):
+csrc/state_space.cu), the delta rule on its own (csrc/delta_rule.cu; the prompts of a bfloat16 run on csrc/delta_chunk.cu):
 
     S_t = diag(a_t) S_(t-1) + b_t k_t v_t^T,   o_t = S_t^T q_t
 
@@ -26,6 +26,8 @@ from .base import MIXERS, Mixer, ParamInfo, StateNeed
 
 # prompt steps whose longest sequence brings fewer tokens than this go token by token like a decode step
 _CHUNKED_MIN_TOKENS = 32
+# the most scratch that the delta rule's chunks may take (2 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it token by token
+_CHUNKED_MAX_FLOATS = 1 << 29
 
 
 def _recurrence(mixer, q, k, v, log_decay, in_scale, state, step, ext: bool):
@@ -312,8 +314,18 @@ class GatedDeltaRule(Mixer):
         conv = ops.short_conv(proj[:, :C], self.w_conv, None if inputs is None else inputs.state, step.slot_ids, step.seq_start, step.tok_seq,
                               single=step.decode_only)
         gate, ba = proj[:, C : C + vd], proj[:, C + vd : C + vd + 2 * H]
-        qn, kn, kq, beta, decay = ops.delta_prep(conv[:, : 2 * self.qd], ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps, self.q_scale)
-        o = ops.delta_rule(qn, kn, kq, conv[:, 2 * self.qd :], beta, decay, memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim)
+        chunked, floats = False, 0
+        if xn.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS and ops.delta_chunked_takes(self.dim, self.vdim):
+            floats = ops.delta_chunked_scratch_floats(step.n_tokens, step.n_seqs, H, self.dim, self.vdim)
+            chunked = floats <= _CHUNKED_MAX_FLOATS
+        qn, kn, kq, beta, decay = ops.delta_prep(conv[:, : 2 * self.qd], ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps, self.q_scale,
+                                                 log_decay=chunked)
+        if chunked:  # a prompt of a bfloat16 run, all chunks side by side but for the walk through the state
+            scratch = self.rt.workspace.get("delta_chunks", floats, torch.float32)
+            o = ops.delta_chunked(qn, kn, conv[:, 2 * self.qd :], beta, decay, memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim,
+                                  step.max_q_len, scratch)
+        else:
+            o = ops.delta_rule(qn, kn, kq, conv[:, 2 * self.qd :], beta, decay, memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim)
         a = ops.head_norm_gate(o, H, self.vdim, self.w_norm, self.eps, gate, ops.GATE_SILU, xn.dtype, out_scale=self.out_scale, out=out)
         return a, self.w_o
 

@@ -1,0 +1,105 @@
+"""The gated delta rule chunk by chunk against the recurrence in 64 bits and beside the token-by-token kernel: portions that are no
+multiple of the chunk, sequences of one token beside long ones, several heads on one q/k head, sizes that leave tiles partly empty, decays
+from none to ones that underflow inside a chunk, repeated keys; and the rule that takes a step there."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def recurrence(q, k, v, beta, decay, S):
+    """One sequence in 64 bits: q, k [T, H, n], v [T, H, m], beta, decay [T, H], S [H, n, m]."""
+    o = torch.empty(v.shape, dtype=torch.float64)
+    for t in range(q.shape[0]):
+        S = S * decay[t, :, None, None]
+        u = beta[t, :, None] * (v[t] - torch.einsum("hnm,hn->hm", S, k[t]))
+        S = S + k[t, :, :, None] * u[:, None, :]
+        o[t] = torch.einsum("hnm,hn->hm", S, q[t])
+    return o, S
+
+
+def inputs(lens, H, G, dim, vdim, seed, kind):
+    g = torch.Generator().manual_seed(seed)
+    T = sum(lens)
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)  # noqa: E731
+    q, k = unit(torch.randn(T, G, dim, generator=g)) * dim ** -0.5, unit(torch.randn(T, G, dim, generator=g))
+    v = torch.randn(T, H, vdim, generator=g).to(torch.bfloat16)
+    beta = torch.rand(T, H, generator=g)
+    logd = -torch.rand(T, H, generator=g) * {"slow": 1e-3, "usual": 1.0, "fast": 60.0}.get(kind, 0.5)
+    if kind == "repeated":  # the same few keys over and over, written at full strength: the system's entries are close to one
+        k = k[torch.randint(0, 3, (T,), generator=g)]
+        beta, logd = torch.ones(T, H), torch.zeros(T, H)
+    return q, k, v, beta, logd
+
+
+@pytest.mark.parametrize("kind", ["slow", "usual", "fast", "repeated"])
+@pytest.mark.parametrize("lens, H, G, dim, vdim", [
+    ([200, 64, 1, 63], 4, 2, 128, 128), ([65], 2, 2, 64, 20), ([130, 33], 3, 1, 36, 72), ([400], 2, 1, 100, 132), ([64, 128], 1, 1, 4, 4),
+])
+def test_against_64_bits_and_the_token_kernel(lens, H, G, dim, vdim, kind):
+    from rusty_llama_b200.kernels import ops
+
+    q, k, v, beta, logd = inputs(lens, H, G, dim, vdim, sum(lens) + dim, kind)
+    T, S = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(1)
+    start_state = torch.randn(S + 1, H, dim, vdim, generator=g)
+    slots, starts = [S - i for i in range(S)], [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    wide = torch.zeros(T, H * vdim + 8, dtype=torch.bfloat16, device=DEV)
+    wide[:, 8:] = v.view(T, -1).to(DEV)
+    qd, kd = q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV)
+    state, state1 = start_state.to(DEV), start_state.to(DEV)
+    scratch = torch.full((ops.delta_chunked_scratch_floats(T, S, H, dim, vdim),), float("nan"), device=DEV)
+    out = ops.delta_chunked(qd, kd, wide[:, 8:], beta.to(DEV), logd.to(DEV), state, i32(slots), i32(starts), H, G, dim, vdim, max(lens), scratch)
+    one = ops.delta_rule(qd, kd, (q * k).sum(-1).contiguous().to(DEV), wide[:, 8:], beta.to(DEV), logd.exp().to(DEV), state1, i32(slots), i32(starts), H, G, dim, vdim)
+    rep = H // G
+    refs = [recurrence(*(t[a:b].double() for t in (q.repeat_interleave(rep, 1), k.repeat_interleave(rep, 1), v, beta, logd.exp().double())), start_state[slot].double())
+            for a, b, slot in zip(starts, starts[1:], slots)]
+    want, want_S = torch.cat([o for o, _ in refs]).reshape(T, -1), torch.stack([s for _, s in refs])
+    rel = lambda x, y: float((x.double().cpu() - y).norm() / y.norm())  # noqa: E731
+    # no worse than token by token (which rounds once a token), or a few roundings of 32 bits
+    assert rel(out, want) <= max(1.5 * rel(one, want), 8 * 2.0 ** -24)
+    assert rel(state[slots], want_S) <= max(1.5 * rel(state1[slots], want_S), 8 * 2.0 ** -24)
+    assert torch.equal(state[0].cpu(), start_state[0])  # (nobody's record)
+
+
+def test_which_steps_go_chunk_by_chunk():
+    """A prompt of a bfloat16 run does, a short portion and a 32-bit run do not, and the layer's results agree within the run's rounding."""
+    from rusty_llama_b200.cache import Cache
+    from rusty_llama_b200.kernels import ops
+    from rusty_llama_b200.parts import MIXERS, Runtime
+    from rusty_llama_b200.spec import PartSpec
+
+    from test_parts import ctx_for
+
+    part = MIXERS.build(PartSpec("gated_delta", {"hidden_size": 64, "num_heads": 2, "num_qk_heads": 1, "dim": 32, "vdim": 48, "taps": 4, "eps": 1e-5}), Runtime.create(DEV, torch.bfloat16))
+    g = torch.Generator().manual_seed(0)
+    w = {}
+    for name, info in part.param_infos().items():
+        t = torch.randn(info.shape, generator=g) * (0.2 if len(info.shape) > 1 else 0.5) + (1.0 if name == "norm" else 0.0)
+        w[name] = (t if info.kind == "scalars" else t.to(torch.bfloat16)).to(DEV)
+    part.load(w)
+    x = torch.randn(150, 64, generator=g).to(torch.bfloat16).to(DEV)
+    called, before = [], ops.delta_chunked
+    ops.delta_chunked = lambda *a, **k: called.append(1) or before(*a, **k)
+    try:
+        outs = []
+        for cuts in ([150], [100, 31, 19], [31] * 4 + [26]):
+            cache = Cache([(0, part.cache_need())], 64, 1, torch.bfloat16, DEV)
+            slot, at, parts = cache.open_sequence(), 0, []
+            for n in cuts:
+                step, tables = ctx_for(cache, [slot], [at], [n])
+                y = part.forward(x[at : at + n], step, cache.view(0, tables))
+                parts.append(y.float().sum(0) if y.dim() == 3 else y.float())
+                cache.commit([slot], [n])
+                at += n
+            outs.append((torch.cat(parts), len(called)))
+    finally:
+        ops.delta_chunked = before
+    assert [n for _, n in outs] == [1, 2, 2]
+    for y, _ in outs[1:]:
+        assert float((y - outs[0][0]).norm() / outs[0][0].norm()) < 1e-2
