@@ -92,6 +92,81 @@ __global__ void short_conv_rows8_kernel(const bf16* __restrict__ x, int x_stride
   *reinterpret_cast<uint4*>(out + (size_t)t * out_stride + c) = packed;
 }
 
+// The same for long prompts and up to CONV_ROW_TAPS taps: a thread takes CONV_RUN tokens of its 8 channels, one after the other, with the
+// last taps - 1 inputs and the taps' weights in registers, so that an input row is read once (and the rows of a run are all asked
+// for before the first is used) and not once per tap with the weights again: 41 us for 2048 tokens of 6144 channels and 4 taps, now
+// 25 (30 with runs of 8, whose registers leave an SM 12 warps); memory's work is 8.  Below two blocks an SM the runs leave too few
+// threads, and every token keeps its own.
+#define CONV_RUN 4
+#define CONV_ROW_TAPS 4
+template <int TAPS>
+__global__ void __launch_bounds__(128, 5)
+short_conv_runs_kernel(const bf16* __restrict__ x, int x_stride, const float* __restrict__ w, const float* __restrict__ bias,
+                       const float* __restrict__ state, const int* __restrict__ slot_ids, const int* __restrict__ seq_start,
+                       const int* __restrict__ tok_seq, bf16* __restrict__ out, int out_stride, int n_tokens, int C, int silu) {
+  pdl_trigger();
+  pdl_wait();
+  const unsigned c8s = C >> 3, idx = blockIdx.x * 128 + threadIdx.x;
+  const int run = (int)(idx / c8s), c = (int)(idx - run * c8s) * 8, t0 = run * CONV_RUN;
+  if (t0 >= n_tokens) return;
+  const int n = min(CONV_RUN, n_tokens - t0);
+  uint4 rows[CONV_RUN];
+  int seqs[CONV_RUN];
+#pragma unroll
+  for (int j = 0; j < CONV_RUN; ++j)
+    if (j < n) {
+      rows[j] = __ldcg(reinterpret_cast<const uint4*>(x + (size_t)(t0 + j) * x_stride + c));
+      seqs[j] = __ldcg(tok_seq + t0 + j);
+    }
+  float wt[TAPS][8], v[TAPS][8], b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < TAPS; ++i) {
+    load4<float>(w + (size_t)i * C + c, wt[i]);
+    load4<float>(w + (size_t)i * C + c + 4, wt[i] + 4);
+  }
+  if (bias) {
+    load4<float>(bias + c, b);
+    load4<float>(bias + c + 4, b + 4);
+  }
+#pragma unroll
+  for (int j = 0; j < CONV_RUN; ++j) {
+    if (j >= n) break;
+    if (j == 0 || seqs[j] != seqs[j > 0 ? j - 1 : 0]) {  // the inputs before this token: the sequence's own, or its record's
+      const int start = __ldcg(seq_start + seqs[j]), local = t0 + j - start;
+      const float* rec = state + (size_t)__ldcg(slot_ids + seqs[j]) * (TAPS - 1) * C;
+#pragma unroll
+      for (int i = 0; i < TAPS - 1; ++i) {
+        const int src = local - (TAPS - 1) + i;
+        if (src >= 0) {
+          bf16x8_to_f32(__ldcg(reinterpret_cast<const uint4*>(x + (size_t)(start + src) * x_stride + c)), v[i]);
+        } else {
+          const float4 lo = __ldcg(reinterpret_cast<const float4*>(rec + (size_t)(TAPS - 1 + src) * C + c));
+          const float4 hi = __ldcg(reinterpret_cast<const float4*>(rec + (size_t)(TAPS - 1 + src) * C + c + 4));
+          v[i][0] = lo.x; v[i][1] = lo.y; v[i][2] = lo.z; v[i][3] = lo.w; v[i][4] = hi.x; v[i][5] = hi.y; v[i][6] = hi.z; v[i][7] = hi.w;
+        }
+      }
+    }
+    bf16x8_to_f32(rows[j], v[TAPS - 1]);
+    uint4 packed;
+    __nv_bfloat162* p2 = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      float lo = b[e], hi = b[e + 1];
+#pragma unroll
+      for (int i = 0; i < TAPS; ++i) {
+        lo += wt[i][e] * v[i][e];
+        hi += wt[i][e + 1] * v[i][e + 1];
+      }
+      p2[e / 2] = __floats2bfloat162_rn(silu ? dr_silu(lo) : lo, silu ? dr_silu(hi) : hi);
+    }
+    *reinterpret_cast<uint4*>(out + (size_t)(t0 + j) * out_stride + c) = packed;
+#pragma unroll
+    for (int i = 0; i < TAPS - 1; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[i][e] = v[i + 1][e];
+  }
+}
+
 // One thread per (sequence, channel): the record after the step's tokens.
 template <typename T>
 __global__ void short_conv_state_kernel(const T* __restrict__ x, int x_stride, float* __restrict__ state, const int* __restrict__ slot_ids,
@@ -162,14 +237,24 @@ RL_API int rl_short_conv(const void* x, int dtype, int x_stride, const float* w,
   }
   const int blocks = (int)((total + threads - 1) / threads), blocks_s = (int)((total_s + threads - 1) / threads);
   if (dtype == RL_BF16) {
-    // (which of the two kernels runs depends on sizes and addresses only, never on the batch)
+    // (all three kernels add up the same sums in the same order)
     const bool rows8 = C % 8 == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 && ((((uintptr_t)x | (uintptr_t)out | (uintptr_t)state | (uintptr_t)w | (uintptr_t)bias) & 15) == 0);
-    if (rows8)
+    const long long runs = (long long)((n_tokens + CONV_RUN - 1) / CONV_RUN) * (C / 8);
+#define RL_CONV_RUNS(TAPS)                                                                                                             \
+  RL_LAUNCH_CHECK(rl_launch(short_conv_runs_kernel<TAPS>, (int)((runs + 127) / 128), 128, 0, stream, (const bf16*)x, x_stride, w, bias, \
+                            (const float*)state, slot_ids, seq_start, tok_seq, (bf16*)out, out_stride, n_tokens, C, silu))
+    if (rows8 && taps <= CONV_ROW_TAPS && runs >= 2 * 148 * 128 && runs < (1LL << 31)) {
+      if (taps == 1) RL_CONV_RUNS(1);
+      else if (taps == 2) RL_CONV_RUNS(2);
+      else if (taps == 3) RL_CONV_RUNS(3);
+      else RL_CONV_RUNS(4);
+    } else if (rows8)
       short_conv_rows8_kernel<<<(int)((total / 8 + threads - 1) / threads), threads, 0, stream>>>((const bf16*)x, x_stride, w, bias, state, slot_ids, seq_start,
                                                                                                    tok_seq, (bf16*)out, out_stride, n_tokens, C, taps, silu);
     else
       short_conv_kernel<bf16><<<blocks, threads, 0, stream>>>((const bf16*)x, x_stride, w, bias, state, slot_ids, seq_start, tok_seq, (bf16*)out,
                                                               out_stride, n_tokens, C, taps, silu);
+#undef RL_CONV_RUNS
     if (taps > 1)
       short_conv_state_kernel<bf16><<<blocks_s, threads, 0, stream>>>((const bf16*)x, x_stride, state, slot_ids, seq_start, n_seqs, C, taps);
   } else if (dtype == RL_F32) {
