@@ -1,4 +1,5 @@
-// Latent attention on the tensor cores (bfloat16): prompts and decode steps with one kernel.
+// Latent attention on the tensor cores (bfloat16): decode steps, short portions and prompts whose cached rows are too many to be
+// expanded per head (the other prompts take attention_prefill_tc.cu over expanded keys and values), with one kernel.
 //
 // A query row is a (token, head) pair; all heads of a token read the same cached rows [rank latent | rot shared
 // key part], so a block takes 16 * MT consecutive rows of one sequence (row = token * H + head: in a decode step
