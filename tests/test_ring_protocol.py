@@ -160,3 +160,73 @@ def test_prompt_attention_with_one_barrier_for_the_probabilities_can_stall():
     first; the parity of a single barrier is then back where it was, and the producer ends waiting for a value stage."""
     problem = _explore_attention(4, p_barriers=1)
     assert problem is not None and "nothing can move" in problem and "('V'" in problem
+
+
+def _explore_stream(S: int, T: int, warps: int, landed: bool):
+    """csrc/gemv_stream.cu's ring: the copying lane refills stage i % S once every product warp has handed fill i - S back; a product warp
+    waits for a fill, asks for its pieces, and hands the stage back: behind the loads' issue or, `landed`, not before the pieces are there.
+    What was asked for lands at any later time and is then what the stage holds at that moment.  Returns the first problem found or None."""
+    programme = lambda i: [("wait", i), ("ask", i)] + ([("need", i)] if landed else []) + [("hand", i)]  # noqa: E731
+    flat = [s for i in range(T) for s in programme(i)]
+    # copies started, held[stage] = the fill it holds (-1: being written), arrivals per stage, per warp (place, pieces on their way)
+    start = (0, (-2,) * S, (0,) * S, ((0, ()),) * warps)
+    seen, queue = {start}, deque([start])
+    while queue:
+        started, held, arrived, ws = queue.popleft()
+        nxt = []
+        if started < T:
+            s = started % S
+            if started < S or arrived[s] == warps * (started // S):
+                nxt.append((started + 1, held[:s] + (-1 - started - 2,) + held[s + 1:], arrived, ws))
+        for s in range(S):
+            if held[s] < -2:  # the copy lands
+                nxt.append((started, held[:s] + (-held[s] - 3,) + held[s + 1:], arrived, ws))
+        for w, (at, flying) in enumerate(ws):
+            put = lambda new, a=arrived: nxt.append((started, held, a, ws[:w] + (new,) + ws[w + 1:]))  # noqa: B023, E731
+            for i in flying:
+                if held[i % S] != i:
+                    return f"a piece of fill {i} is read after the next copy into its stage has begun"
+                put((at, tuple(f for f in flying if f != i)))
+            if at < len(flat):
+                what, i = flat[at]
+                if what == "wait" and held[i % S] == i or what == "need" and i not in flying:
+                    put((at + 1, flying))
+                elif what == "ask":
+                    put((at + 1, flying + (i,)))
+                elif what == "hand":
+                    put((at + 1, flying), arrived[: i % S] + (arrived[i % S] + 1,) + arrived[i % S + 1:])
+        if not nxt and any(at < len(flat) for at, _ in ws):
+            return f"nothing can move: {started} copies started, warps at {[flat[at] for at, _ in ws if at < len(flat)]}"
+        for n in nxt:
+            if n not in seen:
+                seen.add(n)
+                queue.append(n)
+    return None
+
+
+@pytest.mark.parametrize("S, T", [(2, 6), (3, 8)])
+@pytest.mark.parametrize("warps", [1, 2, 3])
+def test_a_stage_handed_back_from_what_was_loaded_is_never_read_too_late(S, T, warps):
+    assert _explore_stream(S, T, warps, landed=True) is None
+
+
+def test_a_stage_handed_back_when_its_pieces_were_only_asked_for_is_read_too_late():
+    problem = _explore_stream(2, 4, 2, landed=False)
+    assert problem is not None and "is read after" in problem
+
+
+def _code(name):
+    import pathlib
+    import re
+
+    return re.sub(r"//[^\n]*", "", (pathlib.Path(__file__).parent.parent / "rusty_llama_b200" / "csrc" / name).read_text())
+
+
+def test_every_hand_over_of_the_streaming_product_is_made_from_what_was_loaded():
+    """The model above against the source: the only arrival on an `empty` barrier is `hand_back`'s, whose address holds a vote over the
+    loaded words."""
+    helper = _code("tc_common.cuh").split("void hand_back(")[1].split("\n}")[0]
+    assert "landed = __any_sync(0xffffffffu, (pieces & zero_bits) != 0)" in helper and "mbar_arrive_s(bar + landed)" in helper
+    code = _code("gemv_stream.cu")
+    assert "mbar_arrive_s(" not in code and "mbar_arrive(&bars.empty" not in code
+    assert code.count("hand_back(") == code.count("hand_back(empty0 + 8 * st, b[0].x ^ b[KB_PER_WARP - 1].x, zero_bits, lane)") == 1
