@@ -462,14 +462,15 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
 
     // ---- O^T += V^T P^T: head size (16-row tiles) x 8 heads over the warp's 16 keys
+    uint32_t pieces = pb0 ^ pb1;  // depends on all that this lane loads from the stage (the keys came through the scores); n_splits is at most 64
 #pragma unroll
     for (int dt = 0; dt < VD / 16; ++dt) {
       uint32_t a[4];
       ldmatrix_x4_trans(a, v_s + (dt >> 2) * HALF_BYTES + swz(v_row, ((dt & 3) << 1) | v_piece));
       mma_bf16(o_acc[dt], a, pb0, pb1);
+      pieces ^= a[0];
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&bars.empty[st]);
+    hand_back(smem_u32(&bars.empty[st]), pieces, (uint32_t)n_splits >> 8, lane);
   }
 
   // ---- the four warps' partial results meet in the ring's memory, which nobody reads any more once

@@ -230,3 +230,10 @@ def test_every_hand_over_of_the_streaming_product_is_made_from_what_was_loaded()
     code = _code("gemv_stream.cu")
     assert "mbar_arrive_s(" not in code and "mbar_arrive(&bars.empty" not in code
     assert code.count("hand_back(") == code.count("hand_back(empty0 + 8 * st, b[0].x ^ b[KB_PER_WARP - 1].x, zero_bits, lane)") == 1
+
+
+def test_every_hand_over_of_the_decode_attention_is_made_from_what_was_loaded():
+    code = _code("attention_decode_tma.cu")
+    assert "mbar_arrive_s(" not in code and "mbar_arrive(&bars.empty" not in code
+    assert code.count("hand_back(smem_u32(&bars.empty[st]), pieces, (uint32_t)n_splits >> 8, lane)") == 1
+    assert "pieces = pb0 ^ pb1;" in code and "pieces ^= a[0];" in code
