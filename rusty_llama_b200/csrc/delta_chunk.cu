@@ -36,10 +36,16 @@ __device__ __forceinline__ void dc_cp_async16(float* dst, const float* src, bool
 }
 
 // Running sums of 64 log decays (zero past the chunk's last token) by one warp, two to a lane.  In 64 bits: what is used of them are
-// differences, and those of fast decays are small beside the sums.
+// differences, and those of fast decays are small beside the sums.  A log decay may be minus infinity, whose differences are no numbers:
+// from DC_LOG_LEAST down, where the exponential has long been zero, all are the same.
+#define DC_LOG_LEAST (-16384.f)
+__device__ __forceinline__ double dc_log(const float* __restrict__ log_decay) {
+  const float l = __ldcg(log_decay);
+  return (double)(l < DC_LOG_LEAST ? DC_LOG_LEAST : l);  // (what is no number stays so)
+}
 __device__ __forceinline__ void dc_log_sums(const float* __restrict__ log_decay, int t0, int n, int H, int h, double* L, int lane) {
-  const double a = 2 * lane < n ? (double)__ldcg(log_decay + (size_t)(t0 + 2 * lane) * H + h) : 0.0;
-  const double b = 2 * lane + 1 < n ? (double)__ldcg(log_decay + (size_t)(t0 + 2 * lane + 1) * H + h) : 0.0;
+  const double a = 2 * lane < n ? dc_log(log_decay + (size_t)(t0 + 2 * lane) * H + h) : 0.0;
+  const double b = 2 * lane + 1 < n ? dc_log(log_decay + (size_t)(t0 + 2 * lane + 1) * H + h) : 0.0;
   double run = a + b;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {

@@ -103,3 +103,28 @@ def test_which_steps_go_chunk_by_chunk():
     assert [n for _, n in outs] == [1, 2, 2]
     for y, _ in outs[1:]:
         assert float((y - outs[0][0]).norm() / outs[0][0].norm()) < 1e-2
+
+
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (36, 72)])
+def test_decays_of_zero(dim, vdim):
+    """A log decay of minus infinity (or far below what an exponential of 32 bits can hold) empties the state and the tokens after it go on
+    from there, inside a chunk, at its first and last token and several times over."""
+    from rusty_llama_b200.kernels import ops
+
+    lens, H, G = [200, 64], 2, 1
+    q, k, v, beta, logd = inputs(lens, H, G, dim, vdim, 5, "usual")
+    for t, h, value in ((5, 0, float("-inf")), (6, 0, float("-inf")), (63, 0, float("-inf")), (64, 1, float("-inf")), (130, 1, -1e30), (200, 0, float("-inf")), (263, 1, -3e38)):
+        logd[t, h] = value
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    T = sum(lens)
+    state = torch.randn(2, H, dim, vdim, generator=torch.Generator().manual_seed(2))
+    sd = state.to(DEV)
+    scratch = torch.empty(ops.delta_chunked_scratch_floats(T, 2, H, dim, vdim), device=DEV)
+    out = ops.delta_chunked(q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV), v.view(T, -1).to(DEV), beta.to(DEV), logd.to(DEV), sd, i32([0, 1]), i32([0, 200, 264]),
+                            H, G, dim, vdim, max(lens), scratch)
+    rep = H // G
+    refs = [recurrence(*(t[a:b].double() for t in (q.repeat_interleave(rep, 1), k.repeat_interleave(rep, 1), v, beta, logd.double().exp())), state[i].double())
+            for i, (a, b) in enumerate(((0, 200), (200, 264)))]
+    want, want_S = torch.cat([o for o, _ in refs]).reshape(T, -1), torch.stack([s for _, s in refs])
+    assert float((out.double().cpu() - want).norm() / want.norm()) <= 32 * 2.0 ** -24
+    assert float((sd.double().cpu() - want_S).norm() / want_S.norm()) <= 32 * 2.0 ** -24
