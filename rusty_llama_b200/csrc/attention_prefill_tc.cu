@@ -59,8 +59,11 @@
 // exponent's constant.
 //
 // Keys of up to 192 beside values of up to 128 (latent attention whose keys and values were expanded for the call, with its output gate in
-// the way out): two blocks still fit an SM with one value stage, whose next tile is asked for behind the next key tile.  16 heads, 2048
-// tokens: 63 us, 21.5 GFLOP at 340 TFLOP/s; the same layer on its latents with mma.sync 468 us.
+// the way out): two blocks still fit an SM with one value stage, whose next tile is asked for behind the next key tile.  There the
+// probabilities go into P V as the sum of two bfloat16 numbers, the second ones in the half of the S buffer that the first leave free: rounded
+// once, under a maximum that is only raised by factors of 2^8, they put the result 5 to 10 % further from 64 bits than the kernel on the latents
+// (whose row maximum is exact, so that a row's largest probability is 1), in two parts 1 to 6 % nearer.  16 heads, 2048 tokens: 63 us with one
+// part (340 TFLOP/s), 74 with two; the same layer on its latents with mma.sync 468 us.
 //
 // Every mbarrier wait is bounded; on expiry a code goes to status[0] and the block drains.
 #include "tc_common.cuh"
@@ -249,36 +252,57 @@ __device__ __forceinline__ uint32_t qk_block(uint32_t tmem_s, uint64_t q_desc, u
   return ready;
 }
 // The same for O (+)= P V: four MMAs of 16 keys each, P from tensor memory (8 columns a step), V as the M/N-contiguous
-// operand (2048 bytes = 128 units a step).
+// operand (2048 bytes = 128 units a step).  TWO_PARTS: P as the sum of two bfloat16 numbers, whose second ones lie 32 columns further on.
+#define RL_PV_ADDRESSES         \
+  "{\n"                         \
+  ".reg .pred t, p, q;\n"       \
+  ".reg .b64 b1, b2, b3;\n"     \
+  ".reg .b32 a1, a2, a3, c0, c1, c2, c3;\n" \
+  "mbarrier.test_wait.parity.shared::cta.b64 q, [%7], %8;\n" \
+  "setp.eq.b32 t, 0, 0;\n"      \
+  "setp.ne.b32 p, %5, 0;\n"     \
+  "add.u32 a1, %2, 8;\n"        \
+  "add.u64 b1, %3, 128;\n"      \
+  "add.u32 a2, %2, 16;\n"       \
+  "add.u64 b2, %3, 256;\n"      \
+  "add.u32 a3, %2, 24;\n"       \
+  "add.u64 b3, %3, 384;\n"
+#define RL_PV_PRODUCTS          \
+  "tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, p;\n" \
+  "tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], b1, %4, t;\n" \
+  "tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], b2, %4, t;\n" \
+  "tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], b3, %4, t;\n"
+#define RL_PV_END               \
+  "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n" \
+  "selp.u32 %0, 1, 0, q;\n"     \
+  "}\n"
+template <bool TWO_PARTS>
 __device__ __forceinline__ uint32_t pv_block(uint32_t tmem_o, uint32_t tmem_p, uint64_t v_desc, uint32_t idesc, uint32_t accumulate_first,
                                              uint32_t commit_bar, uint32_t peek_bar, uint32_t peek_parity) {
   uint32_t ready;
-  asm volatile(
-      "{\n"
-      ".reg .pred t, p, q;\n"
-      ".reg .b64 b1, b2, b3;\n"
-      ".reg .b32 a1, a2, a3;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 q, [%7], %8;\n"
-      "setp.eq.b32 t, 0, 0;\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "add.u32 a1, %2, 8;\n"
-      "add.u64 b1, %3, 128;\n"
-      "add.u32 a2, %2, 16;\n"
-      "add.u64 b2, %3, 256;\n"
-      "add.u32 a3, %2, 24;\n"
-      "add.u64 b3, %3, 384;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, p;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], b1, %4, t;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], b2, %4, t;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], b3, %4, t;\n"
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n"
-      "selp.u32 %0, 1, 0, q;\n"
-      "}\n"
-      : "=r"(ready)
-      : "r"(tmem_o), "r"(tmem_p), "l"(v_desc), "r"(idesc), "r"(accumulate_first), "r"(commit_bar), "r"(peek_bar), "r"(peek_parity)
-      : "memory");
+  if (TWO_PARTS)
+    asm volatile(RL_PV_ADDRESSES
+                 "add.u32 c0, %2, 32;\n"
+                 "add.u32 c1, %2, 40;\n"
+                 "add.u32 c2, %2, 48;\n"
+                 "add.u32 c3, %2, 56;\n" RL_PV_PRODUCTS
+                 "tcgen05.mma.cta_group::1.kind::f16 [%1], [c0], %3, %4, t;\n"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%1], [c1], b1, %4, t;\n"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%1], [c2], b2, %4, t;\n"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%1], [c3], b3, %4, t;\n" RL_PV_END
+                 : "=r"(ready)
+                 : "r"(tmem_o), "r"(tmem_p), "l"(v_desc), "r"(idesc), "r"(accumulate_first), "r"(commit_bar), "r"(peek_bar), "r"(peek_parity)
+                 : "memory");
+  else
+    asm volatile(RL_PV_ADDRESSES RL_PV_PRODUCTS RL_PV_END
+                 : "=r"(ready)
+                 : "r"(tmem_o), "r"(tmem_p), "l"(v_desc), "r"(idesc), "r"(accumulate_first), "r"(commit_bar), "r"(peek_bar), "r"(peek_parity)
+                 : "memory");
   return ready;
 }
+#undef RL_PV_ADDRESSES
+#undef RL_PV_PRODUCTS
+#undef RL_PV_END
 
 // KD, VD: the padded sizes of a key and a value; kdim, vdim: the sizes themselves.
 // MAPS 2: query heads 2h and 2h + 1 are the two halves of the KD numbers of row h (the values are the same for both); the row's
@@ -471,7 +495,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         tc_fence_after();
         // O += P(j) V(j); asks for key tile j + 2
         const int jk = j + 2;
-        k_ready = pv_block(tmem_base + O_COL, tmem_base + (uint32_t)((j & 1) * BNK),
+        k_ready = pv_block<EXPANDED>(tmem_base + O_COL, tmem_base + (uint32_t)((j & 1) * BNK),
                                make_smem_desc_mn(smem_u32(v_s + (size_t)st * V_BYTES), SUBK_BYTES, 1024), idesc_pv, j > 0 ? 1u : 0u,
                                smem_u32(&pv_done[j & 1]), smem_u32(&k_full[jk % KV_STAGES]), (uint32_t)((jk / KV_STAGES) & 1));
         if (jk < n_tiles) {
@@ -596,7 +620,7 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       // The probabilities, rounded to bfloat16, go back into tensor memory two to a column, over the first half of
       // this row of S, and the product reads them there.  (The S buffer's next product comes after this tile's P V in
       // the issuing thread's order, and the tensor core keeps that order.)
-      uint32_t pk[BNK / 2];
+      uint32_t pk[BNK / 2], rest[EXPANDED ? BNK / 2 : 1];
       float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int i = 0; i < BNK / 2; ++i) {
@@ -604,8 +628,10 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const float p1 = exp2_fast(fmaf(__uint_as_float(v[2 * i + 1]), exp_scale, neg_m));
         sum4[i & 3] += p0 + p1;
         pk[i] = pack2(p0, p1);
+        if (EXPANDED) rest[i] = pack2(p0 - __uint_as_float(pk[i] << 16), p1 - __uint_as_float(pk[i] & 0xffff0000u));
       }
       tmem_st_32x32b_x32(s_addr, pk);
+      if constexpr (EXPANDED) tmem_st_32x32b_x32(s_addr + BNK / 2, rest);
       l_run = l_run * a + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
       tmem_st_wait();
       // P is complete (and the accumulator rescaled if it had to be): hand both to the tensor core

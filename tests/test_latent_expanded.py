@@ -137,3 +137,28 @@ def test_a_role_gives_up_with_keys_of_192(code, text):
     expect_give_up(ops, code, "flash_prefill_tc: .*" + text, run)
     assert torch.equal(run(), before)
     ops.tc_status_check()
+
+
+@pytest.mark.parametrize("H, dim, rot, vdim, rank", [(8, 64, 32, 64, 256), (4, 128, 64, 128, 512)])
+def test_expanding_loses_nothing_against_64_bits(H, dim, rot, vdim, rank):
+    """The gated sums of both forms of a step against 64 bits: rounding keys and values per head costs what rounding queries and sums in the
+    latent space costs, and the probabilities must not cost more."""
+    import rusty_llama_b200.parts.latent_attention as module
+    from rusty_llama_b200.cache import Cache
+
+    part, w = make(H, dim, rot, vdim, rank, 256)
+    g = torch.Generator().manual_seed(17)
+    lens = [41, 64, 222, 300]
+    xs = [(2 * torch.randn(n, 256, generator=g)).to(torch.bfloat16) for n in lens]
+    want = torch.cat([plain(dict(w, o=torch.eye(H * vdim, dtype=torch.float64)), x.double(), H, dim, rot, vdim, rank, 0, True, True, 0) for x in xs])
+    off = []
+    for least in (module._EXPAND_MIN_TOKENS, 10**9):
+        cache = Cache([(0, part.cache_need())], 64 * 12, 4, torch.bfloat16, DEV)
+        step, tables = ctx_for(cache, [cache.open_sequence() for _ in lens], [0] * 4, lens)
+        before, module._EXPAND_MIN_TOKENS = module._EXPAND_MIN_TOKENS, least
+        try:
+            a, _ = part.forward_unprojected(torch.cat(xs).to(DEV), step, cache.view(0, tables))
+        finally:
+            module._EXPAND_MIN_TOKENS = before
+        off.append(float((a.double().cpu() - want).norm() / want.norm()))
+    assert off[0] <= off[1], off
