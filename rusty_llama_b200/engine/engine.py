@@ -50,6 +50,8 @@ class StepContext:
     seq_pos0[S] (positions held before the step), seq_len[S] (positions held after),
     slot_ids[S], rows[W] (packed indices of the tokens whose logits are wanted).
 
+    pos0: what seq_pos0 holds, on the host, for choices between forms of a step (None: not told).
+
     shared: what one run of the schedule leaves for later runs of the same step (a mixer that hands the values it projected
     to the layers after it); the model empties it before the first run."""
 
@@ -70,6 +72,7 @@ class StepContext:
     slot_ids: torch.Tensor
     rows: Optional[torch.Tensor]
     shared: Dict[str, torch.Tensor] = field(default_factory=dict)
+    pos0: Optional[List[int]] = None
 
 
 def _pad4(n: int) -> int:
@@ -242,6 +245,7 @@ class Engine:
             seq_len=meta.dev_part(5),
             slot_ids=meta.dev_part(6),
             rows=meta.dev_part(7)[:n_rows] if n_rows else None,
+            pos0=[int(p) for p in pos0],
         )
         tables = [meta.dev_part(8 + g).view(S, w) for g, w in enumerate(meta.widths)]
         return step, tables

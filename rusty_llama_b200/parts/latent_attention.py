@@ -13,13 +13,13 @@ from ..kernels.linear import linear, linear_to_stream
 from ..spec import PartSpec
 from .base import MIXERS, POSITIONS, KVNeed, Mixer, ParamInfo
 
-# A step expands keys and values per head from so many tokens on (above the head products' few-row form), while there are at most so many
-# rows to expand for each of them: a row costs 0.26 million operations a head at the sizes below, a pair on the latents 1.5 thousand more
-# at about a quarter of the rate, so that 43 rows a query break even where every row is seen once; a chunk of a prompt sees each of them
-# from every query.  And they have to fit so many bytes for the call.
+# A step may expand keys and values per head from so many tokens on (above the head products' few-row form), if the rows fit so many bytes
+# for the call.
 _EXPAND_MIN_TOKENS = 33
-_EXPAND_MAX_ROWS_PER_TOKEN = 64
 _EXPAND_MAX_BYTES = 1 << 30
+# What an operation of the attention on the latents (156 TFLOP/s) and of the one over expanded rows (290) takes in operations of the head
+# products (540)
+_LATENT_OPERATION, _EXPANDED_OPERATION = 3.5, 1.9
 
 _NAMES = {"q": "q", "q_down": "dq", "q_norm": "dq.norm", "q_up": "uq", "kv": "dkv", "kv_norm": "dkv.norm", "k_up": "uk", "v_up": "uv", "sink": "sink", "gate": "g", "out": "o"}
 
@@ -148,10 +148,12 @@ class LatentAttention(Mixer):
     def _expands(self, step, q: torch.Tensor, gate) -> int:
         """How many rows a sequence's keys and values are expanded to (a multiple of the page size), or 0: the step works on the latents.
 
-        Expanding costs 2 rank (dim + vdim) operations a head and cached position; working on the latents costs 2 (2 rank - dim - vdim)
-        more a head and (query, key) pair and 2 rank (dim + vdim) a head and token, on mma.sync.  Measured, 16 heads of 128 + 64 / 128, rank
-        512, one prompt of 2048: 468 us on the latents and 25 us for the two products around it; expanded, 16 us for the products, 5 for the
-        rows, 63 for the attention."""
+        The work decides.  Expanding costs 2 rank (dim + vdim) operations a head and held position; working on the latents costs the same a
+        head and token of the step, for the products around it, and 2 (2 rank + rot) instead of 2 (dim + rot + vdim) slower ones a head and
+        (query, key) pair.  So a sequence's earlier positions pay for themselves where enough tokens of the step see them: 41 with
+        128 + 64 / 128 and rank 512, 21 with 64 + 32 / 64 and rank 256, unless a window hides them.  Measured, 16 heads of 128 + 64 / 128, rank
+        512, one prompt of 2048: 468 us on the latents (156 TFLOP/s) and 25 us for the two products around it; expanded, 16 us for the
+        products (540 TFLOP/s), 5 for the rows, 74 for the attention (290 TFLOP/s)."""
         if step.decode_only or self.w_vk is None or step.n_tokens < _EXPAND_MIN_TOKENS or not q.is_cuda:
             return 0
         if not ops.flash_expanded_takes(self.dim + self.rot, self.vdim) or self.dim % 8 or self.rot % 8 or self.rank % 8 or self.dim == 0:
@@ -159,9 +161,18 @@ class LatentAttention(Mixer):
         if q.stride(0) % 8 or q.data_ptr() % 16 or (gate is not None and (gate.stride(0) % 8 or gate.data_ptr() % 16)):
             return 0
         seq_rows = (step.max_kv_len + ops.PAGE_SIZE - 1) // ops.PAGE_SIZE * ops.PAGE_SIZE
-        rows = step.n_seqs * seq_rows
-        small = rows * self.H * (self.vdim + self.dim + self.rot) * 2 <= _EXPAND_MAX_BYTES
-        return seq_rows if small and rows <= _EXPAND_MAX_ROWS_PER_TOKEN * step.n_tokens else 0
+        if step.n_seqs * seq_rows * (self.H * (self.vdim + self.dim + self.rot) + self.rank) * 2 > _EXPAND_MAX_BYTES:
+            return 0
+        # (a caller that does not say what each sequence held: what they all held if they are equally long)
+        pos0 = step.pos0 if step.pos0 is not None else [step.max_kv_len - step.max_q_len] * step.n_seqs
+        earlier = pairs = 0
+        for p, n in zip(pos0, step.q_lens):
+            earlier += p
+            growing = min(n, max(self.window - p, 0)) if self.window else n  # tokens that the window does not cut short
+            pairs += growing * p + growing * (growing + 1) // 2 + (n - growing) * self.window
+        a_row = self.rank * (self.dim + self.vdim)
+        a_pair = _LATENT_OPERATION * (2 * self.rank + self.rot) - _EXPANDED_OPERATION * (self.dim + self.rot + self.vdim)
+        return seq_rows if earlier * a_row <= a_pair * pairs else 0
 
     def forward_unprojected(self, xn: torch.Tensor, step, cache, shared_cache: bool = False):
         if shared_cache == self.own_kv:
