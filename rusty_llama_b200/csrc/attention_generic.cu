@@ -25,13 +25,13 @@ RL_DEFINE_ERROR_TEXT()
 
 #define WARPS 8  // part of the summation order
 
-// DPL: value dimensions per lane (head sizes up to 32 DPL); HB: query heads per block
+// DPL: value dimensions per lane (head sizes up to 32 DPL); HB: query heads per block; by4: the keys' rows can be read four numbers at a time
 template <typename T, int DPL, int HB>
 __global__ void __launch_bounds__(WARPS * 32)
 attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages,
                     const T* __restrict__ v_pages, const int* __restrict__ block_table, int table_width,
                     const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, T* __restrict__ out, int out_stride,
-                    int H, int K, int hd, int page_size, int window, float scale) {
+                    int H, int K, int hd, int page_size, int window, float scale, bool by4) {
   extern __shared__ __align__(16) float sm[];
   const int hd4 = (hd + 3) & ~3;
   float* q_s = sm;                              // [HB][hd4]
@@ -53,7 +53,6 @@ attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__
 
   // keep when pos - key < window (src/backend/cpu.rs:404-409)
   const int first = (window != 0 && pos + 1 > window) ? pos + 1 - window : 0;
-  const bool by4 = (hd & 3) == 0;  // rows that can be read four numbers at a time
   float m[HB], l[HB], acc[HB][DPL];
 #pragma unroll
   for (int h = 0; h < HB; ++h) {
@@ -174,9 +173,10 @@ static int launch_attn_generic(const void* q, int q_stride, const void* k_pages,
   auto kern = attn_generic_kernel<T, DPL, HB>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     RL_REFUSE(7, "attn_generic: cannot get %zu bytes of shared memory", smem);
+  const bool by4 = hd % 4 == 0 && (uintptr_t)k_pages % (4 * sizeof(T)) == 0;
   kern<<<dim3(n_tokens, gy), WARPS * 32, smem, stream>>>((const T*)q, q_stride, (const T*)k_pages, (const T*)v_pages, block_table,
                                                          table_width, tok_seq, tok_pos, (T*)out, out_stride, H, K, hd, page_size,
-                                                         window, scale);
+                                                         window, scale, by4);
   RL_LAUNCH_RESULT();
 }
 

@@ -80,3 +80,20 @@ def test_attention_of_few_and_of_many_tokens(ops, H, K, hd, window):
     for i in (0, 1, 31, 32, 99, 100, n - 1):  # one token: other heads per block, the same bits
         one = ops.attn_generic(q[i : i + 1].to(DEV), *args, seq[i : i + 1].to(DEV), pos[i : i + 1].to(DEV), H, K, hd, window=window)
         assert torch.equal(one[0], many[i])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_over_pages_that_start_anywhere(ops, dtype):
+    """Pages in the middle of a larger buffer, off the boundary that four numbers at a time need: the same bits."""
+    H, K, hd, L = 8, 2, 64, 150
+    g = torch.Generator().manual_seed(3)
+    pages = torch.randn(3, K, 64, hd, generator=g).to(dtype).to(DEV)
+    q = torch.randn(L, H * hd, generator=g).to(dtype).to(DEV)
+    table, seq = torch.arange(3, dtype=torch.int32, device=DEV)[None], torch.zeros(L, dtype=torch.int32, device=DEV)
+    pos = torch.arange(L, dtype=torch.int32, device=DEV)
+    want = ops.attn_generic(q, pages, pages, table, seq, pos, H, K, hd)
+    for off in (1, 2, 3):
+        buffer = torch.zeros(pages.numel() + off, dtype=dtype, device=DEV)
+        moved = buffer[off:].view(pages.shape)
+        moved.copy_(pages)
+        assert torch.equal(ops.attn_generic(q, moved, moved, table, seq, pos, H, K, hd), want)
