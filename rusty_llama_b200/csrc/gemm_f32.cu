@@ -343,7 +343,7 @@ RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* 
   if (M <= GEMV_ROWS && vec && nch <= GEMV_MAX_ITEMS) {
     int R = (N + 2 * sms - 1) / (2 * sms);
     if (R > GEMV_MAX_ITEMS / nch) R = GEMV_MAX_ITEMS / nch;
-    // as many rows of x a block as there are, up to four, while two blocks fit an SM; else one row (up to K of about 34000)
+    // as many rows of x a block as there are, up to four, while two blocks fit an SM; else one row (up to 327 chunks: K of 41856)
     int mb = M == 1 ? 1 : M == 2 ? 2 : 4;
     while (mb > 1 && gemv_f32_smem(mb, nch, R) > 112 * 1024) mb /= 2;
     const size_t smem = gemv_f32_smem(mb, nch, R);

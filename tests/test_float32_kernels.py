@@ -43,12 +43,16 @@ def test_product_in_every_form(ops, M, N, K):
 
 
 def test_product_of_a_very_long_k(ops):
-    """Rows too long for the few-row kernel's shared memory (K above 34000) go to the tile kernel."""
+    """The longest rows of the few-row kernel (327 chunks of 128 and one row of a block's shared memory) and ones too long for it, which go to
+    the tile kernel however few they are: the same bits as among many rows."""
     g = torch.Generator().manual_seed(5)
-    x, w = torch.randn(3, 40000, generator=g), torch.randn(9, 40000, generator=g)
-    out = ops.gemm_f32(x.to(DEV), w.to(DEV))
-    assert bool(((out.cpu().double() - x.double() @ w.double().T).abs() <= product_bound(x, w)).all())
-    assert torch.equal(ops.gemm_f32(x[:, :20000].to(DEV), w[:, :20000].to(DEV))[1], ops.gemm_f32(x[1:2, :20000].to(DEV), w[:, :20000].to(DEV))[0])
+    for K in (20000, 41856, 41860, 44000, 70000):
+        x, w = torch.randn(12, K, generator=g), torch.randn(9, K, generator=g)
+        xd, wd = x.to(DEV), w.to(DEV)
+        many = ops.gemm_f32(xd, wd)
+        assert bool(((many.cpu().double() - x.double() @ w.double().T).abs() <= product_bound(x, w)).all())
+        for rows in (1, 3, 8):
+            assert torch.equal(ops.gemm_f32(xd[:rows], wd), many[:rows])
 
 
 @pytest.mark.parametrize("window", [0, 70])
