@@ -28,9 +28,10 @@ RL_DEFINE_ERROR_TEXT()
 
 // ---------------------------------------------------------------- norm, rotation, cache write
 // Pair i of a rotated part, dimensions (2i, 2i+1) or, not `interleaved`, (i, i + n_pairs), turns by pos * freq[i]; cos and sin are
-// multiplied by `mag`; dimensions from 2 n_pairs on pass unchanged.  Everything in 32-bit, rounded once when stored.
+// multiplied by `mag`; dimensions from 2 n_pairs on pass unchanged.  Everything in 32-bit, rounded once when stored.  dst may be src: a
+// pair is read before it is written, by one thread.
 template <typename T>
-__device__ __forceinline__ void turn_pair(const T* __restrict__ src, T* __restrict__ dst, int i, int n_pairs, int interleaved, int pos,
+__device__ __forceinline__ void turn_pair(const T* src, T* dst, int i, int n_pairs, int interleaved, int pos,
                                           const float* __restrict__ freq, float mag) {
   const bool halves = !interleaved && i < n_pairs;
   const int d0 = halves ? i : 2 * i, d1 = halves ? i + n_pairs : 2 * i + 1;
@@ -48,7 +49,7 @@ __device__ __forceinline__ void turn_pair(const T* __restrict__ src, T* __restri
   dst[d1] = from_f32<T>(v);
 }
 
-// (q may be q_cat: a pair is read before it is written, by one thread)
+// (q may be q_cat: see turn_pair)
 template <typename T>
 __global__ void latent_prep_kernel(const T* q, int ldq, const T* __restrict__ kv, int ldkv,
                                    const float* __restrict__ norm_w, float eps, const float* __restrict__ freq,
