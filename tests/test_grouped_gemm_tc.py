@@ -116,3 +116,21 @@ def test_a_role_gives_up_and_the_next_launch_is_right(ops, code, text):
     expect_give_up(ops, code, "grouped_gemm_tc: " + text, run)
     assert torch.equal(run(), before)
     ops.tc_status_check()
+
+
+@pytest.mark.parametrize("tile_rows", [32, 128, 256])
+def test_a_gate_far_below_zero(ops, tile_rows):
+    """silu and the form with limits where 1 + exp(-gate) is above 2^126: the quotient is small and not zero (an approximate division
+    gives zero there), within the result's rounding to bfloat16 (8 significant bits: 2^-8) and a few of 32 bits before it."""
+    gates = torch.tensor([-1.0, -20.0, -60.0, -80.0, -86.0, -87.5, -88.0, -88.5, 0.0, 3.0, 40.0, 88.0] + [-87.5] * 52)
+    N, K, T = gates.numel(), 8, 3
+    x, w, w2 = torch.zeros(T, K), torch.zeros(2, N, K), torch.zeros(2, N, K)
+    x[:, 0] = 1.0
+    w[:, :, 0], w2[:, :, 0] = gates, 1.0
+    bf = lambda t: t.to(torch.bfloat16).to(DEV)  # noqa: E731
+    ids = torch.tensor([[0], [1], [0]], dtype=torch.int32, device=DEV)
+    order, place, tiles, mt = ops.moe_plan(ids, 2, tile_rows)
+    g = gates.double()
+    for act, want in ((None, g / (1 + torch.exp(-g))), ((1.0, 100.0), g / (1 + torch.exp(-g)) * 2.0)):
+        got = ops.moe_gemm(bf(x), bf(w), tiles, mt, T, order=order, w2=bf(w2), tile_rows=tile_rows, act=act).double().cpu()
+        assert bool(((got - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()), (act, (got[0] / want).tolist()[:12])
