@@ -331,6 +331,35 @@ __device__ __forceinline__ void dc_outer(const float* x, const float* y, int ty,
   }
 }
 
+// The same over the tokens up to each row's own, acc[a][e] += sum_(k <= row) x[row][k] * y[k][4 tx + e], row = ty + 16 a.  What a row does not
+// see is left out and not multiplied by zero: a later token's write may be infinite or no number.
+template <int LX>
+__device__ __forceinline__ void dc_outer_seen(const float* x, const float* y, int ty, int tx, float (&acc)[4][4]) {
+  constexpr int LY = DC_OUT_COLS + DC_PAD;
+#pragma unroll
+  for (int sub = 0; sub < 4; ++sub) {
+#pragma unroll 2
+    for (int k = 0; k < 16; k += 4) {
+      float4 b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(y + (16 * sub + k + j) * LY + 4 * tx);
+#pragma unroll
+      for (int i = sub; i < 4; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(x + (ty + 16 * i) * LX + 16 * sub + k);
+        const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (i > sub || k + j <= ty) {
+            acc[i][0] = fmaf(av[j], b[j].x, acc[i][0]);
+            acc[i][1] = fmaf(av[j], b[j].y, acc[i][1]);
+            acc[i][2] = fmaf(av[j], b[j].z, acc[i][2]);
+            acc[i][3] = fmaf(av[j], b[j].w, acc[i][3]);
+          }
+      }
+    }
+  }
+}
+
 template <int DP>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ log_decay,
@@ -390,7 +419,7 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ k
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[a][e] *= f;
     }
-    dc_outer<DC, LP>(p_s, u_s, ty, tx, acc);
+    dc_outer_seen<LP>(p_s, u_s, ty, tx, acc);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       const int i = ty + 16 * a;

@@ -128,3 +128,28 @@ def test_decays_of_zero(dim, vdim):
     want, want_S = torch.cat([o for o, _ in refs]).reshape(T, -1), torch.stack([s for _, s in refs])
     assert float((out.double().cpu() - want).norm() / want.norm()) <= 32 * 2.0 ** -24
     assert float((sd.double().cpu() - want_S).norm() / want_S.norm()) <= 32 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_what_is_no_number_does_not_reach_earlier_tokens(value):
+    """A value that is infinite or no number spoils its head's outputs from its token on and the state, and nothing before it."""
+    from rusty_llama_b200.kernels import ops
+
+    T, H, n = 150, 2, 64
+    q, k, v, beta, logd = inputs([T], H, 1, n, n, 8, "usual")
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    scratch = torch.empty(ops.delta_chunked_scratch_floats(T, 1, H, n, n), device=DEV)
+
+    def run(v):
+        state = torch.zeros(1, H, n, n, device=DEV)
+        out = ops.delta_chunked(q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV), v.reshape(T, -1).to(DEV), beta.to(DEV), logd.to(DEV), state, i32([0]), i32([0, T]),
+                                H, 1, n, n, T, scratch)
+        return out.view(T, H, n), state[0]
+
+    want, want_S = run(v)
+    for at in (0, 1, 17, 63, 64, 149):
+        bad = v.clone()
+        bad[at, 0] = value
+        out, S = run(bad)
+        assert torch.equal(out[:at], want[:at]) and torch.equal(out[:, 1], want[:, 1]) and torch.equal(S[1], want_S[1]), at
+        assert not bool(out[at:, 0].isfinite().any()) and not bool(S[0].isfinite().any())
