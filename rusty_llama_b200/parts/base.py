@@ -58,6 +58,15 @@ class Workspace:
         return buf
 
 
+def scratch_for_call(shape, dtype: torch.dtype, device) -> Optional[torch.Tensor]:
+    """Scratch that one call uses and gives back, for steps that are never captured (a `Workspace` keeps what it hands out, and what has
+    outgrown it as well).  None where the device has no room for it: the caller has a form of the work that needs none."""
+    try:
+        return torch.empty(shape, dtype=dtype, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 @dataclass
 class Runtime:
     """Where and in which precision a model runs.

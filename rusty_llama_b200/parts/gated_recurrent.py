@@ -22,11 +22,12 @@ import torch
 from ..errors import ConfigError
 from ..kernels import ops
 from ..kernels.linear import linear, linear_to_stream
-from .base import MIXERS, Mixer, ParamInfo, StateNeed
+from .base import MIXERS, Mixer, ParamInfo, StateNeed, scratch_for_call
 
 # prompt steps whose longest sequence brings fewer tokens than this go token by token like a decode step
 _CHUNKED_MIN_TOKENS = 32
-# the most scratch that the delta rule's chunks may take (2 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it token by token
+# the most scratch that the delta rule's chunks may take (2 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it, and where the
+# device has less, token by token
 _CHUNKED_MAX_FLOATS = 1 << 29
 
 
@@ -314,14 +315,15 @@ class GatedDeltaRule(Mixer):
         conv = ops.short_conv(proj[:, :C], self.w_conv, None if inputs is None else inputs.state, step.slot_ids, step.seq_start, step.tok_seq,
                               single=step.decode_only)
         gate, ba = proj[:, C : C + vd], proj[:, C + vd : C + vd + 2 * H]
-        chunked, floats = False, 0
+        scratch = None
         if xn.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS and ops.delta_chunked_takes(self.dim, self.vdim):
             floats = ops.delta_chunked_scratch_floats(step.n_tokens, step.n_seqs, H, self.dim, self.vdim)
-            chunked = floats <= _CHUNKED_MAX_FLOATS
+            if floats <= _CHUNKED_MAX_FLOATS:
+                scratch = scratch_for_call(floats, torch.float32, xn.device)
+        chunked = scratch is not None
         qn, kn, kq, beta, decay = ops.delta_prep(conv[:, : 2 * self.qd], ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps, self.q_scale,
                                                  log_decay=chunked)
         if chunked:  # a prompt of a bfloat16 run, all chunks side by side but for the walk through the state
-            scratch = self.rt.workspace.get("delta_chunks", floats, torch.float32)
             o = ops.delta_chunked(qn, kn, conv[:, 2 * self.qd :], beta, decay, memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim,
                                   step.max_q_len, scratch)
         else:

@@ -153,3 +153,59 @@ def test_what_is_no_number_does_not_reach_earlier_tokens(value):
         out, S = run(bad)
         assert torch.equal(out[:at], want[:at]) and torch.equal(out[:, 1], want[:, 1]) and torch.equal(S[1], want_S[1]), at
         assert not bool(out[at:, 0].isfinite().any()) and not bool(S[0].isfinite().any())
+
+
+def layer(H, G, dim, vdim, d):
+    from rusty_llama_b200.parts import MIXERS, Runtime
+    from rusty_llama_b200.spec import PartSpec
+
+    part = MIXERS.build(PartSpec("gated_delta", {"hidden_size": d, "num_heads": H, "num_qk_heads": G, "dim": dim, "vdim": vdim, "taps": 4, "eps": 1e-5}),
+                        Runtime.create(DEV, torch.bfloat16))
+    g = torch.Generator().manual_seed(0)
+    w = {}
+    for name, info in part.param_infos().items():
+        t = torch.randn(info.shape, generator=g) * (0.2 if len(info.shape) > 1 else 0.5) + (1.0 if name == "norm" else 0.0)
+        w[name] = (t if info.kind == "scalars" else t.to(torch.bfloat16)).to(DEV)
+    part.load(w)
+    return part
+
+
+def test_prompts_of_rising_lengths_leave_no_scratch_behind():
+    from rusty_llama_b200.cache import Cache
+
+    from test_parts import ctx_for
+
+    part = layer(8, 2, 64, 64, 64)
+    cache = Cache([(0, part.cache_need())], 64, 1, torch.bfloat16, DEV)
+    slot = cache.open_sequence()
+
+    def held(n):
+        step, tables = ctx_for(cache, [slot], [0], [n])
+        part.forward(torch.zeros(n, 64, dtype=torch.bfloat16, device=DEV), step, cache.view(0, tables))
+        del step, tables
+        torch.cuda.synchronize()
+        return torch.cuda.memory_allocated()
+
+    first = held(64)
+    assert [held(n) - first for n in (128, 256, 512, 1024, 64)] == [0] * 5
+
+
+def test_a_prompt_without_room_for_the_chunks_goes_token_by_token():
+    from rusty_llama_b200.cache import Cache
+
+    from test_parts import ctx_for
+    from test_waits import with_memory_left
+
+    part = layer(32, 1, 128, 128, 64)
+    x = torch.randn(1024, 64, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16).to(DEV)
+
+    def run():
+        cache = Cache([(0, part.cache_need())], 64, 1, torch.bfloat16, DEV)
+        step, tables = ctx_for(cache, [cache.open_sequence()], [0], [1024])
+        y = part.forward(x, step, cache.view(0, tables))
+        return y.float().sum(0) if y.dim() == 3 else y.float()
+
+    scratch = 4 * (1024 // 64 + 2) * 32 * (64 * 256 + 128 * 128 + 68)
+    got = with_memory_left(scratch, run)  # (the rest of the layer takes some 60 MB of these 75)
+    want = run()
+    assert float((got - want).norm() / want.norm()) < 1e-2

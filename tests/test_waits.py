@@ -43,6 +43,18 @@ def expect_give_up(ops, code, text, launch):
     assert took < 5.0, f"the abandoned launch took {took:.1f} s"
 
 
+def with_memory_left(n_bytes, run):
+    """`run()` while torch's allocator may take `n_bytes` more than what is in use (it says so by an exception on the host)."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + n_bytes) / total)
+    try:
+        return run()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
 def test_gemm_tc_issuer_gives_up_and_the_next_launch_is_right(ops):
     g = torch.Generator().manual_seed(1)
     x = bf16_round(torch.randn(200, 512, generator=g))
