@@ -105,7 +105,7 @@ template <int DP>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_solve_kernel(const float* __restrict__ kn, const bf16* __restrict__ v, int v_stride, const float* __restrict__ beta,
                          const float* __restrict__ log_decay, const int* __restrict__ seq_start, float* __restrict__ W, float* __restrict__ U,
-                         float* __restrict__ tails, int H, int G, int dim, int vdim) {
+                         float* __restrict__ tails, int H, int G, int dim, int vdim, int min_len) {
   extern __shared__ __align__(16) float sm[];
   constexpr int LD = DP + DC_PAD, LA = DC + DC_PAD;
   float* k_s = sm;             // [64][LD]
@@ -115,9 +115,9 @@ delta_chunk_solve_kernel(const float* __restrict__ kn, const bf16* __restrict__ 
   pdl_trigger();
   pdl_wait();
   const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z, kh = h / (H / G), tid = threadIdx.x;
-  const int start = __ldcg(seq_start + s), t0 = start + c * DC;
-  const int n = min(DC, __ldcg(seq_start + s + 1) - t0);
-  if (n <= 0) return;
+  const int start = __ldcg(seq_start + s), end = __ldcg(seq_start + s + 1), t0 = start + c * DC;
+  const int n = min(DC, end - t0);
+  if (n <= 0 || end - start < min_len) return;
   dc_load_rows<DP, 256>(k_s, kn + ((size_t)t0 * G + kh) * dim, (size_t)G * dim, n, dim);
   if (tid < 32) dc_log_sums(log_decay, t0, n, H, h, L, tid);
   if (tid >= 64 && tid < 64 + DC) be[tid - 64] = tid - 64 < n ? __ldcg(beta + (size_t)(t0 + tid - 64) * H + h) : 0.f;
@@ -182,7 +182,7 @@ template <int DP>
 __global__ void __launch_bounds__(4 * DP)
 delta_chunk_walk_kernel(const float* __restrict__ kn, const float* __restrict__ tails, float* __restrict__ state,
                         const int* __restrict__ slot_ids, const int* __restrict__ seq_start, const float* __restrict__ W, float* __restrict__ U,
-                        float* __restrict__ states, int H, int G, int dim, int vdim) {
+                        float* __restrict__ states, int H, int G, int dim, int vdim, int min_len) {
   extern __shared__ __align__(16) float sm[];
   constexpr int LD = DP + DC_PAD, PARTS = DP / 32, LS = DC_COLS + DC_PAD, THREADS = 4 * DP;
   float* w_s = sm;                      // [2][64][LD]
@@ -196,7 +196,7 @@ delta_chunk_walk_kernel(const float* __restrict__ kn, const float* __restrict__ 
   const int col0 = blockIdx.x * DC_COLS, h = blockIdx.y, s = blockIdx.z, kh = h / (H / G);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int start = __ldcg(seq_start + s), len = __ldcg(seq_start + s + 1) - start, n_chunks = (len + DC - 1) / DC;
-  if (n_chunks <= 0) return;
+  if (n_chunks <= 0 || len < min_len) return;
   const int chunk0 = dc_first_chunk(start, s);
   auto load = [&](int c) {
     const size_t slot = (size_t)(chunk0 + c) * H + h;
@@ -364,7 +364,7 @@ template <int DP>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ log_decay,
                        const int* __restrict__ seq_start, const float* __restrict__ U, const float* __restrict__ states, float* __restrict__ out,
-                       int out_stride, int H, int G, int dim, int vdim) {
+                       int out_stride, int H, int G, int dim, int vdim, int min_len) {
   extern __shared__ __align__(16) float sm[];
   constexpr int LD = DP + DC_PAD, LP = DC + DC_PAD, LY = DC_OUT_COLS + DC_PAD;
   constexpr int K_FLOATS = DC * LD > DP * LY ? DC * LD : DP * LY;
@@ -376,9 +376,9 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const float* __restrict__ k
   pdl_trigger();
   pdl_wait();
   const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z, kh = h / (H / G), tid = threadIdx.x;
-  const int start = __ldcg(seq_start + s), t0 = start + c * DC;
-  const int n = min(DC, __ldcg(seq_start + s + 1) - t0);
-  if (n <= 0) return;
+  const int start = __ldcg(seq_start + s), end = __ldcg(seq_start + s + 1), t0 = start + c * DC;
+  const int n = min(DC, end - t0);
+  if (n <= 0 || end - start < min_len) return;
   const size_t at = ((size_t)t0 * G + kh) * dim, ld = (size_t)G * dim;
   dc_load_rows<DP, 256>(q_s, qn + at, ld, n, dim);
   dc_load_rows<DP, 256>(k_s, kn + at, ld, n, dim);
@@ -439,11 +439,12 @@ RL_API long long rl_delta_chunked_scratch(int n_tokens, int n_seqs, int H, int d
 }
 
 // qn, kn: float32 [T, G dim] (unit vectors, the queries times their constant); v: bfloat16 rows of >= H vdim; beta, log_decay: float32
-// [T, H]; state: float32 [slots, H, dim, vdim]; out: float32 [T, >= H vdim].
+// [T, H]; state: float32 [slots, H, dim, vdim]; out: float32 [T, >= H vdim].  Sequences of fewer than min_len tokens (and their rows of out)
+// are left alone.
 template <int DP>
 static int launch_delta_chunked(const float* qn, const float* kn, const bf16* v, int v_stride, const float* beta, const float* log_decay,
                                 float* state, const int* slot_ids, const int* seq_start, float* out, int out_stride, int n_tokens, int n_seqs,
-                                int max_q_len, int H, int G, int dim, int vdim, float* scratch, cudaStream_t stream) {
+                                int max_q_len, int H, int G, int dim, int vdim, int min_len, float* scratch, cudaStream_t stream) {
   constexpr int LD = DP + DC_PAD, LY = DC_OUT_COLS + DC_PAD;
   constexpr size_t smem1 = (size_t)(DC * LD + DC * (DC + DC_PAD)) * 4;
   constexpr size_t smem2 = (size_t)(4 * DC * LD + DP * (DC_COLS + DC_PAD) + DC * DC_COLS + DP / 32 * DC * DC_COLS) * 4;
@@ -458,17 +459,17 @@ static int launch_delta_chunked(const float* qn, const float* kn, const bf16* v,
   float* states = U + chunks * H * DC * vdim;
   float* tails = states + chunks * H * dim * vdim;  // [chunk][head][64 + 4]
   const dim3 per_chunk((max_q_len + DC - 1) / DC, H, n_seqs), per_tile((vdim + DC_COLS - 1) / DC_COLS, H, n_seqs);
-  RL_LAUNCH_CHECK(rl_launch<false>(delta_chunk_solve_kernel<DP>, per_chunk, 256, smem1, stream, kn, v, v_stride, beta, log_decay, seq_start, W, U, tails, H, G, dim, vdim));
+  RL_LAUNCH_CHECK(rl_launch<false>(delta_chunk_solve_kernel<DP>, per_chunk, 256, smem1, stream, kn, v, v_stride, beta, log_decay, seq_start, W, U, tails, H, G, dim, vdim, min_len));
   RL_LAUNCH_CHECK(rl_launch(delta_chunk_walk_kernel<DP>, per_tile, 4 * DP, smem2, stream, kn, (const float*)tails, state, slot_ids, seq_start, (const float*)W, U, states,
-                            H, G, dim, vdim));
+                            H, G, dim, vdim, min_len));
   RL_LAUNCH_CHECK(rl_launch(delta_chunk_out_kernel<DP>, per_chunk, 256, smem3, stream, qn, kn, log_decay, seq_start, (const float*)U,
-                            (const float*)states, out, out_stride, H, G, dim, vdim));
+                            (const float*)states, out, out_stride, H, G, dim, vdim, min_len));
   return 0;
 }
 
 RL_API int rl_delta_chunked(const float* qn, const float* kn, const void* v, int v_stride, const float* beta, const float* log_decay, float* state,
                             const int* slot_ids, const int* seq_start, float* out, int out_stride, int n_tokens, int n_seqs, int max_q_len, int H,
-                            int G, int dim, int vdim, float* scratch, cudaStream_t stream) {
+                            int G, int dim, int vdim, int min_len, float* scratch, cudaStream_t stream) {
   if (n_tokens <= 0 || n_seqs <= 0 || max_q_len <= 0 || H <= 0 || G <= 0) RL_REFUSE(1, "delta_chunked: T=%d S=%d max_q=%d H=%d G=%d", n_tokens, n_seqs, max_q_len, H, G);
   if (!rl_delta_chunked_takes(dim, vdim)) RL_REFUSE(2, "delta_chunked: sizes %d / %d (multiples of 4, keys up to 128)", dim, vdim);
   if (H % G) RL_REFUSE(3, "delta_chunked: %d heads are not a multiple of %d q/k heads", H, G);
@@ -477,7 +478,7 @@ RL_API int rl_delta_chunked(const float* qn, const float* kn, const void* v, int
   if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)state | (uintptr_t)out | (uintptr_t)scratch) & 15) RL_REFUSE(6, "delta_chunked: operands must be 16-byte aligned");
   if (dim <= 64)
     return launch_delta_chunked<64>(qn, kn, (const bf16*)v, v_stride, beta, log_decay, state, slot_ids, seq_start, out, out_stride, n_tokens, n_seqs,
-                                    max_q_len, H, G, dim, vdim, scratch, stream);
+                                    max_q_len, H, G, dim, vdim, min_len, scratch, stream);
   return launch_delta_chunked<128>(qn, kn, (const bf16*)v, v_stride, beta, log_decay, state, slot_ids, seq_start, out, out_stride, n_tokens, n_seqs,
-                                   max_q_len, H, G, dim, vdim, scratch, stream);
+                                   max_q_len, H, G, dim, vdim, min_len, scratch, stream);
 }

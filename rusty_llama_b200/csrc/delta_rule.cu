@@ -17,8 +17,8 @@
 //                     meet; the partial sums of a column's row slices (lanes of one warp) are added by shuffles in a fixed
 //                     order, and u_t is folded into the read-out: o_t = (g S)^T q + u (k . q).  Prompts, parts of
 //                     prompts and single tokens run the same code, so a result's bits depend neither on how a sequence
-//                     was cut into steps nor on what else is in the batch.  (The prompts of a bfloat16 run go chunk by chunk
-//                     through delta_chunk.cu instead, equal within rounding.)
+//                     was cut into steps nor on what else is in the batch.  (Sequences that bring a prompt to a step of a bfloat16
+//                     run go chunk by chunk through delta_chunk.cu instead, equal within rounding.)
 #include "common.cuh"
 
 RL_DEFINE_ERROR_TEXT()
@@ -275,7 +275,7 @@ template <typename T>
 __global__ void delta_prep_kernel(const T* __restrict__ qk, int qk_stride, const T* __restrict__ ba, int ba_stride,
                                   const float* __restrict__ a_log, const float* __restrict__ dt_bias, float unit_eps, float q_scale,
                                   float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ kq, float* __restrict__ beta,
-                                  float* __restrict__ decay, int G, int H, int dim, int log_decay) {
+                                  float* __restrict__ decay, float* __restrict__ log_decay, int G, int H, int dim) {
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const T* row = qk + (size_t)t * qk_stride;
@@ -307,23 +307,24 @@ __global__ void delta_prep_kernel(const T* __restrict__ qk, int qk_stride, const
     const float z = to_f32(bar[H + h]) + dt_bias[h];
     const float sp = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
     const float l = -expf(a_log[h]) * sp;
-    decay[(size_t)t * H + h] = log_decay ? l : expf(l);
+    decay[(size_t)t * H + h] = expf(l);
+    if (log_decay != nullptr) log_decay[(size_t)t * H + h] = l;
   }
 }
 
 RL_API int rl_delta_prep(const void* qk, int dtype, int qk_stride, const void* ba, int ba_stride, const float* a_log, const float* dt_bias,
-                         float unit_eps, float q_scale, float* qn, float* kn, float* kq, float* beta, float* decay, int n_tokens, int G, int H,
-                         int dim, int log_decay, cudaStream_t stream) {
+                         float unit_eps, float q_scale, float* qn, float* kn, float* kq, float* beta, float* decay, float* log_decay, int n_tokens, int G,
+                         int H, int dim, cudaStream_t stream) {
   if (n_tokens <= 0 || G <= 0 || H <= 0 || dim <= 0) RL_REFUSE(1, "delta_prep: T=%d G=%d H=%d dim=%d", n_tokens, G, H, dim);
   if (qk_stride < 2 * G * dim || ba_stride < 2 * H) RL_REFUSE(2, "delta_prep: rows too short");
   int threads = 32 * (G < 8 ? G : 8);
   if (threads < 64) threads = 64;
   if (dtype == RL_BF16)
     delta_prep_kernel<bf16><<<n_tokens, threads, 0, stream>>>((const bf16*)qk, qk_stride, (const bf16*)ba, ba_stride, a_log, dt_bias, unit_eps,
-                                                              q_scale, qn, kn, kq, beta, decay, G, H, dim, log_decay);
+                                                              q_scale, qn, kn, kq, beta, decay, log_decay, G, H, dim);
   else if (dtype == RL_F32)
     delta_prep_kernel<float><<<n_tokens, threads, 0, stream>>>((const float*)qk, qk_stride, (const float*)ba, ba_stride, a_log, dt_bias, unit_eps,
-                                                               q_scale, qn, kn, kq, beta, decay, G, H, dim, log_decay);
+                                                               q_scale, qn, kn, kq, beta, decay, log_decay, G, H, dim);
   else
     RL_REFUSE(3, "delta_prep: unknown dtype %d", dtype);
   RL_LAUNCH_RESULT();
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(DR_COLS * DR_MAX_SLICES)
 delta_rule_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ kq, const T* __restrict__ v,
                   int v_stride, const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ state,
                   const int* __restrict__ slot_ids, const int* __restrict__ seq_start, float* __restrict__ out, int out_stride, int H, int G,
-                  int dim, int vdim, int P) {
+                  int dim, int vdim, int P, int max_len) {
   // two stages of DR_TOKENS tokens each: q [DR_TOKENS][skewed dim], k likewise, then per token beta, decay, k . q;
   // then v [2][DR_TOKENS][DR_COLS] as 32-bit numbers
   extern __shared__ __align__(16) float sm[];
@@ -369,6 +370,8 @@ delta_rule_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   const int col_l = tid / P, slice = tid - col_l * P;
   const int h = blockIdx.y, s = blockIdx.z, kh = h / (H / G);
   const int col = blockIdx.x * DR_COLS + col_l;
+  const int t0 = seq_start[s], t1 = seq_start[s + 1];
+  if (max_len > 0 && t1 - t0 > max_len) return;
   const bool col_ok = col < vdim;
   const int row0 = slice * DR_ROWS;
   const int padded = P * DR_ROWS;
@@ -382,7 +385,6 @@ delta_rule_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
   // rows past the key size stay zero in both stages for good (their state is zero and stays so)
   for (int i = tid; i < 2 * stage_floats; i += nthreads) sm[i] = 0.f;
   __syncthreads();
-  const int t0 = seq_start[s], t1 = seq_start[s + 1];
   auto stage_in = [&](int tb, int st) {  // the copies of up to DR_TOKENS tokens from tb on, asynchronously
     const int nt = min(DR_TOKENS, t1 - tb);
     float* base = sm + st * stage_floats;
@@ -485,9 +487,10 @@ delta_rule_kernel(const float* __restrict__ qn, const float* __restrict__ kn, co
     if (col_ok && row0 + r < dim) S_g[(size_t)(row0 + r) * vdim + col] = S[r];
 }
 
+// max_len: 0, or the most tokens of a sequence that is worked; longer ones (and their rows of out) are left alone.
 RL_API int rl_delta_rule(const float* qn, const float* kn, const float* kq, const void* v, int dtype, int v_stride, const float* beta,
                          const float* decay, float* state, const int* slot_ids, const int* seq_start, float* out, int out_stride, int n_seqs,
-                         int H, int G, int dim, int vdim, cudaStream_t stream) {
+                         int H, int G, int dim, int vdim, int max_len, cudaStream_t stream) {
   if (n_seqs <= 0 || H <= 0 || G <= 0 || dim <= 0 || vdim <= 0) RL_REFUSE(1, "delta_rule: S=%d H=%d G=%d dim=%d vdim=%d", n_seqs, H, G, dim, vdim);
   if (H % G) RL_REFUSE(2, "delta_rule: %d heads are not a multiple of %d q/k heads", H, G);
   int P = 1;
@@ -503,10 +506,10 @@ RL_API int rl_delta_rule(const float* qn, const float* kn, const float* kq, cons
   }
   if (dtype == RL_BF16)
     delta_rule_kernel<bf16><<<grid, block, smem, stream>>>(qn, kn, kq, (const bf16*)v, v_stride, beta, decay, state, slot_ids, seq_start, out,
-                                                           out_stride, H, G, dim, vdim, P);
+                                                           out_stride, H, G, dim, vdim, P, max_len);
   else if (dtype == RL_F32)
     delta_rule_kernel<float><<<grid, block, smem, stream>>>(qn, kn, kq, (const float*)v, v_stride, beta, decay, state, slot_ids, seq_start, out,
-                                                            out_stride, H, G, dim, vdim, P);
+                                                            out_stride, H, G, dim, vdim, P, max_len);
   else
     RL_REFUSE(6, "delta_rule: unknown dtype %d", dtype);
   RL_LAUNCH_RESULT();

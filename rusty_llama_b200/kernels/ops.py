@@ -2214,7 +2214,8 @@ def delta_prep(
 ):
     """What the gated delta rule's recurrence takes, all float32: qk [T, 2 G dim] rows (G q heads, then G k heads) -> unit vectors
     qn (times q_scale) and kn [T, G dim], their products kq [T, G]; ba [T, >= 2 H] rows (b, then a) -> beta = logistic(b) and
-    decay = exp(-exp(a_log) softplus(a + dt_bias)) (log_decay: its logarithm), both [T, H]."""
+    decay = exp(-exp(a_log) softplus(a + dt_bias)), both [T, H].  Returns (qn, kn, kq, beta, decay) and, with log_decay, the decay's
+    logarithm behind them."""
     _cuda(qk, "delta_prep qk", contiguous=False)
     _cuda(ba, "delta_prep ba", qk.dtype, contiguous=False)
     T = qk.shape[0]
@@ -2226,23 +2227,26 @@ def delta_prep(
     f32 = dict(dtype=torch.float32, device=qk.device)
     qn, kn = torch.empty((T, G * dim), **f32), torch.empty((T, G * dim), **f32)
     kq, beta, decay = torch.empty((T, G), **f32), torch.empty((T, H), **f32), torch.empty((T, H), **f32)
+    log = torch.empty((T, H), **f32) if log_decay else None
     lib = build.load("delta_rule")
     rc = lib.rl_delta_prep(
         _p(qk), c_int(_dt(qk, "delta_prep")), c_int(_rows(qk, "delta_prep qk")), _p(ba), c_int(_rows(ba, "delta_prep ba")), _p(a_log), _p(dt_bias),
-        c_float(unit_eps), c_float(q_scale), _p(qn), _p(kn), _p(kq), _p(beta), _p(decay), c_int(T), c_int(G), c_int(H), c_int(dim),
-        c_int(1 if log_decay else 0), _stream(),
+        c_float(unit_eps), c_float(q_scale), _p(qn), _p(kn), _p(kq), _p(beta), _p(decay), _p(log), c_int(T), c_int(G), c_int(H),
+        c_int(dim), _stream(),
     )
     _check(lib, rc, "delta_prep")
-    return qn, kn, kq, beta, decay
+    return (qn, kn, kq, beta, decay, log) if log_decay else (qn, kn, kq, beta, decay)
 
 
 def delta_rule(
     qn: torch.Tensor, kn: torch.Tensor, kq: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
-    slot_ids: torch.Tensor, seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int,
+    slot_ids: torch.Tensor, seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int, max_len: int = 0,
+    out: Optional[torch.Tensor] = None,
 ) -> torch.Tensor:
     """The gated delta rule through the sequences' states, token by token: S <- g S; u = beta (v - S^T k); S <- S + k u^T;
     o = S^T q.  qn, kn: float32 [T, G dim]; kq = k . q: float32 [T, G]; v: [T, H vdim] rows of the run's type; beta, decay:
-    float32 [T, H]; state: float32 [slots, H, dim, vdim].  Head h reads q/k head h // (H / G).  Returns float32 [T, H vdim]."""
+    float32 [T, H]; state: float32 [slots, H, dim, vdim].  Head h reads q/k head h // (H / G).  Returns float32 [T, H vdim].
+    max_len: 0, or sequences of more tokens than this are left alone, states and rows of `out` (made if not given) alike."""
     T = qn.shape[0]
     H, G = num_heads, num_qk_heads
     for name, t, n in (("qn", qn, G * dim), ("kn", kn, G * dim), ("kq", kq, G), ("beta", beta, H), ("decay", decay, H)):
@@ -2260,11 +2264,14 @@ def delta_rule(
     _cuda(seq_start, "delta_rule seq_start", torch.int32)
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "delta_rule: seq_start must hold one more entry than there are sequences")
-    out = torch.empty((T, H * vdim), dtype=torch.float32, device=qn.device)
+    if out is None:
+        out = torch.empty((T, H * vdim), dtype=torch.float32, device=qn.device)
+    _cuda(out, "delta_rule out", torch.float32)
+    _need(tuple(out.shape) == (T, H * vdim), "delta_rule: out must be [T, H vdim]")
     lib = build.load("delta_rule")
     rc = lib.rl_delta_rule(
         _p(qn), _p(kn), _p(kq), _p(v), c_int(_dt(v, "delta_rule v")), c_int(_rows(v, "delta_rule v")), _p(beta), _p(decay), _p(state), _p(slot_ids),
-        _p(seq_start), _p(out), c_int(out.stride(0)), c_int(S), c_int(H), c_int(G), c_int(dim), c_int(vdim), _stream(),
+        _p(seq_start), _p(out), c_int(out.stride(0)), c_int(S), c_int(H), c_int(G), c_int(dim), c_int(vdim), c_int(max_len), _stream(),
     )
     _check(lib, rc, "delta_rule")
     return out
@@ -2283,10 +2290,11 @@ def delta_chunked_scratch_floats(n_tokens: int, n_seqs: int, num_heads: int, dim
 
 def delta_chunked(
     qn: torch.Tensor, kn: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log_decay: torch.Tensor, state: torch.Tensor, slot_ids: torch.Tensor,
-    seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int, max_q_len: int, scratch: torch.Tensor,
+    seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int, max_q_len: int, scratch: torch.Tensor, min_len: int = 1,
 ) -> torch.Tensor:
     """`delta_rule` chunk by chunk, for prompts of bfloat16 runs: the same result within 32-bit rounding.  log_decay: float32 [T, H], the
-    logarithms of the decays; v: bfloat16 rows; scratch: float32, `delta_chunked_scratch_floats` numbers."""
+    logarithms of the decays; v: bfloat16 rows; scratch: float32, `delta_chunked_scratch_floats` numbers.  Sequences of fewer than min_len
+    tokens are left alone, and their rows of the result undefined."""
     T, H, G = qn.shape[0], num_heads, num_qk_heads
     for name, t, n in (("qn", qn, G * dim), ("kn", kn, G * dim), ("beta", beta, H), ("log_decay", log_decay, H)):
         _cuda(t, "delta_chunked rows", torch.float32)
@@ -2307,7 +2315,7 @@ def delta_chunked(
     lib = build.load("delta_chunk")
     rc = lib.rl_delta_chunked(
         _p(qn), _p(kn), _p(v), c_int(_rows(v, "delta_chunked v")), _p(beta), _p(log_decay), _p(state), _p(slot_ids), _p(seq_start), _p(out), c_int(out.stride(0)),
-        c_int(T), c_int(S), c_int(max_q_len), c_int(H), c_int(G), c_int(dim), c_int(vdim), _p(scratch), _stream(),
+        c_int(T), c_int(S), c_int(max_q_len), c_int(H), c_int(G), c_int(dim), c_int(vdim), c_int(min_len), _p(scratch), _stream(),
     )
     _check(lib, rc, "delta_chunked", kernels=3)
     return out

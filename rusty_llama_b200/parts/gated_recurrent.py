@@ -24,7 +24,8 @@ from ..kernels import ops
 from ..kernels.linear import linear, linear_to_stream
 from .base import MIXERS, Mixer, ParamInfo, StateNeed, scratch_for_call
 
-# prompt steps whose longest sequence brings fewer tokens than this go token by token like a decode step
+# prompt steps whose longest sequence brings fewer tokens than this go token by token like a decode step; with the delta rule every sequence
+# that brings fewer does
 _CHUNKED_MIN_TOKENS = 32
 # the most scratch that the delta rule's chunks may take (2 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it, and where the
 # device has less, token by token
@@ -321,13 +322,15 @@ class GatedDeltaRule(Mixer):
             if floats <= _CHUNKED_MAX_FLOATS:
                 scratch = scratch_for_call(floats, torch.float32, xn.device)
         chunked = scratch is not None
-        qn, kn, kq, beta, decay = ops.delta_prep(conv[:, : 2 * self.qd], ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps, self.q_scale,
-                                                 log_decay=chunked)
-        if chunked:  # a prompt of a bfloat16 run, all chunks side by side but for the walk through the state
-            o = ops.delta_chunked(qn, kn, conv[:, 2 * self.qd :], beta, decay, memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim,
-                                  step.max_q_len, scratch)
-        else:
-            o = ops.delta_rule(qn, kn, kq, conv[:, 2 * self.qd :], beta, decay, memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim)
+        qn, kn, kq, beta, decay, *log = ops.delta_prep(conv[:, : 2 * self.qd], ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps,
+                                                       self.q_scale, log_decay=chunked)
+        v, o = conv[:, 2 * self.qd :], None
+        where = (memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim)
+        if chunked:  # prompts of a bfloat16 run, all chunks side by side but for the walk through the state
+            o = ops.delta_chunked(qn, kn, v, beta, *log, *where, step.max_q_len, scratch, min_len=_CHUNKED_MIN_TOKENS)
+        if not chunked or min(step.q_lens) < _CHUNKED_MIN_TOKENS:
+            # (a sequence's own length decides: its bits do not depend on whether a prompt shares the step)
+            o = ops.delta_rule(qn, kn, kq, v, beta, decay, *where, max_len=_CHUNKED_MIN_TOKENS - 1 if chunked else 0, out=o)
         a = ops.head_norm_gate(o, H, self.vdim, self.w_norm, self.eps, gate, ops.GATE_SILU, xn.dtype, out_scale=self.out_scale, out=out)
         return a, self.w_o
 

@@ -209,3 +209,49 @@ def test_a_prompt_without_room_for_the_chunks_goes_token_by_token():
     got = with_memory_left(scratch, run)  # (the rest of the layer takes some 60 MB of these 75)
     want = run()
     assert float((got - want).norm() / want.norm()) < 1e-2
+
+
+def test_a_short_sequence_gets_the_token_kernels_bits_beside_a_prompt():
+    """Which kernel takes a sequence's tokens depends on its own length: beside a prompt a single token and a short portion keep the bits
+    that they have alone."""
+    from rusty_llama_b200.cache import Cache
+    from rusty_llama_b200.kernels import ops
+
+    from test_parts import ctx_for
+
+    part = layer(4, 2, 32, 48, 64)
+    lens = [1, 100, 31, 64, 5]
+    cache = Cache([(0, part.cache_need())], 64, len(lens), torch.bfloat16, DEV)
+    slots = [cache.open_sequence() for _ in lens]
+    x = torch.randn(sum(lens), 64, generator=torch.Generator().manual_seed(4)).to(torch.bfloat16).to(DEV)
+    step, tables = ctx_for(cache, slots, [0] * len(lens), lens)
+    view = cache.view(0, tables)
+    records = next(v.state for v in (view if isinstance(view, tuple) else (view,)) if v.state.dim() == 4)
+    records.normal_(generator=torch.Generator(device=DEV).manual_seed(3))
+    start, seen = records.clone(), {}
+    spied = {name: getattr(ops, name) for name in ("delta_prep", "short_conv", "head_norm_gate")}
+
+    def spy(name):
+        def call(*a, **k):
+            seen[name] = (a, k, spied[name](*a, **k))
+            return seen[name][2]
+        return call
+
+    try:
+        for name in spied:
+            setattr(ops, name, spy(name))
+        part.forward(x, step, view)
+    finally:
+        for name, f in spied.items():
+            setattr(ops, name, f)
+    a, k, _ = seen["delta_prep"]
+    qn, kn, kq, beta, decay = spied["delta_prep"](*a, **dict(k, log_decay=False))
+    alone = ops.delta_rule(qn, kn, kq, seen["short_conv"][2][:, 2 * part.qd :], beta, decay, start, step.slot_ids, step.seq_start, 4, 2, 32, 48)
+    o, at = seen["head_norm_gate"][0][0], 0
+    for i, n in enumerate(lens):
+        same = torch.equal(o[at : at + n], alone[at : at + n]) and torch.equal(records[slots[i]], start[slots[i]])
+        if n < 32:
+            assert same, f"{n} tokens"
+        else:
+            assert float((o[at : at + n] - alone[at : at + n]).norm() / alone[at : at + n].norm()) < 1e-5
+        at += n
