@@ -1228,11 +1228,15 @@ def head_linear(
     return out
 
 
-def latent_expand(pages: torch.Tensor, block_table: torch.Tensor, seq_len: torch.Tensor, seq_rows: int, w_vk: torch.Tensor, rot: int) -> torch.Tensor:
+def latent_expand(
+    pages: torch.Tensor, block_table: torch.Tensor, seq_len: torch.Tensor, seq_rows: int, w_vk: torch.Tensor, rot: int,
+    latents: Optional[torch.Tensor] = None, kv: Optional[torch.Tensor] = None,
+) -> torch.Tensor:
     """Keys and values of every head for the positions that the sequences hold, bfloat16 [S * seq_rows, H, vdim + dim + rot]: row
     (s, j) holds position j of sequence s, a head's value and plain key part = w_vk[h] (rows: vdim, then dim) . latent, then the turned
     key part that all heads share.  Rows a sequence does not hold are zeros up to a multiple of 64 and undefined behind it.
-    pages [pages, 1, PAGE_SIZE, rank + rot]; seq_rows: a multiple of 64, at least every sequence's length."""
+    pages [pages, 1, PAGE_SIZE, rank + rot]; seq_rows: a multiple of 64, at least every sequence's length; latents: scratch
+    [S * seq_rows, rank]; kv: where the result goes (both made if not given)."""
     _cuda(pages, "latent_expand pages", torch.bfloat16)
     _cuda(block_table, "latent_expand block_table", torch.int32)
     _cuda(seq_len, "latent_expand seq_len", torch.int32)
@@ -1242,8 +1246,13 @@ def latent_expand(pages: torch.Tensor, block_table: torch.Tensor, seq_len: torch
     if not (pages.dim() == 4 and tuple(pages.shape[1:]) == (1, PAGE_SIZE, rank + rot) and seq_len.numel() == S):
         raise KernelError(f"latent_expand: pages {tuple(pages.shape)} and {seq_len.numel()} lengths for {S} sequences of latents of {rank} + {rot}")
     rows = S * seq_rows
-    latents = torch.empty((rows, rank), dtype=pages.dtype, device=pages.device)
-    kv = torch.empty((rows, H, n + rot), dtype=pages.dtype, device=pages.device)
+    if latents is None:
+        latents = torch.empty((rows, rank), dtype=pages.dtype, device=pages.device)
+    if kv is None:
+        kv = torch.empty((rows, H, n + rot), dtype=pages.dtype, device=pages.device)
+    _cuda(latents, "latent_expand latents", torch.bfloat16)
+    _cuda(kv, "latent_expand kv", torch.bfloat16)
+    _need(tuple(latents.shape) == (rows, rank) and tuple(kv.shape) == (rows, H, n + rot), "latent_expand: latents or kv of the wrong size")
     lib = build.load("latent_attention")
     rc = lib.rl_latent_rows(
         _p(pages), _p(block_table), c_int(width), _p(seq_len), c_int(S), c_int(seq_rows), _p(latents), _p(kv), c_int(H), c_int(n + rot), c_int(n),

@@ -11,7 +11,7 @@ from ..kernels import ops
 from ..kernels.device import sm_count
 from ..kernels.linear import linear, linear_to_stream
 from ..spec import PartSpec
-from .base import MIXERS, POSITIONS, KVNeed, Mixer, ParamInfo
+from .base import MIXERS, POSITIONS, KVNeed, Mixer, ParamInfo, scratch_for_call
 
 # A step may expand keys and values per head from so many tokens on (above the head products' few-row form), if the rows fit so many bytes
 # for the call.
@@ -189,10 +189,14 @@ class LatentAttention(Mixer):
             # the queries' latent is normed beside the row that is cached; the queries exist after the product with it
             c_q = ops.latent_prep(None, kv, self.w_norm, self.eps, *turn, None, *sizes, q_latent=q, q_norm=self.w_q_norm)
             q, kv = linear(c_q, self.w_uq), None
-        seq_rows = self._expands(step, q, g)
-        if seq_rows:
+        seq_rows, latents, expanded = self._expands(step, q, g), None, None
+        if seq_rows:  # (asked for before anything is done in place; without room for both the step works on the latents)
+            rows = step.n_seqs * seq_rows
+            latents = scratch_for_call((rows, self.rank), xn.dtype, xn.device)
+            expanded = scratch_for_call((rows, self.H, self.vdim + self.dim + self.rot), xn.dtype, xn.device)
+        if latents is not None and expanded is not None:
             ops.latent_prep(q, kv, self.w_norm, self.eps, *turn, None, *sizes, in_place=True)
-            expanded = ops.latent_expand(cache.k_pages, cache.block_table, step.seq_len, seq_rows, self.w_vk, self.rot)
+            ops.latent_expand(cache.k_pages, cache.block_table, step.seq_len, seq_rows, self.w_vk, self.rot, latents, expanded)
             a = ops.flash_expanded(q, expanded, seq_rows, step.seq_start, step.seq_pos0, step.max_q_len, self.vdim, self.window, self.scale,
                                    sink=self.sink, gate=g)
             return a, self.w_o

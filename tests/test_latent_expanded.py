@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from test_parts import ctx_for
-from test_waits import expect_give_up
+from test_waits import expect_give_up, with_memory_left
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -162,3 +162,27 @@ def test_expanding_loses_nothing_against_64_bits(H, dim, rot, vdim, rank):
             module._EXPAND_MIN_TOKENS = before
         off.append(float((a.double().cpu() - want).norm() / want.norm()))
     assert off[0] <= off[1], off
+
+
+def test_a_step_without_room_for_the_rows_works_on_the_latents():
+    import rusty_llama_b200.parts.latent_attention as module
+    from rusty_llama_b200.cache import Cache
+
+    part, w = make(16, 128, 64, 128, 512, 96)
+    held, n = 8000, 256
+    cache = Cache([(0, part.cache_need())], 64 * 130, 1, torch.bfloat16, DEV)
+    cache.kv_groups[0].k.normal_(generator=torch.Generator(device=DEV).manual_seed(1))
+    slot = cache.open_sequence()
+    cache.reserve([slot], [held])
+    cache.commit([slot], [held])
+    step, tables = ctx_for(cache, [slot], [held], [n])
+    x = torch.randn(n, 96, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).to(DEV)
+    run = lambda: part.forward(x, step, cache.view(0, tables))  # noqa: E731
+    before, module._EXPAND_MIN_TOKENS = module._EXPAND_MIN_TOKENS, 10**9
+    try:
+        want = run()
+    finally:
+        module._EXPAND_MIN_TOKENS = before
+    assert part._expands(step, torch.empty(1, 8, device=DEV, dtype=torch.bfloat16), None)
+    scratch = 2 * (held + n) * (16 * 320 + 512)
+    assert torch.equal(with_memory_left(scratch - (8 << 20), run), want)
