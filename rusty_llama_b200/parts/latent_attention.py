@@ -87,6 +87,9 @@ class LatentAttention(Mixer):
         self.n_pairs = rotary_dim // 2
         self.magnitude = float(getattr(self.position, "magnitude", 1.0))
         self.qd, self.vd, self.kvd = self.H * (self.dim + self.rot), self.H * self.vdim, self.rank + self.rot
+        # halves of operations a head, in those of the head products: a row to expand, and a pair that need not be taken on the latents (`_expands`)
+        self.row_costs = self.rank * (self.dim + self.vdim)
+        self.pair_saves = _LATENT_OPERATION * (2 * self.rank + self.rot) - _EXPANDED_OPERATION * (self.dim + self.rot + self.vdim)
         self.w_in = self.w_o = self.w_ukT = self.w_uv = self.w_vk = self.w_norm = self.sink = self.w_uq = self.w_q_norm = None
 
     def cache_need(self):
@@ -165,14 +168,14 @@ class LatentAttention(Mixer):
             return 0
         # (a caller that does not say what each sequence held: what they all held if they are equally long)
         pos0 = step.pos0 if step.pos0 is not None else [step.max_kv_len - step.max_q_len] * step.n_seqs
-        earlier = pairs = 0
+        earlier = sum(pos0)
+        if earlier == 0 and self.pair_saves > 0:
+            return seq_rows
+        pairs = 0
         for p, n in zip(pos0, step.q_lens):
-            earlier += p
             growing = min(n, max(self.window - p, 0)) if self.window else n  # tokens that the window does not cut short
             pairs += growing * p + growing * (growing + 1) // 2 + (n - growing) * self.window
-        a_row = self.rank * (self.dim + self.vdim)
-        a_pair = _LATENT_OPERATION * (2 * self.rank + self.rot) - _EXPANDED_OPERATION * (self.dim + self.rot + self.vdim)
-        return seq_rows if earlier * a_row <= a_pair * pairs else 0
+        return seq_rows if earlier * self.row_costs <= self.pair_saves * pairs else 0
 
     def forward_unprojected(self, xn: torch.Tensor, step, cache, shared_cache: bool = False):
         if shared_cache == self.own_kv:
