@@ -311,6 +311,13 @@ static cudaError_t rl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Streaming multiprocessors of the current device (0: it cannot be asked).
+static inline int rl_sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  return sms;
+}
+
 #define RL_LAUNCH_CHECK(expr)                                                      \
   do {                                                                             \
     cudaError_t rl_e = (expr);                                                     \

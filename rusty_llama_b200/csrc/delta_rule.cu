@@ -243,7 +243,7 @@ RL_API int rl_short_conv(const void* x, int dtype, int x_stride, const float* w,
 #define RL_CONV_RUNS(TAPS)                                                                                                             \
   RL_LAUNCH_CHECK(rl_launch(short_conv_runs_kernel<TAPS>, (int)((runs + 127) / 128), 128, 0, stream, (const bf16*)x, x_stride, w, bias, \
                             (const float*)state, slot_ids, seq_start, tok_seq, (bf16*)out, out_stride, n_tokens, C, silu))
-    if (rows8 && taps <= CONV_ROW_TAPS && runs >= 2 * 148 * 128 && runs < (1LL << 31)) {
+    if (rows8 && taps <= CONV_ROW_TAPS && runs >= 2LL * 128 * rl_sm_count() && runs < (1LL << 31)) {
       if (taps == 1) RL_CONV_RUNS(1);
       else if (taps == 2) RL_CONV_RUNS(2);
       else if (taps == 3) RL_CONV_RUNS(3);

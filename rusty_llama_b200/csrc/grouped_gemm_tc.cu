@@ -421,9 +421,8 @@ static int launch_grouped(const void* w, const void* w2, int matrices, void* out
   auto kern = grouped_gemm_tc_kernel<TO, EPI, NT>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::SMEM_BYTES) != cudaSuccess)
     RL_REFUSE(5, "grouped_gemm_tc: cannot get %d bytes of shared memory", SH::SMEM_BYTES);
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    RL_REFUSE(10, "grouped_gemm_tc: cannot count the SMs");
+  const int sms = rl_sm_count();
+  if (sms <= 0) RL_REFUSE(10, "grouped_gemm_tc: cannot count the SMs");
   const int unit_n = EPI == GATED ? FEATURES / 2 : FEATURES;
   const long long units = max_groups * ((g.N + unit_n - 1) / unit_n);
   if (units > 0x7fffffffLL) RL_REFUSE(11, "grouped_gemm_tc: too many units of work");
@@ -467,8 +466,9 @@ RL_API int rl_moe_gather_rows(const void* x, int ldx, int x_rows, const int* ord
                               cudaStream_t stream) {
   if (n_rows <= 0 || K <= 0 || gather_div <= 0 || x_rows <= 0) RL_REFUSE(1, "moe_gather_rows: rows=%d of %d k=%d div=%d", n_rows, x_rows, K, gather_div);
   if (K % 8 || ldx % 8 || (((uintptr_t)x | (uintptr_t)out) & 15)) RL_REFUSE(3, "moe_gather_rows: k = %d or a row stride of %d elements breaks 16-byte alignment", K, ldx);
-  const int blocks = (n_rows + 7) / 8;
-  RL_LAUNCH_CHECK(rl_launch(moe_gather_rows_kernel, dim3(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, stream, (const uint4*)x, (long long)ldx / 8, x_rows,
+  const int blocks = (n_rows + 7) / 8, most = 8 * rl_sm_count();
+  if (most <= 0) RL_REFUSE(10, "moe_gather_rows: cannot count the SMs");
+  RL_LAUNCH_CHECK(rl_launch(moe_gather_rows_kernel, dim3(blocks < most ? blocks : most), 256, 0, stream, (const uint4*)x, (long long)ldx / 8, x_rows,
                             order, gather_div, (uint4*)out, n_rows, K / 8));
   return 0;
 }
