@@ -65,7 +65,8 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))  # (without making a Stream object)
+    # (without making a Stream object: 0.3 us a launch, `torch.cuda.current_stream().cuda_stream` takes 3.3)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 _launches = 0
@@ -132,11 +133,11 @@ def add_rmsnorm(
     delta_dt = _DT[act_dtype]
     if delta is not None:
         _cuda(delta, "add_rmsnorm delta")
-        if not (delta.dtype in (act_dtype, torch.float32)):
+        if delta.dtype not in (act_dtype, torch.float32):
             raise KernelError(f"add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
         delta_dt = _DT[delta.dtype]
         if delta.dim() == 2:
-            if not (tuple(delta.shape) == (T, d)):
+            if tuple(delta.shape) != (T, d):
                 raise KernelError(f"add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
             n_parts = 1
         else:
@@ -150,7 +151,7 @@ def add_rmsnorm(
     w_dt = _F32
     if weight is not None:
         _cuda(weight, "add_rmsnorm weight")
-        if not (tuple(weight.shape) == (d,)):
+        if tuple(weight.shape) != (d,):
             raise KernelError(f"add_rmsnorm: weight {tuple(weight.shape)} does not match d={d}")
         w_dt = _dt(weight, "add_rmsnorm weight")
         if out is None:
@@ -165,7 +166,7 @@ def add_rmsnorm(
     if n_rows == 0:
         return out
     for name, t in (("x", x), ("delta", delta), ("weight", weight), ("out", out)):
-        if not (t is None or t.data_ptr() % 16 == 0):
+        if t is not None and t.data_ptr() % 16 != 0:
             raise KernelError(f"add_rmsnorm: {name} is not 16-byte aligned")
     lib = build.load("elementwise")
     rc = lib.rl_add_rmsnorm(
@@ -205,7 +206,7 @@ def seq_begin_decode(state: torch.Tensor, slot_ids: torch.Tensor, tok_pos: torch
     S = slot_ids.numel()
     for name, t in (("slot_ids", slot_ids), ("tok_pos", tok_pos), ("seq_pos0", seq_pos0), ("seq_len", seq_len)):
         _cuda(t, f"seq_begin_decode {name}", torch.int32)
-        if not (t.numel() == S):
+        if t.numel() != S:
             raise KernelError(f"seq_begin_decode: {name} has {t.numel()} entries for {S} sequences")
     lib = build.load("elementwise")
     rc = lib.rl_seq_begin_decode(_p(state), _p(slot_ids), c_int(S), _p(tok_pos), _p(seq_pos0), _p(seq_len), _stream())
@@ -325,7 +326,7 @@ def attn_tma_takes(kdim: int, vdim: int) -> bool:
 def _check_sink(sink, num_heads: int, what: str) -> None:
     if sink is not None:
         _cuda(sink, f"{what} sink", torch.float32)
-        if not (sink.numel() == num_heads):
+        if sink.numel() != num_heads:
             raise KernelError(f"{what}: one sink per head")
 
 
@@ -403,7 +404,7 @@ def attn_decode(
     _need(block_table.dim() == 2 and block_table.shape[0] >= S and seq_len.numel() == S, "attn_decode: metadata sizes")
     _cuda(scratch, "attn_decode scratch", torch.float32)
     need = attn_decode_scratch_floats(S, num_heads, vdim, n_splits)
-    if not (scratch.numel() >= need):
+    if scratch.numel() < need:
         raise KernelError(f"attn_decode: scratch holds {scratch.numel()} floats, {need} needed")
     if out is None:
         out = torch.empty((S, num_heads // maps * vdim), dtype=act, device=q.device)
@@ -414,11 +415,11 @@ def attn_decode(
     n_o = S * num_heads * n_splits * vdim
     part_o = c_void_p(scratch.data_ptr())
     part_ml = c_void_p(scratch.data_ptr() + 4 * n_o)
-    if not (impl in ("auto", "warp", "tma")):
+    if impl not in ("auto", "warp", "tma"):
         raise KernelError(f"attn_decode: unknown impl {impl!r}")
     if impl == "auto":
         impl = "tma" if (act == torch.bfloat16 and (head_dim in ATTN_DECODE_TMA_HEAD_DIMS or vdim != head_dim)) else "warp"
-    if not (fuse in (0, 1, 2)):
+    if fuse not in (0, 1, 2):
         raise KernelError(f"attn_decode: fuse={fuse}")
     if fuse:
         _need(impl == "tma", "attn_decode: only the TMA kernel fuses the position encoding")
@@ -431,7 +432,7 @@ def attn_decode(
         _need(impl == "tma", "attn_decode: only the TMA kernel adds the splits up itself")
         _cuda(counters, "attn_decode counters", torch.int32)
         groups = num_kv_heads * ((num_heads // num_kv_heads + 7) // 8)
-        if not (counters.numel() >= S * groups):
+        if counters.numel() < S * groups:
             raise KernelError(f"attn_decode: {counters.numel()} counters, {S * groups} needed")
     _need(q_parts is None or impl == "tma", "attn_decode: only the TMA kernel takes partial sums")
     _check_sink(sink, num_heads, "attn_decode")
@@ -515,7 +516,7 @@ def flash_prefill_tc(
     if not (maps in (1, 2) and num_heads % maps == 0):
         raise KernelError(f"flash_prefill_tc: {maps} maps in {num_heads} heads")
     vdim = value_dim or head_dim
-    if not (attn_tma_takes(head_dim, vdim)):
+    if not attn_tma_takes(head_dim, vdim):
         raise KernelError(f"flash_prefill_tc: key and value sizes {head_dim} / {vdim}, this kernel is built for multiples of 8 up to 128")
     _cuda(q, "flash_prefill_tc q", torch.bfloat16, contiguous=False)
     qs = _rows(q, "flash_prefill_tc q")
@@ -558,7 +559,7 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     ldx, ldw = _rows(x, "gemm_f32 x"), _rows(w, "gemm_f32 w")
     M, K = x.shape
     N = w.shape[0]
-    if not (w.shape[1] == K):
+    if w.shape[1] != K:
         raise KernelError(f"gemm_f32: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=x.device)
@@ -601,7 +602,7 @@ def gemm_bf16_any(
     ldx, ldw = _rows(x, "gemm_bf16_any x"), _rows(w, "gemm_bf16_any w")
     M, K = x.shape
     N = w.shape[0]
-    if not (w.shape[1] == K):
+    if w.shape[1] != K:
         raise KernelError(f"gemm_bf16_any: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     out = torch.empty((M, N // 2 if swiglu else N), dtype=out_dtype, device=x.device)
     lib = build.load("gemm_f32")
@@ -629,7 +630,7 @@ def gemv_bf16(
     ldx, ldw = _rows(x, "gemv_bf16 x"), _rows(w, "gemv_bf16 w")
     M, K = x.shape
     N = w.shape[0]
-    if not (w.shape[1] == K):
+    if w.shape[1] != K:
         raise KernelError(f"gemv_bf16: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     _need(x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0, "gemv_bf16: operands must be 16-byte aligned")
     n_out = N // 2 if swiglu else N
@@ -684,7 +685,7 @@ def gemv_stream_into_stream(
         raise KernelError(f"gemv_stream_into_stream: x{tuple(x.shape)} w{tuple(w.shape)} resid{tuple(resid.shape)} next_w{tuple(next_w.shape)} do not fit")
     lib = build.load("gemv_stream")
     blocks = int(lib.rl_gemv_stream_blocks(c_int(N), c_int(K)))
-    if not (blocks > 0):
+    if blocks <= 0:
         raise KernelError(f"gemv_stream_into_stream: the kernel does not take N={N}, K={K}")
     if xw is None:
         xw = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
@@ -701,7 +702,7 @@ def gemv_stream_into_stream(
         c_int(_rows(xw, "gemv_stream_into_stream xw")), _p(sumsq), c_int(M), c_int(N), c_int(K), ctypes.byref(used), _p(status), *_wt(), _stream(),
     )
     _check(lib, rc, "gemv_stream_into_stream")
-    if not (used.value == blocks):
+    if used.value != blocks:
         raise KernelError(f"gemv_stream_into_stream: the kernel ran {used.value} blocks, the wrapper planned {blocks}")
     return xw, sumsq, blocks
 
@@ -724,7 +725,7 @@ def gemv_stream(
     ldx, ldw = _rows(x, "gemv_stream x"), _rows(w, "gemv_stream w")
     M, K = x.shape
     N = w.shape[0]
-    if not (w.shape[1] == K):
+    if w.shape[1] != K:
         raise KernelError(f"gemv_stream: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     n_out = N // 2 if swiglu else N
     used = c_int(1)
@@ -732,7 +733,7 @@ def gemv_stream(
           "gemv_stream: an activation of one argument goes with a plain product and whole sums")
     _need(act not in GATED_ACTS or swiglu, "gemv_stream: a gate's activation goes with a gate/up product")
     slices = max(1, gemv_stream_slices(M, K, k_splits))  # (0: the launcher says what it does not take)
-    if not (k_splits > 1 or slices == 1):
+    if k_splits <= 1 and slices != 1:
         raise KernelError(f"gemv_stream: k = {K} comes in {slices} slices, whose float32 partial sums have to be asked for (k_splits > 1)")
     if k_splits > 1 and slices > 1:
         _need(out is None and out_dtype == torch.float32 and not swiglu, "gemv_stream: partial sums over k slices are float32, without activation")
@@ -761,7 +762,7 @@ def gemv_stream(
         c_int(M), c_int(N), c_int(K), c_int(1 if swiglu else 0), *_act(act), c_int(k_splits), ctypes.byref(used), _p(status), *_wt(), _stream(),
     )
     _check(lib, rc, "gemv_stream")
-    if not (used.value == slices):
+    if used.value != slices:
         raise KernelError(f"gemv_stream: kernel used {used.value} slices, the wrapper planned {slices}")
     return out
 
@@ -848,7 +849,7 @@ def gemm_tc(
     ldx, ldw = _rows(x, "gemm_tc x"), _rows(w, "gemm_tc w")
     M, K = x.shape
     N = w.shape[0]
-    if not (w.shape[1] == K):
+    if w.shape[1] != K:
         raise KernelError(f"gemm_tc: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     n_out = N // 2 if swiglu else N
     used = c_int(1)
@@ -873,7 +874,7 @@ def gemm_tc(
     )
     _check(lib, rc, "gemm_tc")
     if k_splits > 1:
-        if not (used.value == k_splits):
+        if used.value != k_splits:
             raise KernelError(f"gemm_tc: kernel used {used.value} slices, the wrapper planned {k_splits}")
     return out
 
@@ -908,7 +909,7 @@ def sample(
     _cuda(rng_index, "sample rng_index", torch.int32)
     _need(rng_index.numel() == R, "sample: one random-state index per row")
     _cuda(scratch, "sample scratch", torch.float32)
-    if not (scratch.numel() >= R * n):
+    if scratch.numel() < R * n:
         raise KernelError(f"sample: scratch holds {scratch.numel()} floats, {R * n} needed")
     if out is None:
         out = torch.empty((R,), dtype=torch.int32, device=logits.device)
@@ -957,7 +958,7 @@ def sample_chain(
         raise KernelError(f"sample_chain: history must be [slots, {SAMPLE_HISTORY_MAX}] with one count per slot")
     _cuda(work, "sample_chain work", torch.float32)
     need = R * 2 * ((n + 3) // 4 * 4)
-    if not (work.numel() >= need):
+    if work.numel() < need:
         raise KernelError(f"sample_chain: work holds {work.numel()} floats, {need} needed")
     _need(work.data_ptr() % 16 == 0, "sample_chain: work must be 16-byte aligned")
     if out is None:
@@ -998,10 +999,10 @@ def normed_add_rmsnorm(
     _cuda(x, "normed_add_rmsnorm x", torch.float32)
     T, d = x.shape
     _cuda(delta, "normed_add_rmsnorm delta")
-    if not (delta.dtype in (act_dtype, torch.float32)):
+    if delta.dtype not in (act_dtype, torch.float32):
         raise KernelError(f"normed_add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
     if delta.dim() == 2:
-        if not (tuple(delta.shape) == (T, d)):
+        if tuple(delta.shape) != (T, d):
             raise KernelError(f"normed_add_rmsnorm: delta {tuple(delta.shape)} does not match x {(T, d)}")
         n_parts, part_stride = 1, 0
     else:
@@ -1049,7 +1050,7 @@ def gated_add_rmsnorm(
     n_parts, part_stride, delta_dt = 0, 0, _DT[act_dtype]
     if delta is not None:
         _cuda(delta, "gated_add_rmsnorm delta")
-        if not (delta.dtype in (act_dtype, torch.float32)):
+        if delta.dtype not in (act_dtype, torch.float32):
             raise KernelError(f"gated_add_rmsnorm: delta is {delta.dtype} in a run of {act_dtype}")
         delta_dt = _DT[delta.dtype]
         if not (tuple(delta.shape[-2:]) == (T, d) and delta.dim() in (2, 3)):
@@ -1062,7 +1063,7 @@ def gated_add_rmsnorm(
         _need(delta is not None, "gated_add_rmsnorm: a gate but nothing to gate")
         _cuda(z, "gated_add_rmsnorm gate", act_dtype, contiguous=False)
         zs = _rows(z, "gated_add_rmsnorm gate")
-        if not (tuple(z.shape) == (T, d)):
+        if tuple(z.shape) != (T, d):
             raise KernelError(f"gated_add_rmsnorm: gate {tuple(z.shape)} does not match x {(T, d)}")
         _cuda(bias, "gated_add_rmsnorm bias", torch.float32)
         _need(tuple(bias.shape) == (d,), "gated_add_rmsnorm: bias does not match d")
@@ -1336,7 +1337,7 @@ def latent_attn(
 
 # ------------------------------------------------------------------ routed feed-forward
 def grouped_gemm_takes(K: int, ldx: int, head_stride: int) -> bool:
-    """Whether the tensor-core products of `grouped_gemm.cu` take operands with this k and these strides (in elements)."""
+    """Whether the products of `grouped_gemm_tc.cu` and `grouped_gemm.cu` take operands with this k and these strides (in elements)."""
     return bool(build.load("grouped_gemm").rl_grouped_gemm_takes(c_int(K), c_int(ldx), c_int(head_stride)))
 
 
@@ -1485,7 +1486,7 @@ def moe_gemm(
         )
         _check(lib, rc, "moe_gemm_tc")
         return out
-    if not (tile_rows == moe_tile_rows()):
+    if tile_rows != moe_tile_rows():
         raise KernelError(f"moe_gemm: the plain kernel wants tiles of {moe_tile_rows()} rows, the plan has {tile_rows}")
     lib = build.load("moe")
     rc = lib.rl_moe_gemm(
@@ -1566,7 +1567,7 @@ def latent_attn_mma(
     if n_splits > 1:
         _cuda(scratch, "latent_attn_mma scratch", torch.float32)
         need = latent_attn_mma_scratch_floats(T * H, rank, n_splits)
-        if not (scratch.numel() >= need):
+        if scratch.numel() < need:
             raise KernelError(f"latent_attn_mma: scratch holds {scratch.numel()} floats, {need} needed")
     if out is None:
         out = torch.empty((T, H, rank), dtype=torch.bfloat16, device=q_cat.device)
@@ -1622,11 +1623,11 @@ def qkv_prep(
     else:
         block_table = k_pages = v_pages = None
     coef, every = temperature or (0.0, 0)
-    if not (temperature is None or int(every) > 0):
+    if temperature is not None and int(every) <= 0:
         raise KernelError(f"qkv_prep: a temperature that grows every {every} positions")
     if bias is not None:
         _cuda(bias, "qkv_prep bias", torch.float32)
-        if not (bias.numel() == cols):
+        if bias.numel() != cols:
             raise KernelError(f"qkv_prep: bias has {bias.numel()} numbers for {cols} columns")
     if rotary_dim:
         _cuda(inv_freq, "qkv_prep inv_freq", torch.float32)
@@ -1635,13 +1636,13 @@ def qkv_prep(
         if w is not None:
             _cuda(w, f"qkv_prep {name}", torch.float32)
             want = heads * kdim if norm_whole else kdim
-            if not (w.numel() == want):
+            if w.numel() != want:
                 raise KernelError(f"qkv_prep: {name} must hold one weight per number of {'all heads' if norm_whole else 'a head'} ({want})")
     vs_stride = 0
     if v_src is not None:
         _cuda(v_src, "qkv_prep v_src", qkv.dtype, contiguous=False)
         vs_stride = _rows(v_src, "qkv_prep v_src")
-        if not (tuple(v_src.shape) == (T, num_kv_heads * vdim)):
+        if tuple(v_src.shape) != (T, num_kv_heads * vdim):
             raise KernelError(f"qkv_prep: v_src {tuple(v_src.shape)} is not [T, {num_kv_heads * vdim}]")
         _cuda(v_lambda, "qkv_prep v_lambda", torch.float32)
         _need(v_lambda.numel() == 1, "qkv_prep: v_lambda is one number")
@@ -1797,7 +1798,7 @@ def sigmoid_attn_mma(
     qs = _rows(q, "sigmoid_attn_mma q")
     T = q.shape[0]
     _need(q.shape[1] >= num_heads * kdim, "sigmoid_attn_mma: q rows too short")
-    if not (sigmoid_attn_mma_takes(kdim, vdim, num_heads)):
+    if not sigmoid_attn_mma_takes(kdim, vdim, num_heads):
         raise KernelError(f"sigmoid_attn_mma: sizes {kdim}, {vdim} with {num_heads} heads are not built")
     _check_kv_pages(k_pages, v_pages, q.dtype, num_kv_heads, kdim, vdim, "sigmoid_attn_mma")
     _cuda(block_table, "sigmoid_attn_mma block_table", torch.int32)
@@ -1877,7 +1878,7 @@ def decay_attn(
     lib = build.load("recurrent")
     if max_q_len > 0 and scratch is not None:
         _cuda(scratch, "decay_attn scratch", torch.float32)
-        if not (dim <= DECAY_CHUNKED_MAX_DIM):
+        if dim > DECAY_CHUNKED_MAX_DIM:
             raise KernelError(f"decay_attn: the chunked kernels take key sizes up to {DECAY_CHUNKED_MAX_DIM}")
         _need(scratch.numel() >= decay_attn_chunked_scratch_floats(S, max_q_len, num_heads, dim, vdim), "decay_attn: scratch too small")
         rc = lib.rl_decay_attn_chunked(
@@ -1942,7 +1943,7 @@ def min_gru(
     for name, b in (("z_bias", z_bias), ("x_bias", x_bias)):
         if b is not None:
             _cuda(b, f"min_gru {name}", torch.float32)
-            if not (b.numel() == width):
+            if b.numel() != width:
                 raise KernelError(f"min_gru: {name} does not match the width")
     _cuda(state, "min_gru state", torch.float32)
     if not (state.dim() == 2 and state.shape[1] == width):
@@ -2028,7 +2029,7 @@ def gated_attn(
     (a per head), a = exp(log_decay).  in_scale: float32 [T, H] (b) or None (1).  ext: the state has one more column, fed with
     v = 1, and so has the result.  state: float32 [slots, H, dim, vdim (+1)].  Returns float32 [T, H (vdim (+1))]."""
     qk_heads = qk_heads or num_heads
-    if not (num_heads % qk_heads == 0):
+    if num_heads % qk_heads != 0:
         raise KernelError(f"gated_attn: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
     for name, t, n in (("q", q, qk_heads * dim), ("k", k, qk_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"gated_attn {name}", q.dtype, contiguous=False)
@@ -2085,7 +2086,7 @@ def gated_attn_chunked(
     """`gated_attn` chunk by chunk (64 tokens, all chunks side by side, 32-bit arithmetic): equal within rounding, for prompts.
     max_q_len: the most tokens a sequence of the step brings; scratch: float32, at least `gated_attn_chunked_scratch_floats(...)`."""
     qk_heads = qk_heads or num_heads
-    if not (num_heads % qk_heads == 0):
+    if num_heads % qk_heads != 0:
         raise KernelError(f"gated_attn_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
     for name, t, n in (("q", q, qk_heads * dim), ("k", k, qk_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"gated_attn_chunked {name}", q.dtype, contiguous=False)
@@ -2093,7 +2094,7 @@ def gated_attn_chunked(
             raise KernelError(f"gated_attn_chunked: {name} has the wrong shape or stride")
     T = q.shape[0]
     vcols = vdim + (1 if ext else 0)
-    if not (gated_attn_chunked_takes(dim, vcols)):
+    if not gated_attn_chunked_takes(dim, vcols):
         raise KernelError(f"gated_attn_chunked: key size {dim} is too large for the chunked kernels")
     _cuda(log_decay, "gated_attn_chunked log_decay", torch.float32)
     per_channel = log_decay.numel() == T * num_heads * dim
@@ -2138,7 +2139,7 @@ def head_norm_gate(
     xs = _rows(x, "head_norm_gate x")
     T = x.shape[0]
     xh = n + (1 if m is not None else 0)
-    if not (x.shape[1] == num_heads * xh):
+    if x.shape[1] != num_heads * xh:
         raise KernelError(f"head_norm_gate: x {tuple(x.shape)} is not [T, {num_heads} * {xh}]")
     per_head = 0
     if weight is not None:
@@ -2205,7 +2206,7 @@ def short_conv(
     if bias is not None:
         _cuda(bias, "short_conv bias", torch.float32)
         _need(bias.numel() == C, "short_conv: one bias per channel")
-    if not (not single or T == S):
+    if single and T != S:
         raise KernelError(f"short_conv: {T} tokens of {S} sequences are not one each")
     out = torch.empty((T, C), dtype=x.dtype, device=x.device)
     lib = build.load("delta_rule")
@@ -2260,11 +2261,11 @@ def delta_rule(
     H, G = num_heads, num_qk_heads
     for name, t, n in (("qn", qn, G * dim), ("kn", kn, G * dim), ("kq", kq, G), ("beta", beta, H), ("decay", decay, H)):
         _cuda(t, f"delta_rule {name}", torch.float32)
-        if not (tuple(t.shape) == (T, n)):
+        if tuple(t.shape) != (T, n):
             raise KernelError(f"delta_rule: {name} {tuple(t.shape)} is not [{T}, {n}]")
     _cuda(v, "delta_rule v", contiguous=False)
     _need(tuple(v.shape) == (T, H * vdim), "delta_rule: v must be [T, H vdim]")
-    if not (dim <= DELTA_RULE_MAX_DIM):
+    if dim > DELTA_RULE_MAX_DIM:
         raise KernelError(f"delta_rule: key size {dim} exceeds {DELTA_RULE_MAX_DIM}")
     _cuda(state, "delta_rule state", torch.float32)
     if not (state.dim() == 4 and tuple(state.shape[1:]) == (H, dim, vdim)):
@@ -2337,7 +2338,7 @@ def ssm_gates(raw: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor):
     T, H = raw.shape
     for name, t in (("a_log", a_log), ("dt_bias", dt_bias)):
         _cuda(t, f"ssm_gates {name}", torch.float32)
-        if not (t.numel() == H):
+        if t.numel() != H:
             raise KernelError(f"ssm_gates: one {name} per head")
     log_a, dt = (torch.empty((T, H), dtype=torch.float32, device=raw.device) for _ in range(2))
     lib = build.load("state_space")
@@ -2356,7 +2357,7 @@ def ssm_gate_norm(
     T, n = y.shape
     for name, t in (("x", x), ("z", z)):
         _cuda(t, f"ssm_gate_norm {name}", act_dtype, contiguous=False)
-        if not (tuple(t.shape) == (T, n)):
+        if tuple(t.shape) != (T, n):
             raise KernelError(f"ssm_gate_norm: {name} {tuple(t.shape)} does not match y {(T, n)}")
     _cuda(skip, "ssm_gate_norm skip", torch.float32)
     _cuda(weight, "ssm_gate_norm weight", torch.float32)
@@ -2398,17 +2399,17 @@ def scalar_decay_chunked(
     value sizes up to 128: equal within rounding, for prompts.  max_q_len: the most tokens a sequence of the step brings; scratch:
     float32, `scalar_decay_chunked_scratch_floats(...)` numbers.  Returns float32 [T, H vdim]."""
     qk_heads = qk_heads or num_heads
-    if not (num_heads % qk_heads == 0):
+    if num_heads % qk_heads != 0:
         raise KernelError(f"scalar_decay_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
     for name, t, n in (("q", q, qk_heads * dim), ("k", k, qk_heads * dim), ("v", v, num_heads * vdim)):
         _cuda(t, f"scalar_decay_chunked {name}", torch.bfloat16, contiguous=False)
         if not (_rows(t, f"scalar_decay_chunked {name}") == q.stride(0) and t.shape[1] == n and t.shape[0] == q.shape[0]):
             raise KernelError(f"scalar_decay_chunked: {name} has the wrong shape or stride")
     T = q.shape[0]
-    if not (scalar_decay_chunked_takes(dim, vdim)):
+    if not scalar_decay_chunked_takes(dim, vdim):
         raise KernelError(f"scalar_decay_chunked: sizes {dim} x {vdim} are not built")
     _cuda(log_decay, "scalar_decay_chunked log_decay", torch.float32)
-    if not (log_decay.numel() == T * num_heads):
+    if log_decay.numel() != T * num_heads:
         raise KernelError(f"scalar_decay_chunked: log_decay {tuple(log_decay.shape)} is not [T, H]")
     if in_scale is not None:
         _cuda(in_scale, "scalar_decay_chunked in_scale", torch.float32)
@@ -2495,7 +2496,7 @@ def flash_mix(
     if not (maps in (1, 2) and num_heads % maps == 0 and kdim % (8 * maps) == 0):
         raise KernelError(f"flash_mix: {maps} maps in {num_heads} heads of {kdim}")
     _need(q.shape[1] >= num_heads // maps * parts * kdim, "flash_mix: q rows too short")
-    if not (flash_mix_takes(kdim, vdim, parts)):
+    if not flash_mix_takes(kdim, vdim, parts):
         raise KernelError(f"flash_mix: sizes {kdim} / {vdim} with {parts} query parts are not built")
     _check_kv_pages(k_pages, v_pages, torch.bfloat16, num_kv_heads, kdim, vdim, "flash_mix")
     _cuda(block_table, "flash_mix block_table", torch.int32)
@@ -2550,7 +2551,7 @@ def flash_mix_decode(
     _cuda(qf, "flash_mix_decode qf", torch.bfloat16)
     S = qf.shape[0]
     _need(qf.dim() == 2 and qf.shape[1] == num_heads * num_kv_heads * kdim, "flash_mix_decode: qf must be [S, H K kdim]")
-    if not (flash_mix_decode_takes(num_heads, num_kv_heads, kdim, vdim)):
+    if not flash_mix_decode_takes(num_heads, num_kv_heads, kdim, vdim):
         raise KernelError(f"flash_mix_decode: sizes {num_heads} / {num_kv_heads} / {kdim} / {vdim} are not built")
     _check_kv_pages(k_pages, v_pages, torch.bfloat16, num_kv_heads, kdim, vdim, "flash_mix_decode")
     _cuda(block_table, "flash_mix_decode block_table", torch.int32)
