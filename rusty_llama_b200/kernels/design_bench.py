@@ -122,7 +122,8 @@ def kernel_table(z: dict, T: int, batch: int, ctx: int, peaks: dict) -> Dict[str
         if like:
             out[name]["like"] = like
 
-    # ---- attention: prompt
+    # ---- attention: prompt, over keys and values that the step expands per head (`LatentAttention._expands`); beside it the kernel on the
+    # latents, which takes short portions and steps whose earlier rows would not pay
     pages_n = (T + 63) // 64
     pages = torch.randn(pages_n, 1, 64, Dk, device=dev, dtype=bf)
     table = torch.randperm(pages_n, device=dev).to(torch.int32).view(1, -1).contiguous()
@@ -131,6 +132,17 @@ def kernel_table(z: dict, T: int, batch: int, ctx: int, peaks: dict) -> Dict[str
     start = torch.tensor([0, T], dtype=torch.int32, device=dev)
     pos0 = torch.zeros(1, dtype=torch.int32, device=dev)
     scale = 1.0 / math.sqrt(dim + rot)
+    seq_rows, held = 64 * pages_n, torch.tensor([T], dtype=torch.int32, device=dev)
+    w_vk = torch.randn(H, vdim + dim, rank, device=dev, dtype=bf)
+    latents, kv = torch.empty(seq_rows, rank, device=dev, dtype=bf), torch.empty(seq_rows, H, vdim + dim + rot, device=dev, dtype=bf)
+    us = mb._time(lambda i: ops.latent_expand(pages, table, held, seq_rows, w_vk, rot, latents, kv), 1, **it)
+    note("prefill_expand_keys_and_values", us, (T * (Dk + H * (vdim + dim + rot)) + w_vk.numel()) * 2, 2.0 * T * H * (vdim + dim) * rank)
+    qp, gate = torch.randn(T, H * (dim + rot), device=dev, dtype=bf), torch.randn(T, H * vdim, device=dev, dtype=bf)
+    us = mb._time(lambda i: ops.flash_expanded(qp, kv, seq_rows, start, pos0, T, vdim, 0, scale, sink=sink, gate=gate), 1, **it)
+    expanded_flops = 2.0 * T * T / 2 * H * (dim + rot + vdim)
+    note("prefill_expanded_attention", us, 0, expanded_flops)
+    out["prefill_expanded_attention"]["TFLOPs"] = round(expanded_flops / us / 1e6, 1)
+    del kv, latents
     us = mb._time(lambda i: ops.latent_attn_mma(q_cat, pages, table, start, pos0, T, sink, rank, rot, scale), 1, **it)
     flops = 2.0 * T * T / 2 * H * (Dk + rank)
     r = mb.bench_flash_prefill(SimpleNamespace(tokens=T, impl="auto", heads=H, kv_heads=H, head_dim=vdim, splits=0, **it))
@@ -153,7 +165,7 @@ def kernel_table(z: dict, T: int, batch: int, ctx: int, peaks: dict) -> Dict[str
          like={"kernel": "attn_decode", "us": r["us"], "frac": round(r["GBps"] / peaks["hbm_gbs"], 3)})
     out["decode_latent_attention"]["cache_bytes_vs_like"] = round(Dk / (2.0 * H * vdim), 4)
     del pools
-    # ---- the two per-head maps, norm + rotation + cache write
+    # ---- the two per-head maps of a step on the latents (every decode step), norm + rotation + cache write
     for rows, tag in ((T, "prefill"), (batch, "decode")):
         qp = torch.randn(rows, H * (dim + rot) + H * vdim + Dk, device=dev, dtype=bf)
         w_uk = torch.randn(H, rank, dim, device=dev, dtype=bf)

@@ -141,9 +141,14 @@ def kernel_table(z: dict, T: int, batch: int, ctx: int, peaks: dict) -> Dict[str
         a_log, dt = torch.zeros(H, device=dev), torch.zeros(H, device=dev)
         us = mb._time(lambda i: ops.delta_prep(conv[:, : 2 * qd], ba, a_log, dt, H, H, hd, 1e-6, hd ** -0.5), 1, **it)
         note(f"{tag}_delta_unit_vectors_scalars", us, rows * 2 * qd * (2 + 4), 0)
-        qn, kn, kq, beta, dec = ops.delta_prep(conv[:, : 2 * qd], ba, a_log, dt, H, H, hd, 1e-6, hd ** -0.5)
-        st3 = torch.zeros(n_seqs, H, hd, hd, device=dev)
-        us = mb._time(lambda i: ops.delta_rule(qn, kn, kq, conv[:, 2 * qd:], beta, dec, st3, step.slot_ids, step.seq_start, H, H, hd, hd), 1, **it)
+        qn, kn, kq, beta, dec, log = ops.delta_prep(conv[:, : 2 * qd], ba, a_log, dt, H, H, hd, 1e-6, hd ** -0.5, log_decay=True)
+        st3, v3 = torch.zeros(n_seqs, H, hd, hd, device=dev), conv[:, 2 * qd:]
+        where = (st3, step.slot_ids, step.seq_start, H, H, hd, hd)
+        if prompt:  # chunk by chunk, as `GatedDeltaRule` takes a prompt
+            room = torch.empty(ops.delta_chunked_scratch_floats(rows, n_seqs, H, hd, hd), device=dev)
+            us = mb._time(lambda i: ops.delta_chunked(qn, kn, v3, beta, log, *where, per, room), 1, **it)
+        else:
+            us = mb._time(lambda i: ops.delta_rule(qn, kn, kq, v3, beta, dec, *where), 1, **it)
         note(f"{tag}_delta_recurrence", us, rows * qd * (2 * 4 + 2 + 4) + 2 * st3.numel() * 4, 6.0 * rows * qd * hd, like=like_decay)
     ops.tc_status_check()
     return out
