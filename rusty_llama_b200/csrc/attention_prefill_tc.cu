@@ -63,7 +63,7 @@
 // probabilities go into P V as the sum of two bfloat16 numbers, the second ones in the half of the S buffer that the first leave free: rounded
 // once, under a maximum that is only raised by factors of 2^8, they put the result 5 to 10 % further from 64 bits than the kernel on the latents
 // (whose row maximum is exact, so that a row's largest probability is 1), in two parts 1 to 6 % nearer.  16 heads, 2048 tokens: 63 us with one
-// part (340 TFLOP/s), 74 with two; the same layer on its latents with mma.sync 468 us.
+// part (340 TFLOP/s), 75 with two; the same layer on its latents with mma.sync 468 us.
 //
 // Every mbarrier wait is bounded; on expiry a code goes to status[0] and the block drains.
 #include "tc_common.cuh"

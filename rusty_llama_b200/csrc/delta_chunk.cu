@@ -16,7 +16,7 @@
 //
 // Token by token every token was one chain of dependent steps per column (760 cycles with nothing to hide them); here only (2) is
 // serial, with 64 tokens a step.  Bound: the FMA pipe and the shared-memory reads that feed it, 1.1 billion multiply-adds for 16 heads
-// of 128 x 128 and 2048 tokens in (2) and about as many in (1) and (3) each.  Sequences of 1029, 700 and 319 tokens: 62, 106 and 74 us
+// of 128 x 128 and 2048 tokens in (2) and about as many in (1) and (3) each.  Sequences of 1029, 700 and 319 tokens: 62, 106 and 72 us
 // against 444 us token by token.
 #include "common.cuh"
 

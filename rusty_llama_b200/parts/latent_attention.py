@@ -17,7 +17,7 @@ from .base import MIXERS, POSITIONS, KVNeed, Mixer, ParamInfo, scratch_for_call
 # for the call.
 _EXPAND_MIN_TOKENS = 33
 _EXPAND_MAX_BYTES = 1 << 30
-# What an operation of the attention on the latents (156 TFLOP/s) and of the one over expanded rows (290) takes in operations of the head
+# What an operation of the attention on the latents (156 TFLOP/s) and of the one over expanded rows (285) takes in operations of the head
 # products (540)
 _LATENT_OPERATION, _EXPANDED_OPERATION = 3.5, 1.9
 
@@ -156,7 +156,7 @@ class LatentAttention(Mixer):
         (query, key) pair.  So a sequence's earlier positions pay for themselves where enough tokens of the step see them: 41 with
         128 + 64 / 128 and rank 512, 21 with 64 + 32 / 64 and rank 256, unless a window hides them.  Measured, 16 heads of 128 + 64 / 128, rank
         512, one prompt of 2048: 468 us on the latents (156 TFLOP/s) and 25 us for the two products around it; expanded, 16 us for the
-        products (540 TFLOP/s), 5 for the rows, 74 for the attention (290 TFLOP/s)."""
+        products (540 TFLOP/s), 5 for the rows, 75 for the attention (285 TFLOP/s)."""
         if step.decode_only or self.w_vk is None or step.n_tokens < _EXPAND_MIN_TOKENS or not q.is_cuda:
             return 0
         if not ops.flash_expanded_takes(self.dim + self.rot, self.vdim) or self.dim % 8 or self.rot % 8 or self.rank % 8 or self.dim == 0:
@@ -197,7 +197,9 @@ class LatentAttention(Mixer):
             rows = step.n_seqs * seq_rows
             latents = scratch_for_call((rows, self.rank), xn.dtype, xn.device)
             expanded = scratch_for_call((rows, self.H, self.vdim + self.dim + self.rot), xn.dtype, xn.device)
-        if latents is not None and expanded is not None:
+            if latents is None or expanded is None:
+                latents = expanded = None
+        if latents is not None:
             ops.latent_prep(q, kv, self.w_norm, self.eps, *turn, None, *sizes, in_place=True)
             ops.latent_expand(cache.k_pages, cache.block_table, step.seq_len, seq_rows, self.w_vk, self.rot, latents, expanded)
             a = ops.flash_expanded(q, expanded, seq_rows, step.seq_start, step.seq_pos0, step.max_q_len, self.vdim, self.window, self.scale,
