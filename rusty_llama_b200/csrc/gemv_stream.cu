@@ -305,6 +305,11 @@ gemv_stream_kernel(const bf16* __restrict__ x, int ldx, const __grid_constant__ 
     }
   } else {
     // ---------------- products
+    // A stage is handed back when its pieces are in registers (hand_back).  Where three registers are left for it, that is behind the loads of
+    // the next stage (an item's last stage: behind its products), so that nobody waits for the youngest loads.  Decode products of 8B sizes at
+    // 8 rows, at once / late: QKV 13.0 / 12.8, attention output 10.0 / 9.7, gate/up 38.4 / 38.2 us; the build with five stages' activations
+    // spills for it (down 21.8 / 26.3).
+    constexpr bool LATE = !HI && SLICE_STAGES * KC == SHORT_SLICE;
     const int g = lane >> 2, t4 = lane & 3;
     // row g of a stage; k block kb = warp + 16 j lies in 64-k block kb / 2 as 16-byte pieces
     // (kb & 1) * 4 + t4, swizzled by the 64-k block's number
@@ -352,6 +357,7 @@ gemv_stream_kernel(const bf16* __restrict__ x, int ldx, const __grid_constant__ 
         unit = 0;
         ++slice;
       }
+      uint32_t back = empty0, piece0 = 0, piece1 = 0;
       float acc[2 * KB_PER_WARP][4];
 #pragma unroll
       for (int i = 0; i < 2 * KB_PER_WARP; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -364,15 +370,20 @@ gemv_stream_kernel(const bf16* __restrict__ x, int ldx, const __grid_constant__ 
             uint4 b[KB_PER_WARP];
 #pragma unroll
             for (int j = 0; j < KB_PER_WARP; ++j) b[j] = lds128(w_off[j] + st_off);
+            if (LATE && s > 0) hand_back(back, piece0 ^ piece1, zero_bits, lane);
 #pragma unroll
             for (int j = 0; j < KB_PER_WARP; ++j) {
               const uint4 lo = xa[s][j], hi = HI ? xb[s][j] : zero;
               mma_bf16_16x8x16(acc[2 * j], lo.x, hi.x, lo.y, hi.y, b[j].x, b[j].y);
               mma_bf16_16x8x16(acc[2 * j + 1], lo.z, hi.z, lo.w, hi.w, b[j].z, b[j].w);
             }
-            // (decode products of 8B sizes at 8 rows, down 21.9, gate/up 38.4, attention output 10.2 us; handed back one stage late, behind the
-            // next stage's loads, 22.6, 38.6 and 10.3: the products wait for the pieces at once in any case)
-            hand_back(empty0 + 8 * st, b[0].x ^ b[KB_PER_WARP - 1].x, zero_bits, lane);
+            if (LATE) {
+              back = empty0 + 8 * st;
+              piece0 = b[0].x;
+              piece1 = b[KB_PER_WARP - 1].x;
+            } else {
+              hand_back(empty0 + 8 * st, b[0].x ^ b[KB_PER_WARP - 1].x, zero_bits, lane);
+            }
             if (warp == 0 && lane == 0 && item == first_item && s == 0) rl_trace_event(5);  // first stage consumed
             st_off += STAGE_BYTES;
             if (++st == STAGES) {
@@ -384,6 +395,7 @@ gemv_stream_kernel(const bf16* __restrict__ x, int ldx, const __grid_constant__ 
         }
       }
       if (!ok) break;
+      if (LATE) hand_back(back, piece0 ^ piece1, zero_bits, lane);
       // leave the partial sums to the storing warps; the buffer was last read two items ago
       const int buf = done_items & 1;
       if (done_items >= 2 && !mbar_wait_role(&bars.red_free[buf], ((done_items >> 1) - 1) & 1, ctl, 37)) {

@@ -162,12 +162,23 @@ def test_prompt_attention_with_one_barrier_for_the_probabilities_can_stall():
     assert problem is not None and "nothing can move" in problem and "('V'" in problem
 
 
-def _explore_stream(S: int, T: int, warps: int, landed: bool):
+def _explore_stream(S: int, items, warps: int, how: str):
     """csrc/gemv_stream.cu's ring: the copying lane refills stage i % S once every product warp has handed fill i - S back; a product warp
-    waits for a fill, asks for its pieces, and hands the stage back: behind the loads' issue or, `landed`, not before the pieces are there.
-    What was asked for lands at any later time and is then what the stage holds at that moment.  Returns the first problem found or None."""
-    programme = lambda i: [("wait", i), ("ask", i)] + ([("need", i)] if landed else []) + [("hand", i)]  # noqa: E731
-    flat = [s for i in range(T) for s in programme(i)]
+    waits for a fill, asks for its pieces, and hands the stage back: behind the loads' issue ("asked"), not before the pieces are there
+    ("landed"), or not before they are there and behind the next stage's loads, an item's last stage at its end ("late").  `items`: stages of
+    each item.  What was asked for lands at any later time and is then what the stage holds at that moment.  Returns the first problem
+    found or None."""
+    T, flat, i = sum(items), [], 0
+    for n in items:
+        for s in range(n):
+            flat += [("wait", i), ("ask", i)]
+            if how != "late":
+                flat += ([("need", i)] if how == "landed" else []) + [("hand", i)]
+            elif s > 0:
+                flat += [("need", i - 1), ("hand", i - 1)]
+            i += 1
+        if how == "late":
+            flat += [("need", i - 1), ("hand", i - 1)]
     # copies started, held[stage] = the fill it holds (-1: being written), arrivals per stage, per warp (place, pieces on their way)
     start = (0, (-2,) * S, (0,) * S, ((0, ()),) * warps)
     seen, queue = {start}, deque([start])
@@ -204,14 +215,15 @@ def _explore_stream(S: int, T: int, warps: int, landed: bool):
     return None
 
 
-@pytest.mark.parametrize("S, T", [(2, 6), (3, 8)])
-@pytest.mark.parametrize("warps", [1, 2, 3])
-def test_a_stage_handed_back_from_what_was_loaded_is_never_read_too_late(S, T, warps):
-    assert _explore_stream(S, T, warps, landed=True) is None
+@pytest.mark.parametrize("S, items", [(2, (1, 1, 1, 1)), (2, (3, 2)), (3, (4, 4)), (3, (1, 3, 2))])
+@pytest.mark.parametrize("warps", [1, 2])
+@pytest.mark.parametrize("how", ["landed", "late"])
+def test_a_stage_handed_back_from_what_was_loaded_is_never_read_too_late(S, items, warps, how):
+    assert _explore_stream(S, items, warps, how) is None
 
 
 def test_a_stage_handed_back_when_its_pieces_were_only_asked_for_is_read_too_late():
-    problem = _explore_stream(2, 4, 2, landed=False)
+    problem = _explore_stream(2, (2, 2), 2, "asked")
     assert problem is not None and "is read after" in problem
 
 
@@ -223,13 +235,14 @@ def _code(name):
 
 
 def test_every_hand_over_of_the_streaming_product_is_made_from_what_was_loaded():
-    """The model above against the source: the only arrival on an `empty` barrier is `hand_back`'s, whose address holds a vote over the
-    loaded words."""
+    """The model above against the source: the only arrivals on an `empty` barrier are `hand_back`'s, whose address holds the loaded words."""
     helper = _code("tc_common.cuh").split("void hand_back(")[1].split("\n}")[0]
-    assert "landed = __any_sync(0xffffffffu, (pieces & zero_bits) != 0)" in helper and "mbar_arrive_s(bar + landed)" in helper
+    assert "__syncwarp();" in helper and "mbar_arrive_s(bar + (pieces & zero_bits))" in helper
     code = _code("gemv_stream.cu")
     assert "mbar_arrive_s(" not in code and "mbar_arrive(&bars.empty" not in code
-    assert code.count("hand_back(") == code.count("hand_back(empty0 + 8 * st, b[0].x ^ b[KB_PER_WARP - 1].x, zero_bits, lane)") == 1
+    assert code.count("hand_back(empty0 + 8 * st, b[0].x ^ b[KB_PER_WARP - 1].x, zero_bits, lane)") == 1
+    assert code.count("hand_back(back, piece0 ^ piece1, zero_bits, lane)") == 2 and "piece0 = b[0].x;" in code and "piece1 = b[KB_PER_WARP - 1].x;" in code
+    assert code.count("hand_back(") == 3
 
 
 def test_every_hand_over_of_the_decode_attention_is_made_from_what_was_loaded():
