@@ -16,7 +16,8 @@
 //   gla_log_decay     log a = logsigmoid(z + bias) / tau, 32-bit, from the projection in the run's element type
 //   mlstm_gates       the capped log gates, the running maximum through the sequences' records, a's logarithm, b and m per token
 //   gated_attn        the recurrence token by token (decode steps, 32-bit runs, short prompts): equal bits however a sequence is cut
-//   gated_attn chunked   prompts of bfloat16 runs: chunks of 64 tokens, sub-chunks of 16 (see below)
+//   gated_attn chunked   prompts of bfloat16 runs: chunks of 64 tokens, sub-chunks of 16 (see below; a decay per channel on the tensor
+//                     cores, gated_chunk_mma.cuh)
 //   head_norm_gate    per head: the normaliser, the RMS norm over the head's values, weight, gate; writes the run's element type
 //
 // Everything between the projections and the state is 32-bit: decays and their logarithms, gates, the maximum, the state, the sums.
@@ -879,6 +880,8 @@ gated_chunk_out_kernel(const T* __restrict__ q, const T* __restrict__ k, const T
   }
 }
 
+#include "gated_chunk_mma.cuh"
+
 RL_API long long rl_gated_attn_chunked_scratch_floats(int n_seqs, int max_q_len, int H, int dim, int vcols) {
   return (long long)n_seqs * H * ((max_q_len + GC - 1) / GC) * dim * (vcols + 1);
 }
@@ -890,10 +893,14 @@ static size_t gated_chunk_out_smem(int dim) {
 
 RL_API int rl_gated_attn_chunked_takes(int dim) { return dim > 0 && gated_chunk_out_smem(dim) <= 227 * 1024; }
 
+// norm_w: null, or the heads' norm weights [vdim]; result is then bfloat16 rows that have been through what head_norm_gate does (gate may
+// be null; gate_act as there), where the tensor-core kernels take the call, and nothing is launched and RL_NOT_FUSED returned where
+// they do not.  Without it result is float32.
 RL_API int rl_gated_attn_chunked(const void* q, const void* k, const void* v, int dtype, int in_stride, const float* log_decay,
                                  int per_channel, const float* in_scale, float q_scale, float* state, const int* slot_ids,
-                                 const int* seq_start, float* scratch, float* out, int out_stride, int n_seqs, int max_q_len, int H,
-                                 int QH, int dim, int vdim, int ext, cudaStream_t stream) {
+                                 const int* seq_start, float* scratch, void* result, int out_stride, int n_seqs, int max_q_len, int H,
+                                 int QH, int dim, int vdim, int ext, const float* norm_w, float eps, const void* gate, int gate_stride,
+                                 int gate_act, float out_scale, cudaStream_t stream) {
   if (QH <= 0 || H % QH) RL_REFUSE(6, "gated_attn_chunked: %d heads are not a multiple of %d q/k heads", H, QH);
   if (n_seqs <= 0 || max_q_len <= 0 || H <= 0 || dim <= 0 || vdim <= 0 || (ext != 0 && ext != 1) || !log_decay || !scratch)
     RL_REFUSE(1, "gated_attn_chunked: S=%d max_q=%d H=%d dim=%d vdim=%d ext=%d", n_seqs, max_q_len, H, dim, vdim, ext);
@@ -906,13 +913,38 @@ RL_API int rl_gated_attn_chunked(const void* q, const void* k, const void* v, in
   const int elems = dim * vcols;
   // Rows are read four numbers at a time where each of them starts on four of its type and is whole fours long.
   const uintptr_t four = dtype == RL_BF16 ? 7 : 15;
+  float* out = (float*)result;
   int wide = 0;
   if (dim % 4 == 0 && in_stride % 4 == 0 && (((uintptr_t)q | (uintptr_t)k) & four) == 0) wide |= GC_WIDE_QK;
   if (vdim % 4 == 0 && in_stride % 4 == 0 && ((uintptr_t)v & four) == 0) wide |= GC_WIDE_V;
   if (dim % 4 == 0 && ((uintptr_t)log_decay & 15) == 0) wide |= GC_WIDE_DECAY;
-  if (vcols % 4 == 0 && out_stride % 4 == 0 && (((uintptr_t)state | (uintptr_t)scratch | (uintptr_t)out) & 15) == 0) wide |= GC_WIDE_STATE;
+  if (vcols % 4 == 0 && (((uintptr_t)state | (uintptr_t)scratch) & 15) == 0 && (norm_w || (out_stride % 4 == 0 && ((uintptr_t)out & 15) == 0))) wide |= GC_WIDE_STATE;
   const int scan_elems = wide & GC_WIDE_STATE ? 4 : 1;
   dim3 grid((unsigned)sh, max_chunks, col_tiles), grid2((unsigned)sh, (elems / scan_elems + 255) / 256), grid3((unsigned)sh, max_chunks);
+  if (norm_w && (out_stride % 2 || ((uintptr_t)result & 3) || gate_stride % 2 || ((uintptr_t)gate & 3) || ((uintptr_t)norm_w & 7))) return RL_NOT_FUSED;
+  // A decay per channel on bfloat16 rows in 16-byte pieces goes to the tensor cores (gated_chunk_mma.cuh): 2048 tokens, 16 heads of
+  // 128 x 128: 97 instead of 185 us for the three steps.  One decay per head comes with a normaliser column, whose odd rows do not fit.
+  if (dtype == RL_BF16 && per_channel && !in_scale && !ext && (wide & GC_WIDE_STATE) && gated_mma_takes(q, k, v, in_stride, log_decay, dim, vdim)) {
+#define RL_GM(DP)                                                                                                                     \
+  do {                                                                                                                                \
+    constexpr size_t s1 = (size_t)GC * (DP + 8) * 4 + GC * (GM_COLS + 8) * 2, s3 = GmOut<DP>::BYTES;                                  \
+    if (cudaFuncSetAttribute(gated_mma_state_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1) != cudaSuccess ||      \
+        cudaFuncSetAttribute(gated_mma_out_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3) != cudaSuccess)          \
+      RL_REFUSE(4, "gated_attn_chunked: %zu bytes of shared memory refused", s3);                                                     \
+    RL_LAUNCH_CHECK(rl_launch(gated_mma_state_kernel<DP>, grid3, 256, s1, stream, (const bf16*)k, (const bf16*)v, in_stride, log_decay, \
+                              seq_start, scratch, chunk_decay, max_chunks, H, QH, dim, vdim));                                        \
+    RL_LAUNCH_CHECK(rl_launch(gated_chunk_scan_kernel<4>, grid2, 256, 0, stream, state, slot_ids, seq_start, scratch,                 \
+                              (const float*)chunk_decay, max_chunks, H, dim, vcols));                                                 \
+    RL_LAUNCH_CHECK(rl_launch(gated_mma_out_kernel<DP>, grid3, 256, s3, stream, (const bf16*)q, (const bf16*)k, (const bf16*)v,       \
+                              in_stride, log_decay, q_scale, seq_start, (const float*)scratch, max_chunks, result, out_stride, H, QH, \
+                              dim, vdim, SplNorm{norm_w, eps, (const bf16*)gate, gate_stride, gate_act, out_scale}));                 \
+  } while (0)
+    if (dim <= 64) RL_GM(64);
+    else RL_GM(128);
+#undef RL_GM
+    return 0;
+  }
+  if (norm_w) return RL_NOT_FUSED;
   const size_t smem1 = ((size_t)GC * gc_row(dim) + GC * GC_COLS + GC * 4) * sizeof(float), smem3 = gated_chunk_out_smem(dim);
 #define RL_GC(T)                                                                                                                     \
   do {                                                                                                                               \

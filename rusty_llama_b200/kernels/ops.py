@@ -2078,13 +2078,36 @@ def gated_attn_chunked_scratch_floats(n_seqs: int, max_q_len: int, num_heads: in
     return n_seqs * num_heads * ((max_q_len + GATED_CHUNK - 1) // GATED_CHUNK) * dim * (vcols + 1)
 
 
+def _norm_args(norm, what: str, T: int, H: int, n: int):
+    """(weight, eps, gate, gate's row stride, gate_act, out_scale, out) of a norm that chunked kernels are to take along; a weight that the
+    heads do not share becomes None (the kernels have no form for it)."""
+    if norm is None:
+        return None, 0.0, None, 0, GATE_NONE, 1.0, None
+    weight, eps, gate, gate_act, out_scale, out = norm
+    _cuda(weight, f"{what} norm weight", torch.float32)
+    gs = 0
+    if gate is not None:
+        _cuda(gate, f"{what} gate", torch.bfloat16, contiguous=False)
+        gs = _rows(gate, f"{what} gate")
+        if gate.shape[0] != T or gate.shape[1] < H * n:
+            raise KernelError(f"{what}: gate rows too short")
+    if out is not None:
+        _cuda(out, f"{what} out", torch.bfloat16, contiguous=False)
+        if tuple(out.shape) != (T, H * n) or _rows(out, f"{what} out") < H * n:
+            raise KernelError(f"{what}: out must be [T, H vdim]")
+    return weight if weight.numel() == n else None, eps, gate, gs, gate_act, out_scale, out
+
+
 def gated_attn_chunked(
     q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, log_decay: torch.Tensor, in_scale: Optional[torch.Tensor], state: torch.Tensor,
     slot_ids: torch.Tensor, seq_start: torch.Tensor, num_heads: int, dim: int, vdim: int, max_q_len: int, scratch: torch.Tensor,
-    q_scale: float = 1.0, ext: bool = False, qk_heads: int = 0,
-) -> torch.Tensor:
+    q_scale: float = 1.0, ext: bool = False, qk_heads: int = 0, norm=None,
+) -> Optional[torch.Tensor]:
     """`gated_attn` chunk by chunk (64 tokens, all chunks side by side, 32-bit arithmetic): equal within rounding, for prompts.
-    max_q_len: the most tokens a sequence of the step brings; scratch: float32, at least `gated_attn_chunked_scratch_floats(...)`."""
+    max_q_len: the most tokens a sequence of the step brings; scratch: float32, at least `gated_attn_chunked_scratch_floats(...)`.
+
+    norm: None, or (weight [vdim], eps, gate, gate_act, out_scale, out) as `head_norm_gate` takes them (out may be None): returns what
+    `head_norm_gate` would make of the result, in q's type, in the same kernels; None where they do not take the sizes (nothing is launched)."""
     qk_heads = qk_heads or num_heads
     if num_heads % qk_heads != 0:
         raise KernelError(f"gated_attn_chunked: {num_heads} heads are not a multiple of {qk_heads} q/k heads")
@@ -2112,18 +2135,26 @@ def gated_attn_chunked(
     _need(seq_start.numel() == S + 1, "gated_attn_chunked: seq_start must hold one more entry than there are sequences")
     _cuda(scratch, "gated_attn_chunked scratch", torch.float32)
     _need(max_q_len >= 1 and scratch.numel() >= gated_attn_chunked_scratch_floats(S, max_q_len, num_heads, dim, vcols), "gated_attn_chunked: scratch too small")
-    out = torch.empty((T, num_heads * vcols), dtype=torch.float32, device=q.device)
+    weight, eps, gate, gs, gate_act, out_scale, out = _norm_args(norm, "gated_attn_chunked", T, num_heads, vdim)
+    if norm is not None and (weight is None or q.dtype != torch.bfloat16 or ext):
+        return None
+    if out is None:
+        out = torch.empty((T, num_heads * vcols), dtype=torch.float32 if norm is None else q.dtype, device=q.device)
     lib = build.load("gated_recurrent")
     rc = lib.rl_gated_attn_chunked(
         _p(q), _p(k), _p(v), c_int(_dt(q, "gated_attn_chunked")), c_int(q.stride(0)), _p(log_decay), c_int(1 if per_channel else 0), _p(in_scale),
         c_float(q_scale), _p(state), _p(slot_ids), _p(seq_start), _p(scratch), _p(out), c_int(out.stride(0)), c_int(S), c_int(max_q_len),
-        c_int(num_heads), c_int(qk_heads), c_int(dim), c_int(vdim), c_int(1 if ext else 0), _stream(),
+        c_int(num_heads), c_int(qk_heads), c_int(dim), c_int(vdim), c_int(1 if ext else 0), _p(weight), c_float(eps), _p(gate), c_int(gs),
+        c_int(gate_act), c_float(out_scale), _stream(),
     )
+    if rc == _NOT_FUSED:
+        return None
     _check(lib, rc, "gated_attn_chunked", kernels=3)
     return out
 
 
 GATE_NONE, GATE_SIGMOID, GATE_SILU = 0, 1, 2
+_NOT_FUSED = -20  # what the launcher of `gated_attn_chunked` answers where it cannot take the norm along
 
 
 def head_norm_gate(

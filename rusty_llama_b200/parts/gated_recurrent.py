@@ -32,20 +32,23 @@ _CHUNKED_MIN_TOKENS = 32
 _CHUNKED_MAX_FLOATS = 1 << 29
 
 
-def _recurrence(mixer, q, k, v, log_decay, in_scale, state, step, ext: bool):
-    """The recurrence over a step's tokens: chunk by chunk for the prompts of a bfloat16 run (all chunks side by side, equal
-    within rounding), token by token otherwise (equal bits however a sequence is cut into steps)."""
+def _recurrence(mixer, q, k, v, log_decay, in_scale, state, step, ext: bool, norm=None):
+    """(o, normed): the recurrence over a step's tokens: chunk by chunk for the prompts of a bfloat16 run (all chunks side by side, equal
+    within rounding), token by token otherwise (equal bits however a sequence is cut into steps).  norm: as `gated_attn_chunked` takes
+    it; normed says whether o has been through it."""
     chunked = (q.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS and ops.gated_attn_chunked_takes(mixer.dim, mixer.vdim + (1 if ext else 0)))
     if chunked:
         need = ops.gated_attn_chunked_scratch_floats(step.n_seqs, step.max_q_len, mixer.H, mixer.dim, mixer.vdim + (1 if ext else 0))
         scratch = mixer.rt.workspace.get("gated_attn_chunks", need, torch.float32)
-        return ops.gated_attn_chunked(
-            q, k, v, log_decay, in_scale, state, step.slot_ids, step.seq_start, mixer.H, mixer.dim, mixer.vdim, step.max_q_len, scratch,
-            q_scale=mixer.q_scale, ext=ext,
-        )
+        args = (q, k, v, log_decay, in_scale, state, step.slot_ids, step.seq_start, mixer.H, mixer.dim, mixer.vdim, step.max_q_len, scratch)
+        if norm is not None:
+            a = ops.gated_attn_chunked(*args, q_scale=mixer.q_scale, ext=ext, norm=norm)
+            if a is not None:
+                return a, True
+        return ops.gated_attn_chunked(*args, q_scale=mixer.q_scale, ext=ext), False
     return ops.gated_attn(
         q, k, v, log_decay, in_scale, state, step.slot_ids, step.seq_start, mixer.H, mixer.dim, mixer.vdim, q_scale=mixer.q_scale, ext=ext,
-    )
+    ), False
 
 
 @MIXERS.register("gated_linear_attention")
@@ -131,8 +134,10 @@ class GatedLinearAttention(Mixer):
             inner = inner.contiguous()
         z = linear(inner, self.w_a2)
         log_decay = ops.gla_log_decay(z, self.b_a, self.tau)
-        o = _recurrence(self, q, k, v, log_decay, None, cache.state, step, ext=False)
-        a = ops.head_norm_gate(o, self.H, self.vdim, self.w_norm, self.eps, gate, ops.GATE_SILU, xn.dtype, out_scale=self.out_scale, out=out)
+        a, normed = _recurrence(self, q, k, v, log_decay, None, cache.state, step, ext=False,
+                                norm=(self.w_norm, self.eps, gate, ops.GATE_SILU, self.out_scale, out))
+        if not normed:
+            a = ops.head_norm_gate(a, self.H, self.vdim, self.w_norm, self.eps, gate, ops.GATE_SILU, xn.dtype, out_scale=self.out_scale, out=out)
         return a, self.w_o
 
 
@@ -218,7 +223,7 @@ class MatrixMemory(Mixer):
         gi, gf = proj[:, 2 * qd + 2 * vd : 2 * qd + 2 * vd + H], proj[:, 2 * qd + 2 * vd + H :]
         log_a, b, m = ops.mlstm_gates(gi, gf, self.b_i, self.b_f, self.cap, maximum.state, step.slot_ids, step.seq_start,
                                       scan=xn.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS)
-        o = _recurrence(self, q, k, v, log_a, b, memory.state, step, ext=True)
+        o, _ = _recurrence(self, q, k, v, log_a, b, memory.state, step, ext=True)
         a = ops.head_norm_gate(
             o, H, self.vdim, self.w_norm, self.eps, gate, ops.GATE_SIGMOID, xn.dtype, m=m, den_eps=self.den_eps, out_scale=self.out_scale, out=out,
         )
