@@ -2154,7 +2154,7 @@ def gated_attn_chunked(
 
 
 GATE_NONE, GATE_SIGMOID, GATE_SILU = 0, 1, 2
-_NOT_FUSED = -20  # what the launcher of `gated_attn_chunked` answers where it cannot take the norm along
+_NOT_FUSED = -20  # what the launchers of `gated_attn_chunked` and `delta_chunked` answer where they cannot take the norm along
 
 
 def head_norm_gate(
@@ -2332,10 +2332,14 @@ def delta_chunked_scratch_floats(n_tokens: int, n_seqs: int, num_heads: int, dim
 def delta_chunked(
     qn: torch.Tensor, kn: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log_decay: torch.Tensor, state: torch.Tensor, slot_ids: torch.Tensor,
     seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int, max_q_len: int, scratch: torch.Tensor, min_len: int = 1,
-) -> torch.Tensor:
+    norm=None,
+) -> Optional[torch.Tensor]:
     """`delta_rule` chunk by chunk, for prompts of bfloat16 runs: the same result within 32-bit rounding.  log_decay: float32 [T, H], the
     logarithms of the decays; v: bfloat16 rows; scratch: float32, `delta_chunked_scratch_floats` numbers.  Sequences of fewer than min_len
-    tokens are left alone, and their rows of the result undefined."""
+    tokens are left alone, and their rows of the result undefined.
+
+    norm: None, or (weight [vdim], eps, gate, gate_act, out_scale, out) as `head_norm_gate` takes them (out may be None): returns what
+    `head_norm_gate` would make of the result, in bfloat16, in the same kernels; None where they cannot (nothing is launched)."""
     T, H, G = qn.shape[0], num_heads, num_qk_heads
     for name, t, n in (("qn", qn, G * dim), ("kn", kn, G * dim), ("beta", beta, H), ("log_decay", log_decay, H)):
         _cuda(t, "delta_chunked rows", torch.float32)
@@ -2352,12 +2356,19 @@ def delta_chunked(
     _need(seq_start.numel() == S + 1, "delta_chunked: seq_start must hold one more entry than there are sequences")
     _cuda(scratch, "delta_chunked scratch", torch.float32)
     _need(scratch.numel() >= delta_chunked_scratch_floats(T, S, H, dim, vdim), "delta_chunked: scratch too small")
-    out = torch.empty((T, H * vdim), dtype=torch.float32, device=qn.device)
+    weight, eps, gate, gs, gate_act, out_scale, out = _norm_args(norm, "delta_chunked", T, H, vdim)
+    if norm is not None and weight is None:
+        return None
+    if out is None:
+        out = torch.empty((T, H * vdim), dtype=torch.float32 if norm is None else torch.bfloat16, device=qn.device)
     lib = build.load("delta_chunk")
     rc = lib.rl_delta_chunked(
         _p(qn), _p(kn), _p(v), c_int(_rows(v, "delta_chunked v")), _p(beta), _p(log_decay), _p(state), _p(slot_ids), _p(seq_start), _p(out), c_int(out.stride(0)),
-        c_int(T), c_int(S), c_int(max_q_len), c_int(H), c_int(G), c_int(dim), c_int(vdim), c_int(min_len), _p(scratch), _stream(),
+        c_int(T), c_int(S), c_int(max_q_len), c_int(H), c_int(G), c_int(dim), c_int(vdim), c_int(min_len), _p(scratch), _p(weight), c_float(eps),
+        _p(gate), c_int(gs), c_int(gate_act), c_float(out_scale), _stream(),
     )
+    if rc == _NOT_FUSED:
+        return None
     _check(lib, rc, "delta_chunked", kernels=3)
     return out
 

@@ -27,9 +27,9 @@ from .base import MIXERS, Mixer, ParamInfo, StateNeed, scratch_for_call
 # prompt steps whose longest sequence brings fewer tokens than this go token by token like a decode step; with the delta rule every sequence
 # that brings fewer does
 _CHUNKED_MIN_TOKENS = 32
-# the most scratch that the delta rule's chunks may take (2 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it, and where the
+# the most scratch that the delta rule's chunks may take (3 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it, and where the
 # device has less, token by token
-_CHUNKED_MAX_FLOATS = 1 << 29
+_CHUNKED_MAX_FLOATS = 3 << 28
 
 
 def _recurrence(mixer, q, k, v, log_decay, in_scale, state, step, ext: bool, norm=None):
@@ -331,9 +331,15 @@ class GatedDeltaRule(Mixer):
                                                        self.q_scale, log_decay=chunked)
         v, o = conv[:, 2 * self.qd :], None
         where = (memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim)
+        short = min(step.q_lens) < _CHUNKED_MIN_TOKENS
         if chunked:  # prompts of a bfloat16 run, all chunks side by side but for the walk through the state
-            o = ops.delta_chunked(qn, kn, v, beta, *log, *where, step.max_q_len, scratch, min_len=_CHUNKED_MIN_TOKENS)
-        if not chunked or min(step.q_lens) < _CHUNKED_MIN_TOKENS:
+            args = (qn, kn, v, beta, *log, *where, step.max_q_len, scratch)
+            if not short:
+                a = ops.delta_chunked(*args, norm=(self.w_norm, self.eps, gate, ops.GATE_SILU, self.out_scale, out))
+                if a is not None:
+                    return a, self.w_o
+            o = ops.delta_chunked(*args, min_len=_CHUNKED_MIN_TOKENS)
+        if not chunked or short:
             # (a sequence's own length decides: its bits do not depend on whether a prompt shares the step)
             o = ops.delta_rule(qn, kn, kq, v, beta, decay, *where, max_len=_CHUNKED_MIN_TOKENS - 1 if chunked else 0, out=o)
         a = ops.head_norm_gate(o, H, self.vdim, self.w_norm, self.eps, gate, ops.GATE_SILU, xn.dtype, out_scale=self.out_scale, out=out)

@@ -255,3 +255,56 @@ def test_a_short_sequence_gets_the_token_kernels_bits_beside_a_prompt():
         else:
             assert float((o[at : at + n] - alone[at : at + n]).norm() / alone[at : at + n].norm()) < 1e-5
         at += n
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("what", ["k", "beta", "logd"])
+def test_what_is_no_number_does_not_reach_earlier_tokens_from_elsewhere(what, value):
+    """The same for a token's key, its strength and its decay (one that grows without bound is no number either)."""
+    from rusty_llama_b200.kernels import ops
+
+    T, H, n = 150, 2, 64
+    q, k, v, beta, logd = inputs([T], H, 2, n, n, 9, "usual")
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    scratch = torch.empty(ops.delta_chunked_scratch_floats(T, 1, H, n, n), device=DEV)
+
+    def run(k, beta, logd):
+        state = torch.zeros(1, H, n, n, device=DEV)
+        out = ops.delta_chunked(q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV), v.reshape(T, -1).to(DEV), beta.to(DEV), logd.to(DEV), state, i32([0]), i32([0, T]),
+                                H, 2, n, n, T, scratch)
+        return out.view(T, H, n), state[0]
+
+    want, want_S = run(k, beta, logd)
+    for at in (0, 1, 17, 63, 64, 149):
+        bad = {"k": k.clone(), "beta": beta.clone(), "logd": logd.clone()}
+        if what == "k":
+            bad["k"][at, 0, 5] = value
+        else:
+            bad[what][at, 0] = value
+        out, S = run(**bad)
+        assert torch.equal(out[:at], want[:at]) and torch.equal(out[:, 1], want[:, 1]) and torch.equal(S[1], want_S[1]), at
+        assert not bool(out[at:, 0].isfinite().any()) and not bool(S[0].isfinite().any()), at
+
+
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (36, 72), (64, 20)])
+def test_the_norm_taken_along(dim, vdim):
+    """The same sums through the norm inside the last kernel and behind it: a rounding of each of two 32-bit chains apart, then rounded to
+    bfloat16 (2^-8 at most where that falls on different sides); wider values than a block has columns for are left to the caller."""
+    from rusty_llama_b200.kernels import ops
+
+    lens, H, G = [130, 40], 2, 1
+    q, k, v, beta, logd = inputs(lens, H, G, dim, vdim, 11, "usual")
+    T, g = sum(lens), torch.Generator().manual_seed(3)
+    gate, w = torch.randn(T, H * vdim, generator=g).to(torch.bfloat16).to(DEV), torch.randn(vdim, generator=g).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    scratch = torch.empty(ops.delta_chunked_scratch_floats(T, 2, H, dim, vdim), device=DEV)
+
+    def run(norm):
+        return ops.delta_chunked(q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV), v.reshape(T, -1).to(DEV), beta.to(DEV), logd.to(DEV),
+                                 torch.zeros(2, H, dim, vdim, device=DEV), i32([0, 1]), i32([0, 130, 170]), H, G, dim, vdim, 130, scratch, norm=norm)
+
+    got = run((w, 1e-5, gate, ops.GATE_SILU, 0.5, None))
+    want = ops.head_norm_gate(run(None), H, vdim, w, 1e-5, gate, ops.GATE_SILU, torch.bfloat16, out_scale=0.5)
+    assert got.dtype == torch.bfloat16 and float(((got.float() - want.float()).abs() / (want.float().abs() + 1e-3)).max()) <= 2.0 ** -7
+    assert float((got != want).float().mean()) <= 0.01
+    assert run((w, 1e-5, gate, ops.GATE_SILU, 0.5, torch.empty(T, H * vdim + 1, dtype=torch.bfloat16, device=DEV)[:, 1:])) is None
