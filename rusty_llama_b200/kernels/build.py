@@ -145,6 +145,75 @@ def build(name: str, verbose: bool = True) -> str:
     return out
 
 
+# ------------------------------------------------------------------ the host's module (csrc/host_calls.cpp)
+HOST_CALLS = "_rl_host_calls"
+
+
+def _host_command(out: str) -> List[str]:
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
+    flags = ["-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for inc in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"], cuda):
+        flags += ["-isystem", inc]
+    libs = ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return [shutil.which("g++") or "c++"] + flags + ["-o", out, os.path.join(CSRC_DIR, "host_calls.cpp")] + libs
+
+
+def _host_fingerprint() -> str:
+    import torch
+
+    with open(os.path.join(CSRC_DIR, "host_calls.cpp"), "rb") as f:
+        return hashlib.sha256(f.read() + f"{sys.version}|{torch.__version__}".encode()).hexdigest()
+
+
+def build_host_calls(verbose: bool = True) -> str:
+    """Compile `csrc/host_calls.cpp` against this Python and this PyTorch if that has not been done; returns the path."""
+    out = os.path.join(_build_dir(), HOST_CALLS + ".so")
+    want = _host_fingerprint()
+    if _host_is_built(out, want):
+        return out
+    if verbose:
+        _say("compiling host_calls.cpp ...")
+    tmp = f"{out}.{os.getpid()}.tmp"
+    proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if proc.returncode != 0:
+        if os.path.exists(tmp):
+            os.remove(tmp)
+        raise KernelError(f"compiling host_calls.cpp failed (exit {proc.returncode}):\n{proc.stdout}")
+    os.replace(tmp, out)
+    with open(out + ".sha256", "w") as f:
+        f.write(want)
+    return out
+
+
+def _host_is_built(out: str, want: str) -> bool:
+    try:
+        with open(out + ".sha256") as f:
+            return os.path.isfile(out) and f.read().strip() == want
+    except OSError:
+        return False
+
+
+def load_host_calls(may_build: bool):
+    """The module of `csrc/host_calls.cpp`; None where it is not built and may not be."""
+    import importlib.machinery
+    import importlib.util
+
+    out = os.path.join(_build_dir(), HOST_CALLS + ".so")
+    if not _host_is_built(out, _host_fingerprint()):
+        if not may_build:
+            return None
+        build_host_calls()
+    loader = importlib.machinery.ExtensionFileLoader(HOST_CALLS, out)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(HOST_CALLS, loader))
+    loader.exec_module(module)
+    return module
+
+
 def build_all(verbose: bool = True) -> List[str]:
     """Every source, a few at a time in parallel."""
     names = source_names()
@@ -168,7 +237,7 @@ def build_all(verbose: bool = True) -> List[str]:
     for n in names:
         if isinstance(results[n], Exception):
             raise results[n]
-    return [results[n] for n in names]
+    return [results[n] for n in names] + [build_host_calls(verbose)]
 
 
 def load(name: str) -> ctypes.CDLL:

@@ -1,0 +1,120 @@
+"""What a launch costs the host: calling the kernel libraries' launchers, checking their tensors, and the few tensor operations in between.
+
+`csrc/host_calls.cpp` does this natively (an `add_rmsnorm` with the tensor of its result: 6.2 us instead of 10.9, of which the driver has 3; a
+sublayer of nine kernels: 92 us a pass instead of 165, which is the host's time); the classes and functions below are the same in Python,
+used where that module cannot be built (no Python or PyTorch headers) and where there is no GPU to launch on.  Results and errors are the same.
+"""
+
+from __future__ import annotations
+
+import ctypes
+from typing import Dict
+
+import torch
+
+from ..errors import KernelError
+from . import build
+
+
+class PythonLauncher:
+    """A launcher called with tensors, numbers and None as they are (a float is the launcher's float, anything else an integer or pointer)."""
+
+    def __init__(self, address: int, wide: bool):
+        self.fn = ctypes.CFUNCTYPE(ctypes.c_longlong if wide else ctypes.c_int)(address)
+
+    def __call__(self, *args):
+        given = []
+        for a in args:
+            if isinstance(a, float):
+                given.append(ctypes.c_float(a))
+            elif a is None:
+                given.append(ctypes.c_void_p(0))
+            elif isinstance(a, torch.Tensor):
+                given.append(ctypes.c_void_p(a.data_ptr()))
+            else:
+                given.append(ctypes.c_longlong(a))
+        return self.fn(*given)
+
+
+def python_cuda(t: torch.Tensor, what: str, dtype=None, contiguous=True) -> torch.Tensor:
+    if not isinstance(t, torch.Tensor):
+        raise KernelError(f"{what}: not a tensor")
+    if not t.is_cuda:
+        raise KernelError(f"{what}: tensor is on {t.device}, the kernels run on CUDA only")
+    if dtype is not None and t.dtype != dtype:
+        raise KernelError(f"{what}: dtype {t.dtype}, expected {dtype}")
+    if contiguous and not t.is_contiguous():
+        raise KernelError(f"{what}: tensor is not contiguous")
+    return t
+
+
+def python_rows(t: torch.Tensor, what: str) -> int:
+    """Row stride of a 2-D tensor whose rows are dense."""
+    if t.dim() != 2 or t.stride(1) != 1:
+        raise KernelError(f"{what}: expected a 2-D tensor with dense rows")
+    return t.stride(0)
+
+
+def python_odd(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether rows of the two cannot be moved in 16-byte pieces (eight 16-bit numbers)."""
+    return bool(x.shape[1] % 8 or x.stride(0) % 8 or w.stride(0) % 8 or x.data_ptr() % 16 or w.data_ptr() % 16)
+
+
+def python_stream() -> int:
+    # (without making a Stream object: 0.3 us a launch, `torch.cuda.current_stream().cuda_stream` takes 3.3)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def python_empty(like: torch.Tensor, dtype, *sizes: int) -> torch.Tensor:
+    return torch.empty(sizes, dtype=dtype, device=like.device)
+
+
+def python_columns(t: torch.Tensor, first: int, end: int) -> torch.Tensor:
+    return t[:, first:end]
+
+
+def _native():
+    """The native module, or None.  It is built here if there is a GPU whose launches would gain from it; never for shape-only runs."""
+    try:
+        return build.load_host_calls(torch.cuda.is_available())
+    except Exception as e:  # whatever is missing on this machine: the Python side does the same
+        build._say(f"host_calls.cpp is not used: {str(e).strip().splitlines()[-1][:200] if str(e).strip() else type(e).__name__}")
+        return None
+
+
+_module = _native()
+if _module is not None:
+    _module.set_error(KernelError)
+    cuda, rows, odd, stream = _module.cuda, _module.rows, _module.odd, _module.stream
+    empty, columns, launcher = _module.empty, _module.columns, _module.launcher
+else:
+    cuda, rows, odd, stream = python_cuda, python_rows, python_odd, python_stream
+    empty, columns, launcher = python_empty, python_columns, PythonLauncher
+
+
+class Library:
+    """A kernel library's launchers as attributes, made when first asked for."""
+
+    _WIDE = ("rl_delta_chunked_scratch",)  # (what returns long long; everything else returns int)
+
+    def __init__(self, name: str):
+        self._cdll = build.load(name)
+
+    def __getattr__(self, name: str):
+        fn = launcher(ctypes.cast(getattr(self._cdll, name), ctypes.c_void_p).value, name in self._WIDE)
+        setattr(self, name, fn)
+        return fn
+
+    def rl_error_text(self) -> bytes:
+        return self._cdll.rl_error_text()
+
+
+_libraries: Dict[str, Library] = {}
+
+
+def library(name: str) -> Library:
+    """The library of `csrc/<name>.cu`, built first if need be."""
+    lib = _libraries.get(name)
+    if lib is None:
+        lib = _libraries[name] = Library(name)
+    return lib

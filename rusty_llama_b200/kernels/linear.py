@@ -19,6 +19,7 @@ import torch
 from ..errors import KernelError
 from . import ops
 from .device import sm_count
+from .host import odd as _odd  # whether the operands' rows cannot be moved in 16-byte pieces
 
 _library_gemm = False
 
@@ -33,13 +34,6 @@ def _streams(M: int, K: int, whole: bool) -> bool:
     slice (the result goes on as it is, not as partial sums)."""
     slices = ops.gemv_stream_slices(M, K, 1)
     return slices == 1 or (slices > 1 and not whole)
-
-
-def _odd(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the operands' rows cannot be moved in 16-byte pieces."""
-    return bool(
-        x.shape[1] % 8 or x.stride(0) % 8 or w.stride(0) % 8 or x.data_ptr() % 16 or w.data_ptr() % 16
-    )
 
 
 def use_library_gemm(on: bool) -> None:

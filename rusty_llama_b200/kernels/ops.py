@@ -18,6 +18,8 @@ import torch
 from ..errors import KernelError
 from . import build
 from .device import sm_count
+from .host import columns, library  # noqa: F401  (columns is for the parts)
+from .host import cuda as _cuda, empty as _empty, rows as _rows, stream as _stream
 
 PAGE_SIZE = 64  # tokens per cache page; the attention kernels' key tile
 
@@ -39,34 +41,8 @@ def _need(cond: bool, msg: str) -> None:
         raise KernelError(msg)
 
 
-def _cuda(t: torch.Tensor, what: str, dtype=None, contiguous=True) -> torch.Tensor:
-    # (a message is made only when it is raised, here and below: a launch asks several such questions of every tensor, and
-    # formatting sizes and devices for nobody took as long as the launch itself)
-    if not isinstance(t, torch.Tensor):
-        raise KernelError(f"{what}: not a tensor")
-    if not t.is_cuda:
-        raise KernelError(f"{what}: tensor is on {t.device}, the kernels run on CUDA only")
-    if dtype is not None and t.dtype != dtype:
-        raise KernelError(f"{what}: dtype {t.dtype}, expected {dtype}")
-    if contiguous and not t.is_contiguous():
-        raise KernelError(f"{what}: tensor is not contiguous")
-    return t
-
-
-def _rows(t: torch.Tensor, what: str) -> int:
-    """Row stride of a 2-D tensor whose rows are dense."""
-    if t.dim() != 2 or t.stride(1) != 1:
-        raise KernelError(f"{what}: expected a 2-D tensor with dense rows")
-    return t.stride(0)
-
-
-def _p(t: Optional[torch.Tensor]):
+def _ptr(t: Optional[torch.Tensor]):
     return c_void_p(0 if t is None else t.data_ptr())
-
-
-def _stream():
-    # (without making a Stream object: 0.3 us a launch, `torch.cuda.current_stream().cuda_stream` takes 3.3)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 _launches = 0
@@ -99,12 +75,12 @@ def embed_gather(tokens: torch.Tensor, table: torch.Tensor, out: Optional[torch.
     _need(tokens.dim() == 1 and table.dim() == 2, "embed_gather: tokens[T] and table[V, d] expected")
     T, d = tokens.numel(), table.shape[1]
     if out is None:
-        out = torch.empty((T, d), dtype=torch.float32, device=table.device)
+        out = _empty(table, torch.float32, T, d)
     _cuda(out, "embed_gather out", torch.float32)
     _need(tuple(out.shape) == (T, d), "embed_gather: out has the wrong shape")
     _need(table.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0, "embed_gather: tensors must be 16-byte aligned")
-    lib = build.load("elementwise")
-    rc = lib.rl_embed_gather(_p(tokens), _p(table), c_int(_dt(table, "embed_gather table")), _p(out), c_int(T), c_int(d), c_float(scale), _stream())
+    lib = library("elementwise")
+    rc = lib.rl_embed_gather(tokens, table, _dt(table, "embed_gather table"), out, T, d, float(scale), _stream())
     _check(lib, rc, "embed_gather")
     return out
 
@@ -155,11 +131,11 @@ def add_rmsnorm(
             raise KernelError(f"add_rmsnorm: weight {tuple(weight.shape)} does not match d={d}")
         w_dt = _dt(weight, "add_rmsnorm weight")
         if out is None:
-            out = torch.empty((n_rows, d), dtype=act_dtype, device=x.device)
+            out = _empty(x, act_dtype, n_rows, d)
         _cuda(out, "add_rmsnorm out", act_dtype)
         _need(tuple(out.shape) == (n_rows, d), "add_rmsnorm: out has the wrong shape")
     elif plain_out:
-        out = torch.empty((n_rows, d), dtype=act_dtype, device=x.device)
+        out = _empty(x, act_dtype, n_rows, d)
     else:
         _need(delta is not None, "add_rmsnorm: neither a delta nor a weight, nothing to do")
         out = None
@@ -168,10 +144,10 @@ def add_rmsnorm(
     for name, t in (("x", x), ("delta", delta), ("weight", weight), ("out", out)):
         if t is not None and t.data_ptr() % 16 != 0:
             raise KernelError(f"add_rmsnorm: {name} is not 16-byte aligned")
-    lib = build.load("elementwise")
+    lib = library("elementwise")
     rc = lib.rl_add_rmsnorm(
-        _p(x), _p(delta), c_int(delta_dt), c_int(n_parts), c_ll(part_stride), _p(weight), c_int(w_dt), _p(out),
-        c_int(_DT[act_dtype]), _p(rows), c_int(n_rows), c_int(d), c_float(eps), c_int(1 if write_x else 0), _stream(),
+        x, delta, delta_dt, n_parts, part_stride, weight, w_dt, out,
+        _DT[act_dtype], rows, n_rows, d, float(eps), 1 if write_x else 0, _stream(),
     )
     _check(lib, rc, "add_rmsnorm")
     return out
@@ -183,11 +159,11 @@ def swiglu(gate_up: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.T
     _need(gate_up.dim() == 2 and gate_up.shape[1] % 2 == 0, "swiglu: input must be [T, 2*ff]")
     T, ff = gate_up.shape[0], gate_up.shape[1] // 2
     if out is None:
-        out = torch.empty((T, ff), dtype=gate_up.dtype, device=gate_up.device)
+        out = _empty(gate_up, gate_up.dtype, T, ff)
     _cuda(out, "swiglu out", gate_up.dtype)
     _need(tuple(out.shape) == (T, ff), "swiglu: out has the wrong shape")
-    lib = build.load("elementwise")
-    rc = lib.rl_swiglu(_p(gate_up), _p(out), c_int(_dt(gate_up, "swiglu")), c_int(T), c_int(ff), _stream())
+    lib = library("elementwise")
+    rc = lib.rl_swiglu(gate_up, out, _dt(gate_up, "swiglu"), T, ff, _stream())
     _check(lib, rc, "swiglu")
     return out
 
@@ -208,8 +184,8 @@ def seq_begin_decode(state: torch.Tensor, slot_ids: torch.Tensor, tok_pos: torch
         _cuda(t, f"seq_begin_decode {name}", torch.int32)
         if t.numel() != S:
             raise KernelError(f"seq_begin_decode: {name} has {t.numel()} entries for {S} sequences")
-    lib = build.load("elementwise")
-    rc = lib.rl_seq_begin_decode(_p(state), _p(slot_ids), c_int(S), _p(tok_pos), _p(seq_pos0), _p(seq_len), _stream())
+    lib = library("elementwise")
+    rc = lib.rl_seq_begin_decode(state, slot_ids, S, tok_pos, seq_pos0, seq_len, _stream())
     _check(lib, rc, "seq_begin_decode")
 
 
@@ -221,8 +197,8 @@ def seq_set_len(state: torch.Tensor, slot_ids: torch.Tensor, seq_len: torch.Tens
     _cuda(slot_ids, "seq_set_len slot_ids", torch.int32)
     _cuda(seq_len, "seq_set_len seq_len", torch.int32)
     _need(slot_ids.numel() == seq_len.numel(), "seq_set_len: one length per sequence")
-    lib = build.load("elementwise")
-    rc = lib.rl_seq_set_len(_p(state), _p(slot_ids), _p(seq_len), c_int(slot_ids.numel()), _stream())
+    lib = library("elementwise")
+    rc = lib.rl_seq_set_len(state, slot_ids, seq_len, slot_ids.numel(), _stream())
     _check(lib, rc, "seq_set_len")
 
 
@@ -267,11 +243,11 @@ def rope_kv_write(
     if rotary_dim:
         _cuda(inv_freq, "rope_kv_write inv_freq", torch.float32)
         _need(inv_freq.numel() == rotary_dim // 2, "rope_kv_write: inv_freq must hold rotary_dim/2 values")
-    lib = build.load("rope")
+    lib = library("rope")
     rc = lib.rl_rope_kv_write(
-        _p(qkv), c_int(_dt(qkv, "rope_kv_write")), c_int(stride), _p(tok_pos), _p(tok_seq), _p(block_table), c_int(width),
-        _p(k_pages), _p(v_pages), _p(inv_freq), c_int(T), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim),
-        c_int(rotary_dim), c_int(1 if interleaved else 0), c_int(PAGE_SIZE), c_int(1 if write_kv else 0), _stream(),
+        qkv, _dt(qkv, "rope_kv_write"), stride, tok_pos, tok_seq, block_table, width,
+        k_pages, v_pages, inv_freq, T, num_heads, num_kv_heads, head_dim,
+        rotary_dim, 1 if interleaved else 0, PAGE_SIZE, 1 if write_kv else 0, _stream(),
     )
     _check(lib, rc, "rope_kv_write")
 
@@ -301,15 +277,15 @@ def attn_generic(
     _cuda(tok_pos, "attn_generic tok_pos", torch.int32)
     _need(tok_seq.numel() == T and tok_pos.numel() == T and block_table.dim() == 2, "attn_generic: metadata sizes")
     if out is None:
-        out = torch.empty((T, num_heads * head_dim), dtype=q.dtype, device=q.device)
+        out = _empty(q, q.dtype, T, num_heads * head_dim)
     _cuda(out, "attn_generic out", q.dtype)
     if scale is None:
         scale = 1.0 / math.sqrt(head_dim)
-    lib = build.load("attention_generic")
+    lib = library("attention_generic")
     rc = lib.rl_attn_generic(
-        _p(q), c_int(_dt(q, "attn_generic")), c_int(qs), _p(k_pages), _p(v_pages), _p(block_table),
-        c_int(block_table.shape[1]), _p(tok_seq), _p(tok_pos), _p(out), c_int(out.stride(0)), c_int(T),
-        c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(PAGE_SIZE), c_int(window), c_float(scale), c_int(sm_count(q.device)), _stream(),
+        q, _dt(q, "attn_generic"), qs, k_pages, v_pages, block_table,
+        block_table.shape[1], tok_seq, tok_pos, out, out.stride(0), T,
+        num_heads, num_kv_heads, head_dim, PAGE_SIZE, window, float(scale), sm_count(q.device), _stream(),
     )
     _check(lib, rc, "attn_generic")
     return out
@@ -334,11 +310,11 @@ def _bias_args(bias, num_heads: int, what: str):
     """A learned bias by head and distance: None, or float32 [H, L]; a score of head h and a key n positions behind its query is
     raised by bias[h, min(n, L - 1)], after everything else that makes the score."""
     if bias is None:
-        return c_void_p(0), c_int(0)
+        return None, 0
     _cuda(bias, f"{what} bias", torch.float32)
     if not (bias.dim() == 2 and bias.shape[0] == num_heads and bias.shape[1] > 0):
         raise KernelError(f"{what}: bias {tuple(bias.shape)} for {num_heads} heads")
-    return _p(bias), c_int(bias.shape[1])
+    return bias, bias.shape[1]
 
 
 def attn_decode_scratch_floats(n_seqs: int, num_heads: int, head_dim: int, n_splits: int) -> int:
@@ -407,14 +383,14 @@ def attn_decode(
     if scratch.numel() < need:
         raise KernelError(f"attn_decode: scratch holds {scratch.numel()} floats, {need} needed")
     if out is None:
-        out = torch.empty((S, num_heads // maps * vdim), dtype=act, device=q.device)
+        out = _empty(q, act, S, num_heads // maps * vdim)
     _cuda(out, "attn_decode out", act, contiguous=False)
     _need(_rows(out, "attn_decode out") >= out.shape[1] and tuple(out.shape) == (S, num_heads // maps * vdim), "attn_decode: out must be [S, H value_dim] rows")
     if scale is None:
         scale = 1.0 / math.sqrt(head_dim)
     n_o = S * num_heads * n_splits * vdim
-    part_o = c_void_p(scratch.data_ptr())
-    part_ml = c_void_p(scratch.data_ptr() + 4 * n_o)
+    part_o = scratch.data_ptr()
+    part_ml = scratch.data_ptr() + 4 * n_o
     if impl not in ("auto", "warp", "tma"):
         raise KernelError(f"attn_decode: unknown impl {impl!r}")
     if impl == "auto":
@@ -439,27 +415,27 @@ def attn_decode(
     if impl == "tma":
         _need(act == torch.bfloat16, "attn_decode: the TMA kernel is bfloat16 only")
         status = _tc_status_word(q.device)
-        lib = build.load("attention_decode_tma")
+        lib = library("attention_decode_tma")
         rc = lib.rl_attn_decode_tma(
-            c_void_p(0) if q_parts is not None else _p(q), c_int(qs), _p(k_pages), _p(v_pages), c_int(k_pages.shape[0]), _p(block_table),
-            c_int(block_table.shape[1]), _p(seq_len), part_o, part_ml, _p(out), c_int(out.stride(0)), c_int(S),
-            c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(vdim), c_int(PAGE_SIZE), c_int(window), c_float(scale),
-            c_int(n_splits), _p(status), c_int(fuse), _p(inv_freq) if (fuse and rotary_dim) else c_void_p(0), c_int(rotary_dim if fuse else 0),
-            c_int(1 if interleaved else 0), _p(counters) if counters is not None else c_void_p(0),
-            _p(q_parts) if q_parts is not None else c_void_p(0), c_int(0 if q_parts is None else q_parts.shape[0]),
-            c_ll(0 if q_parts is None else q_parts.stride(0)), *_wt(), _p(sink), c_int(chunk), c_float(softcap), c_int(maps),
-            *(c_float(x) for x in (pair or (0.0, 0.0, 0.0))), *_bias_args(bias, num_heads, "attn_decode"), _stream(),
+            None if q_parts is not None else q, qs, k_pages, v_pages, k_pages.shape[0], block_table,
+            block_table.shape[1], seq_len, part_o, part_ml, out, out.stride(0), S,
+            num_heads, num_kv_heads, head_dim, vdim, PAGE_SIZE, window, float(scale),
+            n_splits, status, fuse, inv_freq if (fuse and rotary_dim) else None, rotary_dim if fuse else 0,
+            1 if interleaved else 0, counters if counters is not None else None,
+            q_parts if q_parts is not None else None, 0 if q_parts is None else q_parts.shape[0],
+            0 if q_parts is None else q_parts.stride(0), *_wt(), sink, chunk, float(softcap), maps,
+            *(float(x) for x in (pair or (0.0, 0.0, 0.0))), *_bias_args(bias, num_heads, "attn_decode"), _stream(),
         )
         _check(lib, rc, "attn_decode_tma", kernels=1 if counters is not None else 2)
         return out
     _need(chunk == 0 and softcap == 0.0 and pair is None and bias is None and vdim == head_dim,
           "attn_decode: only the TMA kernel takes chunks, capped scores, a bias, values of another size and two maps per head")
-    lib = build.load("attention_decode")
+    lib = library("attention_decode")
     rc = lib.rl_attn_decode_sink(
-        _p(q), c_int(_dt(q, "attn_decode")), c_int(qs), _p(k_pages), _p(v_pages), _p(block_table),
-        c_int(block_table.shape[1]), _p(seq_len), part_o, part_ml, _p(out), c_int(out.stride(0)), c_int(S),
-        c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(PAGE_SIZE), c_int(window), c_float(scale),
-        c_int(n_splits), _p(sink), _stream(),
+        q, _dt(q, "attn_decode"), qs, k_pages, v_pages, block_table,
+        block_table.shape[1], seq_len, part_o, part_ml, out, out.stride(0), S,
+        num_heads, num_kv_heads, head_dim, PAGE_SIZE, window, float(scale),
+        n_splits, sink, _stream(),
     )
     _check(lib, rc, "attn_decode", kernels=2)
     return out
@@ -483,16 +459,16 @@ def flash_prefill(
     S = seq_pos0.numel()
     _need(seq_start.numel() == S + 1 and block_table.dim() == 2 and block_table.shape[0] >= S, "flash_prefill: metadata sizes")
     if out is None:
-        out = torch.empty((T, num_heads * head_dim), dtype=torch.bfloat16, device=q.device)
+        out = _empty(q, torch.bfloat16, T, num_heads * head_dim)
     _cuda(out, "flash_prefill out", torch.bfloat16)
     if scale is None:
         scale = 1.0 / math.sqrt(head_dim)
     _check_sink(sink, num_heads, "flash_prefill")
-    lib = build.load("attention_prefill")
+    lib = library("attention_prefill")
     rc = lib.rl_flash_prefill(
-        _p(q), c_int(qs), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]), _p(seq_start),
-        _p(seq_pos0), _p(out), c_int(out.stride(0)), c_int(S), c_int(max_q_len), c_int(num_heads),
-        c_int(num_kv_heads), c_int(head_dim), c_int(PAGE_SIZE), c_int(window), c_float(scale), _p(sink), _stream(),
+        q, qs, k_pages, v_pages, block_table, block_table.shape[1], seq_start,
+        seq_pos0, out, out.stride(0), S, max_q_len, num_heads,
+        num_kv_heads, head_dim, PAGE_SIZE, window, float(scale), sink, _stream(),
     )
     _check(lib, rc, "flash_prefill")
     return out
@@ -530,19 +506,19 @@ def flash_prefill_tc(
     S = seq_pos0.numel()
     _need(seq_start.numel() == S + 1 and block_table.dim() == 2 and block_table.shape[0] >= S, "flash_prefill_tc: metadata sizes")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=torch.bfloat16, device=q.device)
+        out = _empty(q, torch.bfloat16, T, num_heads * vdim)
     _cuda(out, "flash_prefill_tc out", torch.bfloat16, contiguous=False)
     _need(_rows(out, "flash_prefill_tc out") % 8 == 0 and tuple(out.shape) == (T, num_heads * vdim), "flash_prefill_tc: out must be [T, H value_dim] rows at 16-byte steps")
     if scale is None:
         scale = 1.0 / math.sqrt(head_dim)
     _check_sink(sink, num_heads, "flash_prefill_tc")
     status = _tc_status_word(q.device)
-    lib = build.load("attention_prefill_tc")
+    lib = library("attention_prefill_tc")
     rc = lib.rl_flash_prefill_tc(
-        _p(q), c_int(qs), c_int(T), _p(k_pages), _p(v_pages), c_int(k_pages.shape[0]), _p(block_table),
-        c_int(block_table.shape[1]), _p(seq_start), _p(seq_pos0), _p(out), c_int(out.stride(0)), c_int(S), c_int(max_q_len),
-        c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(vdim), c_int(PAGE_SIZE), c_int(window), c_float(scale), _p(status), *_wt(), _p(sink),
-        c_int(chunk), c_float(softcap), c_int(maps), *_bias_args(bias, num_heads, "flash_prefill_tc"), _stream(),
+        q, qs, T, k_pages, v_pages, k_pages.shape[0], block_table,
+        block_table.shape[1], seq_start, seq_pos0, out, out.stride(0), S, max_q_len,
+        num_heads, num_kv_heads, head_dim, vdim, PAGE_SIZE, window, float(scale), status, *_wt(), sink,
+        chunk, float(softcap), maps, *_bias_args(bias, num_heads, "flash_prefill_tc"), _stream(),
     )
     _check(lib, rc, "flash_prefill_tc")
     return out
@@ -562,12 +538,12 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     if w.shape[1] != K:
         raise KernelError(f"gemm_f32: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
     if out is None:
-        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+        out = _empty(x, torch.float32, M, N)
     _cuda(out, "gemm_f32 out", torch.float32, contiguous=False)
     _need(tuple(out.shape) == (M, N), "gemm_f32: out has the wrong shape")
-    lib = build.load("gemm_f32")
-    rc = lib.rl_gemm_f32(_p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_rows(out, "gemm_f32 out")), c_int(M), c_int(N), c_int(K),
-                         c_int(sm_count(x.device)), _stream())
+    lib = library("gemm_f32")
+    rc = lib.rl_gemm_f32(x, ldx, w, ldw, out, _rows(out, "gemm_f32 out"), M, N, K,
+                         sm_count(x.device), _stream())
     _check(lib, rc, "gemm_f32")
     return out
 
@@ -579,15 +555,15 @@ def _act(act):
     """(alpha, limit) of a gate/up product's activation as the launchers take it: None is silu(gate) * up.
     "relu2": the code with which a product that is NOT a gate/up product sends its sums through relu(x)^2."""
     if act is None:
-        return c_float(1.0), c_float(0.0)
+        return 1.0, 0.0
     if act == "relu2":
-        return c_float(0.0), c_float(-2.0)
+        return 0.0, -2.0
     if act == "gelu_tanh":  # gelu(gate) * up, the tanh form (RL_GATED_GELU_TANH of csrc/common.cuh)
-        return c_float(0.0), c_float(-3.0)
+        return 0.0, -3.0
     alpha, limit = act
     if not (limit > 0):
         raise KernelError(f"a gated activation with limits needs a positive limit, got {limit}")
-    return c_float(alpha), c_float(limit)
+    return float(alpha), float(limit)
 
 
 def gemm_bf16_any(
@@ -604,11 +580,11 @@ def gemm_bf16_any(
     N = w.shape[0]
     if w.shape[1] != K:
         raise KernelError(f"gemm_bf16_any: x[{M}, {K}] against w[{N}, {w.shape[1]}]")
-    out = torch.empty((M, N // 2 if swiglu else N), dtype=out_dtype, device=x.device)
-    lib = build.load("gemm_f32")
+    out = _empty(x, out_dtype, M, N // 2 if swiglu else N)
+    lib = library("gemm_f32")
     rc = lib.rl_gemm_bf16_any(
-        _p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_dt(out, "gemm_bf16_any out")), c_int(out.shape[1]),
-        c_int(M), c_int(N), c_int(K), c_int(1 if swiglu else 0), *_act(act), _stream(),
+        x, ldx, w, ldw, out, _dt(out, "gemm_bf16_any out"), out.shape[1],
+        M, N, K, 1 if swiglu else 0, *_act(act), _stream(),
     )
     _check(lib, rc, "gemm_bf16_any")
     return out
@@ -637,20 +613,20 @@ def gemv_bf16(
     if k_splits > 1:
         _need(out_dtype == torch.float32 and not swiglu, "gemv_bf16: partial sums over k slices are float32, without activation")
         if out is None:
-            out = torch.empty((k_splits, M, n_out), dtype=torch.float32, device=x.device)
+            out = _empty(x, torch.float32, k_splits, M, n_out)
         _cuda(out, "gemv_bf16 out", torch.float32)
         _need(tuple(out.shape) == (k_splits, M, n_out), "gemv_bf16: out has the wrong shape")
         ldo = n_out
     else:
         if out is None:
-            out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+            out = _empty(x, out_dtype, M, n_out)
         _cuda(out, "gemv_bf16 out", out_dtype, contiguous=False)
         _need(tuple(out.shape) == (M, n_out), "gemv_bf16: out has the wrong shape")
         ldo = _rows(out, "gemv_bf16 out")
-    lib = build.load("gemv_bf16")
+    lib = library("gemv_bf16")
     rc = lib.rl_gemv_bf16(
-        _p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_dt(out, "gemv_bf16 out")), c_int(ldo),
-        c_int(M), c_int(N), c_int(K), c_int(1 if swiglu else 0), *_act(act), c_int(k_splits), _stream(),
+        x, ldx, w, ldw, out, _dt(out, "gemv_bf16 out"), ldo,
+        M, N, K, 1 if swiglu else 0, *_act(act), k_splits, _stream(),
     )
     _check(lib, rc, "gemv_bf16")
     return out
@@ -660,8 +636,8 @@ def gemv_stream_slices(M: int, K: int, k_splits: int = 1) -> int:
     """How many slices of k `gemv_stream` produces for these arguments: 1 is a finished result, more
     are float32 partial sums, 0 means that the kernel does not take the shape (more than 16 rows, k
     no multiple of 64).  A slice is at most 4096 long, or 5120 when k is longer than 4096, so longer k always comes in slices."""
-    lib = build.load("gemv_stream")
-    return int(lib.rl_gemv_stream_slices(c_int(M), c_int(K), c_int(k_splits)))
+    lib = library("gemv_stream")
+    return int(lib.rl_gemv_stream_slices(M, K, k_splits))
 
 
 def gemv_stream_into_stream(
@@ -683,23 +659,23 @@ def gemv_stream_into_stream(
     N = w.shape[0]
     if not (w.shape[1] == K and tuple(resid.shape) == (M, N) and tuple(next_w.shape) == (N,)):
         raise KernelError(f"gemv_stream_into_stream: x{tuple(x.shape)} w{tuple(w.shape)} resid{tuple(resid.shape)} next_w{tuple(next_w.shape)} do not fit")
-    lib = build.load("gemv_stream")
-    blocks = int(lib.rl_gemv_stream_blocks(c_int(N), c_int(K)))
+    lib = library("gemv_stream")
+    blocks = int(lib.rl_gemv_stream_blocks(N, K))
     if blocks <= 0:
         raise KernelError(f"gemv_stream_into_stream: the kernel does not take N={N}, K={K}")
     if xw is None:
-        xw = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+        xw = _empty(x, torch.bfloat16, M, N)
     if sumsq is None:
-        sumsq = torch.empty(blocks * 8, dtype=torch.float32, device=x.device)
+        sumsq = _empty(x, torch.float32, blocks * 8)
     _cuda(xw, "gemv_stream_into_stream xw", torch.bfloat16, contiguous=False)
     _cuda(sumsq, "gemv_stream_into_stream sumsq", torch.float32)
     _need(tuple(xw.shape) == (M, N) and sumsq.numel() >= blocks * 8, "gemv_stream_into_stream: xw or sumsq of the wrong size")
     used = c_int(0)
     status = _tc_status_word(x.device)
     rc = lib.rl_gemv_stream_into_stream(
-        _p(x), c_int(_rows(x, "gemv_stream_into_stream x")), _p(w), c_int(_rows(w, "gemv_stream_into_stream w")), _p(resid),
-        c_int(_rows(resid, "gemv_stream_into_stream resid")), _p(next_w), c_int(_dt(next_w, "gemv_stream_into_stream next_w")), _p(xw),
-        c_int(_rows(xw, "gemv_stream_into_stream xw")), _p(sumsq), c_int(M), c_int(N), c_int(K), ctypes.byref(used), _p(status), *_wt(), _stream(),
+        x, _rows(x, "gemv_stream_into_stream x"), w, _rows(w, "gemv_stream_into_stream w"), resid,
+        _rows(resid, "gemv_stream_into_stream resid"), next_w, _dt(next_w, "gemv_stream_into_stream next_w"), xw,
+        _rows(xw, "gemv_stream_into_stream xw"), sumsq, M, N, K, ctypes.addressof(used), status, *_wt(), _stream(),
     )
     _check(lib, rc, "gemv_stream_into_stream")
     if used.value != blocks:
@@ -737,29 +713,29 @@ def gemv_stream(
         raise KernelError(f"gemv_stream: k = {K} comes in {slices} slices, whose float32 partial sums have to be asked for (k_splits > 1)")
     if k_splits > 1 and slices > 1:
         _need(out is None and out_dtype == torch.float32 and not swiglu, "gemv_stream: partial sums over k slices are float32, without activation")
-        out = torch.empty((slices, M, n_out), dtype=torch.float32, device=x.device)
+        out = _empty(x, torch.float32, slices, M, n_out)
         ldo = n_out
     else:
         if out is None:
-            out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+            out = _empty(x, out_dtype, M, n_out)
         _cuda(out, "gemv_stream out", out_dtype, contiguous=False)
         _need(tuple(out.shape) == (M, n_out), "gemv_stream: out has the wrong shape")
         ldo = _rows(out, "gemv_stream out")
     status = _tc_status_word(x.device)
-    lib = build.load("gemv_stream")
+    lib = library("gemv_stream")
     if row_scale is not None:
         sumsq, blocks, norm_k, eps = row_scale
         _cuda(sumsq, "gemv_stream row_scale", torch.float32)
         _need(k_splits == 1 and slices == 1 and sumsq.numel() >= blocks * 8, "gemv_stream: a row scale goes with whole sums and needs its shares")
         rc = lib.rl_gemv_stream_scaled(
-            _p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_dt(out, "gemv_stream out")), c_int(ldo), c_int(M), c_int(N), c_int(K),
-            c_int(1 if swiglu else 0), *_act(act), _p(sumsq), c_int(blocks), c_int(norm_k), c_float(eps), _p(status), *_wt(), _stream(),
+            x, ldx, w, ldw, out, _dt(out, "gemv_stream out"), ldo, M, N, K,
+            1 if swiglu else 0, *_act(act), sumsq, blocks, norm_k, float(eps), status, *_wt(), _stream(),
         )
         _check(lib, rc, "gemv_stream")
         return out
     rc = lib.rl_gemv_stream(
-        _p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_dt(out, "gemv_stream out")), c_int(ldo),
-        c_int(M), c_int(N), c_int(K), c_int(1 if swiglu else 0), *_act(act), c_int(k_splits), ctypes.byref(used), _p(status), *_wt(), _stream(),
+        x, ldx, w, ldw, out, _dt(out, "gemv_stream out"), ldo,
+        M, N, K, 1 if swiglu else 0, *_act(act), k_splits, ctypes.addressof(used), status, *_wt(), _stream(),
     )
     _check(lib, rc, "gemv_stream")
     if used.value != slices:
@@ -792,14 +768,14 @@ class short_wait:
 
 
 def _wt():
-    return c_int(_wait_test[0]), ctypes.c_uint(_wait_test[1])
+    return _wait_test[0], _wait_test[1]
 
 
 def _tc_status_word(device: torch.device) -> torch.Tensor:
-    key = (device.type, device.index)
-    if key not in _tc_status:
-        _tc_status[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _tc_status[key]
+    word = _tc_status.get(device)
+    if word is None:
+        word = _tc_status[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return word
 
 
 _STATUS_NAMES = {
@@ -858,19 +834,19 @@ def gemm_tc(
         slices = (K + 63) // 64
         per = (slices + min(k_splits, slices) - 1) // min(k_splits, slices)
         k_splits = (slices + per - 1) // per
-        out = torch.empty((k_splits, M, n_out), dtype=torch.float32, device=x.device)
+        out = _empty(x, torch.float32, k_splits, M, n_out)
         ldo = n_out
     else:
         if out is None:
-            out = torch.empty((M, n_out), dtype=out_dtype, device=x.device)
+            out = _empty(x, out_dtype, M, n_out)
         _cuda(out, "gemm_tc out", out_dtype, contiguous=False)
         _need(tuple(out.shape) == (M, n_out), "gemm_tc: out has the wrong shape")
         ldo = _rows(out, "gemm_tc out")
     status = _tc_status_word(x.device)
-    lib = build.load("gemm_tc")
+    lib = library("gemm_tc")
     rc = lib.rl_gemm_tc(
-        _p(x), c_int(ldx), _p(w), c_int(ldw), _p(out), c_int(_dt(out, "gemm_tc out")), c_int(ldo),
-        c_int(M), c_int(N), c_int(K), c_int(1 if swiglu else 0), *_act(act), c_int(k_splits), ctypes.byref(used), c_int(tile_n), _p(status), *_wt(), _stream(),
+        x, ldx, w, ldw, out, _dt(out, "gemm_tc out"), ldo,
+        M, N, K, 1 if swiglu else 0, *_act(act), k_splits, ctypes.addressof(used), tile_n, status, *_wt(), _stream(),
     )
     _check(lib, rc, "gemm_tc")
     if k_splits > 1:
@@ -886,10 +862,10 @@ def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Te
     stride = _rows(logits, "argmax logits")
     R, n = logits.shape
     if out is None:
-        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        out = _empty(logits, torch.int32, R)
     _cuda(out, "argmax out", torch.int32)
-    lib = build.load("sampling")
-    rc = lib.rl_argmax(_p(logits), c_ll(stride), c_int(R), c_int(n), _p(out), _stream())
+    lib = library("sampling")
+    rc = lib.rl_argmax(logits, stride, R, n, out, _stream())
     _check(lib, rc, "argmax")
     return out
 
@@ -912,12 +888,12 @@ def sample(
     if scratch.numel() < R * n:
         raise KernelError(f"sample: scratch holds {scratch.numel()} floats, {R * n} needed")
     if out is None:
-        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        out = _empty(logits, torch.int32, R)
     _cuda(out, "sample out", torch.int32)
-    lib = build.load("sampling")
+    lib = library("sampling")
     rc = lib.rl_sample(
-        _p(logits), c_ll(stride), c_int(R), c_int(n), c_float(temperature), c_float(top_p), _p(rng_states),
-        _p(rng_index), _p(scratch), _p(out), _stream(),
+        logits, stride, R, n, float(temperature), float(top_p), rng_states,
+        rng_index, scratch, out, _stream(),
     )
     _check(lib, rc, "sample")
     return out
@@ -962,7 +938,7 @@ def sample_chain(
         raise KernelError(f"sample_chain: work holds {work.numel()} floats, {need} needed")
     _need(work.data_ptr() % 16 == 0, "sample_chain: work must be 16-byte aligned")
     if out is None:
-        out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+        out = _empty(logits, torch.int32, R)
     _cuda(out, "sample_chain out", torch.int32)
     if mirostat:
         _need(mirostat_mu is not None, "sample_chain: mirostat needs its state")
@@ -973,15 +949,15 @@ def sample_chain(
         _cuda(xtc_states, "sample_chain xtc_states", torch.int64)
         _need(xtc_states.numel() == history_count.numel(), "sample_chain: one XTC state per slot")
     breakers = (ctypes.c_int * max(len(dry_breakers), 1))(*[int(b) for b in dry_breakers])
-    lib = build.load("sampling")
+    lib = build.load("sampling")  # (more floats than a native call takes)
     rc = lib.rl_sample_chain(
-        _p(logits), c_ll(stride), c_int(R), c_int(n), c_float(temperature), c_float(top_p), c_int(top_k), c_float(min_p),
+        _ptr(logits), c_ll(stride), c_int(R), c_int(n), c_float(temperature), c_float(top_p), c_int(top_k), c_float(min_p),
         c_float(repeat_penalty), c_int(last_n), c_float(frequency_penalty), c_float(presence_penalty), c_int(mirostat),
         c_float(mirostat_tau), c_float(mirostat_eta), c_float(xtc_probability), c_float(xtc_threshold),
         c_float(dry_multiplier), c_float(dry_base), c_int(dry_allowed_length), c_int(dry_last_n), breakers, c_int(len(dry_breakers)),
-        _p(rng_states),
-        _p(slot_of_row), _p(history), _p(history_count), _p(mirostat_mu) if mirostat_mu is not None else c_void_p(0),
-        _p(xtc_states) if xtc_states is not None else c_void_p(0), _p(work), _p(out), _stream(),
+        _ptr(rng_states),
+        _ptr(slot_of_row), _ptr(history), _ptr(history_count), _ptr(mirostat_mu) if mirostat_mu is not None else c_void_p(0),
+        _ptr(xtc_states) if xtc_states is not None else c_void_p(0), _ptr(work), _ptr(out), c_void_p(_stream()),
     )
     _check(lib, rc, "sample_chain")
     return out
@@ -1017,7 +993,7 @@ def normed_add_rmsnorm(
         _cuda(weight, "normed_add_rmsnorm weight", delta_weight.dtype)
         _need(tuple(weight.shape) == (d,), "normed_add_rmsnorm: weight does not match d")
     if weight is not None or plain_out:
-        out = torch.empty((n_rows, d), dtype=act_dtype, device=x.device)
+        out = _empty(x, act_dtype, n_rows, d)
     if rows is not None:
         _cuda(rows, "normed_add_rmsnorm rows", torch.int32)
     if delta_bias is not None:
@@ -1025,11 +1001,11 @@ def normed_add_rmsnorm(
         _need(tuple(delta_bias.shape) == (d,) and delta_bias.data_ptr() % 16 == 0, "normed_add_rmsnorm: delta_bias must be an aligned row of d numbers")
     if n_rows == 0:
         return out
-    lib = build.load("elementwise")
+    lib = library("elementwise")
     rc = lib.rl_normed_add_rmsnorm(
-        _p(x), _p(delta), c_int(_DT[delta.dtype]), c_int(n_parts), c_ll(part_stride), _p(delta_bias), _p(delta_weight), c_float(delta_eps), _p(weight),
-        c_int(_dt(delta_weight, "normed_add_rmsnorm weight")), c_float(eps), _p(out), c_int(_DT[act_dtype]), _p(rows), c_int(n_rows),
-        c_int(d), c_int(1 if write_x else 0), _stream(),
+        x, delta, _DT[delta.dtype], n_parts, part_stride, delta_bias, delta_weight, float(delta_eps), weight,
+        _dt(delta_weight, "normed_add_rmsnorm weight"), float(eps), out, _DT[act_dtype], rows, n_rows,
+        d, 1 if write_x else 0, _stream(),
     )
     _check(lib, rc, "normed_add_rmsnorm")
     return out
@@ -1073,17 +1049,17 @@ def gated_add_rmsnorm(
         _cuda(weight, "gated_add_rmsnorm weight")
         _need(tuple(weight.shape) == (d,), "gated_add_rmsnorm: weight does not match d")
         w_dt = _dt(weight, "gated_add_rmsnorm weight")
-        out = torch.empty((n_rows, d), dtype=act_dtype, device=x.device)
+        out = _empty(x, act_dtype, n_rows, d)
     else:
         _need(delta is not None, "gated_add_rmsnorm: neither a delta nor a weight, nothing to do")
     if rows is not None:
         _cuda(rows, "gated_add_rmsnorm rows", torch.int32)
     if n_rows == 0:
         return out
-    lib = build.load("elementwise")
+    lib = library("elementwise")
     rc = lib.rl_gated_add_rmsnorm(
-        _p(x), _p(delta), c_int(delta_dt), c_int(n_parts), c_ll(part_stride), _p(z), c_int(zs), _p(bias), _p(weight), c_int(w_dt), _p(out),
-        c_int(_DT[act_dtype]), _p(rows), c_int(n_rows), c_int(d), c_int(groups), c_float(eps), c_int(1 if write_x else 0), _stream(),
+        x, delta, delta_dt, n_parts, part_stride, z, zs, bias, weight, w_dt, out,
+        _DT[act_dtype], rows, n_rows, d, groups, float(eps), 1 if write_x else 0, _stream(),
     )
     _check(lib, rc, "gated_add_rmsnorm")
     return out
@@ -1093,8 +1069,8 @@ def scale_softcap(y: torch.Tensor, scale: float, cap: float = 0.0) -> torch.Tens
     """y <- y * scale, then y <- cap tanh(y / cap) if cap > 0; in place, float32 (dense)."""
     _cuda(y, "scale_softcap y", torch.float32)
     if y.numel():
-        lib = build.load("elementwise")
-        rc = lib.rl_scale_softcap(_p(y), c_ll(y.numel()), c_float(scale), c_float(cap), _stream())
+        lib = library("elementwise")
+        rc = lib.rl_scale_softcap(y, y.numel(), float(scale), float(cap), _stream())
         _check(lib, rc, "scale_softcap")
     return y
 
@@ -1103,7 +1079,7 @@ def gated_glu(gate_up: torch.Tensor, act) -> torch.Tensor:
     """h[t, i] = act(gate_up[t, i], gate_up[t, ff + i]) for the activations of a gate/up product (None: silu(gate) * up,
     (alpha, limit): the clamped form, "gelu_tanh": gelu(gate) * up), as a pass of its own behind a plain product."""
     alpha, limit = _act(act)
-    return clamped_glu(gate_up, alpha.value, limit.value)
+    return clamped_glu(gate_up, alpha, limit)
 
 
 def clamped_glu(gate_up: torch.Tensor, alpha: float, limit: float) -> torch.Tensor:
@@ -1111,9 +1087,9 @@ def clamped_glu(gate_up: torch.Tensor, alpha: float, limit: float) -> torch.Tens
     _cuda(gate_up, "clamped_glu input")
     _need(gate_up.dim() == 2 and gate_up.shape[1] % 2 == 0, "clamped_glu: input must be [T, 2*ff]")
     T, ff = gate_up.shape[0], gate_up.shape[1] // 2
-    out = torch.empty((T, ff), dtype=gate_up.dtype, device=gate_up.device)
-    lib = build.load("elementwise")
-    rc = lib.rl_clamped_glu(_p(gate_up), _p(out), c_int(_dt(gate_up, "clamped_glu")), c_int(T), c_int(ff), c_float(alpha), c_float(limit), _stream())
+    out = _empty(gate_up, gate_up.dtype, T, ff)
+    lib = library("elementwise")
+    rc = lib.rl_clamped_glu(gate_up, out, _dt(gate_up, "clamped_glu"), T, ff, float(alpha), float(limit), _stream())
     _check(lib, rc, "clamped_glu")
     return out
 
@@ -1166,13 +1142,13 @@ def latent_prep(
         ldql, q_rank = _rows(q_latent, "latent_prep q_latent"), q_latent.shape[1]
         _cuda(q_norm, "latent_prep q_norm", torch.float32)
         _need(q_latent.shape[0] == T and q_norm.numel() == q_rank, "latent_prep: the query latent's rows or norm weight do not fit")
-        ql_out = torch.empty((T, q_rank), dtype=dt, device=q_latent.device)
-    lib = build.load("latent_attention")
+        ql_out = _empty(q_latent, dt, T, q_rank)
+    lib = library("latent_attention")
     rc = lib.rl_latent_prep(
-        _p(q), c_int(ldq), _p(kv), c_int(ldkv), c_int(_dt(some, "latent_prep")), _p(norm_w), c_float(eps), _p(freq), c_int(n_pairs),
-        c_int(1 if interleaved else 0), c_float(magnitude), _p(tok_pos), _p(tok_seq), _p(block_table) if kv is not None else c_void_p(0), c_int(width),
-        _p(pages) if kv is not None else c_void_p(0), c_int(PAGE_SIZE), _p(q_cat) if q is not None else c_void_p(0), c_int(T), c_int(num_heads),
-        c_int(dim), c_int(rot), c_int(rank), _p(q_latent), c_int(ldql), c_int(q_rank), _p(q_norm), _p(ql_out), c_int(1 if in_place and q is not None else 0), _stream(),
+        q, ldq, kv, ldkv, _dt(some, "latent_prep"), norm_w, float(eps), freq, n_pairs,
+        1 if interleaved else 0, float(magnitude), tok_pos, tok_seq, block_table if kv is not None else None, width,
+        pages if kv is not None else None, PAGE_SIZE, q_cat if q is not None else None, T, num_heads,
+        dim, rot, rank, q_latent, ldql, q_rank, q_norm, ql_out, 1 if in_place and q is not None else 0, _stream(),
     )
     _check(lib, rc, "latent_prep")
     return ql_out
@@ -1206,24 +1182,24 @@ def head_linear(
         _need(gate.shape[0] == M and (H - 1) * gate_head_stride + N <= gate.shape[1], "head_linear: gate rows do not fit")
     if x.dtype == torch.bfloat16 and grouped_gemm_takes(K, ldx, x_head_stride) and x.data_ptr() % 16 == 0:
         if M > HEAD_LINEAR_MMA_MAX_ROWS and w.data_ptr() % 16 == 0:
-            lib = build.load("grouped_gemm_tc")
+            lib = library("grouped_gemm_tc")
             rc = lib.rl_head_linear_tc(
-                _p(x), c_int(ldx), c_int(x_head_stride), _p(w), _p(out), c_int(ldo), c_int(out_head_stride), _p(gate), c_int(ldg),
-                c_int(gate_head_stride), c_int(M), c_int(H), c_int(N), c_int(K), _p(held), c_int(seq_rows), _p(_tc_status_word(x.device)), *_wt(), _stream(),
+                x, ldx, x_head_stride, w, out, ldo, out_head_stride, gate, ldg,
+                gate_head_stride, M, H, N, K, held, seq_rows, _tc_status_word(x.device), *_wt(), _stream(),
             )
             _check(lib, rc, "head_linear_tc")
             return out
-        lib = build.load("grouped_gemm")
+        lib = library("grouped_gemm")
         rc = lib.rl_head_linear_mma(
-            _p(x), c_int(ldx), c_int(x_head_stride), _p(w), _p(out), c_int(ldo), c_int(out_head_stride), _p(gate), c_int(ldg),
-            c_int(gate_head_stride), c_int(M), c_int(H), c_int(N), c_int(K), _stream(),
+            x, ldx, x_head_stride, w, out, ldo, out_head_stride, gate, ldg,
+            gate_head_stride, M, H, N, K, _stream(),
         )
         _check(lib, rc, "head_linear_mma")
         return out
-    lib = build.load("latent_attention")
+    lib = library("latent_attention")
     rc = lib.rl_head_linear(
-        _p(x), c_int(ldx), c_int(x_head_stride), _p(w), c_ll(N * K), c_int(K), c_int(1), _p(out), c_int(ldo), c_int(out_head_stride),
-        _p(gate), c_int(ldg), c_int(gate_head_stride), c_int(_dt(x, "head_linear")), c_int(M), c_int(H), c_int(N), c_int(K), _stream(),
+        x, ldx, x_head_stride, w, N * K, K, 1, out, ldo, out_head_stride,
+        gate, ldg, gate_head_stride, _dt(x, "head_linear"), M, H, N, K, _stream(),
     )
     _check(lib, rc, "head_linear")
     return out
@@ -1248,16 +1224,16 @@ def latent_expand(
         raise KernelError(f"latent_expand: pages {tuple(pages.shape)} and {seq_len.numel()} lengths for {S} sequences of latents of {rank} + {rot}")
     rows = S * seq_rows
     if latents is None:
-        latents = torch.empty((rows, rank), dtype=pages.dtype, device=pages.device)
+        latents = _empty(pages, pages.dtype, rows, rank)
     if kv is None:
-        kv = torch.empty((rows, H, n + rot), dtype=pages.dtype, device=pages.device)
+        kv = _empty(pages, pages.dtype, rows, H, n + rot)
     _cuda(latents, "latent_expand latents", torch.bfloat16)
     _cuda(kv, "latent_expand kv", torch.bfloat16)
     _need(tuple(latents.shape) == (rows, rank) and tuple(kv.shape) == (rows, H, n + rot), "latent_expand: latents or kv of the wrong size")
-    lib = build.load("latent_attention")
+    lib = library("latent_attention")
     rc = lib.rl_latent_rows(
-        _p(pages), _p(block_table), c_int(width), _p(seq_len), c_int(S), c_int(seq_rows), _p(latents), _p(kv), c_int(H), c_int(n + rot), c_int(n),
-        c_int(rot), c_int(rank), _stream(),
+        pages, block_table, width, seq_len, S, seq_rows, latents, kv, H, n + rot, n,
+        rot, rank, _stream(),
     )
     _check(lib, rc, "latent_rows")
     head_linear(latents, 0, w_vk, kv.view(rows, H * (n + rot)), n + rot, held=seq_len, seq_rows=seq_rows)
@@ -1291,12 +1267,12 @@ def flash_expanded(
         _cuda(gate, "flash_expanded gate", torch.bfloat16, contiguous=False)
         ldg = _rows(gate, "flash_expanded gate")
         _need(gate.shape[0] == T and gate.shape[1] >= H * vdim, "flash_expanded: gate rows do not fit")
-    out = torch.empty((T, H * vdim), dtype=torch.bfloat16, device=q.device)
-    lib = build.load("attention_prefill_tc")
+    out = _empty(q, torch.bfloat16, T, H * vdim)
+    lib = library("attention_prefill_tc")
     rc = lib.rl_flash_prefill_tc_expanded(
-        _p(q), c_int(_rows(q, "flash_expanded q")), c_int(T), _p(kv), c_int(seq_rows // PAGE_SIZE), c_int(stride), _p(seq_start), _p(seq_pos0), _p(out),
-        c_int(H * vdim), c_int(S), c_int(max_q_len), c_int(H), c_int(kdim), c_int(vdim), c_int(window), c_float(scale), _p(sink), _p(gate), c_int(ldg),
-        _p(_tc_status_word(q.device)), *_wt(), _stream(),
+        q, _rows(q, "flash_expanded q"), T, kv, seq_rows // PAGE_SIZE, stride, seq_start, seq_pos0, out,
+        H * vdim, S, max_q_len, H, kdim, vdim, window, float(scale), sink, gate, ldg,
+        _tc_status_word(q.device), *_wt(), _stream(),
     )
     _check(lib, rc, "flash_prefill_tc_expanded")
     return out
@@ -1323,13 +1299,13 @@ def latent_attn(
         _cuda(sink, "latent_attn sink", torch.float32)
         _need(sink.numel() == H, "latent_attn: one sink per head")
     if out is None:
-        out = torch.empty((T, H, rank), dtype=q_cat.dtype, device=q_cat.device)
+        out = _empty(q_cat, q_cat.dtype, T, H, rank)
     _cuda(out, "latent_attn out", q_cat.dtype)
     _need(tuple(out.shape) == (T, H, rank), "latent_attn: out has the wrong shape")
-    lib = build.load("latent_attention")
+    lib = library("latent_attention")
     rc = lib.rl_latent_attn(
-        _p(q_cat), _p(pages), c_int(_dt(q_cat, "latent_attn")), _p(block_table), c_int(block_table.shape[1]), _p(tok_seq), _p(tok_pos),
-        _p(sink), _p(out), c_int(T), c_int(H), c_int(rank), c_int(rot), c_int(PAGE_SIZE), c_int(window), c_float(scale), _stream(),
+        q_cat, pages, _dt(q_cat, "latent_attn"), block_table, block_table.shape[1], tok_seq, tok_pos,
+        sink, out, T, H, rank, rot, PAGE_SIZE, window, float(scale), _stream(),
     )
     _check(lib, rc, "latent_attn")
     return out
@@ -1338,11 +1314,11 @@ def latent_attn(
 # ------------------------------------------------------------------ routed feed-forward
 def grouped_gemm_takes(K: int, ldx: int, head_stride: int) -> bool:
     """Whether the products of `grouped_gemm_tc.cu` and `grouped_gemm.cu` take operands with this k and these strides (in elements)."""
-    return bool(build.load("grouped_gemm").rl_grouped_gemm_takes(c_int(K), c_int(ldx), c_int(head_stride)))
+    return bool(library("grouped_gemm").rl_grouped_gemm_takes(K, ldx, head_stride))
 
 
 def moe_tile_rows() -> int:
-    return int(build.load("moe").rl_moe_tile_rows())
+    return int(library("moe").rl_moe_tile_rows())
 
 
 def moe_router(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], n_experts: int, top: int, renormalize: bool = False,
@@ -1361,15 +1337,15 @@ def moe_router(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], n
     if bias is not None:
         _cuda(bias, "moe_router bias", torch.float32)
         _need(bias.numel() == n_experts, "moe_router: one bias per expert")
-    ids = torch.empty((T, top), dtype=torch.int32, device=x.device)
-    weights = torch.empty((T, top), dtype=torch.float32, device=x.device)
-    gate = torch.empty((T,), dtype=torch.float32, device=x.device) if has_gate else None
-    logits = torch.empty((T, w.shape[0]), dtype=torch.float32, device=x.device)
-    lib = build.load("moe")
+    ids = _empty(x, torch.int32, T, top)
+    weights = _empty(x, torch.float32, T, top)
+    gate = _empty(x, torch.float32, T) if has_gate else None
+    logits = _empty(x, torch.float32, T, w.shape[0])
+    lib = library("moe")
     rc = lib.rl_moe_router(
-        _p(x), c_int(_rows(x, "moe_router x")), c_int(_dt(x, "moe_router")), _p(w), _p(bias), c_int(T), c_int(n_experts), c_int(d), c_int(top),
-        c_int(1 if renormalize else 0), c_int(1 if has_gate else 0), _p(logits), _p(ids), _p(weights), _p(gate), c_int(1 if logistic else 0),
-        c_float(renorm_eps), c_float(weight_scale), _stream(),
+        x, _rows(x, "moe_router x"), _dt(x, "moe_router"), w, bias, T, n_experts, d, top,
+        1 if renormalize else 0, 1 if has_gate else 0, logits, ids, weights, gate, 1 if logistic else 0,
+        float(renorm_eps), float(weight_scale), _stream(),
     )
     _check(lib, rc, "moe_router", kernels=2)
     return ids, weights, gate
@@ -1386,12 +1362,12 @@ def moe_choose(logits: torch.Tensor, bias: Optional[torch.Tensor], n_experts: in
     if bias is not None:
         _cuda(bias, "moe_choose bias", torch.float32)
         _need(bias.numel() == n_experts, "moe_choose: one bias per expert")
-    ids = torch.empty((T, top), dtype=torch.int32, device=logits.device)
-    weights = torch.empty((T, top), dtype=torch.float32, device=logits.device)
-    gate = torch.empty((T,), dtype=torch.float32, device=logits.device) if has_gate else None
-    lib = build.load("moe")
-    rc = lib.rl_moe_choose(_p(logits), _p(bias), c_int(T), c_int(n_experts), c_int(top), c_int(1 if renormalize else 0), c_int(1 if has_gate else 0),
-                           _p(ids), _p(weights), _p(gate), c_int(1 if logistic else 0), c_float(renorm_eps), c_float(weight_scale), _stream())
+    ids = _empty(logits, torch.int32, T, top)
+    weights = _empty(logits, torch.float32, T, top)
+    gate = _empty(logits, torch.float32, T) if has_gate else None
+    lib = library("moe")
+    rc = lib.rl_moe_choose(logits, bias, T, n_experts, top, 1 if renormalize else 0, 1 if has_gate else 0,
+                           ids, weights, gate, 1 if logistic else 0, float(renorm_eps), float(weight_scale), _stream())
     _check(lib, rc, "moe_choose")
     return ids, weights, gate
 
@@ -1402,10 +1378,10 @@ def moe_table_lookup(tokens: torch.Tensor, table: torch.Tensor, n_experts: int):
     _cuda(table, "moe_table_lookup table", torch.int32)
     _need(tokens.dim() == 1 and table.dim() == 2, "moe_table_lookup: tokens[T] and table[vocab, top] expected")
     T, top = tokens.numel(), table.shape[1]
-    ids = torch.empty((T, top), dtype=torch.int32, device=tokens.device)
-    weights = torch.empty((T, top), dtype=torch.float32, device=tokens.device)
-    lib = build.load("moe")
-    rc = lib.rl_moe_table_lookup(_p(tokens), _p(table), c_int(top), c_int(T), c_int(n_experts), _p(ids), _p(weights), _stream())
+    ids = _empty(tokens, torch.int32, T, top)
+    weights = _empty(tokens, torch.float32, T, top)
+    lib = library("moe")
+    rc = lib.rl_moe_table_lookup(tokens, table, top, T, n_experts, ids, weights, _stream())
     _check(lib, rc, "moe_table_lookup")
     return ids, weights
 
@@ -1441,11 +1417,11 @@ def moe_plan(ids: torch.Tensor, n_experts: int, tile_rows: int = 0):
     n = ids.numel()
     tile_rows = tile_rows or moe_tile_rows()
     max_tiles = moe_max_tiles(n, n_experts, tile_rows)
-    order = torch.empty((n,), dtype=torch.int32, device=ids.device)
-    place = torch.empty((n,), dtype=torch.int32, device=ids.device)
-    tiles = torch.empty((1 + 3 * max_tiles,), dtype=torch.int32, device=ids.device)
-    lib = build.load("moe")
-    rc = lib.rl_moe_plan(_p(ids), c_int(n), c_int(n_experts), _p(order), _p(place), _p(tiles), c_int(tile_rows), _stream())
+    order = _empty(ids, torch.int32, n)
+    place = _empty(ids, torch.int32, n)
+    tiles = _empty(ids, torch.int32, 1 + 3 * max_tiles)
+    lib = library("moe")
+    rc = lib.rl_moe_plan(ids, n, n_experts, order, place, tiles, tile_rows, _stream())
     _check(lib, rc, "moe_plan")
     return order, place, tiles, max_tiles
 
@@ -1469,29 +1445,29 @@ def moe_gemm(
         _cuda(w2, "moe_gemm w2", x.dtype)
         _need(tuple(w2.shape) == (E, N, K), "moe_gemm: w2 does not match w")
     out_dtype = out_dtype or x.dtype
-    out = torch.empty((n_rows, N), dtype=out_dtype, device=x.device)
+    out = _empty(x, out_dtype, n_rows, N)
     tile_rows = tile_rows or moe_tile_rows()
     _need(act is None or (act == "relu2") == (w2 is None), "moe_gemm: an activation of one argument goes with one matrix, a gate's with two")
     alpha, limit = _act(act)
     if x.dtype == torch.bfloat16 and tile_rows in MOE_MMA_TILE_ROWS and grouped_gemm_takes(K, x.stride(0), 0) and (x.data_ptr() | w.data_ptr()) % 16 == 0:
-        lib = build.load("grouped_gemm_tc")
+        lib = library("grouped_gemm_tc")
         if order is not None and n_rows >= MOE_GATHER_ROWS_PER_EXPERT * E:
-            rows = torch.empty((n_rows, K), dtype=x.dtype, device=x.device)
-            rc = lib.rl_moe_gather_rows(_p(x), c_int(x.stride(0)), c_int(x.shape[0]), _p(order), c_int(gather_div), _p(rows), c_int(n_rows), c_int(K), _stream())
+            rows = _empty(x, x.dtype, n_rows, K)
+            rc = lib.rl_moe_gather_rows(x, x.stride(0), x.shape[0], order, gather_div, rows, n_rows, K, _stream())
             _check(lib, rc, "moe_gather_rows")
             x, order = rows, None
         rc = lib.rl_moe_gemm_tc(
-            _p(x), c_int(x.stride(0)), c_int(x.shape[0]), _p(order), c_int(gather_div), _p(w), _p(w2), _p(out), c_int(_dt(out, "moe_gemm out")), c_int(N),
-            _p(tiles), c_int(max_tiles), c_int(tile_rows), c_int(E), c_int(N), c_int(K), alpha, limit, _p(_tc_status_word(x.device)), *_wt(), _stream(),
+            x, x.stride(0), x.shape[0], order, gather_div, w, w2, out, _dt(out, "moe_gemm out"), N,
+            tiles, max_tiles, tile_rows, E, N, K, alpha, limit, _tc_status_word(x.device), *_wt(), _stream(),
         )
         _check(lib, rc, "moe_gemm_tc")
         return out
     if tile_rows != moe_tile_rows():
         raise KernelError(f"moe_gemm: the plain kernel wants tiles of {moe_tile_rows()} rows, the plan has {tile_rows}")
-    lib = build.load("moe")
+    lib = library("moe")
     rc = lib.rl_moe_gemm(
-        _p(x), c_int(_rows(x, "moe_gemm x")), c_int(_dt(x, "moe_gemm")), _p(order), c_int(gather_div), _p(w), _p(w2), _p(out),
-        c_int(_dt(out, "moe_gemm out")), c_int(N), _p(tiles), c_int(max_tiles), c_int(N), c_int(K), alpha, limit, _stream(),
+        x, _rows(x, "moe_gemm x"), _dt(x, "moe_gemm"), order, gather_div, w, w2, out,
+        _dt(out, "moe_gemm out"), N, tiles, max_tiles, N, K, alpha, limit, _stream(),
     )
     _check(lib, rc, "moe_gemm")
     return out
@@ -1521,11 +1497,11 @@ def moe_combine(
         _cuda(x, "moe_combine x", contiguous=False)
         _need(tuple(x.shape) == (T, d), "moe_combine: x has the wrong shape")
         x_dt, xs = _dt(x, "moe_combine x"), _rows(x, "moe_combine x")
-    out = torch.empty((T, d), dtype=out_dtype, device=y.device)
-    lib = build.load("moe")
+    out = _empty(y, out_dtype, T, d)
+    lib = library("moe")
     rc = lib.rl_moe_combine(
-        _p(y), _p(place), _p(weights), c_int(top), _p(shared), c_int(shared_dt), _p(gate), _p(out), c_int(_dt(out, "moe_combine out")),
-        c_int(T), c_int(d), _p(x), c_int(x_dt), c_int(xs), _stream(),
+        y, place, weights, top, shared, shared_dt, gate, out, _dt(out, "moe_combine out"),
+        T, d, x, x_dt, xs, _stream(),
     )
     _check(lib, rc, "moe_combine")
     return out
@@ -1533,7 +1509,7 @@ def moe_combine(
 
 def latent_attn_mma_takes(rank: int, rot: int) -> bool:
     """Whether the tensor-core latent attention is built for these sizes (else `latent_attn` takes them)."""
-    return bool(build.load("latent_attention_mma").rl_latent_attn_mma_takes(c_int(rank), c_int(rot)))
+    return bool(library("latent_attention_mma").rl_latent_attn_mma_takes(rank, rot))
 
 
 def latent_attn_mma_scratch_floats(n_rows: int, rank: int, n_splits: int) -> int:
@@ -1570,14 +1546,14 @@ def latent_attn_mma(
         if scratch.numel() < need:
             raise KernelError(f"latent_attn_mma: scratch holds {scratch.numel()} floats, {need} needed")
     if out is None:
-        out = torch.empty((T, H, rank), dtype=torch.bfloat16, device=q_cat.device)
+        out = _empty(q_cat, torch.bfloat16, T, H, rank)
     _cuda(out, "latent_attn_mma out", torch.bfloat16)
     _need(tuple(out.shape) == (T, H, rank), "latent_attn_mma: out has the wrong shape")
-    lib = build.load("latent_attention_mma")
+    lib = library("latent_attention_mma")
     rc = lib.rl_latent_attn_mma(
-        _p(q_cat), _p(pages), _p(block_table), c_int(block_table.shape[1]), _p(seq_start), _p(seq_pos0), _p(sink), _p(out),
-        _p(scratch) if n_splits > 1 else c_void_p(0), c_ll(T * H), c_int(S), c_int(max_q_len * H), c_int(H), c_int(rank), c_int(rot),
-        c_int(PAGE_SIZE), c_int(window), c_float(scale), c_int(n_splits), _stream(),
+        q_cat, pages, block_table, block_table.shape[1], seq_start, seq_pos0, sink, out,
+        scratch if n_splits > 1 else None, T * H, S, max_q_len * H, H, rank, rot,
+        PAGE_SIZE, window, float(scale), n_splits, _stream(),
     )
     _check(lib, rc, "latent_attn_mma", kernels=2 if n_splits > 1 else 1)
     return out
@@ -1646,12 +1622,12 @@ def qkv_prep(
             raise KernelError(f"qkv_prep: v_src {tuple(v_src.shape)} is not [T, {num_kv_heads * vdim}]")
         _cuda(v_lambda, "qkv_prep v_lambda", torch.float32)
         _need(v_lambda.numel() == 1, "qkv_prep: v_lambda is one number")
-    lib = build.load("attention_ext")
+    lib = library("attention_ext")
     rc = lib.rl_qkv_prep(
-        _p(qkv), c_int(_dt(qkv, "qkv_prep")), c_int(stride), _p(bias), _p(tok_pos), _p(tok_seq), _p(block_table), c_int(1 if block_table is None else block_table.shape[1]),
-        _p(k_pages), _p(v_pages), _p(inv_freq if rotary_dim else None), c_float(magnitude), _p(q_norm), _p(k_norm), c_float(norm_eps), c_int(T), c_int(num_heads),
-        c_int(num_kv_heads), c_int(kdim), c_int(vdim), c_int(rotary_dim), c_int(1 if interleaved else 0), c_int(PAGE_SIZE),
-        _p(v_src), c_int(vs_stride), _p(v_lambda), c_int(1 if norm_whole else 0), c_int(1 if v_from_k else 0), c_float(coef), c_int(int(every)), _stream(),
+        qkv, _dt(qkv, "qkv_prep"), stride, bias, tok_pos, tok_seq, block_table, 1 if block_table is None else block_table.shape[1],
+        k_pages, v_pages, inv_freq if rotary_dim else None, float(magnitude), q_norm, k_norm, float(norm_eps), T, num_heads,
+        num_kv_heads, kdim, vdim, rotary_dim, 1 if interleaved else 0, PAGE_SIZE,
+        v_src, vs_stride, v_lambda, 1 if norm_whole else 0, 1 if v_from_k else 0, float(coef), int(every), _stream(),
     )
     _check(lib, rc, "qkv_prep")
 
@@ -1698,14 +1674,14 @@ def attn_ext(
         gs = _rows(gate, "attn_ext gate")
         _need(gate.shape[0] == T and gate.shape[1] >= num_heads * vdim, "attn_ext: gate rows too short")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=q.dtype, device=q.device)
+        out = _empty(q, q.dtype, T, num_heads * vdim)
     _cuda(out, "attn_ext out", q.dtype, contiguous=False)
     _need(_rows(out, "attn_ext out") >= num_heads * vdim and tuple(out.shape) == (T, num_heads * vdim), "attn_ext: out must be [T, H vdim]")
-    lib = build.load("attention_ext")
+    lib = library("attention_ext")
     rc = lib.rl_attn_ext(
-        _p(q), c_int(_dt(q, "attn_ext")), c_int(qs), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]), _p(tok_seq),
-        _p(tok_pos), _p(sink), _p(mix), _p(gate), c_int(gs), c_float(out_scale), _p(out), c_int(out.stride(0)), c_int(T), c_int(num_heads),
-        c_int(num_kv_heads), c_int(kdim), c_int(vdim), c_int(PAGE_SIZE), c_int(window), c_float(scale), c_int(chunk), c_float(softcap), c_int(maps),
+        q, _dt(q, "attn_ext"), qs, k_pages, v_pages, block_table, block_table.shape[1], tok_seq,
+        tok_pos, sink, mix, gate, gs, float(out_scale), out, out.stride(0), T, num_heads,
+        num_kv_heads, kdim, vdim, PAGE_SIZE, window, float(scale), chunk, float(softcap), maps,
         *_bias_args(bias, num_heads, "attn_ext"), _stream(),
     )
     _check(lib, rc, "attn_ext")
@@ -1719,12 +1695,12 @@ def map_combine(a: torch.Tensor, num_heads: int, vdim: int, lam: float, eps: flo
     T = a.shape[0]
     _need(a.shape[1] >= 2 * num_heads * vdim, "map_combine: rows too short")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=a.dtype, device=a.device)
+        out = _empty(a, a.dtype, T, num_heads * vdim)
     _cuda(out, "map_combine out", a.dtype, contiguous=False)
     _need(tuple(out.shape) == (T, num_heads * vdim), "map_combine: out must be [T, H vdim]")
-    lib = build.load("attention_ext")
-    rc = lib.rl_map_combine(_p(a), c_int(_dt(a, "map_combine")), c_int(_rows(a, "map_combine a")), c_float(lam), c_float(eps), c_float(factor), _p(out),
-                            c_int(_rows(out, "map_combine out")), c_int(T), c_int(num_heads), c_int(vdim), _stream())
+    lib = library("attention_ext")
+    rc = lib.rl_map_combine(a, _dt(a, "map_combine"), _rows(a, "map_combine a"), float(lam), float(eps), float(factor), out,
+                            _rows(out, "map_combine out"), T, num_heads, vdim, _stream())
     _check(lib, rc, "map_combine")
     return out
 
@@ -1762,14 +1738,14 @@ def sigmoid_attn(
         gs = _rows(gate, "sigmoid_attn gate")
         _need(gate.shape[0] == T and gate.shape[1] >= num_heads, "sigmoid_attn: gate rows too short")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=q.dtype, device=q.device)
+        out = _empty(q, q.dtype, T, num_heads * vdim)
     _cuda(out, "sigmoid_attn out", q.dtype, contiguous=False)
     _need(_rows(out, "sigmoid_attn out") >= num_heads * vdim and tuple(out.shape) == (T, num_heads * vdim), "sigmoid_attn: out must be [T, H vdim]")
-    lib = build.load("attention_sigmoid")
+    lib = library("attention_sigmoid")
     rc = lib.rl_sigmoid_attn(
-        _p(q), c_int(_dt(q, "sigmoid_attn")), c_int(qs), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]), _p(tok_seq),
-        _p(tok_pos), _p(head_bias), _p(mix), _p(gate), c_int(gs), c_float(out_scale), _p(out), c_int(out.stride(0)), c_int(T), c_int(num_heads),
-        c_int(num_kv_heads), c_int(kdim), c_int(vdim), c_int(PAGE_SIZE), c_int(window), c_float(scale), c_int(chunk), c_float(softcap), _stream(),
+        q, _dt(q, "sigmoid_attn"), qs, k_pages, v_pages, block_table, block_table.shape[1], tok_seq,
+        tok_pos, head_bias, mix, gate, gs, float(out_scale), out, out.stride(0), T, num_heads,
+        num_kv_heads, kdim, vdim, PAGE_SIZE, window, float(scale), chunk, float(softcap), _stream(),
     )
     _check(lib, rc, "sigmoid_attn")
     return out
@@ -1821,14 +1797,14 @@ def sigmoid_attn_mma(
     _need(parts >= 1 and scratch.numel() >= sigmoid_attn_mma_scratch_floats(T, num_heads, num_kv_heads, vdim, mix is not None, parts),
           "sigmoid_attn_mma: scratch too small")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=q.dtype, device=q.device)
+        out = _empty(q, q.dtype, T, num_heads * vdim)
     _cuda(out, "sigmoid_attn_mma out", q.dtype, contiguous=False)
     _need(_rows(out, "sigmoid_attn_mma out") >= num_heads * vdim and tuple(out.shape) == (T, num_heads * vdim), "sigmoid_attn_mma: out must be [T, H vdim]")
-    lib = build.load("attention_sigmoid")
+    lib = library("attention_sigmoid")
     rc = lib.rl_sigmoid_attn_mma(
-        _p(q), c_ll(qs), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]), _p(seq_start), _p(seq_pos0), _p(head_bias), _p(mix),
-        _p(gate), c_int(gs), c_float(out_scale), _p(scratch), c_int(parts), _p(out), c_int(out.stride(0)), c_int(T), c_int(S), c_int(max_q_len),
-        c_int(num_heads), c_int(num_kv_heads), c_int(kdim), c_int(vdim), c_int(window), c_float(scale), c_int(chunk), c_float(softcap), _stream(),
+        q, qs, k_pages, v_pages, block_table, block_table.shape[1], seq_start, seq_pos0, head_bias, mix,
+        gate, gs, float(out_scale), scratch, parts, out, out.stride(0), T, S, max_q_len,
+        num_heads, num_kv_heads, kdim, vdim, window, float(scale), chunk, float(softcap), _stream(),
     )
     _check(lib, rc, "sigmoid_attn_mma", kernels=2)
     return out
@@ -1872,24 +1848,24 @@ def decay_attn(
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "decay_attn: seq_start must hold one more entry than there are sequences")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=torch.float32, device=q.device)
+        out = _empty(q, torch.float32, T, num_heads * vdim)
     _cuda(out, "decay_attn out", torch.float32)
     _need(tuple(out.shape) == (T, num_heads * vdim), "decay_attn: out has the wrong shape")
-    lib = build.load("recurrent")
+    lib = library("recurrent")
     if max_q_len > 0 and scratch is not None:
         _cuda(scratch, "decay_attn scratch", torch.float32)
         if dim > DECAY_CHUNKED_MAX_DIM:
             raise KernelError(f"decay_attn: the chunked kernels take key sizes up to {DECAY_CHUNKED_MAX_DIM}")
         _need(scratch.numel() >= decay_attn_chunked_scratch_floats(S, max_q_len, num_heads, dim, vdim), "decay_attn: scratch too small")
         rc = lib.rl_decay_attn_chunked(
-            _p(q), _p(k), _p(v), c_int(_dt(q, "decay_attn")), c_int(q.stride(0)), _p(decay), _p(state), _p(slot_ids), _p(seq_start), _p(scratch),
-            _p(out), c_int(out.stride(0)), c_int(S), c_int(max_q_len), c_int(num_heads), c_int(dim), c_int(vdim), c_int(1 if silu else 0), _stream(),
+            q, k, v, _dt(q, "decay_attn"), q.stride(0), decay, state, slot_ids, seq_start, scratch,
+            out, out.stride(0), S, max_q_len, num_heads, dim, vdim, 1 if silu else 0, _stream(),
         )
         _check(lib, rc, "decay_attn_chunked", kernels=3)
         return out
     rc = lib.rl_decay_attn(
-        _p(q), _p(k), _p(v), c_int(_dt(q, "decay_attn")), c_int(q.stride(0)), _p(decay), _p(state), _p(slot_ids), _p(seq_start), _p(out),
-        c_int(out.stride(0)), c_int(S), c_int(num_heads), c_int(dim), c_int(vdim), c_int(1 if silu else 0), _stream(),
+        q, k, v, _dt(q, "decay_attn"), q.stride(0), decay, state, slot_ids, seq_start, out,
+        out.stride(0), S, num_heads, dim, vdim, 1 if silu else 0, _stream(),
     )
     _check(lib, rc, "decay_attn")
     return out
@@ -1912,13 +1888,13 @@ def rms_gate(
         gs = _rows(gate, "rms_gate gate")
         _need(gate.shape[0] == T and gate.shape[1] >= n, "rms_gate: gate rows too short")
     if out is None:
-        out = torch.empty((T, n), dtype=act_dtype, device=x.device)
+        out = _empty(x, act_dtype, T, n)
     _cuda(out, "rms_gate out", act_dtype, contiguous=False)
     _need(tuple(out.shape) == (T, n) and _rows(out, "rms_gate out") >= n, "rms_gate: out must be [T, n]")
-    lib = build.load("recurrent")
+    lib = library("recurrent")
     rc = lib.rl_rms_gate(
-        _p(x), c_int(xs), _p(weight), c_int(_dt(weight, "rms_gate weight")), c_float(eps), _p(gate), c_int(gs), c_float(out_scale), _p(out),
-        c_int(out.stride(0)), c_int(_DT[act_dtype]), c_int(T), c_int(n), _stream(),
+        x, xs, weight, _dt(weight, "rms_gate weight"), float(eps), gate, gs, float(out_scale), out,
+        out.stride(0), _DT[act_dtype], T, n, _stream(),
     )
     _check(lib, rc, "rms_gate")
     return out
@@ -1953,13 +1929,13 @@ def min_gru(
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "min_gru: seq_start must hold one more entry than there are sequences")
     if out is None:
-        out = torch.empty((T, width), dtype=z.dtype, device=z.device)
+        out = _empty(z, z.dtype, T, width)
     _cuda(out, "min_gru out", z.dtype, contiguous=False)
     _need(tuple(out.shape) == (T, width) and _rows(out, "min_gru out") >= width, "min_gru: out must be [T, width]")
-    lib = build.load("recurrent")
+    lib = library("recurrent")
     rc = lib.rl_min_gru(
-        _p(z), _p(x), _p(g), c_int(_dt(z, "min_gru")), c_int(z.stride(0)), _p(z_bias), _p(x_bias), _p(state), _p(slot_ids), _p(seq_start),
-        c_float(out_scale), _p(out), c_int(out.stride(0)), c_int(S), c_int(width), c_int(max_q_len), _stream(),
+        z, x, g, _dt(z, "min_gru"), z.stride(0), z_bias, x_bias, state, slot_ids, seq_start,
+        float(out_scale), out, out.stride(0), S, width, max_q_len, _stream(),
     )
     _check(lib, rc, "min_gru")
     return out
@@ -1974,9 +1950,9 @@ def gla_log_decay(z: torch.Tensor, bias: Optional[torch.Tensor], tau: float) -> 
     if bias is not None:
         _cuda(bias, "gla_log_decay bias", torch.float32)
         _need(bias.numel() == n, "gla_log_decay: one bias per column")
-    out = torch.empty((T, n), dtype=torch.float32, device=z.device)
-    lib = build.load("gated_recurrent")
-    rc = lib.rl_gla_log_decay(_p(z), c_int(_dt(z, "gla_log_decay")), c_int(zs), _p(bias), c_float(tau), _p(out), c_int(T), c_int(n), _stream())
+    out = _empty(z, torch.float32, T, n)
+    lib = library("gated_recurrent")
+    rc = lib.rl_gla_log_decay(z, _dt(z, "gla_log_decay"), zs, bias, float(tau), out, T, n, _stream())
     _check(lib, rc, "gla_log_decay")
     return out
 
@@ -2006,11 +1982,11 @@ def mlstm_gates(
     _cuda(seq_start, "mlstm_gates seq_start", torch.int32)
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "mlstm_gates: seq_start must hold one more entry than there are sequences")
-    log_a, b, m = (torch.empty((T, H), dtype=torch.float32, device=gi.device) for _ in range(3))
-    lib = build.load("gated_recurrent")
+    log_a, b, m = (_empty(gi, torch.float32, T, H) for _ in range(3))
+    lib = library("gated_recurrent")
     rc = lib.rl_mlstm_gates(
-        _p(gi), _p(gf), c_int(_dt(gi, "mlstm_gates")), c_int(stride), _p(bias_i), _p(bias_f), c_float(cap), _p(m_state), _p(slot_ids),
-        _p(seq_start), _p(log_a), _p(b), _p(m), c_int(S), c_int(H), c_int(1 if scan else 0), _stream(),
+        gi, gf, _dt(gi, "mlstm_gates"), stride, bias_i, bias_f, float(cap), m_state, slot_ids,
+        seq_start, log_a, b, m, S, H, 1 if scan else 0, _stream(),
     )
     _check(lib, rc, "mlstm_gates")
     return log_a, b, m
@@ -2051,12 +2027,12 @@ def gated_attn(
     _cuda(seq_start, "gated_attn seq_start", torch.int32)
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "gated_attn: seq_start must hold one more entry than there are sequences")
-    out = torch.empty((T, num_heads * vcols), dtype=torch.float32, device=q.device)
-    lib = build.load("gated_recurrent")
+    out = _empty(q, torch.float32, T, num_heads * vcols)
+    lib = library("gated_recurrent")
     rc = lib.rl_gated_attn(
-        _p(q), _p(k), _p(v), c_int(_dt(q, "gated_attn")), c_int(q.stride(0)), _p(log_decay), c_int(1 if per_channel else 0), _p(in_scale),
-        c_float(q_scale), _p(state), _p(slot_ids), _p(seq_start), _p(out), c_int(out.stride(0)), c_int(S), c_int(num_heads), c_int(qk_heads),
-        c_int(dim), c_int(vdim), c_int(1 if ext else 0), _stream(),
+        q, k, v, _dt(q, "gated_attn"), q.stride(0), log_decay, 1 if per_channel else 0, in_scale,
+        float(q_scale), state, slot_ids, seq_start, out, out.stride(0), S, num_heads, qk_heads,
+        dim, vdim, 1 if ext else 0, _stream(),
     )
     _check(lib, rc, "gated_attn")
     return out
@@ -2139,13 +2115,13 @@ def gated_attn_chunked(
     if norm is not None and (weight is None or q.dtype != torch.bfloat16 or ext):
         return None
     if out is None:
-        out = torch.empty((T, num_heads * vcols), dtype=torch.float32 if norm is None else q.dtype, device=q.device)
-    lib = build.load("gated_recurrent")
+        out = _empty(q, torch.float32 if norm is None else q.dtype, T, num_heads * vcols)
+    lib = library("gated_recurrent")
     rc = lib.rl_gated_attn_chunked(
-        _p(q), _p(k), _p(v), c_int(_dt(q, "gated_attn_chunked")), c_int(q.stride(0)), _p(log_decay), c_int(1 if per_channel else 0), _p(in_scale),
-        c_float(q_scale), _p(state), _p(slot_ids), _p(seq_start), _p(scratch), _p(out), c_int(out.stride(0)), c_int(S), c_int(max_q_len),
-        c_int(num_heads), c_int(qk_heads), c_int(dim), c_int(vdim), c_int(1 if ext else 0), _p(weight), c_float(eps), _p(gate), c_int(gs),
-        c_int(gate_act), c_float(out_scale), _stream(),
+        q, k, v, _dt(q, "gated_attn_chunked"), q.stride(0), log_decay, 1 if per_channel else 0, in_scale,
+        float(q_scale), state, slot_ids, seq_start, scratch, out, out.stride(0), S, max_q_len,
+        num_heads, qk_heads, dim, vdim, 1 if ext else 0, weight, float(eps), gate, gs,
+        gate_act, float(out_scale), _stream(),
     )
     if rc == _NOT_FUSED:
         return None
@@ -2186,13 +2162,13 @@ def head_norm_gate(
         gs = _rows(gate, "head_norm_gate gate")
         _need(gate.shape[0] == T and gate.shape[1] >= num_heads * n, "head_norm_gate: gate rows too short")
     if out is None:
-        out = torch.empty((T, num_heads * n), dtype=act_dtype, device=x.device)
+        out = _empty(x, act_dtype, T, num_heads * n)
     _cuda(out, "head_norm_gate out", act_dtype, contiguous=False)
     _need(tuple(out.shape) == (T, num_heads * n) and _rows(out, "head_norm_gate out") >= num_heads * n, "head_norm_gate: out must be [T, H n]")
-    lib = build.load("gated_recurrent")
+    lib = library("gated_recurrent")
     rc = lib.rl_head_norm_gate(
-        _p(x), c_int(xs), c_int(xh), _p(m), c_float(den_eps), _p(weight), c_int(per_head), c_float(eps), _p(gate), c_int(gs), c_int(gate_act),
-        c_float(out_scale), _p(out), c_int(out.stride(0)), c_int(_DT[act_dtype]), c_int(T), c_int(num_heads), c_int(n), _stream(),
+        x, xs, xh, m, float(den_eps), weight, per_head, float(eps), gate, gs, gate_act,
+        float(out_scale), out, out.stride(0), _DT[act_dtype], T, num_heads, n, _stream(),
     )
     _check(lib, rc, "head_norm_gate")
     return out
@@ -2239,11 +2215,11 @@ def short_conv(
         _need(bias.numel() == C, "short_conv: one bias per channel")
     if single and T != S:
         raise KernelError(f"short_conv: {T} tokens of {S} sequences are not one each")
-    out = torch.empty((T, C), dtype=x.dtype, device=x.device)
-    lib = build.load("delta_rule")
+    out = _empty(x, x.dtype, T, C)
+    lib = library("delta_rule")
     rc = lib.rl_short_conv(
-        _p(x), c_int(_dt(x, "short_conv")), c_int(xs), _p(w), _p(bias), _p(state if taps > 1 else None), _p(slot_ids), _p(seq_start), _p(tok_seq), _p(out),
-        c_int(out.stride(0)), c_int(T), c_int(S), c_int(C), c_int(taps), c_int(1 if silu else 0), c_int(1 if single else 0), _stream(),
+        x, _dt(x, "short_conv"), xs, w, bias, state if taps > 1 else None, slot_ids, seq_start, tok_seq, out,
+        out.stride(0), T, S, C, taps, 1 if silu else 0, 1 if single else 0, _stream(),
     )
     _check(lib, rc, "short_conv", kernels=2 if taps > 1 and not single else 1)
     return out
@@ -2265,15 +2241,15 @@ def delta_prep(
     _cuda(a_log, "delta_prep a_log", torch.float32)
     _cuda(dt_bias, "delta_prep dt_bias", torch.float32)
     _need(a_log.numel() == H and dt_bias.numel() == H, "delta_prep: one A_log and one dt_bias per head")
-    f32 = dict(dtype=torch.float32, device=qk.device)
-    qn, kn = torch.empty((T, G * dim), **f32), torch.empty((T, G * dim), **f32)
-    kq, beta, decay = torch.empty((T, G), **f32), torch.empty((T, H), **f32), torch.empty((T, H), **f32)
-    log = torch.empty((T, H), **f32) if log_decay else None
-    lib = build.load("delta_rule")
+    f32 = torch.float32
+    qn, kn = _empty(qk, f32, T, G * dim), _empty(qk, f32, T, G * dim)
+    kq, beta, decay = _empty(qk, f32, T, G), _empty(qk, f32, T, H), _empty(qk, f32, T, H)
+    log = _empty(qk, f32, T, H) if log_decay else None
+    lib = library("delta_rule")
     rc = lib.rl_delta_prep(
-        _p(qk), c_int(_dt(qk, "delta_prep")), c_int(_rows(qk, "delta_prep qk")), _p(ba), c_int(_rows(ba, "delta_prep ba")), _p(a_log), _p(dt_bias),
-        c_float(unit_eps), c_float(q_scale), _p(qn), _p(kn), _p(kq), _p(beta), _p(decay), _p(log), c_int(T), c_int(G), c_int(H),
-        c_int(dim), _stream(),
+        qk, _dt(qk, "delta_prep"), _rows(qk, "delta_prep qk"), ba, _rows(ba, "delta_prep ba"), a_log, dt_bias,
+        float(unit_eps), float(q_scale), qn, kn, kq, beta, decay, log, T, G, H,
+        dim, _stream(),
     )
     _check(lib, rc, "delta_prep")
     return (qn, kn, kq, beta, decay, log) if log_decay else (qn, kn, kq, beta, decay)
@@ -2306,13 +2282,13 @@ def delta_rule(
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "delta_rule: seq_start must hold one more entry than there are sequences")
     if out is None:
-        out = torch.empty((T, H * vdim), dtype=torch.float32, device=qn.device)
+        out = _empty(qn, torch.float32, T, H * vdim)
     _cuda(out, "delta_rule out", torch.float32)
     _need(tuple(out.shape) == (T, H * vdim), "delta_rule: out must be [T, H vdim]")
-    lib = build.load("delta_rule")
+    lib = library("delta_rule")
     rc = lib.rl_delta_rule(
-        _p(qn), _p(kn), _p(kq), _p(v), c_int(_dt(v, "delta_rule v")), c_int(_rows(v, "delta_rule v")), _p(beta), _p(decay), _p(state), _p(slot_ids),
-        _p(seq_start), _p(out), c_int(out.stride(0)), c_int(S), c_int(H), c_int(G), c_int(dim), c_int(vdim), c_int(max_len), _stream(),
+        qn, kn, kq, v, _dt(v, "delta_rule v"), _rows(v, "delta_rule v"), beta, decay, state, slot_ids,
+        seq_start, out, out.stride(0), S, H, G, dim, vdim, max_len, _stream(),
     )
     _check(lib, rc, "delta_rule")
     return out
@@ -2324,9 +2300,8 @@ def delta_chunked_takes(dim: int, vdim: int) -> bool:
 
 
 def delta_chunked_scratch_floats(n_tokens: int, n_seqs: int, num_heads: int, dim: int, vdim: int) -> int:
-    lib = build.load("delta_chunk")
-    lib.rl_delta_chunked_scratch.restype = c_ll
-    return int(lib.rl_delta_chunked_scratch(c_int(n_tokens), c_int(n_seqs), c_int(num_heads), c_int(dim), c_int(vdim)))
+    lib = library("delta_chunk")
+    return int(lib.rl_delta_chunked_scratch(n_tokens, n_seqs, num_heads, dim, vdim))
 
 
 def delta_chunked(
@@ -2360,12 +2335,12 @@ def delta_chunked(
     if norm is not None and weight is None:
         return None
     if out is None:
-        out = torch.empty((T, H * vdim), dtype=torch.float32 if norm is None else torch.bfloat16, device=qn.device)
-    lib = build.load("delta_chunk")
+        out = _empty(qn, torch.float32 if norm is None else torch.bfloat16, T, H * vdim)
+    lib = library("delta_chunk")
     rc = lib.rl_delta_chunked(
-        _p(qn), _p(kn), _p(v), c_int(_rows(v, "delta_chunked v")), _p(beta), _p(log_decay), _p(state), _p(slot_ids), _p(seq_start), _p(out), c_int(out.stride(0)),
-        c_int(T), c_int(S), c_int(max_q_len), c_int(H), c_int(G), c_int(dim), c_int(vdim), c_int(min_len), _p(scratch), _p(weight), c_float(eps),
-        _p(gate), c_int(gs), c_int(gate_act), c_float(out_scale), _stream(),
+        qn, kn, v, _rows(v, "delta_chunked v"), beta, log_decay, state, slot_ids, seq_start, out, out.stride(0),
+        T, S, max_q_len, H, G, dim, vdim, min_len, scratch, weight, float(eps),
+        gate, gs, gate_act, float(out_scale), _stream(),
     )
     if rc == _NOT_FUSED:
         return None
@@ -2382,9 +2357,9 @@ def ssm_gates(raw: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor):
         _cuda(t, f"ssm_gates {name}", torch.float32)
         if t.numel() != H:
             raise KernelError(f"ssm_gates: one {name} per head")
-    log_a, dt = (torch.empty((T, H), dtype=torch.float32, device=raw.device) for _ in range(2))
-    lib = build.load("state_space")
-    rc = lib.rl_ssm_gates(_p(raw), c_int(_dt(raw, "ssm_gates")), c_int(_rows(raw, "ssm_gates raw")), _p(a_log), _p(dt_bias), _p(log_a), _p(dt), c_int(T), c_int(H), _stream())
+    log_a, dt = (_empty(raw, torch.float32, T, H) for _ in range(2))
+    lib = library("state_space")
+    rc = lib.rl_ssm_gates(raw, _dt(raw, "ssm_gates"), _rows(raw, "ssm_gates raw"), a_log, dt_bias, log_a, dt, T, H, _stream())
     _check(lib, rc, "ssm_gates")
     return log_a, dt
 
@@ -2407,14 +2382,14 @@ def ssm_gate_norm(
     if not (n % H == 0 and n % groups == 0 and weight.numel() == n):
         raise KernelError(f"ssm_gate_norm: {H} heads, {groups} parts and {weight.numel()} weights for a row of {n}")
     if out is None:
-        out = torch.empty((T, n), dtype=act_dtype, device=y.device)
+        out = _empty(y, act_dtype, T, n)
     _cuda(out, "ssm_gate_norm out", act_dtype, contiguous=False)
     _need(tuple(out.shape) == (T, n), "ssm_gate_norm: out must be [T, n]")
-    lib = build.load("state_space")
+    lib = library("state_space")
     rc = lib.rl_ssm_gate_norm(
-        _p(y), c_int(_rows(y, "ssm_gate_norm y")), _p(x), c_int(_rows(x, "ssm_gate_norm x")), _p(skip), c_int(n // H), _p(z), c_int(_rows(z, "ssm_gate_norm z")),
-        _p(weight), c_float(eps), c_int(groups), _p(out), c_int(_rows(out, "ssm_gate_norm out")), c_int(_DT[act_dtype]), c_int(T), c_int(n),
-        c_float(out_scale), _stream(),
+        y, _rows(y, "ssm_gate_norm y"), x, _rows(x, "ssm_gate_norm x"), skip, n // H, z, _rows(z, "ssm_gate_norm z"),
+        weight, float(eps), groups, out, _rows(out, "ssm_gate_norm out"), _DT[act_dtype], T, n,
+        float(out_scale), _stream(),
     )
     _check(lib, rc, "ssm_gate_norm")
     return out
@@ -2465,11 +2440,11 @@ def scalar_decay_chunked(
     _need(seq_start.numel() == S + 1, "scalar_decay_chunked: seq_start must hold one more entry than there are sequences")
     _cuda(scratch, "scalar_decay_chunked scratch", torch.float32)
     _need(max_q_len >= 1 and scratch.numel() >= scalar_decay_chunked_scratch_floats(S, max_q_len, num_heads, dim, vdim), "scalar_decay_chunked: scratch too small")
-    out = torch.empty((T, num_heads * vdim), dtype=torch.float32, device=q.device)
-    lib = build.load("state_space")
+    out = _empty(q, torch.float32, T, num_heads * vdim)
+    lib = library("state_space")
     rc = lib.rl_scalar_decay_chunked(
-        _p(q), _p(k), _p(v), c_int(q.stride(0)), _p(log_decay), _p(in_scale), _p(state), _p(slot_ids), _p(seq_start), _p(scratch), _p(out),
-        c_int(out.stride(0)), c_int(S), c_int(max_q_len), c_int(num_heads), c_int(qk_heads), c_int(dim), c_int(vdim), _stream(),
+        q, k, v, q.stride(0), log_decay, in_scale, state, slot_ids, seq_start, scratch, out,
+        out.stride(0), S, max_q_len, num_heads, qk_heads, dim, vdim, _stream(),
     )
     _check(lib, rc, "scalar_decay_chunked", kernels=3)
     return out
@@ -2484,8 +2459,8 @@ def unary_act(x: torch.Tensor, kind: int = ACT_RELU2) -> torch.Tensor:
     out = torch.empty_like(x)
     if x.numel() == 0:
         return out
-    lib = build.load("recurrent")
-    rc = lib.rl_unary_act(_p(x), _p(out), c_int(_dt(x, "unary_act")), c_ll(x.numel()), c_int(kind), _stream())
+    lib = library("recurrent")
+    rc = lib.rl_unary_act(x, out, _dt(x, "unary_act"), x.numel(), kind, _stream())
     _check(lib, rc, "unary_act")
     return out
 
@@ -2513,9 +2488,9 @@ def fold_queries(q: torch.Tensor, mix: torch.Tensor, num_heads: int, num_kv_head
     _cuda(mix, "fold_queries mix", torch.float32)
     _need(tuple(mix.shape) == (num_heads, num_heads), "fold_queries: the mixing matrix must be [H, H]")
     T = q.shape[0]
-    out = torch.empty((T, num_heads * num_kv_heads * kdim), dtype=torch.bfloat16, device=q.device)
-    lib = build.load("attention_mix_mma")
-    rc = lib.rl_fold_queries(_p(q), c_int(qs), _p(mix), _p(out), c_int(T), c_int(num_heads), c_int(num_kv_heads), c_int(kdim), c_int(maps), _stream())
+    out = _empty(q, torch.bfloat16, T, num_heads * num_kv_heads * kdim)
+    lib = library("attention_mix_mma")
+    rc = lib.rl_fold_queries(q, qs, mix, out, T, num_heads, num_kv_heads, kdim, maps, _stream())
     _check(lib, rc, "fold_queries")
     return out
 
@@ -2553,15 +2528,15 @@ def flash_mix(
         gs = _rows(gate, "flash_mix gate")
         _need(gate.shape[0] == T and gate.shape[1] >= num_heads * vdim, "flash_mix: gate rows too short")
     if out is None:
-        out = torch.empty((T, num_heads * vdim), dtype=torch.bfloat16, device=q.device)
+        out = _empty(q, torch.bfloat16, T, num_heads * vdim)
     _cuda(out, "flash_mix out", torch.bfloat16, contiguous=False)
     _need(tuple(out.shape) == (T, num_heads * vdim) and _rows(out, "flash_mix out") >= num_heads * vdim, "flash_mix: out must be [T, H vdim]")
-    lib = build.load("attention_mix_mma")
+    lib = library("attention_mix_mma")
     rc = lib.rl_flash_mix(
-        _p(q), c_ll(qs), c_int(parts * kdim), c_int(parts), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]),
-        _p(seq_start), _p(seq_pos0), _p(sink), _p(gate), c_int(gs), c_float(out_scale), _p(out), c_int(out.stride(0)), c_int(S),
-        c_int(max_q_len), c_int(num_heads), c_int(num_kv_heads), c_int(kdim), c_int(vdim), c_int(PAGE_SIZE), c_int(window), c_float(scale),
-        c_int(chunk), c_float(softcap), c_int(maps), *_bias_args(bias, num_heads, "flash_mix"), _stream(),
+        q, qs, parts * kdim, parts, k_pages, v_pages, block_table, block_table.shape[1],
+        seq_start, seq_pos0, sink, gate, gs, float(out_scale), out, out.stride(0), S,
+        max_q_len, num_heads, num_kv_heads, kdim, vdim, PAGE_SIZE, window, float(scale),
+        chunk, float(softcap), maps, *_bias_args(bias, num_heads, "flash_mix"), _stream(),
     )
     _check(lib, rc, "flash_mix")
     return out
@@ -2610,16 +2585,16 @@ def flash_mix_decode(
         gs = _rows(gate, "flash_mix_decode gate")
         _need(gate.shape[0] == S and gate.shape[1] >= num_heads * vdim, "flash_mix_decode: gate rows too short")
     if out is None:
-        out = torch.empty((S, num_heads * vdim), dtype=torch.bfloat16, device=qf.device)
+        out = _empty(qf, torch.bfloat16, S, num_heads * vdim)
     _cuda(out, "flash_mix_decode out", torch.bfloat16, contiguous=False)
     _need(tuple(out.shape) == (S, num_heads * vdim) and _rows(out, "flash_mix_decode out") >= num_heads * vdim, "flash_mix_decode: out must be [S, H vdim]")
     n_o = S * num_heads * n_splits * vdim
-    lib = build.load("attention_mix_mma")
+    lib = library("attention_mix_mma")
     rc = lib.rl_flash_mix_decode(
-        _p(qf), _p(k_pages), _p(v_pages), _p(block_table), c_int(block_table.shape[1]), _p(seq_pos0), _p(sink), _p(gate), c_int(gs),
-        c_float(out_scale), c_void_p(scratch.data_ptr()), c_void_p(scratch.data_ptr() + 4 * n_o), _p(out), c_int(out.stride(0)), c_int(S),
-        c_int(num_heads), c_int(num_kv_heads), c_int(kdim), c_int(vdim), c_int(PAGE_SIZE), c_int(window), c_float(scale), c_int(n_splits),
-        c_int(chunk), c_float(softcap), *_bias_args(bias, num_heads, "flash_mix_decode"), _stream(),
+        qf, k_pages, v_pages, block_table, block_table.shape[1], seq_pos0, sink, gate, gs,
+        float(out_scale), scratch.data_ptr(), scratch.data_ptr() + 4 * n_o, out, out.stride(0), S,
+        num_heads, num_kv_heads, kdim, vdim, PAGE_SIZE, window, float(scale), n_splits,
+        chunk, float(softcap), *_bias_args(bias, num_heads, "flash_mix_decode"), _stream(),
     )
     _check(lib, rc, "flash_mix_decode", kernels=2)
     return out

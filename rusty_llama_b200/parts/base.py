@@ -25,6 +25,7 @@ from typing import List, Callable, Dict, Mapping, Optional, Tuple
 import torch
 
 from ..errors import ConfigError
+from ..kernels import ops
 from ..spec import PartSpec
 
 
@@ -232,8 +233,6 @@ class ResidualStream:
         return out
 
     def flush(self) -> None:
-        from ..kernels import ops
-
         if self.pending is not None:
             if self.pending_norm is not None:
                 ops.normed_add_rmsnorm(self.x, self.pending, self.pending_norm[0], self.pending_norm[1], None, 0.0, self.act_dtype,
@@ -280,8 +279,6 @@ class PositionEncoding(Part):
         return None
 
     def write_qk(self, qkv: torch.Tensor, step, kv, num_heads: int, num_kv_heads: int, head_dim: int, write_kv: bool) -> None:
-        from ..kernels import ops
-
         T = qkv.shape[0]
         q = qkv[:, : num_heads * head_dim].view(T, num_heads, head_dim)
         k = qkv[:, num_heads * head_dim : (num_heads + num_kv_heads) * head_dim].view(T, num_kv_heads, head_dim)

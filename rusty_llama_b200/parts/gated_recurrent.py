@@ -127,9 +127,9 @@ class GatedLinearAttention(Mixer):
             raise ConfigError("gated_linear_attention: a state cannot be another run's")
         proj = linear(xn, self.w_in)
         qd, vd = self.qd, self.vd
-        q, k, v = proj[:, :qd], proj[:, qd : 2 * qd], proj[:, 2 * qd : 2 * qd + vd]
-        gate = proj[:, 2 * qd + vd : 2 * qd + 2 * vd]
-        inner = proj[:, 2 * qd + 2 * vd :]
+        q, k, v = ops.columns(proj, 0, qd), ops.columns(proj, qd, 2 * qd), ops.columns(proj, 2 * qd, 2 * qd + vd)
+        gate = ops.columns(proj, 2 * qd + vd, 2 * qd + 2 * vd)
+        inner = ops.columns(proj, 2 * qd + 2 * vd, proj.shape[1])
         if inner.data_ptr() % 16 or inner.stride(0) % 8:  # the second product moves its rows in 16-byte pieces
             inner = inner.contiguous()
         z = linear(inner, self.w_a2)
@@ -218,9 +218,9 @@ class MatrixMemory(Mixer):
         memory, maximum = cache
         proj = linear(xn, self.w_in)
         qd, vd, H = self.qd, self.vd, self.H
-        q, k, v = proj[:, :qd], proj[:, qd : 2 * qd], proj[:, 2 * qd : 2 * qd + vd]
-        gate = proj[:, 2 * qd + vd : 2 * qd + 2 * vd]
-        gi, gf = proj[:, 2 * qd + 2 * vd : 2 * qd + 2 * vd + H], proj[:, 2 * qd + 2 * vd + H :]
+        q, k, v = ops.columns(proj, 0, qd), ops.columns(proj, qd, 2 * qd), ops.columns(proj, 2 * qd, 2 * qd + vd)
+        gate = ops.columns(proj, 2 * qd + vd, 2 * qd + 2 * vd)
+        gi, gf = ops.columns(proj, 2 * qd + 2 * vd, 2 * qd + 2 * vd + H), ops.columns(proj, 2 * qd + 2 * vd + H, proj.shape[1])
         log_a, b, m = ops.mlstm_gates(gi, gf, self.b_i, self.b_f, self.cap, maximum.state, step.slot_ids, step.seq_start,
                                       scan=xn.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS)
         o, _ = _recurrence(self, q, k, v, log_a, b, memory.state, step, ext=True)
@@ -318,18 +318,18 @@ class GatedDeltaRule(Mixer):
         memory, inputs = cache if self.taps > 1 else (cache, None)
         proj = linear(xn, self.w_in)
         C, vd, H = self.channels, self.vd, self.H
-        conv = ops.short_conv(proj[:, :C], self.w_conv, None if inputs is None else inputs.state, step.slot_ids, step.seq_start, step.tok_seq,
+        conv = ops.short_conv(ops.columns(proj, 0, C), self.w_conv, None if inputs is None else inputs.state, step.slot_ids, step.seq_start, step.tok_seq,
                               single=step.decode_only)
-        gate, ba = proj[:, C : C + vd], proj[:, C + vd : C + vd + 2 * H]
+        gate, ba = ops.columns(proj, C, C + vd), ops.columns(proj, C + vd, C + vd + 2 * H)
         scratch = None
         if xn.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS and ops.delta_chunked_takes(self.dim, self.vdim):
             floats = ops.delta_chunked_scratch_floats(step.n_tokens, step.n_seqs, H, self.dim, self.vdim)
             if floats <= _CHUNKED_MAX_FLOATS:
                 scratch = scratch_for_call(floats, torch.float32, xn.device)
         chunked = scratch is not None
-        qn, kn, kq, beta, decay, *log = ops.delta_prep(conv[:, : 2 * self.qd], ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps,
+        qn, kn, kq, beta, decay, *log = ops.delta_prep(ops.columns(conv, 0, 2 * self.qd), ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps,
                                                        self.q_scale, log_decay=chunked)
-        v, o = conv[:, 2 * self.qd :], None
+        v, o = ops.columns(conv, 2 * self.qd, C), None
         where = (memory.state, step.slot_ids, step.seq_start, H, self.G, self.dim, self.vdim)
         short = min(step.q_lens) < _CHUNKED_MIN_TOKENS
         if chunked:  # prompts of a bfloat16 run, all chunks side by side but for the walk through the state
@@ -429,10 +429,10 @@ class StateSpaceDuality(Mixer):
         memory, inputs = cache if self.taps > 1 else (cache, None)
         proj = linear(xn, self.w_in)
         n = self.inner
-        z, raw_dt = proj[:, :n], proj[:, n + self.channels :]
-        conv = ops.short_conv(proj[:, n : n + self.channels], self.w_conv, None if inputs is None else inputs.state, step.slot_ids, step.seq_start,
+        z, raw_dt = ops.columns(proj, 0, n), ops.columns(proj, n + self.channels, proj.shape[1])
+        conv = ops.short_conv(ops.columns(proj, n, n + self.channels), self.w_conv, None if inputs is None else inputs.state, step.slot_ids, step.seq_start,
                               step.tok_seq, bias=self.b_conv, single=step.decode_only)
-        x, B, C = conv[:, :n], conv[:, n : n + self.bc], conv[:, n + self.bc :]
+        x, B, C = ops.columns(conv, 0, n), ops.columns(conv, n, n + self.bc), ops.columns(conv, n + self.bc, self.channels)
         log_a, dt = ops.ssm_gates(raw_dt, self.a_log, self.dt_bias)
         y = self._recurrence(C, B, x, log_a, dt, memory.state, step)
         a = ops.ssm_gate_norm(y, x, self.skip, z, self.w_norm, self.eps, self.norm_groups, xn.dtype, out_scale=self.out_scale, out=out)

@@ -183,9 +183,9 @@ class LatentAttention(Mixer):
         T = xn.shape[0]
         proj = linear(xn, self.w_in)
         first = self.q_rank or self.qd
-        q = proj[:, :first]
-        g = proj[:, first : first + self.vd] if self.has_gate else None
-        kv = proj[:, proj.shape[1] - self.kvd :] if self.own_kv else None
+        q = ops.columns(proj, 0, first)
+        g = ops.columns(proj, first, first + self.vd) if self.has_gate else None
+        kv = ops.columns(proj, proj.shape[1] - self.kvd, proj.shape[1]) if self.own_kv else None
         turn = (self.freq, self.n_pairs, self.magnitude, step.tok_pos, step.tok_seq, cache.block_table, cache.k_pages)
         sizes = (self.H, self.dim, self.rot, self.rank, self.interleaved)
         if self.q_rank:

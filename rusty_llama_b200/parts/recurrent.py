@@ -130,9 +130,9 @@ class DecayLinearAttention(Mixer):
             # q and k lie side by side at the start of the rows: 2 H heads turned in place, nothing stored anywhere else
             ops.rope_kv_write(proj, step.tok_pos, step.tok_seq, None, None, None, self.position.inv_freq, 2 * self.H, 0, self.dim,
                               self.position.rotary_dim, self.position.interleaved, write_kv=False)
-        q, k = proj[:, : self.qd], proj[:, self.qd : 2 * self.qd]
-        v = proj[:, 2 * self.qd : 2 * self.qd + self.vd]
-        gate = proj[:, 2 * self.qd + self.vd :] if self.has_gate else None
+        q, k = ops.columns(proj, 0, self.qd), ops.columns(proj, self.qd, 2 * self.qd)
+        v = ops.columns(proj, 2 * self.qd, 2 * self.qd + self.vd)
+        gate = ops.columns(proj, 2 * self.qd + self.vd, proj.shape[1]) if self.has_gate else None
         # a prompt step of a bfloat16 run works its sequences chunk by chunk, all chunks at once; 32-bit runs and single
         # tokens go token by token (the same bits however a sequence is cut into steps)
         chunked = xn.dtype == torch.bfloat16 and step.max_q_len >= _CHUNKED_MIN_TOKENS and self.dim <= ops.DECAY_CHUNKED_MAX_DIM
@@ -208,7 +208,7 @@ class MinGRU(Mixer):
         proj = linear(xn, self.w_in)
         w = self.width
         a = ops.min_gru(
-            proj[:, :w], proj[:, w : 2 * w], proj[:, 2 * w :], self.b_z, self.b_x, cache.state, step.slot_ids, step.seq_start,
+            ops.columns(proj, 0, w), ops.columns(proj, w, 2 * w), ops.columns(proj, 2 * w, proj.shape[1]), self.b_z, self.b_x, cache.state, step.slot_ids, step.seq_start,
             out_scale=self.out_scale, out=out, max_q_len=step.max_q_len if xn.dtype == torch.bfloat16 else 0,
         )
         return a, self.w_o

@@ -1,0 +1,109 @@
+"""The native side of a launch against its Python twin: arguments of every kind in the order that a launcher declares them, in registers and
+on the stack, and the checks' results and messages."""
+
+import ctypes
+import shutil
+import subprocess
+
+import pytest
+import torch
+
+from rusty_llama_b200.errors import KernelError
+from rusty_llama_b200.kernels import build, host
+
+SOURCE = """
+#include <math.h>
+#include <stddef.h>
+static double seen[64];
+double* last(void) { return seen; }
+#define S(i, v) seen[i] = (double)(v)
+int few(const void* a, int b, float c) { S(0, a == NULL); S(1, b); S(2, c); return -b; }
+int none(void) { return -7; }
+long long wide(int a) { return ((long long)a << 33) + 1; }
+int many(const void* a, int b, float c, long long d, const void* e, int f, float g, int h, int i, unsigned j, int k, float l, long long m, int n,
+         const void* o, float p, float q, int r, float s, int t, float u, const void* v) {
+  S(0, a == NULL); S(1, b); S(2, c); S(3, d); S(4, e != NULL); S(5, f); S(6, g); S(7, h); S(8, i); S(9, j); S(10, k); S(11, l); S(12, m); S(13, n);
+  S(14, o == NULL); S(15, p); S(16, q); S(17, r); S(18, s); S(19, t); S(20, u); S(21, (size_t)v & 0xffff);
+  return r - t;
+}
+"""
+
+
+def launchers():
+    build.build_host_calls()
+    native = build.load_host_calls(False)
+    native.set_error(KernelError)
+    return native, [native.launcher, host.PythonLauncher]
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    if not shutil.which("gcc"):
+        pytest.skip("no C compiler")
+    d = tmp_path_factory.mktemp("host_calls")
+    (d / "seen.c").write_text(SOURCE)
+    subprocess.run(["gcc", "-O2", "-shared", "-fPIC", "-o", str(d / "seen.so"), str(d / "seen.c")], check=True)
+    lib = ctypes.CDLL(str(d / "seen.so"))
+    lib.last.restype = ctypes.POINTER(ctypes.c_double)
+    return lib
+
+
+def test_arguments_reach_the_launcher_as_declared(library):
+    native, makers = launchers()
+    at = lambda name: ctypes.cast(getattr(library, name), ctypes.c_void_p).value  # noqa: E731
+    t = torch.zeros(8)
+    args = (None, -3, 1.5, -(1 << 40), t, True, -2.25, 7, -8, 4000000000, 10, 0.5, 1 << 35, 13, None, 15.0, -16.0, 17, float("inf"), 19, 0.1, t)
+    want = [1, -3, 1.5, -(1 << 40), 1, 1, -2.25, 7, -8, 4000000000, 10, 0.5, 1 << 35, 13, 1, 15, -16, 17, float("inf"), 19, ctypes.c_float(0.1).value, t.data_ptr() & 0xFFFF]
+    for make in makers:
+        assert make(at("few"), False)(t, 5, 2.5) == -5 and library.last()[:3] == [0.0, 5.0, 2.5]
+        assert make(at("many"), False)(*args) == -2 and library.last()[:22] == want
+        assert make(at("none"), False)() == -7 and make(at("wide"), True)(3) == (3 << 33) + 1
+    few = native.launcher(at("few"), False)
+    for wrong in (("x", 1, 1.0), (t, [1], 1.0), tuple([1.0] * 9), tuple([1] * 57)):
+        with pytest.raises(TypeError):
+            few(*wrong)
+    with pytest.raises(RuntimeError):  # a C++ exception on the way is a Python one
+        few(torch.sparse_coo_tensor(torch.tensor([[0]]), torch.tensor([1.0]), (2,)), 1, 1.0)
+
+
+def test_checks_and_views_agree_with_python():
+    native, _ = launchers()
+
+    def outcome(f, *a, **k):
+        try:
+            return f(*a, **k)
+        except KernelError as e:
+            return str(e)
+
+    t = torch.arange(24, dtype=torch.float32).view(4, 6)
+    for a, k in (((1, "a"), {}), ((t, "b c"), {}), ((t, "b", torch.float32), {}), ((t.t(), "d"), dict(contiguous=False))):
+        assert outcome(native.cuda, *a, **k) == outcome(host.python_cuda, *a, **k)
+    for x in (t, t[:, 2:4], t.t(), t[0]):
+        assert outcome(native.rows, x, "r") == outcome(host.python_rows, x, "r")
+    assert torch.equal(native.columns(t, 1, 4), host.python_columns(t, 1, 4)) and native.columns(t, 1, 4).stride() == (6, 1)
+    e = native.empty(t, torch.bfloat16, 3, 5)
+    assert e.dtype == torch.bfloat16 and tuple(e.shape) == (3, 5) and e.device == t.device
+    w = torch.zeros(64, 64, dtype=torch.bfloat16)
+    for x, y in ((w, w), (w[:, 1:], w), (w, w[:, 4:]), (w[:, :63], w), (w[:, 8:], w), (torch.zeros(4, 60, dtype=torch.bfloat16), w)):
+        assert native.odd(x, y) == host.python_odd(x, y)
+
+
+@pytest.mark.gpu
+def test_the_native_side_is_what_launches():
+    from rusty_llama_b200.kernels import ops
+
+    assert host._module is not None and ops._cuda is host._module.cuda
+    x = torch.zeros(4, 6, device="cuda")
+    for a, k in (((x, "a", torch.bfloat16), {}), ((x.t(), "b"), {}), ((x, "c", torch.float32, True), {}), ((x.t(), "d"), dict(contiguous=False))):
+        results = []
+        for f in (host._module.cuda, host.python_cuda):
+            try:
+                results.append(f(*a, **k) is a[0])
+            except KernelError as e:
+                results.append(str(e))
+        assert results[0] == results[1]
+    assert host._module.stream() == host.python_stream()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        assert host._module.stream() == host.python_stream() == torch.cuda.current_stream().cuda_stream
+    with pytest.raises(torch.OutOfMemoryError):
+        host._module.empty(x, torch.float32, 1 << 45)
