@@ -94,66 +94,123 @@ __global__ void moe_router_logits_kernel(const T* __restrict__ x, int ldx, const
     }
 }
 
+// Ordered as floats are, as unsigned integers (what is no number does not get here).
+__device__ __forceinline__ unsigned moe_key(float v) {
+  const unsigned u = __float_as_uint(v);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+
 // One warp per token (four tokens per block): softmax over the E logits (or the logistic function of each), the `top` largest of
-// score + bias; weights s_e (/ (sum of the chosen s + renorm_eps) if renorm) * weight_scale.
-__global__ void moe_router_choose_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int E, int rows, int top,
-                                         int renorm, int n_tokens, int* __restrict__ ids, float* __restrict__ weights,
-                                         float* __restrict__ gate, int logistic, float renorm_eps, float weight_scale) {
-  extern __shared__ float sm[];  // per warp: E scores, E choice scores
+// score + bias; weights s_e (/ (sum of the chosen s + renorm_eps) if renorm) * weight_scale.  logits: `parts` partial sums
+// [parts, n_tokens, rows], added up here in order.
+// A lane has the experts lane + 32 i in registers (EACH of them); a round of the choice is a warp-wide maximum of keys and a minimum of the
+// indices that have it, two instructions where ten shuffles were, and nothing is read back from memory: 2048 tokens, 6 of 64: 4.4 us instead of 16.
+template <int EACH>
+__global__ void __launch_bounds__(128)
+moe_router_choose_kernel(const float* __restrict__ logits, int parts, const float* __restrict__ bias, int E, int rows, int top,
+                         int renorm, int n_tokens, int* __restrict__ ids, float* __restrict__ weights,
+                         float* __restrict__ gate, int logistic, float renorm_eps, float weight_scale) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x * 4 + warp;
   if (t >= n_tokens) return;
-  float* z = sm + (size_t)warp * 2 * E;
-  float* choice = z + E;
   const float* lg = logits + (size_t)t * rows;
+  const size_t part = (size_t)n_tokens * rows;
+  float z[EACH];
+  float gate_z = 0.f;
+#pragma unroll
+  for (int i = 0; i < EACH; ++i) z[i] = 0.f;
+  for (int p0 = 0; p0 < parts; p0 += 4) {  // four partial sums asked for at once
+    float v[4][EACH], gv[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const bool in = p0 + p < parts;
+#pragma unroll
+      for (int i = 0; i < EACH; ++i) v[p][i] = in && lane + 32 * i < E ? __ldcg(lg + (p0 + p) * part + lane + 32 * i) : 0.f;
+      gv[p] = in && rows > E ? __ldcg(lg + (p0 + p) * part + E) : 0.f;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+#pragma unroll
+      for (int i = 0; i < EACH; ++i) z[i] = p0 + p ? z[i] + v[p][i] : v[p][i];
+      gate_z = p0 + p ? gate_z + gv[p] : gv[p];
+    }
+  }
   float mx = -INFINITY, sum = 0.f;
   if (!logistic) {
-    for (int e = lane; e < E; e += 32) mx = fmaxf(mx, lg[e]);
+#pragma unroll
+    for (int i = 0; i < EACH; ++i)
+      if (lane + 32 * i < E) mx = fmaxf(mx, z[i]);
     mx = warp_max(mx);
-    for (int e = lane; e < E; e += 32) sum += expf(lg[e] - mx);
+#pragma unroll
+    for (int i = 0; i < EACH; ++i)
+      if (lane + 32 * i < E) {
+        z[i] = expf(z[i] - mx);
+        sum += z[i];
+      }
     sum = warp_sum(sum);
   }
-  for (int e = lane; e < E; e += 32) {
-    const float s = logistic ? 1.0f / (1.0f + expf(-lg[e])) : expf(lg[e] - mx) / sum;
-    z[e] = s;
-    choice[e] = fmaxf(s + (bias ? bias[e] : 0.f), -FLT_MAX);  // (also what is not a number: every expert stays one that can be chosen once)
-  }
-  __syncwarp();
-  float chosen_sum = 0.f;
-  for (int j = 0; j < top; ++j) {
-    float best = -INFINITY;
-    int at = 0x7fffffff;
-    for (int e = lane; e < E; e += 32)
-      if (choice[e] > best) {  // ascending e within a lane: the lower index keeps a tie
-        best = choice[e];
-        at = e;
-      }
+  unsigned key[EACH];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
-      if (ob > best || (ob == best && oa < at)) {
-        best = ob;
-        at = oa;
-      }
-    }
-    if (lane == 0) {
-      ids[(size_t)t * top + j] = at;
-      weights[(size_t)t * top + j] = z[at];
-      choice[at] = -INFINITY;
-    }
-    chosen_sum += z[at];
-    __syncwarp();
+  for (int i = 0; i < EACH; ++i) {
+    const int e = lane + 32 * i;
+    z[i] = logistic ? 1.0f / (1.0f + expf(-z[i])) : z[i] / sum;
+    // (also what is not a number: every expert stays one that can be chosen once)
+    key[i] = e < E ? moe_key(fmaxf(z[i] + (bias ? bias[e] : 0.f), -FLT_MAX)) : 0u;
   }
-  if (lane == 0 && (renorm || weight_scale != 1.0f))
-    for (int j = 0; j < top; ++j) {
-      float wj = weights[(size_t)t * top + j];
-      if (renorm) wj /= (chosen_sum + renorm_eps);
-      weights[(size_t)t * top + j] = wj * weight_scale;
+  float chosen_sum = 0.f, mine = 0.f;  // mine: lane j keeps the j-th choice's score (top <= 32), or the last of its round of 32
+  for (int j = 0; j < top; ++j) {
+    unsigned best = 0;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) best = max(best, key[i]);
+    best = __reduce_max_sync(0xffffffffu, best);
+    unsigned at = 0xffffffffu;
+#pragma unroll
+    for (int i = EACH - 1; i >= 0; --i)
+      if (key[i] == best && lane + 32 * i < E) at = lane + 32 * i;  // the lower index keeps a tie
+    at = __reduce_min_sync(0xffffffffu, at);
+    float score = 0.f;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i)
+      if (lane + 32 * i == (int)at) {
+        score = z[i];
+        key[i] = 0u;
+      }
+    score = __shfl_sync(0xffffffffu, score, at & 31);
+    chosen_sum += score;
+    if ((j & 31) == lane) {
+      mine = score;
+      ids[(size_t)t * top + j] = (int)at;
+      if (top > 32) weights[(size_t)t * top + j] = score;
     }
-  if (rows > E && lane == 0) gate[t] = 1.0f / (1.0f + expf(-lg[E]));
+  }
+  if (top <= 32) {
+    if (lane < top) weights[(size_t)t * top + lane] = (renorm ? mine / (chosen_sum + renorm_eps) : mine) * weight_scale;
+  } else {
+    for (int j = lane; j < top; j += 32) {  // (written by this very lane)
+      const float w = weights[(size_t)t * top + j];
+      weights[(size_t)t * top + j] = (renorm ? w / (chosen_sum + renorm_eps) : w) * weight_scale;
+    }
+  }
+  if (rows > E && lane == 0) gate[t] = 1.0f / (1.0f + expf(-gate_z));
+}
+
+#define MOE_MAX_EXPERTS 1536  // as the former kernel's shared memory had room for
+static int launch_choose(const float* logits, int parts, const float* bias, int E, int rows, int top, int renorm, int n_tokens, int* ids,
+                         float* weights, float* gate, int logistic, float renorm_eps, float weight_scale, cudaStream_t stream) {
+  const int blocks = (n_tokens + 3) / 4;
+#define RL_CHOOSE(EACH)                                                                                                                  \
+  RL_LAUNCH_CHECK(rl_launch(moe_router_choose_kernel<EACH>, blocks, 128, 0, stream, logits, parts, bias, E, rows, top, renorm, n_tokens, \
+                            ids, weights, gate, logistic, renorm_eps, weight_scale))
+  if (E <= 32) RL_CHOOSE(1);
+  else if (E <= 64) RL_CHOOSE(2);
+  else if (E <= 128) RL_CHOOSE(4);
+  else if (E <= 256) RL_CHOOSE(8);
+  else if (E <= 512) RL_CHOOSE(16);
+  else RL_CHOOSE(48);
+#undef RL_CHOOSE
+  return 0;
 }
 
 // logits: float32 scratch of n_tokens * (E + has_gate) values.
@@ -162,8 +219,7 @@ RL_API int rl_moe_router(const void* x, int ldx, int dtype, const float* w, cons
                          float renorm_eps, float weight_scale, cudaStream_t stream) {
   if (n_tokens <= 0 || E <= 0 || d <= 0 || top <= 0 || top > E) RL_REFUSE(1, "moe_router: T=%d E=%d d=%d top=%d", n_tokens, E, d, top);
   if (has_gate && gate == nullptr) RL_REFUSE(2, "moe_router: a gate row but nowhere to write the gate");
-  const size_t smem = (size_t)4 * 2 * E * sizeof(float);
-  if (smem > 48 * 1024) RL_REFUSE(3, "moe_router: %d experts exceed the kernel's shared memory", E);
+  if (E > MOE_MAX_EXPERTS) RL_REFUSE(3, "moe_router: %d experts exceed %d", E, MOE_MAX_EXPERTS);
   const int rows = E + (has_gate ? 1 : 0);
   dim3 grid((n_tokens + ROUTER_TOKENS - 1) / ROUTER_TOKENS, (rows + 4 * ROUTER_ROWS - 1) / (4 * ROUTER_ROWS));
   if (grid.y > 65535) RL_REFUSE(5, "moe_router: %d experts exceed the grid", E);
@@ -179,21 +235,17 @@ RL_API int rl_moe_router(const void* x, int ldx, int dtype, const float* w, cons
     RL_LAUNCH_CHECK(rl_launch<false>(moe_router_logits_kernel<float, false>, grid, 128, 0, stream, (const float*)x, ldx, w, rows, d, n_tokens, logits));
   else
     RL_REFUSE(4, "moe_router: unknown dtype %d", dtype);
-  RL_LAUNCH_CHECK(rl_launch<false>(moe_router_choose_kernel, (n_tokens + 3) / 4, 128, smem, stream, (const float*)logits, bias, E, rows, top,
-                                   renorm, n_tokens, ids, weights, gate, logistic, renorm_eps, weight_scale));
-  return 0;
+  return launch_choose(logits, 1, bias, E, rows, top, renorm, n_tokens, ids, weights, gate, logistic, renorm_eps, weight_scale, stream);
 }
 
-// The choice alone, from logits that another product made (float32 [n_tokens, E + has_gate]).
-RL_API int rl_moe_choose(const float* logits, const float* bias, int n_tokens, int E, int top, int renorm, int has_gate, int* ids, float* weights,
+// The choice alone, from logits that another product made (float32 [parts, n_tokens, E + has_gate], partial sums).
+RL_API int rl_moe_choose(const float* logits, int parts, const float* bias, int n_tokens, int E, int top, int renorm, int has_gate, int* ids, float* weights,
                          float* gate, int logistic, float renorm_eps, float weight_scale, cudaStream_t stream) {
   if (n_tokens <= 0 || E <= 0 || top <= 0 || top > E) RL_REFUSE(1, "moe_choose: T=%d E=%d top=%d", n_tokens, E, top);
   if (has_gate && gate == nullptr) RL_REFUSE(2, "moe_choose: a gate column but nowhere to write the gate");
-  const size_t smem = (size_t)4 * 2 * E * sizeof(float);
-  if (smem > 48 * 1024) RL_REFUSE(3, "moe_choose: %d experts exceed the kernel's shared memory", E);
-  RL_LAUNCH_CHECK(rl_launch<false>(moe_router_choose_kernel, (n_tokens + 3) / 4, 128, smem, stream, logits, bias, E, E + (has_gate ? 1 : 0), top,
-                                   renorm, n_tokens, ids, weights, gate, logistic, renorm_eps, weight_scale));
-  return 0;
+  if (E > MOE_MAX_EXPERTS) RL_REFUSE(3, "moe_choose: %d experts exceed %d", E, MOE_MAX_EXPERTS);
+  if (parts <= 0) RL_REFUSE(4, "moe_choose: %d partial sums", parts);
+  return launch_choose(logits, parts, bias, E, E + (has_gate ? 1 : 0), top, renorm, n_tokens, ids, weights, gate, logistic, renorm_eps, weight_scale, stream);
 }
 
 // ---------------------------------------------------------------- plan
@@ -202,62 +254,109 @@ RL_API int rl_moe_choose(const float* logits, const float* bias, int n_tokens, i
 // (expert, first row, rows) per tile.  One block per expert: every block counts all experts' pairs in shared memory
 // (it needs the counts of the experts before its own for its first row and its first tile), then lays out its own
 // expert's pairs, each thread a contiguous piece of the pairs so that their order is kept.
+// `always` further matrices, numbers E and up, take every token (a shared expert in pieces of the others' size): their rows come behind the n
+// of the pairs, row n + j T + t is token t's of the j-th (order: its first pair).  Their tiles stand between the others', evenly: blocks that
+// wait for an expert's weights are then beside blocks whose matrix is in L2 and whose rows are many.
 #define PLAN_THREADS 512
+
+// where the i-th of `few` tiles stands among `all`, and how many of the few stand before place p
+__device__ __forceinline__ int plan_place(int i, int few, int all) { return (int)(((long long)i * all) / few); }
+__device__ __forceinline__ int plan_before(int p, int few, int all) {  // the least i with plan_place(i) >= p
+  return (int)(((long long)p * few + all - 1) / all);
+}
 
 __global__ void __launch_bounds__(PLAN_THREADS)
 moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* __restrict__ order, int* __restrict__ place,
-                int* __restrict__ tiles, int tile_rows) {
+                int* __restrict__ tiles, int tile_rows, int always, int top) {
   extern __shared__ int cnt[];  // E counts
-  __shared__ int scan[PLAN_THREADS];
-  __shared__ int first_row, first_tile;
+  __shared__ int scan[PLAN_THREADS / 32], sums[3];
   pdl_trigger();
   pdl_wait();
-  const int e = blockIdx.x, tid = threadIdx.x;
+  const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < E; i += PLAN_THREADS) cnt[i] = 0;
+  if (tid < 3) sums[tid] = 0;
   __syncthreads();
   const int per = (n + PLAN_THREADS - 1) / PLAN_THREADS;
   const int lo = min(n, tid * per), hi = min(n, lo + per);
   int mine = 0;
-  for (int i = lo; i < hi; ++i) {
-    const int id = ids[i];
-    if (id < E) atomicAdd(&cnt[id], 1);
-    else if (e == 0) place[i] = -1;  // (no expert of the plan: it has no row)
-    mine += id == e;
+  for (int i0 = lo; i0 < hi; i0 += 8) {  // eight asked for at once: one after the other the trips to L2 were most of the kernel
+    int id[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) id[u] = i0 + u < hi ? __ldcg(ids + i0 + u) : 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i0 + u < hi) {
+        if (id[u] < E) atomicAdd(&cnt[id[u]], 1);
+        else if (e == 0) place[i0 + u] = -1;  // (no expert of the plan: it has no row)
+        mine += id[u] == e;
+      }
   }
-  scan[tid] = mine;
+  int before = mine;  // of this warp's threads up to this one
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += v;
+  }
+  if (lane == 31) scan[warp] = before;
   __syncthreads();
-  if (tid == 0) {
-    int at = 0, nt = 0;
-    for (int k = 0; k < e; ++k) {
-      at += cnt[k];
-      nt += (cnt[k] + tile_rows - 1) / tile_rows;
+  for (int k = tid; k < E; k += PLAN_THREADS) {  // rows and tiles of the experts before this one, tiles of all
+    const int c = cnt[k], nt = (c + tile_rows - 1) / tile_rows;
+    if (k < e) {
+      atomicAdd(&sums[0], c);
+      atomicAdd(&sums[1], nt);
     }
-    first_row = at;
-    first_tile = nt;
-    if (e == E - 1) tiles[0] = nt + (cnt[e] + tile_rows - 1) / tile_rows;
+    atomicAdd(&sums[2], nt);
   }
-  // exclusive scan of the threads' counts (Hillis-Steele over the block)
-  for (int o = 1; o < PLAN_THREADS; o <<= 1) {
-    const int v = tid >= o ? scan[tid - o] : 0;
-    __syncthreads();
-    scan[tid] += v;
-    __syncthreads();
-  }
-  int r = first_row + scan[tid] - mine;
-  for (int i = lo; i < hi; ++i)
-    if (ids[i] == e) {
-      order[r] = i;
-      place[i] = r;
-      ++r;
+  __syncthreads();
+  const int T = n / top, per_always = (T + tile_rows - 1) / tile_rows, few = always * per_always, all = sums[2] + few;
+  if (e == 0 && tid == 0) tiles[0] = all;
+  int first_row, first_tile, c;
+  if (e < E) {
+    first_row = sums[0];
+    first_tile = sums[1];
+    c = cnt[e];
+    int r = first_row + before - mine;
+    for (int w = 0; w < warp; ++w) r += scan[w];
+    for (int i0 = lo; i0 < hi && mine > 0; i0 += 8) {
+      int id[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) id[u] = i0 + u < hi ? __ldcg(ids + i0 + u) : -1;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i0 + u < hi && id[u] == e) {
+          order[r] = i0 + u;
+          place[i0 + u] = r;
+          ++r;
+          --mine;
+        }
     }
+  } else {
+    first_row = n + (e - E) * T;
+    first_tile = (e - E) * per_always;
+    c = T;
+    for (int t = tid; t < T; t += PLAN_THREADS) order[first_row + t] = t * top;
+  }
   // As few tiles as hold the expert's rows.  Where the products take tiles of any multiple of 16 rows (the heights from 128 on) they
   // are equally high: 300 rows in two tiles of 160 and 140 instead of 256 and 44 (no last tile is empty: the others hold at most
   // tile_rows each).
-  const int c = cnt[e], n_tiles = (c + tile_rows - 1) / tile_rows;
+  const int n_tiles = (c + tile_rows - 1) / tile_rows;
   int high = tile_rows;
   if (tile_rows >= 128 && n_tiles > 0) high = min(tile_rows, ((c + n_tiles - 1) / n_tiles + 15) & ~15);
   for (int k = tid; k < n_tiles; k += PLAN_THREADS) {
-    int* t = tiles + 1 + 3 * (first_tile + k);
+    int at = first_tile + k;
+    if (e >= E) {
+      at = plan_place(at, few, all);
+    } else if (few > 0) {
+      // the at-th place that none of the few has: places before p that are free are p - plan_before(p); find the first p with at + 1 of them
+      int lo_p = at, hi_p = at + few;
+      while (lo_p < hi_p) {
+        const int p = (lo_p + hi_p) >> 1;
+        if (p + 1 - plan_before(p + 1, few, all) >= at + 1) hi_p = p;
+        else lo_p = p + 1;
+      }
+      at = lo_p;
+    }
+    int* t = tiles + 1 + 3 * at;
     t[0] = e;
     t[1] = first_row + k * high;
     t[2] = min(high, c - k * high);
@@ -287,11 +386,11 @@ RL_API int rl_moe_table_lookup(const int* tokens, const int* table, int top, int
 
 RL_API int rl_moe_tile_rows() { return MOE_TM; }
 
-RL_API int rl_moe_plan(const int* ids, int n, int E, int* order, int* place, int* tiles, int tile_rows, cudaStream_t stream) {
-  if (n <= 0 || E <= 0 || tile_rows <= 0) RL_REFUSE(1, "moe_plan: n=%d E=%d tile_rows=%d", n, E, tile_rows);
+RL_API int rl_moe_plan(const int* ids, int n, int E, int* order, int* place, int* tiles, int tile_rows, int always, int top, cudaStream_t stream) {
+  if (n <= 0 || E <= 0 || tile_rows <= 0 || always < 0 || top <= 0 || n % top) RL_REFUSE(1, "moe_plan: n=%d E=%d tile_rows=%d always=%d top=%d", n, E, tile_rows, always, top);
   const size_t smem = (size_t)E * sizeof(int);
   if (smem > 40 * 1024) RL_REFUSE(2, "moe_plan: %d experts exceed the kernel's shared memory", E);
-  RL_LAUNCH_CHECK(rl_launch<false>(moe_plan_kernel, E, PLAN_THREADS, smem, stream, ids, n, E, order, place, tiles, tile_rows));
+  RL_LAUNCH_CHECK(rl_launch(moe_plan_kernel, E + always, PLAN_THREADS, smem, stream, ids, n, E, order, place, tiles, tile_rows, always, top));
   return 0;
 }
 
@@ -400,11 +499,12 @@ RL_API int rl_moe_gemm(const void* x, int ldx, int dtype, const int* order, int 
 
 // ---------------------------------------------------------------- weighted sum of a token's experts
 // out[t, :] = sum_j weights[t, j] * y[place[t * top + j], :]  (+ gate[t] * shared[t, :]); y is float32.  A negative place takes
-// x[t, :], the experts' input (of type TS, like `shared`), in the place of y.
+// x[t, :], the experts' input (of type TS, like `shared`), in the place of y.  The rows of `always` further matrices (see the plan) are
+// y[T top + j T + t, :] and count gate[t] (1 without a gate) each.
 template <typename TS, typename TO>
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
                                    int top, const TS* __restrict__ shared, const float* __restrict__ gate, TO* __restrict__ out, int d,
-                                   const TS* __restrict__ x, int ldx) {
+                                   const TS* __restrict__ x, int ldx, int always) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x;
@@ -415,6 +515,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
       v += weights[(size_t)t * top + j] * (p >= 0 ? y[(size_t)p * d + i] : x != nullptr ? to_f32(x[(size_t)t * ldx + i]) : 0.f);
     }
     if (shared) v += (gate ? gate[t] : 1.f) * to_f32(shared[(size_t)t * d + i]);
+    for (int j = 0; j < always; ++j) v += (gate ? gate[t] : 1.f) * y[((size_t)gridDim.x * (top + j) + t) * d + i];
     out[(size_t)t * d + i] = from_f32<TO>(v);
   }
 }
@@ -425,30 +526,32 @@ template <typename TS, typename TO>
 __global__ void __launch_bounds__(256)
 moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights, int top,
                        const TS* __restrict__ shared, const float* __restrict__ gate, TO* __restrict__ out, int d,
-                       const TS* __restrict__ x, int ldx) {
+                       const TS* __restrict__ x, int ldx, int always) {
   pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (i >= d) return;
   float v[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int j0 = 0; j0 < top; j0 += COMBINE_AHEAD) {
+  const int all = top + always;
+  for (int j0 = 0; j0 < all; j0 += COMBINE_AHEAD) {
     int p[COMBINE_AHEAD];
     float w[COMBINE_AHEAD], f[COMBINE_AHEAD][4];
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u) {
-      const bool in = j0 + u < top;
-      p[u] = in ? __ldcg(place + (size_t)t * top + j0 + u) : -1;
-      w[u] = in ? __ldcg(weights + (size_t)t * top + j0 + u) : 0.f;
+      const int j = j0 + u;
+      const bool in = j < top;
+      p[u] = in ? __ldcg(place + (size_t)t * top + j) : j < all ? (int)gridDim.x * j + t : -1;
+      w[u] = in ? __ldcg(weights + (size_t)t * top + j) : j < all && gate ? __ldcg(gate + t) : 1.f;
     }
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u) {
-      if (j0 + u >= top || (p[u] < 0 && x == nullptr)) f[u][0] = f[u][1] = f[u][2] = f[u][3] = 0.f;
+      if (j0 + u >= all || (p[u] < 0 && x == nullptr)) f[u][0] = f[u][1] = f[u][2] = f[u][3] = 0.f;
       else if (p[u] >= 0) load4_g<float>(y + (size_t)p[u] * d + i, f[u]);
       else load4_g<TS>(x + (size_t)t * ldx + i, f[u]);
     }
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u)
-      if (j0 + u < top)
+      if (j0 + u < all)
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] += w[u] * f[u][e];
   }
@@ -463,9 +566,10 @@ moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ plac
 }
 
 RL_API int rl_moe_combine(const float* y, const int* place, const float* weights, int top, const void* shared, int shared_dtype,
-                          const float* gate, void* out, int out_dtype, int n_tokens, int d, const void* x, int x_dtype, int ldx,
+                          const float* gate, void* out, int out_dtype, int n_tokens, int d, const void* x, int x_dtype, int ldx, int always,
                           cudaStream_t stream) {
-  if (n_tokens <= 0 || d <= 0 || top <= 0) RL_REFUSE(1, "moe_combine: T=%d d=%d top=%d", n_tokens, d, top);
+  if (n_tokens <= 0 || d <= 0 || top <= 0 || always < 0) RL_REFUSE(1, "moe_combine: T=%d d=%d top=%d always=%d", n_tokens, d, top, always);
+  if ((long long)n_tokens * (top + always) > 0x7fffffffLL) RL_REFUSE(4, "moe_combine: %d tokens of %d choices are too many", n_tokens, top + always);
   if (shared == nullptr && x != nullptr) shared_dtype = x_dtype;
   if (x != nullptr && shared_dtype != x_dtype) RL_REFUSE(3, "moe_combine: shared result of type %d beside an input of type %d", shared_dtype, x_dtype);
   // (which kernel runs depends on sizes and addresses only; both add in the same order)
@@ -474,10 +578,10 @@ RL_API int rl_moe_combine(const float* y, const int* place, const float* weights
 #define RL_MC(TS, TO)                                                                                                          \
   if (vec)                                                                                                                     \
     RL_LAUNCH_CHECK(rl_launch(moe_combine_vec_kernel<TS, TO>, grid, 256, 0, stream, y, place, weights, top, (const TS*)shared, gate, \
-                              (TO*)out, d, (const TS*)x, ldx));                                                                \
+                              (TO*)out, d, (const TS*)x, ldx, always));                                                        \
   else                                                                                                                         \
   RL_LAUNCH_CHECK(rl_launch<false>(moe_combine_kernel<TS, TO>, n_tokens, 256, 0, stream, y, place, weights, top, (const TS*)shared, \
-                                   gate, (TO*)out, d, (const TS*)x, ldx))
+                                   gate, (TO*)out, d, (const TS*)x, ldx, always))
   if (shared_dtype == RL_BF16 && out_dtype == RL_F32) { RL_MC(bf16, float); }
   else if (shared_dtype == RL_F32 && out_dtype == RL_F32) { RL_MC(float, float); }
   else if (shared_dtype == RL_BF16 && out_dtype == RL_BF16) { RL_MC(bf16, bf16); }

@@ -1353,12 +1353,13 @@ def moe_router(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], n
 
 def moe_choose(logits: torch.Tensor, bias: Optional[torch.Tensor], n_experts: int, top: int, renormalize: bool = False,
                logistic: bool = False, renorm_eps: float = 0.0, weight_scale: float = 1.0):
-    """`moe_router` behind its product: logits float32 [T, E (+1)] that another product made."""
+    """`moe_router` behind its product: logits float32 [T, E (+1)] that another product made, or partial sums [parts, T, E (+1)] of them."""
     _cuda(logits, "moe_choose logits", torch.float32)
-    if not (logits.dim() == 2 and logits.shape[1] in (n_experts, n_experts + 1)):
+    parts = 1 if logits.dim() == 2 else logits.shape[0]
+    if not (logits.dim() in (2, 3) and logits.shape[-1] in (n_experts, n_experts + 1)):
         raise KernelError(f"moe_choose: logits {tuple(logits.shape)} for {n_experts} experts")
-    T = logits.shape[0]
-    has_gate = logits.shape[1] == n_experts + 1
+    T = logits.shape[-2]
+    has_gate = logits.shape[-1] == n_experts + 1
     if bias is not None:
         _cuda(bias, "moe_choose bias", torch.float32)
         _need(bias.numel() == n_experts, "moe_choose: one bias per expert")
@@ -1366,7 +1367,7 @@ def moe_choose(logits: torch.Tensor, bias: Optional[torch.Tensor], n_experts: in
     weights = _empty(logits, torch.float32, T, top)
     gate = _empty(logits, torch.float32, T) if has_gate else None
     lib = library("moe")
-    rc = lib.rl_moe_choose(logits, bias, T, n_experts, top, 1 if renormalize else 0, 1 if has_gate else 0,
+    rc = lib.rl_moe_choose(logits, parts, bias, T, n_experts, top, 1 if renormalize else 0, 1 if has_gate else 0,
                            ids, weights, gate, 1 if logistic else 0, float(renorm_eps), float(weight_scale), _stream())
     _check(lib, rc, "moe_choose")
     return ids, weights, gate
@@ -1409,19 +1410,23 @@ def moe_max_tiles(n_pairs: int, n_experts: int, tile_rows: int = 0) -> int:
     return min(n_pairs, n_pairs // rows + n_experts)
 
 
-def moe_plan(ids: torch.Tensor, n_experts: int, tile_rows: int = 0):
-    """ids int32 [T, top] -> (order [T top], place [T top], tiles [1 + 3 max_tiles], max_tiles), all on the device.
+def moe_plan(ids: torch.Tensor, n_experts: int, tile_rows: int = 0, always: int = 0):
+    """ids int32 [T, top] -> (order [T (top + always)], place [T top], tiles [1 + 3 max_tiles], max_tiles), all on the device.
     A pair whose id is n_experts or more names no expert of the plan: it has no row, and its place is -1.
-    tile_rows: the height of a row tile (0: the plain product's)."""
+    tile_rows: the height of a row tile (0: the plain product's).  always: matrices behind the experts' that take every token: row
+    T top + j T + t of the layout is token t's of the j-th."""
     _cuda(ids, "moe_plan ids", torch.int32)
     n = ids.numel()
     tile_rows = tile_rows or moe_tile_rows()
     max_tiles = moe_max_tiles(n, n_experts, tile_rows)
-    order = _empty(ids, torch.int32, n)
+    top = ids.shape[-1]
+    if always:
+        max_tiles += always * ((n // top + tile_rows - 1) // tile_rows)
+    order = _empty(ids, torch.int32, n + always * (n // top))
     place = _empty(ids, torch.int32, n)
     tiles = _empty(ids, torch.int32, 1 + 3 * max_tiles)
     lib = library("moe")
-    rc = lib.rl_moe_plan(ids, n, n_experts, order, place, tiles, tile_rows, _stream())
+    rc = lib.rl_moe_plan(ids, n, n_experts, order, place, tiles, tile_rows, always, top, _stream())
     _check(lib, rc, "moe_plan")
     return order, place, tiles, max_tiles
 
@@ -1475,16 +1480,17 @@ def moe_gemm(
 
 def moe_combine(
     y: torch.Tensor, place: torch.Tensor, weights: torch.Tensor, shared: Optional[torch.Tensor], gate: Optional[torch.Tensor],
-    out_dtype: torch.dtype = torch.float32, x: Optional[torch.Tensor] = None,
+    out_dtype: torch.dtype = torch.float32, x: Optional[torch.Tensor] = None, always: int = 0,
 ) -> torch.Tensor:
-    """out[t] = sum_j weights[t, j] * y[place[t, j]] (+ gate[t] * shared[t]); y float32 [T top, d].  Where place is negative the
-    term is weights[t, j] * x[t] (x [T, d], the experts' input: a choice that hands the input on)."""
+    """out[t] = sum_j weights[t, j] * y[place[t, j]] (+ gate[t] * shared[t]); y float32 [T (top + always), d].  Where place is negative the
+    term is weights[t, j] * x[t] (x [T, d], the experts' input: a choice that hands the input on).  always: the rows of that many
+    matrices that take every token stand behind the pairs' (`moe_plan`) and are added like `shared`."""
     _cuda(y, "moe_combine y", torch.float32)
     _cuda(weights, "moe_combine weights", torch.float32)
     _cuda(place, "moe_combine place", torch.int32)
     T, top = weights.shape
     d = y.shape[1]
-    _need(y.shape[0] == T * top and place.numel() == T * top, "moe_combine: sizes do not fit")
+    _need(y.shape[0] == T * (top + always) and place.numel() == T * top, "moe_combine: sizes do not fit")
     shared_dt = _F32
     if shared is not None:
         _cuda(shared, "moe_combine shared")
@@ -1501,7 +1507,7 @@ def moe_combine(
     lib = library("moe")
     rc = lib.rl_moe_combine(
         y, place, weights, top, shared, shared_dt, gate, out, _dt(out, "moe_combine out"),
-        T, d, x, x_dt, xs, _stream(),
+        T, d, x, x_dt, xs, always, _stream(),
     )
     _check(lib, rc, "moe_combine")
     return out

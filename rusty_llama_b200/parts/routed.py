@@ -8,6 +8,7 @@ import torch
 
 from ..errors import ConfigError
 from ..kernels import ops
+from ..kernels.device import sm_count
 from ..kernels.linear import linear, linear_swiglu
 from .base import FEED_FORWARDS, FeedForward, ParamInfo
 
@@ -129,6 +130,14 @@ class RoutedExperts(FeedForward):
             exact = self.rt.dtype == torch.bfloat16 and self.d % 8 == 0 and torch.equal(narrow.to(torch.float32), self.w_router)
             self.w_router16 = narrow if exact else None
         self.bias = tensors[self.prefix + self.names["bias"]].contiguous() if self.has_bias else None
+        # A shared expert of a multiple of the others' size is that many experts more that take every token: for steps that `_joins` names
+        # its matrices stand behind the others', too.
+        self.always = 0
+        if self.shared_ff and self.shared_ff % self.ff == 0 and self.rt.dtype == torch.bfloat16 and self.d % 8 == 0 and self.ff % 8 == 0:
+            n = self.always = self.shared_ff // self.ff
+            self.w_gate = torch.cat([self.w_gate, tensors[self._shared("gate")].view(n, self.ff, self.d)])
+            self.w_up = torch.cat([self.w_up, tensors[self._shared("up")].view(n, self.ff, self.d)])
+            self.w_down = torch.cat([self.w_down, tensors[self._shared("down")].view(self.d, n, self.ff).transpose(0, 1)])
         if self.shared_ff:
             gate, up = tensors[self._shared("gate")], tensors[self._shared("up")]
             self.shared_fused = self.rt.dtype == torch.bfloat16
@@ -146,21 +155,23 @@ class RoutedExperts(FeedForward):
         else:
             how = dict(renormalize=self.renormalize, logistic=self.router == "sigmoid", renorm_eps=self.renorm_eps, weight_scale=self.weight_scale)
             if self.w_router16 is not None:
-                ids, weights, gate = ops.moe_choose(linear(xn, self.w_router16, out_dtype=torch.float32), self.bias, self.choices, self.top, **how)
+                ids, weights, gate = ops.moe_choose(self._logits(xn), self.bias, self.choices, self.top, **how)
             else:
                 ids, weights, gate = ops.moe_router(xn, self.w_router, self.bias, self.choices, self.top, **how)
         # the height of a row tile; the plain kernels (32-bit runs, sizes that break 16-byte rows) have their own
         tile_rows = 0
         if xn.dtype == torch.bfloat16 and self.d % 8 == 0 and self.ff % 8 == 0:
             tile_rows = ops.moe_mma_tile_rows(T * self.top, self.E)
-        order, place, tiles, max_tiles = ops.moe_plan(ids, self.E, tile_rows)
+        always = self.always if self._joins(T) else 0
+        order, place, tiles, max_tiles = ops.moe_plan(ids, self.E, tile_rows, always)
+        n_rows = T * (self.top + always)
         if self.gated:
-            h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, T * self.top, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act)
+            h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, n_rows, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act)
         else:
-            h = ops.moe_gemm(xn, self.w_up, tiles, max_tiles, T * self.top, order=order, gather_div=self.top, tile_rows=tile_rows, act="relu2")
-        y = ops.moe_gemm(h, self.w_down, tiles, max_tiles, T * self.top, out_dtype=torch.float32, tile_rows=tile_rows)
+            h = ops.moe_gemm(xn, self.w_up, tiles, max_tiles, n_rows, order=order, gather_div=self.top, tile_rows=tile_rows, act="relu2")
+        y = ops.moe_gemm(h, self.w_down, tiles, max_tiles, n_rows, out_dtype=torch.float32, tile_rows=tile_rows)
         shared = None
-        if self.shared_ff:
+        if self.shared_ff and not always:
             if self.shared_fused:
                 hs = linear_swiglu(xn, self.ws_gate_up, act=self.act)
             elif self.act is not None:
@@ -168,4 +179,22 @@ class RoutedExperts(FeedForward):
             else:
                 hs = ops.swiglu(linear(xn, self.ws_gate_up))
             shared = linear(hs, self.ws_down)
-        return ops.moe_combine(y, place, weights, shared, gate, x=xn if self.identity else None)
+        return ops.moe_combine(y, place, weights, shared, gate, x=xn if self.identity else None, always=always)
+
+    def _joins(self, T: int) -> bool:
+        """Whether a shared expert's rows go through the experts' two products: where both stream weights, which two launches less and one tail
+        instead of three help (a part alone, us: 64 experts of 1408 x 2048 and two more, 64 tokens 222 instead of 245, 16 tokens 173 instead of
+        198; 32 of 2048 x 4096 and one, 96 tokens 312 instead of 332, 8 tokens 202 instead of 209).  One token has too few tiles for that (64 and 92
+        instead of 59 and 80), and many tokens' products of one matrix are dense ones, where the prompt product is the faster kernel (1400 and
+        2048 tokens: level)."""
+        return T >= 8 and T * self.top <= 64 * self.E
+
+    def _logits(self, xn: torch.Tensor) -> torch.Tensor:
+        """The router's product, as partial sums over ranges of 256 of k where whole sums would give no more than half of the SMs a tile of
+        the output (32 experts of width 4096, 96 tokens: 6 us instead of 24; 64 of width 2048, 2048 tokens: 7 instead of 15)."""
+        M, K = xn.shape
+        rows = self.w_router16.shape[0]
+        parts = K // 256
+        if M <= 32 or parts < 2 or 2 * ((M + 127) // 128) * ((rows + 255) // 256) > sm_count(xn.device) or xn.stride(0) % 8 or xn.data_ptr() % 16:
+            return linear(xn, self.w_router16, out_dtype=torch.float32)
+        return ops.gemm_tc(xn, self.w_router16, torch.float32, k_splits=parts)
