@@ -324,8 +324,9 @@ scalar_chunk_state_kernel(const bf16* __restrict__ k, const bf16* __restrict__ v
   }
 }
 
-// (2): V numbers of a (sequence, head)'s state per thread; leaves in every chunk's place the state BEFORE that chunk.
-template <int V>
+// (2): V numbers of a (sequence, head)'s state per thread; leaves in every chunk's place the state BEFORE that chunk.  HALVES (V = 4): as the
+// two bfloat16 halves that (3) multiplies with, those of four neighbouring numbers side by side in the 16 bytes that the four had.
+template <int V, bool HALVES>
 __global__ void scalar_chunk_scan_kernel(float* __restrict__ state, const int* __restrict__ slot_ids, const int* __restrict__ seq_start,
                                          float* __restrict__ scratch, const float* __restrict__ chunk_decay, int max_chunks, int H, int elems) {
   pdl_trigger();
@@ -353,7 +354,13 @@ __global__ void scalar_chunk_scan_kernel(float* __restrict__ state, const int* _
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (c0 + j < n_chunks) {
-        if (V == 4) store4<float>(u + (size_t)(c0 + j) * elems, S);
+        if constexpr (HALVES) {
+          bf16 hi[4], lo[4];
+#pragma unroll
+          for (int v = 0; v < 4; ++v) sc_split(S[v], hi[v], lo[v]);
+          *reinterpret_cast<uint4*>(u + (size_t)(c0 + j) * elems) =
+              make_uint4(sc_pack(hi[0], hi[1]), sc_pack(hi[2], hi[3]), sc_pack(lo[0], lo[1]), sc_pack(lo[2], lo[3]));
+        } else if (V == 4) store4<float>(u + (size_t)(c0 + j) * elems, S);
         else u[(size_t)(c0 + j) * elems] = S[0];
 #pragma unroll
         for (int v = 0; v < V; ++v) S[v] = d[j] * S[v] + add[j][v];
@@ -364,8 +371,11 @@ __global__ void scalar_chunk_scan_kernel(float* __restrict__ state, const int* _
 }
 
 // (3): a block of four warps per (sequence, head, chunk), a warp per 16 tokens.  The state before the chunk takes the place of the
-// chunk's keys and values in shared memory, one bfloat16 half of it after the other.
-template <int HDK, int HDV>
+// chunk's keys and values in shared memory, one bfloat16 half of it after the other; with HALVES (as (2) leaves them) both at once and without
+// another look at them: eight columns of the tile are the halves of four, and the sums over both meet by a shuffle (1200 and 848
+// tokens, 64 heads of 128 x 64: 52 us instead of 67, and the scan 17 instead of 23).  One walk of a block per head through all chunks, its sums
+// in registers, in the place of (1) and (2), took 77 us where they take 53: 6 us a chunk, latencies one after the other.
+template <int HDK, int HDV, bool HALVES>
 __global__ void __launch_bounds__(128)
 scalar_chunk_out_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, int in_stride,
                         const float* __restrict__ log_decay, const float* __restrict__ in_scale, const int* __restrict__ seq_start,
@@ -453,47 +463,89 @@ scalar_chunk_out_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, 
 #pragma unroll
   for (int i = 0; i < HDV / 8; ++i) inter[i][0] = inter[i][1] = inter[i][2] = inter[i][3] = 0.f;
   const float* sp = scratch + ((size_t)blockIdx.x * max_chunks + c) * dim * vdim;
-  bf16* st_s = k_s;  // [HDK][VS]
-  for (int pass = 0; pass < 2; ++pass) {
-    __syncthreads();  // the keys and values (or the first half) are no longer read
-    if ((vdim & 3) == 0) {  // four numbers a load, four loads in flight
-#pragma unroll 4
-      for (int idx = tid; idx < HDK * (HDV / 4); idx += 128) {
-        const int r = idx / (HDV / 4), cc = 4 * (idx - r * (HDV / 4));
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < dim && cc < vdim) t = __ldcg(reinterpret_cast<const float4*>(sp + (size_t)r * vdim + cc));
-        const float f[4] = {t.x, t.y, t.z, t.w};
-        bf16 o[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          bf16 hi, lo;
-          sc_split(f[e], hi, lo);
-          o[e] = pass == 0 ? hi : lo;
-        }
-        uint2 raw;
-        raw.x = sc_pack(o[0], o[1]);
-        raw.y = sc_pack(o[2], o[3]);
-        *reinterpret_cast<uint2*>(st_s + r * VS + cc) = raw;
-      }
-    } else {
-      for (int idx = tid; idx < HDK * HDV; idx += 128) {
-        const int r = idx / HDV, cc = idx - r * HDV;
-        bf16 hi = __float2bfloat16_rn(0.f), lo = hi;
-        if (r < dim && cc < vdim) sc_split(__ldcg(sp + (size_t)r * vdim + cc), hi, lo);
-        st_s[r * VS + cc] = pass == 0 ? hi : lo;
-      }
+  bf16* st_s = k_s;  // [HDK][VS]; with halves [HDK][2 HDV + 8]
+  if constexpr (HALVES) {
+    constexpr int HS = 2 * HDV + 8;
+    __syncthreads();  // the keys and values are no longer read
+#pragma unroll 8
+    for (int idx = tid; idx < HDK * (HDV / 4); idx += 128) {
+      const int r = idx / (HDV / 4), q4 = idx % (HDV / 4);
+      const bool here = r < dim && 4 * q4 < vdim;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(st_s + r * HS + 8 * q4)), "l"(here ? sp + (size_t)r * vdim + 4 * q4 : scratch), "r"(here ? 16 : 0) : "memory");
     }
+    sc_cp_async_wait_all();
     __syncthreads();
+    // (a quarter of the columns at a time, so that the sums over both halves fit the registers beside the others)
 #pragma unroll
-    for (int kk = 0; kk < HDK / 16; ++kk) {
-      uint32_t a[4];
-      sc_ldmatrix_x4(a, qa + kk * 16);
+    for (int part = 0; part < HDV / 32; ++part) {
+      float both[8][4];
 #pragma unroll
-      for (int dp = 0; dp < HDV / 16; ++dp) {
-        uint32_t b[4];
-        sc_ldmatrix_x4_trans(b, st_s + (size_t)(kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * VS + dp * 16 + 8 * (lane >> 4));
-        sc_mma(inter[2 * dp], a, b[0], b[1]);
-        sc_mma(inter[2 * dp + 1], a, b[2], b[3]);
+      for (int i = 0; i < 8; ++i) both[i][0] = both[i][1] = both[i][2] = both[i][3] = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < HDK / 16; ++kk) {
+        uint32_t a[4];
+        sc_ldmatrix_x4(a, qa + kk * 16);
+#pragma unroll
+        for (int dp = 0; dp < 4; ++dp) {
+          uint32_t b[4];
+          sc_ldmatrix_x4_trans(b, st_s + (size_t)(kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * HS + part * 64 + dp * 16 + 8 * (lane >> 4));
+          sc_mma(both[2 * dp], a, b[0], b[1]);
+          sc_mma(both[2 * dp + 1], a, b[2], b[3]);
+        }
+      }
+      // piece i: lanes t4 < 2 have columns 4 i + 2 t4 and one on of the rounded halves, lanes t4 >= 2 the same of what the rounding left
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) both[i][e] += __shfl_xor_sync(0xffffffffu, both[i][e], 2);
+      // to where the scores' product has them: piece j's columns 8 j + 2 t4 are in pieces 2 j (lanes t4 < 2) and 2 j + 1, at the place t4 & 1
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) inter[4 * part + j][e] = t4 < 2 ? both[2 * j][e] : both[2 * j + 1][e];
+    }
+  } else {
+  for (int pass = 0; pass < 2; ++pass) {
+      __syncthreads();  // the keys and values (or the first half) are no longer read
+      if ((vdim & 3) == 0) {  // four numbers a load, four loads in flight
+  #pragma unroll 4
+        for (int idx = tid; idx < HDK * (HDV / 4); idx += 128) {
+          const int r = idx / (HDV / 4), cc = 4 * (idx - r * (HDV / 4));
+          float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (r < dim && cc < vdim) t = __ldcg(reinterpret_cast<const float4*>(sp + (size_t)r * vdim + cc));
+          const float f[4] = {t.x, t.y, t.z, t.w};
+          bf16 o[4];
+  #pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            bf16 hi, lo;
+            sc_split(f[e], hi, lo);
+            o[e] = pass == 0 ? hi : lo;
+          }
+          uint2 raw;
+          raw.x = sc_pack(o[0], o[1]);
+          raw.y = sc_pack(o[2], o[3]);
+          *reinterpret_cast<uint2*>(st_s + r * VS + cc) = raw;
+        }
+      } else {
+        for (int idx = tid; idx < HDK * HDV; idx += 128) {
+          const int r = idx / HDV, cc = idx - r * HDV;
+          bf16 hi = __float2bfloat16_rn(0.f), lo = hi;
+          if (r < dim && cc < vdim) sc_split(__ldcg(sp + (size_t)r * vdim + cc), hi, lo);
+          st_s[r * VS + cc] = pass == 0 ? hi : lo;
+        }
+      }
+      __syncthreads();
+  #pragma unroll
+      for (int kk = 0; kk < HDK / 16; ++kk) {
+        uint32_t a[4];
+        sc_ldmatrix_x4(a, qa + kk * 16);
+  #pragma unroll
+        for (int dp = 0; dp < HDV / 16; ++dp) {
+          uint32_t b[4];
+          sc_ldmatrix_x4_trans(b, st_s + (size_t)(kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * VS + dp * 16 + 8 * (lane >> 4));
+          sc_mma(inter[2 * dp], a, b[0], b[1]);
+          sc_mma(inter[2 * dp + 1], a, b[2], b[3]);
+        }
       }
     }
   }
@@ -528,9 +580,13 @@ template <int HDK, int HDV>
 static int launch_scalar_chunked(const bf16* q, const bf16* k, const bf16* v, int in_stride, const float* log_decay, const float* in_scale,
                                  float* state, const int* slot_ids, const int* seq_start, float* scratch, float* chunk_decay, float* out,
                                  int out_stride, int n_seqs, int max_chunks, int H, int QH, int dim, int vdim, cudaStream_t stream) {
-  const size_t smem1 = (size_t)SC * ((HDK + 8) + 2 * (HDV + 8)) * sizeof(bf16), smem3 = (size_t)SC * (2 * (HDK + 8) + (HDV + 8)) * sizeof(bf16);
+  // (rows of whole fours, which the scan can leave as halves and (3) fetch 16 bytes at a time)
+  const bool halves = vdim % 4 == 0;
+  const size_t rows = (size_t)SC * (HDK + 8), tiles = (size_t)SC * (HDK + 8 + HDV + 8), state_tile = (size_t)HDK * (2 * HDV + 8);
+  const size_t smem1 = (size_t)SC * ((HDK + 8) + 2 * (HDV + 8)) * sizeof(bf16), smem3 = (rows + (halves && state_tile > tiles ? state_tile : tiles)) * sizeof(bf16);
+  auto out3 = halves ? scalar_chunk_out_kernel<HDK, HDV, true> : scalar_chunk_out_kernel<HDK, HDV, false>;
   if ((smem1 > 48 * 1024 && cudaFuncSetAttribute(scalar_chunk_state_kernel<HDK, HDV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) ||
-      (smem3 > 48 * 1024 && cudaFuncSetAttribute(scalar_chunk_out_kernel<HDK, HDV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess))
+      (smem3 > 48 * 1024 && cudaFuncSetAttribute(out3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess))
     RL_REFUSE(5, "scalar_decay_chunked: %zu bytes of shared memory refused", smem3);
   const int elems = dim * vdim;
   dim3 grid(n_seqs * H, max_chunks);
@@ -538,14 +594,14 @@ static int launch_scalar_chunked(const bf16* q, const bf16* k, const bf16* v, in
                             chunk_decay, max_chunks, H, QH, dim, vdim));
   if (elems % 4 == 0) {
     dim3 grid2(n_seqs * H, (elems / 4 + 127) / 128);
-    RL_LAUNCH_CHECK(rl_launch(scalar_chunk_scan_kernel<4>, grid2, 128, 0, stream, state, slot_ids, seq_start, scratch, (const float*)chunk_decay,
+    RL_LAUNCH_CHECK(rl_launch(halves ? scalar_chunk_scan_kernel<4, true> : scalar_chunk_scan_kernel<4, false>, grid2, 128, 0, stream, state, slot_ids, seq_start, scratch, (const float*)chunk_decay,
                               max_chunks, H, elems));
   } else {
     dim3 grid2(n_seqs * H, (elems + 127) / 128);
-    RL_LAUNCH_CHECK(rl_launch(scalar_chunk_scan_kernel<1>, grid2, 128, 0, stream, state, slot_ids, seq_start, scratch, (const float*)chunk_decay,
+    RL_LAUNCH_CHECK(rl_launch(scalar_chunk_scan_kernel<1, false>, grid2, 128, 0, stream, state, slot_ids, seq_start, scratch, (const float*)chunk_decay,
                               max_chunks, H, elems));
   }
-  RL_LAUNCH_CHECK(rl_launch(scalar_chunk_out_kernel<HDK, HDV>, grid, 128, smem3, stream, q, k, v, in_stride, log_decay, in_scale, seq_start,
+  RL_LAUNCH_CHECK(rl_launch(out3, grid, 128, smem3, stream, q, k, v, in_stride, log_decay, in_scale, seq_start,
                             (const float*)scratch, max_chunks, out, out_stride, H, QH, dim, vdim));
   return 0;
 }
