@@ -37,6 +37,39 @@ __global__ void embed_gather_kernel(const int* __restrict__ tokens, const TW* __
   }
 }
 
+// The same for the many rows of a prompt step: a thread takes up to PIECES pieces of eight numbers, all asked for before the first is stored, so
+// that an SM has twice the bytes on their way (2048 rows of 4096: 13 us instead of 15, of 2048: 7.0 instead of 8.4; memory's work is 8 and 4).
+#define EMBED_ROWS_MIN 64
+#define EMBED_THREADS 128
+template <int PIECES>
+__global__ void __launch_bounds__(EMBED_THREADS)
+embed_gather_rows_kernel(const int* __restrict__ tokens, const bf16* __restrict__ table, float* __restrict__ out, int d, float scale) {
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const bf16* row = table + (size_t)__ldcg(tokens + t) * d;
+  float* o = out + (size_t)t * d;
+  for (int i0 = threadIdx.x * 8; i0 < d; i0 += PIECES * EMBED_THREADS * 8) {
+    uint4 raw[PIECES];
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      const int i = i0 + p * EMBED_THREADS * 8;
+      if (i < d) raw[p] = __ldcg(reinterpret_cast<const uint4*>(row + i));
+    }
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      const int i = i0 + p * EMBED_THREADS * 8;
+      if (i >= d) break;
+      float f[8];
+      bf16x8_to_f32(raw[p], f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] *= scale;
+      store4<float>(o + i, f);
+      store4<float>(o + i + 4, f + 4);
+    }
+  }
+}
+
 static int row_threads(int d) {
   int t = ((d / 4 + 31) / 32) * 32;
   return t < 32 ? 32 : (t > 1024 ? 1024 : t);
@@ -46,7 +79,9 @@ RL_API int rl_embed_gather(const int* tokens, const void* table, int table_dtype
                            int d, float scale, cudaStream_t stream) {
   if (n_tokens <= 0 || d <= 0) RL_REFUSE(1, "embed_gather: n_tokens=%d d=%d", n_tokens, d);
   const int th = row_threads(d);
-  if (table_dtype == RL_BF16 && d % 4 == 0)
+  if (table_dtype == RL_BF16 && d % 8 == 0 && n_tokens >= EMBED_ROWS_MIN && (((uintptr_t)table | (uintptr_t)out) & 15) == 0)
+    RL_LAUNCH_CHECK(rl_launch(embed_gather_rows_kernel<4>, n_tokens, EMBED_THREADS, 0, stream, tokens, (const bf16*)table, out, d, scale));
+  else if (table_dtype == RL_BF16 && d % 4 == 0)
     RL_LAUNCH_CHECK(rl_launch(embed_gather_kernel<bf16, true>, n_tokens, th, 0, stream, tokens, (const bf16*)table, out, d, scale));
   else if (table_dtype == RL_BF16)
     RL_LAUNCH_CHECK(rl_launch<false>(embed_gather_kernel<bf16, false>, n_tokens, 256, 0, stream, tokens, (const bf16*)table, out, d, scale));
@@ -278,6 +313,7 @@ template <typename TA, typename TW, typename TD>
 static int launch_add_rmsnorm(float* x, const void* delta, int n_parts, long long part_stride, const void* w,
                               void* out, const int* rows, int n_rows, int d, float eps, int write_x,
                               cudaStream_t stream) {
+  if (n_parts == 0) write_x = 0;  // (the stream is what it was: a third of the pass's bytes for the norm that opens a model)
   const bool vec = d % 4 == 0;
   if (vec && !std::is_same<TA, float>::value && n_rows >= ROWS_KERNEL_MIN_ROWS && d <= 256 * 4 * ROWS_KERNEL_CHUNKS) {
     RL_LAUNCH_CHECK(rl_launch(add_rmsnorm_rows_kernel<TA, TW, TD, ROWS_KERNEL_CHUNKS>, n_rows, 256, 0, stream, x,
