@@ -63,7 +63,7 @@
 // probabilities go into P V as the sum of two bfloat16 numbers, the second ones in the half of the S buffer that the first leave free: rounded
 // once, under a maximum that is only raised by factors of 2^8, they put the result 5 to 10 % further from 64 bits than the kernel on the latents
 // (whose row maximum is exact, so that a row's largest probability is 1), in two parts 1 to 6 % nearer.  16 heads, 2048 tokens: 63 us with one
-// part (340 TFLOP/s), 75 with two; the same layer on its latents with mma.sync 468 us.
+// part, 75 with two (before the way out was shortened, which took 65 to 59); the same layer on its latents with mma.sync 468 us.
 //
 // Every mbarrier wait is bounded; on expiry a code goes to status[0] and the block drains.
 #include "tc_common.cuh"
@@ -639,6 +639,21 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[j & 1]);
     }
+    const int rows_valid = rows_here - warp * 32;  // (may be <= 0: nothing is written then)
+    // The gate's numbers come as whole lines too, eight lanes to a row of 64, the first of them under the wait for the last product: read by the
+    // threads that own the rows, 16 bytes of 32 lines at a time, and divided with a branch in each (common.cuh), they held a block up for 13 us
+    // after its last tile instead of 7.
+    uint4 gates[EXPANDED ? 8 : 1];
+    const bf16* gate_rows = nullptr;
+    if (EXPANDED && gate != nullptr) gate_rows = gate + (size_t)(tok0 + row0 + warp * 32) * gate_stride + (size_t)h * vdim;
+    auto load_gates = [&](int c) {
+#pragma unroll
+      for (int it = 0; it < (EXPANDED ? 8 : 0); ++it) {
+        const int rr = it * 4 + (lane >> 3), at = c * 64 + (lane & 7) * 8;
+        gates[it] = rr < rows_valid && at < vdim ? __ldcg(reinterpret_cast<const uint4*>(gate_rows + (size_t)rr * gate_stride + at)) : make_uint4(0, 0, 0, 0);
+      }
+    };
+    if (EXPANDED && gate_rows != nullptr && ok) load_gates(0);
     if (ok && !mbar_wait_role(&pv_done[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, ctl, 20)) give_up(20);
     ok = __all_sync(0xffffffffu, ok);  // (the way out below works as a warp)
     if (ok) {
@@ -647,7 +662,6 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       // This thread holds a row of the output; the warp turns 64 dims of its 32 rows at a time through the
       // queries' buffer, which no product reads any more, and writes whole 128-byte rows (see tc_common.cuh).
       const uint32_t stage = smem_u32(q_s) + (uint32_t)(warp * ROW_STAGE_BYTES);
-      const int rows_valid = rows_here - warp * 32;  // (may be <= 0: nothing is written then)
       bf16* o = out + (size_t)(tok0 + row0 + warp * 32) * out_stride + (size_t)h * vdim;
 #pragma unroll 1
       for (int c = 0; c < VD / 64; ++c) {
@@ -655,24 +669,33 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         tmem_ld_32x32b_x32(o_addr + c * 64, v0);
         tmem_ld_32x32b_x32(o_addr + c * 64 + 32, v1);
         tmem_ld_wait();
+        if (EXPANDED && gate_rows != nullptr) {  // every number times the logistic function of its gate's, which turn through the same memory
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          v0[i] = __float_as_uint(__uint_as_float(v0[i]) * inv);
-          v1[i] = __float_as_uint(__uint_as_float(v1[i]) * inv);
-        }
-        if (EXPANDED && gate != nullptr && r < rows_here) {  // every number times the logistic function of its gate's
-          const bf16* g = gate + (size_t)(tok0 + row0 + r) * gate_stride + (size_t)h * vdim + c * 64;
-          const int cols = min(64, vdim - c * 64);  // (a multiple of 8)
+          for (int it = 0; it < (EXPANDED ? 8 : 0); ++it) {
+            const int rr = it * 4 + (lane >> 3);
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(stage + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4)), "r"(gates[it].x),
+                         "r"(gates[it].y), "r"(gates[it].z), "r"(gates[it].w) : "memory");
+          }
+          __syncwarp();
+          if ((c + 1) * 64 < vdim) load_gates(c + 1);
 #pragma unroll
           for (int i = 0; i < 64; i += 8) {
-            if (i >= cols) break;
+            uint4 g;
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(g.x), "=r"(g.y), "=r"(g.z), "=r"(g.w) : "r"(stage + lane * 128 + (((i >> 3) ^ (lane & 7)) << 4)) : "memory");
             float f[8];
-            bf16x8_to_f32(__ldcg(reinterpret_cast<const uint4*>(g + i)), f);
+            bf16x8_to_f32(g, f);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               uint32_t& x = i < 32 ? v0[(i + e) & 31] : v1[(i + e) & 31];
-              x = __float_as_uint(__uint_as_float(x) / (1.0f + expf(-f[e])));
+              x = __float_as_uint(__uint_as_float(x) * divide_by_1up(inv, 1.0f + expf(-f[e])));
             }
+          }
+          __syncwarp();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            v0[i] = __float_as_uint(__uint_as_float(v0[i]) * inv);
+            v1[i] = __float_as_uint(__uint_as_float(v1[i]) * inv);
           }
         }
         store_rows64_bf16(o + c * 64, out_stride, rows_valid, v0, v1, stage, lane, vdim - c * 64);

@@ -26,7 +26,7 @@ RL_DEFINE_ERROR_TEXT()
 // ---------------------------------------------------------------- short convolution
 #define CONV_MAX_TAPS 16
 
-__device__ __forceinline__ float dr_silu(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float dr_silu(float z) { return divide_by_1up(z, 1.0f + expf(-z)); }
 
 // One thread per (token, channel).  x: [T, >= C] rows; w: [taps][C] (tap i of every channel side by side, the last row the
 // current token's); state: [slots][taps - 1][C], entry j the input at (first position of the step) - (taps - 1) + j.

@@ -30,7 +30,7 @@ RL_DEFINE_ERROR_TEXT()
 template <typename T>
 __device__ __forceinline__ float gr_load(const T* p) { return to_f32(__ldcg(p)); }
 
-__device__ __forceinline__ float gr_logistic(float x) { return 1.0f / (1.0f + expf(-x)); }
+__device__ __forceinline__ float gr_logistic(float x) { return logistic_no_branch(x); }
 __device__ __forceinline__ float gr_log_logistic(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
 // Four neighbouring numbers of a row, `left` of them there (the others are zero); `wide`: the row's start and its length allow one load.

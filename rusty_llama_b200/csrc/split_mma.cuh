@@ -158,7 +158,7 @@ struct SplNorm {
   int gate_stride, act;  // 0 the gate itself, 1 the logistic function of it, 2 silu
   float scale;
 };
-__device__ __forceinline__ float spl_logistic(float x) { return 1.0f / (1.0f + expf(-x)); }
+__device__ __forceinline__ float spl_logistic(float x) { return logistic_no_branch(x); }
 __device__ __forceinline__ void spl_finish(const float (&acc)[2][2][2][1][4], float* ss, int n, int t0, int h, int vdim, int col0, void* out, int out_stride,
                                            const SplNorm& norm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;

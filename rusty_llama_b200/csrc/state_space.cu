@@ -79,7 +79,7 @@ ssm_gate_norm_kernel(const float* __restrict__ y, int y_stride, const T* __restr
     float ss = 0.f;
 #pragma unroll
     for (int e = 0; e < U; ++e) {
-      v[c][e] = (yv[e] + d * xv[e]) * (zv[e] / (1.0f + expf(-zv[e])));
+      v[c][e] = (yv[e] + d * xv[e]) * divide_by_1up(zv[e], 1.0f + expf(-zv[e]));
       ss += v[c][e] * v[c][e];
     }
     unit_ss[u] = ss;
