@@ -119,9 +119,9 @@ __device__ __forceinline__ float gated_act(float g, float u, float alpha, float 
   if (limit > 0.f) {
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit) + 1.0f;
-    return g * (1.0f / (1.0f + expf(-alpha * g))) * u;
+    return g * logistic_no_branch(alpha * g) * u;
   }
-  return g * (1.0f / (1.0f + expf(-g))) * u;
+  return g * logistic_no_branch(g) * u;
 }
 // the same with the hardware's approximations of exp and of the division (a few units in the last place of 32 bits)
 __device__ __forceinline__ float gated_act_fast(float g, float u, float alpha, float limit) {
