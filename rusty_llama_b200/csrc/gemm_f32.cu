@@ -15,7 +15,7 @@
 // tile kernel: 32 of them for the 2048 features of an output projection).  A chunk
 // per thread gives K / 128 times the threads and chains of 128.
 //
-//   gemv_f32_kernel  up to GEMV_ROWS rows: bound by reading the weights.  One row of 11264 x 2048: 17.4 us, 5.3 TB/s; 2048 x 5632: 12 us, 3.9 TB/s.
+//   gemv_f32_kernel  up to GEMV_ROWS rows: bound by reading the weights.  One row of 11264 x 2048: 18.6 us, 5.0 TB/s; 2048 x 5632: 11.9 us, 3.9 TB/s.
 //   gemm_f32_kernel  more rows, and operands that cannot be moved 16 bytes at a time: bound by the FMA pipe.  283 rows of
 //                    11264 x 2048: 344 us, 38 TFLOP/s; of 2048 x 2048, where the tiles are few: 84 us, 28 TFLOP/s.
 // Prompts of 219 and 64 tokens and twelve decode steps of both on three layers of d 2048 and ff 5632: 60.9 ms in one kernel that
@@ -97,14 +97,12 @@ gemm_fma_kernel(const TA* __restrict__ x, int ldx, const TA* __restrict__ w, int
 
 // ------------------------------------------------------------------ 32-bit, few rows
 #define KCHUNK 128        // the summation order's chunk of k: part of the result, not a tuning knob
-#define GEMV_ROWS 8       // rows up to which the weights are streamed (measured, gate/up of 11264 x 2048: 8 rows 65 us, 16 rows 109 us; 17 rows in tiles 71 us)
+#define GEMV_ROWS 8       // rows up to which the weights are streamed (measured, gate/up of 11264 x 2048: 8 rows 43 us; 17 rows in tiles 71 us)
 #define GEMV_THREADS 128  // one (feature, chunk) pair each
-#define GEMV_STAGES 3
-#define GEMV_SUB 32       // k of a chunk that a stage of the ring holds
-#define GEMV_ITEM (GEMV_SUB + 4)      // floats per item in a stage: 144 bytes, so that eight lanes' 16-byte reads meet all banks
-#define GEMV_XCHUNK (KCHUNK + 4)      // the same for the rows of x, per chunk
-#define GEMV_MAX_ITEMS 512            // items of a block, whose sums wait in shared memory
-#define GEMV_RING_BYTES (GEMV_STAGES * GEMV_THREADS * GEMV_ITEM * 4)
+#define GEMV_SUB 32       // k of a chunk that a stage of the ring holds: 128 bytes of an item, whose 16-byte pieces lie swizzled by the item
+#define GEMV_XCHUNK (KCHUNK + 4)      // the rows of x, per chunk: eight chunks' same places meet all banks
+#define GEMV_MAX_ITEMS 2048           // items of a block, whose sums wait in shared memory
+#define GEMV_STAGE_BYTES (GEMV_THREADS * GEMV_SUB * 4)
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
@@ -113,17 +111,22 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 // MB rows of x (blockIdx.y names which) against R features a block.  A thread owns a (feature, chunk) pair at a time and walks
 // its 128 k's; 128 such pairs go through the ring side by side, 32 k's a stage, copied so that eight lanes take a 128-byte line.
 // The ring's first stages are asked for before the kernel before this one has ended: no kernel writes weights.
-// Bound: the weights' bytes.  Two blocks an SM keep 64 KB in flight; every block has R = ceil(N / (2 SMs)) features (a grid of
-// one wave) until their sums take more shared memory than that leaves.
-template <int MB>
+// Bound: the weights' bytes.  Two blocks an SM keep 96 KB in flight.  A warp's pairs are of neighbouring features, so that its
+// lanes read few places of x and not 32, and a whole stage's reads run ahead of its sums.  Before (pairs of neighbouring chunks, a
+// question before every four k's, three stages padded to 144 bytes a pair, x by way of registers), in us, before / now:
+//   rows    2560 x 2048    2048 x 2048    11264 x 2048    2048 x 5632    32000 x 2048    2048 x 14336
+//      1      8.0 / 5.6      5.5 / 5.6     19.1 / 18.6    12.9 / 11.9     51.6 / 45.8     62.5 / 26.6
+//      2     10.4 / 6.0      7.2 / 5.7     22.9 / 17.9    16.6 / 12.5     60.8 / 46.6      124 / 46.7
+//      8     21.2 / 15.0    14.8 / 13.5    67.9 / 42.9    64.2 / 41.5      151 / 102       452 / 165
+template <int MB, int STAGES>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, int ldw, float* __restrict__ out, int ldo,
                 int M, int N, int K, int R) {
   extern __shared__ __align__(16) float sm[];
   const int nch = (K + KCHUNK - 1) / KCHUNK;
   float* ring = sm;
-  float* xs = ring + GEMV_STAGES * GEMV_THREADS * GEMV_ITEM;  // [MB][nch][GEMV_XCHUNK]
-  float* part = xs + MB * nch * GEMV_XCHUNK;                  // [MB][R * nch]
+  float* xs = ring + STAGES * GEMV_THREADS * GEMV_SUB;  // [MB][nch][GEMV_XCHUNK]
+  float* part = xs + MB * nch * GEMV_XCHUNK;                 // [MB][nch * rows]
   const int tid = threadIdx.x;
   const int n0 = blockIdx.x * R, rows = min(R, N - n0);
   const int m0 = blockIdx.y * MB, mb = min(MB, M - m0);
@@ -132,67 +135,72 @@ gemv_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
   pdl_trigger();
 
   // eight 16-byte pieces a thread and stage: piece tid % 8 of items tid / 8 + 16 j
-  const int piece = (tid & 7) * 4;
+  const int piece = (tid & 7) * 4, swizzled = ((tid & 7) ^ (tid / 8 & 7)) * 4;
   const float* src[8];
   int k_at[8];
   auto load = [&](int step) {
     const int sub = step % (KCHUNK / GEMV_SUB);
-    float* dst = ring + (size_t)(step % GEMV_STAGES) * GEMV_THREADS * GEMV_ITEM;
+    float* dst = ring + (size_t)(step % STAGES) * GEMV_THREADS * GEMV_SUB;
     if (sub == 0) {
       const int base = step / (KCHUNK / GEMV_SUB) * GEMV_THREADS + tid / 8;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int item = base + 16 * j;
-        const int r = item / nch, c = item - r * nch;
+        const int c = item / rows, r = item - c * rows;
         k_at[j] = item < items ? c * KCHUNK + piece : K;
-        src[j] = w + (size_t)(n0 + min(r, rows - 1)) * ldw + c * KCHUNK + piece;
+        src[j] = w + (size_t)(n0 + r) * ldw + c * KCHUNK + piece;
       }
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (k_at[j] + sub * GEMV_SUB < K) cp_async16(dst + (tid / 8 + 16 * j) * GEMV_ITEM + piece, src[j] + sub * GEMV_SUB);
+      if (k_at[j] + sub * GEMV_SUB < K) cp_async16(dst + (tid / 8 + 16 * j) * GEMV_SUB + swizzled, src[j] + sub * GEMV_SUB);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int i = 0; i < GEMV_STAGES - 1; ++i) {
+  for (int i = 0; i < STAGES - 1; ++i) {
     if (i < steps) load(i);
     else asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();
-  for (int i = tid; i < MB * (K / 4); i += GEMV_THREADS) {
-    const int m = i / (K / 4), k = (i - m * (K / 4)) * 4;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (m < mb) load4_g(x + (size_t)(m0 + m) * ldx + k, v);
-    store4(xs + (m * nch + k / KCHUNK) * GEMV_XCHUNK + k % KCHUNK, v);
-  }
+#pragma unroll
+  for (int m = 0; m < MB; ++m)
+    for (int k = tid * 4; k < K; k += GEMV_THREADS * 4) {
+      float* at = xs + (m * nch + k / KCHUNK) * GEMV_XCHUNK + k % KCHUNK;
+      if (m < mb) cp_async16(at, x + (size_t)(m0 + m) * ldx + k);
+      else *reinterpret_cast<float4*>(at) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");  // (the ring's first stages too: they were asked for long before)
 
   float acc[MB];
 #pragma unroll
   for (int m = 0; m < MB; ++m) acc[m] = 0.f;
   for (int step = 0; step < steps; ++step) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(GEMV_STAGES - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();  // everyone's pieces of this stage (and, first, x) are there, and the stage before it is free
-    if (step + GEMV_STAGES - 1 < steps) load(step + GEMV_STAGES - 1);
+    if (step + STAGES - 1 < steps) load(step + STAGES - 1);
     else asm volatile("cp.async.commit_group;" ::: "memory");
     const int sub = step % (KCHUNK / GEMV_SUB);
     const int item = step / (KCHUNK / GEMV_SUB) * GEMV_THREADS + tid;
-    const int c = item % nch;
-    const float* wr = ring + (size_t)(step % GEMV_STAGES) * GEMV_THREADS * GEMV_ITEM + tid * GEMV_ITEM;
+    const int c = min(item, items - 1) / rows;
+    const float* wr = ring + (size_t)(step % STAGES) * GEMV_THREADS * GEMV_SUB + tid * GEMV_SUB;
     const float* xr = xs + c * GEMV_XCHUNK + sub * GEMV_SUB;
     const int left = item < items ? (K - c * KCHUNK - sub * GEMV_SUB) : 0;  // k's of this stage that exist (a multiple of 4)
+    auto four = [&](int i, const float4& a) {
 #pragma unroll
-    for (int i = 0; i < GEMV_SUB; i += 4) {
-      if (i < left) {
-        const float4 a = *reinterpret_cast<const float4*>(wr + i);
-#pragma unroll
-        for (int m = 0; m < MB; ++m) {
-          const float4 b = *reinterpret_cast<const float4*>(xr + m * nch * GEMV_XCHUNK + i);
-          acc[m] = fmaf(b.x, a.x, acc[m]);
-          acc[m] = fmaf(b.y, a.y, acc[m]);
-          acc[m] = fmaf(b.z, a.z, acc[m]);
-          acc[m] = fmaf(b.w, a.w, acc[m]);
-        }
+      for (int m = 0; m < MB; ++m) {
+        const float4 b = *reinterpret_cast<const float4*>(xr + m * nch * GEMV_XCHUNK + i);
+        acc[m] = fmaf(b.x, a.x, acc[m]);
+        acc[m] = fmaf(b.y, a.y, acc[m]);
+        acc[m] = fmaf(b.z, a.z, acc[m]);
+        acc[m] = fmaf(b.w, a.w, acc[m]);
       }
+    };
+    if (left >= GEMV_SUB) {  // (without a question in between, so that the reads run ahead of the sums)
+#pragma unroll
+      for (int i = 0; i < GEMV_SUB; i += 4) four(i, *reinterpret_cast<const float4*>(wr + (i ^ (tid & 7) * 4)));
+    } else {
+      for (int i = 0; i < left; i += 4) four(i, *reinterpret_cast<const float4*>(wr + (i ^ (tid & 7) * 4)));
     }
     if (sub == KCHUNK / GEMV_SUB - 1) {
 #pragma unroll
@@ -206,7 +214,8 @@ gemv_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
   for (int i = tid; i < rows * mb; i += GEMV_THREADS) {
     const int m = i / rows, r = i - m * rows;
     float total = 0.f;
-    for (int c = 0; c < nch; ++c) total += part[m * most + r * nch + c];
+#pragma unroll 8
+    for (int c = 0; c < nch; ++c) total += part[m * most + c * rows + r];
     out[(size_t)(m0 + m) * ldo + n0 + r] = total;
   }
 }
@@ -308,13 +317,14 @@ gemm_f32_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ 
   }
 }
 
-template <int MB>
+template <int MB, int STAGES>
 static int launch_gemv_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K, int R,
                            size_t smem, cudaStream_t stream) {
-  if (cudaFuncSetAttribute(gemv_f32_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  auto kern = gemv_f32_kernel<MB, STAGES>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     RL_REFUSE(4, "gemm_f32: cannot get %zu bytes of shared memory", smem);
   dim3 grid((N + R - 1) / R, (M + MB - 1) / MB);
-  RL_LAUNCH_CHECK(rl_launch(gemv_f32_kernel<MB>, grid, GEMV_THREADS, smem, stream, x, ldx, w, ldw, out, ldo, M, N, K, R));
+  RL_LAUNCH_CHECK(rl_launch(kern, grid, GEMV_THREADS, smem, stream, x, ldx, w, ldw, out, ldo, M, N, K, R));
   return 0;
 }
 
@@ -332,7 +342,9 @@ static int launch_gemm_f32(const float* x, int ldx, const float* w, int ldw, flo
   RL_LAUNCH_RESULT();
 }
 
-static size_t gemv_f32_smem(int mb, int nch, int R) { return GEMV_RING_BYTES + (size_t)mb * nch * (GEMV_XCHUNK + R) * sizeof(float); }
+static size_t gemv_f32_smem(int stages, int mb, int nch, int R) {
+  return (size_t)stages * GEMV_STAGE_BYTES + (size_t)mb * nch * (GEMV_XCHUNK + R) * sizeof(float);
+}
 
 RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K, int sms,
                        cudaStream_t stream) {
@@ -341,16 +353,30 @@ RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* 
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
   const int nch = (K + KCHUNK - 1) / KCHUNK;
   if (M <= GEMV_ROWS && vec && nch <= GEMV_MAX_ITEMS) {
-    int R = (N + 2 * sms - 1) / (2 * sms);
-    if (R > GEMV_MAX_ITEMS / nch) R = GEMV_MAX_ITEMS / nch;
-    // as many rows of x a block as there are, up to four, while two blocks fit an SM; else one row (up to 327 chunks: K of 41856)
+    // features a block: as many as make one wave of two blocks an SM, or of three where that is less to walk through (2560 x 2048 with 2 rows: 9
+    // features of 16 chunks are 144 pairs, two passes of 128; 6 are one: 7.9 and 6.0 us) and three fit
+    auto features = [&](int per_sm) {
+      const int R = (N + per_sm * sms - 1) / (per_sm * sms);
+      return R < GEMV_MAX_ITEMS / nch ? R : GEMV_MAX_ITEMS / nch;
+    };
+    auto passes = [&](int R) { return (R * nch + GEMV_THREADS - 1) / GEMV_THREADS; };
+    const int R2 = features(2), R3 = features(3);
+    // as many rows of x a block as there are, up to four, while two blocks fit an SM; else one row (up to 338 chunks: K of 43264)
+    const size_t half = 112 * 1024, third = 74 * 1024;
     int mb = M == 1 ? 1 : M == 2 ? 2 : 4;
-    while (mb > 1 && gemv_f32_smem(mb, nch, R) > 112 * 1024) mb /= 2;
-    const size_t smem = gemv_f32_smem(mb, nch, R);
+    while (mb > 1 && gemv_f32_smem(3, mb, nch, R2) > half) mb /= 2;
+    const bool three = 3 * passes(R3) < 2 * passes(R2) && gemv_f32_smem(3, mb, nch, R3) <= third;
+    const int R = three ? R3 : R2, stages = three || gemv_f32_smem(4, mb, nch, R) > half ? 3 : 4;
+    const size_t smem = gemv_f32_smem(stages, mb, nch, R);
     if (smem <= 224 * 1024) {
-      if (mb == 1) return launch_gemv_f32<1>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
-      if (mb == 2) return launch_gemv_f32<2>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
-      return launch_gemv_f32<4>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream);
+#define RL_GEMV(MB, STAGES) return launch_gemv_f32<MB, STAGES>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream)
+      if (mb == 1 && stages == 4) RL_GEMV(1, 4);
+      if (mb == 1) RL_GEMV(1, 3);
+      if (mb == 2 && stages == 4) RL_GEMV(2, 4);
+      if (mb == 2) RL_GEMV(2, 3);
+      if (stages == 4) RL_GEMV(4, 4);
+      RL_GEMV(4, 3);
+#undef RL_GEMV
     }
   }
   // the tile with the least work on the busiest SM: its blocks there, times the tile's outputs, times what an output costs with

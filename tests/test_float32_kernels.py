@@ -55,6 +55,16 @@ def test_product_of_a_very_long_k(ops):
             assert torch.equal(ops.gemm_f32(xd[:rows], wd), many[:rows])
 
 
+@pytest.mark.parametrize("N, K", [(2560, 2048), (2553, 1924), (11264, 2048), (40001, 2048), (2048, 5632), (2047, 14336)])
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8])
+def test_few_rows_of_large_matrices(ops, M, N, K):
+    """Three blocks an SM and two, one pass and many, the most sums a block holds, the last block's fewer features: the same bits as among
+    many rows."""
+    g = torch.Generator(device=DEV).manual_seed(M * 7919 + N + K)
+    x, w = torch.randn(40, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    assert torch.equal(ops.gemm_f32(x[:M], w), ops.gemm_f32(x, w)[:M])
+
+
 @pytest.mark.parametrize("window", [0, 70])
 @pytest.mark.parametrize("H, K, hd", [(8, 1, 64), (6, 2, 40), (16, 2, 128), (5, 5, 30), (6, 1, 256), (12, 4, 18)])
 def test_attention_of_few_and_of_many_tokens(ops, H, K, hd, window):
