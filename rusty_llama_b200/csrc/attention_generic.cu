@@ -14,8 +14,9 @@
 // read once serves HB heads.  Bounds: a prompt, the rows' way from L2 (hence several
 // heads a block); a decode step, the chain of one warp's groups (hence WARPS warps, and
 // fewer heads a block until every SM has two).  32 heads of 64 on 4: prompts of 219 and
-// 64 tokens 66 us a layer, a decode step of both 13 us (one warp per token and head, which
-// read a key number by number: 166 us on average over both).
+// 64 tokens 66 us a layer, a decode step of both 8.4 us and 16 from HBM (9.6 and 18 before a head
+// alone read ahead; one warp per token and head, which read a key number by number: 166 us on
+// average over prompts and decode steps).
 //
 // Cache layout of one layer: pages[page][kv_head][slot_in_page][hd]; the page of
 // position p of batch sequence s is block_table[s][p / page_size].
@@ -25,13 +26,16 @@ RL_DEFINE_ERROR_TEXT()
 
 #define WARPS 8  // part of the summation order
 
-// DPL: value dimensions per lane (head sizes up to 32 DPL); HB: query heads per block; by4: the keys' rows can be read four numbers at a time
-template <typename T, int DPL, int HB>
+// DPL: value dimensions per lane (head sizes up to 32 DPL); HB: query heads per block; by4: the keys' rows can be read four numbers at a time;
+// ALONE: see rl_attn_generic
+template <typename T, int DPL, int HB, bool ALONE>
 __global__ void __launch_bounds__(WARPS * 32)
 attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_pages,
                     const T* __restrict__ v_pages, const int* __restrict__ block_table, int table_width,
                     const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, T* __restrict__ out, int out_stride,
                     int H, int K, int hd, int page_size, int window, float scale, bool by4) {
+  static_assert(!ALONE || HB == 1, "a head alone");
+  constexpr int AHEAD = 32 / DPL;  // rows of values that a lane asks for at a time
   extern __shared__ __align__(16) float sm[];
   const int hd4 = (hd + 3) & ~3;
   float* q_s = sm;                              // [HB][hd4]
@@ -69,9 +73,26 @@ attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__
     float s[HB];
 #pragma unroll
     for (int h = 0; h < HB; ++h) s[h] = 0.f;
+    const size_t row = valid ? (((size_t)table[key / page_size] * K + kh) * page_size + key % page_size) * hd : 0;
     if (valid) {
-      const T* kr = k_pages + (((size_t)table[key / page_size] * K + kh) * page_size + key % page_size) * hd;
-      if (by4) {
+      const T* kr = k_pages + row;
+      if (ALONE && by4) {  // sixteen pieces of the row on their way at a time
+        for (int i0 = 0; i0 < hd; i0 += 64) {
+          float kv[16][4];
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (i0 + 4 * j < hd) load4(kr + i0 + 4 * j, kv[j]);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (i0 + 4 * j >= hd) break;
+            const float4 qv = *reinterpret_cast<const float4*>(q_s + i0 + 4 * j);
+            s[0] = fmaf(qv.x, kv[j][0], s[0]);
+            s[0] = fmaf(qv.y, kv[j][1], s[0]);
+            s[0] = fmaf(qv.z, kv[j][2], s[0]);
+            s[0] = fmaf(qv.w, kv[j][3], s[0]);
+          }
+        }
+      } else if (by4) {
 #pragma unroll 4
         for (int i = 0; i < hd; i += 4) {
           float kv[4];
@@ -93,6 +114,21 @@ attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__
         }
       }
     }
+    // a head alone: the values' rows do not wait for the probabilities, nor a row's place for the table (the lane that has its key knows it)
+    const int count = min(32, pos - base + 1);
+    float ahead[ALONE ? AHEAD : 1][DPL];
+    auto ask = [&](int j0) {
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j) {
+        const T* vr = v_pages + __shfl_sync(0xffffffffu, (unsigned long long)row, j0 + j);
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) {
+          const int dim = lane + 32 * i;
+          ahead[ALONE ? j : 0][i] = (dim < hd && j0 + j < count) ? to_f32(vr[dim]) : 0.f;
+        }
+      }
+    };
+    if constexpr (ALONE) ask(0);
 #pragma unroll
     for (int h = 0; h < HB; ++h) {
       const float v = valid ? __fmul_rn(s[h], scale) : -INFINITY;  // (rounded here in every form of this kernel, not inside a later sum)
@@ -106,7 +142,25 @@ attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__
       for (int i = 0; i < DPL; ++i) acc[h][i] *= alpha;
     }
     __syncwarp();
-    const int count = min(32, pos - base + 1);
+    if constexpr (ALONE) {
+      for (int j0 = 0; j0 < count; j0 += AHEAD) {
+        if (j0) ask(j0);
+#pragma unroll
+        for (int j = 0; j < AHEAD; j += 4) {
+          if (j0 + j >= count) break;
+          const float4 p = *reinterpret_cast<const float4*>(ps + j0 + j);
+#pragma unroll
+          for (int i = 0; i < DPL; ++i) {
+            acc[0][i] = fmaf(p.x, ahead[ALONE ? j : 0][i], acc[0][i]);
+            acc[0][i] = fmaf(p.y, ahead[ALONE ? j + 1 : 0][i], acc[0][i]);
+            acc[0][i] = fmaf(p.z, ahead[ALONE ? j + 2 : 0][i], acc[0][i]);
+            acc[0][i] = fmaf(p.w, ahead[ALONE ? j + 3 : 0][i], acc[0][i]);
+          }
+        }
+      }
+      __syncwarp();
+      continue;
+    }
 #pragma unroll 2
     for (int j0 = 0; j0 < count; j0 += 4) {
       float v[4][DPL];
@@ -163,14 +217,14 @@ attn_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__
   }
 }
 
-template <typename T, int DPL, int HB>
+template <typename T, int DPL, int HB, bool ALONE = false>
 static int launch_attn_generic(const void* q, int q_stride, const void* k_pages, const void* v_pages, const int* block_table,
                                int table_width, const int* tok_seq, const int* tok_pos, void* out, int out_stride, int n_tokens,
                                int H, int K, int hd, int page_size, int window, float scale, cudaStream_t stream) {
   const int G = H / K, gy = K * ((G + HB - 1) / HB);
   if (gy > 65535) RL_REFUSE(4, "attn_generic: %d heads exceed the grid", H);
   const size_t smem = (size_t)(HB * ((hd + 3) & ~3) + WARPS * HB * (32 + hd + 2)) * sizeof(float);
-  auto kern = attn_generic_kernel<T, DPL, HB>;
+  auto kern = attn_generic_kernel<T, DPL, HB, ALONE>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     RL_REFUSE(7, "attn_generic: cannot get %zu bytes of shared memory", smem);
   const bool by4 = hd % 4 == 0 && (uintptr_t)k_pages % (4 * sizeof(T)) == 0;
@@ -195,6 +249,14 @@ RL_API int rl_attn_generic(const void* q, int dtype, int q_stride, const void* k
   const int dpl = hd <= 64 ? 2 : hd <= 128 ? 4 : 8, G = H / K;
   int hb = 16 / dpl;
   while (hb > 1 && (hb / 2 >= G || (long long)n_tokens * K * ((G + hb - 1) / hb) < 2LL * sms)) hb /= 2;
+  // A head alone and no more blocks than the SMs hold at once (two each, at 128 registers a thread): all of a key's pieces and the values' rows are
+  // asked for ahead.  One token in 32 heads of 64 over 2000 keys 58 and 44 us, eight over 300 19.7 and 15.2; 384 blocks over 300 keys 24 and 26,
+  // 1600 94 and 126, where the registers cost more blocks at a time than the waits.  (Of larger heads none gained: 40 of 128 over 300 keys 19.5 both.)
+  if (dpl == 2 && hb == 1 && (long long)n_tokens * H <= 2LL * sms)
+    return dtype == RL_BF16 ? launch_attn_generic<bf16, 2, 1, true>(q, q_stride, k_pages, v_pages, block_table, table_width, tok_seq, tok_pos, out, out_stride,
+                                                                    n_tokens, H, K, hd, page_size, window, scale, stream)
+                            : launch_attn_generic<float, 2, 1, true>(q, q_stride, k_pages, v_pages, block_table, table_width, tok_seq, tok_pos, out, out_stride,
+                                                                     n_tokens, H, K, hd, page_size, window, scale, stream);
 #define RL_GENERIC(D, B)                                                                                                              \
   if (dpl == D && hb == B)                                                                                                            \
     return dtype == RL_BF16 ? launch_attn_generic<bf16, D, B>(q, q_stride, k_pages, v_pages, block_table, table_width, tok_seq, tok_pos, \

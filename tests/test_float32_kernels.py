@@ -111,3 +111,24 @@ def test_attention_over_pages_that_start_anywhere(ops, dtype):
         moved = buffer[off:].view(pages.shape)
         moved.copy_(pages)
         assert torch.equal(ops.attn_generic(q, moved, moved, table, seq, pos, H, K, hd), want)
+
+
+@pytest.mark.parametrize("hd, H, K", [(64, 4, 1), (60, 2, 2), (33, 3, 3), (4, 6, 2)])
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_head_alone_asks_ahead(ops, hd, H, K, window, dtype):
+    """Single tokens (reads ahead, no more blocks than the SMs hold) at the borders of the groups of 32 keys and of the warps' rounds: the same
+    bits as among 400 tokens (no reads ahead)."""
+    g = torch.Generator().manual_seed(hd + window)
+    n, page = 560, 64
+    pages = -(-n // page)
+    k, v = (torch.randn(pages, K, page, hd, generator=g).to(DEV, dtype) for _ in range(2))
+    table = torch.randperm(pages, generator=g).to(torch.int32).view(1, -1).to(DEV)
+    at = [0, 1, 30, 31, 32, 33, 63, 64, 255, 256, 257, 288, 511, 512, 559]
+    q = torch.randn(400, H * hd, generator=g).to(DEV, dtype)
+    pos = torch.tensor((at * 27)[:400], dtype=torch.int32, device=DEV)
+    run = lambda lo, hi: ops.attn_generic(  # noqa: E731
+        q[lo:hi], k, v, table, torch.zeros(hi - lo, dtype=torch.int32, device=DEV), pos[lo:hi], H, K, hd, window=window, scale=hd ** -0.5)
+    many = run(0, 400)
+    for i in range(len(at)):
+        assert torch.equal(run(i, i + 1)[0], many[i]), at[i]
