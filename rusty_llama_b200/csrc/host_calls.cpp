@@ -60,39 +60,43 @@ struct Launcher {
   vectorcallfunc call;
   Fn fn;
   int wide;  // returns long long
+  int n;     // arguments, or -1: nobody said, and each goes by its own type
+  char kinds[HC_INTS + HC_FLOATS];  // of each: 'p' a pointer, 'i' a whole number, 'f' a float
 };
 
 static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   const Launcher* l = reinterpret_cast<Launcher*>(self);
   const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
   if (kwnames && PyTuple_GET_SIZE(kwnames)) return PyErr_Format(PyExc_TypeError, "a launcher takes no keywords");
+  if (l->n >= 0 && n != l->n) return PyErr_Format(PyExc_TypeError, "this launcher takes %d arguments, not %zd", l->n, n);
   L i[HC_INTS] = {};
   float f[HC_FLOATS] = {};
   int ni = 0, nf = 0;
   HC_TRY
   for (Py_ssize_t k = 0; k < n; ++k) {
     PyObject* a = args[k];
-    if (PyFloat_Check(a)) {
+    const char kind = l->n >= 0 ? l->kinds[k] : PyFloat_Check(a) ? 'f' : a == Py_None || THPVariable_Check(a) ? 'p' : 'i';
+    if (kind == 'f') {
       if (nf == HC_FLOATS) return PyErr_Format(PyExc_TypeError, "a launcher takes %d floats at most", HC_FLOATS);
-      f[nf++] = (float)PyFloat_AS_DOUBLE(a);
+      const double x = PyFloat_AsDouble(a);
+      if (x == -1.0 && PyErr_Occurred()) return nullptr;
+      f[nf++] = (float)x;
       continue;
     }
     if (ni == HC_INTS) return PyErr_Format(PyExc_TypeError, "a launcher takes %d integers and tensors at most", HC_INTS);
-    if (a == Py_None) {
-      i[ni++] = 0;
-    } else if (PyLong_Check(a)) {
+    if (PyLong_Check(a)) {  // (a pointer's, too: an address)
       i[ni] = (L)PyLong_AsUnsignedLongLongMask(a);
       if (i[ni] == -1 && PyErr_Occurred()) return nullptr;
       ++ni;
-    } else if (THPVariable_Check(a)) {
-      i[ni++] = (L)(uintptr_t)THPVariable_Unpack(a).data_ptr();
-    } else if (PyIndex_Check(a)) {
-      PyObject* whole = PyNumber_Index(a);
+    } else if (kind == 'p') {
+      if (THPVariable_Check(a)) i[ni++] = (L)(uintptr_t)THPVariable_Unpack(a).data_ptr();
+      else if (a == Py_None) i[ni++] = 0;
+      else return PyErr_Format(PyExc_TypeError, "argument %zd of a launcher is a tensor, an address or None, not %s", k + 1, Py_TYPE(a)->tp_name);
+    } else {
+      PyObject* whole = PyNumber_Index(a);  // (refuses floats and None)
       if (!whole) return nullptr;
       i[ni++] = (L)PyLong_AsUnsignedLongLongMask(whole);
       Py_DECREF(whole);
-    } else {
-      return PyErr_Format(PyExc_TypeError, "a launcher takes tensors, numbers and None, not %s", Py_TYPE(a)->tp_name);
     }
   }
   L r;
@@ -107,16 +111,27 @@ static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nar
 
 static PyTypeObject launcher_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// launcher(address, returns long long) -> callable
+// launcher(address, returns long long, kinds=None) -> callable.  Kinds are what every call's arguments are checked against, in number and in
+// kind: without the check an argument of another kind moves all behind it to other places of their rows.
 static PyObject* make_launcher(PyObject*, PyObject* args) {
   unsigned long long address;
   int wide;
-  if (!PyArg_ParseTuple(args, "Kp", &address, &wide)) return nullptr;
+  const char* kinds = nullptr;
+  if (!PyArg_ParseTuple(args, "Kp|z", &address, &wide, &kinds)) return nullptr;
+  int floats = 0, n = 0;
+  for (; kinds && kinds[n]; ++n) {
+    if (kinds[n] == 'f') ++floats;
+    else if (kinds[n] != 'p' && kinds[n] != 'i') return PyErr_Format(PyExc_ValueError, "unknown kind of argument in '%s'", kinds);
+  }
+  if (floats > HC_FLOATS || n - floats > HC_INTS)
+    return PyErr_Format(PyExc_TypeError, "a launcher takes %d floats and %d integers and tensors at most", HC_FLOATS, HC_INTS);
   Launcher* l = PyObject_New(Launcher, &launcher_type);
   if (!l) return nullptr;
   l->call = launcher_call;
   l->fn = reinterpret_cast<Fn>((uintptr_t)address);
   l->wide = wide;
+  l->n = kinds ? n : -1;
+  for (int k = 0; k < n; ++k) l->kinds[k] = kinds[k];
   return reinterpret_cast<PyObject*>(l);
 }
 

@@ -8,7 +8,10 @@ used where that module cannot be built (no Python or PyTorch headers) and where 
 from __future__ import annotations
 
 import ctypes
-from typing import Dict
+import operator
+import os
+import re
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -17,22 +20,33 @@ from . import build
 
 
 class PythonLauncher:
-    """A launcher called with tensors, numbers and None as they are (a float is the launcher's float, anything else an integer or pointer)."""
+    """A launcher called with tensors, numbers and None as they are.  kinds: of every argument 'p' (a pointer: a tensor, an address or
+    None), 'i' (a whole number) or 'f' (a float); calls are checked against it.  Without kinds each argument goes by its own type."""
 
-    def __init__(self, address: int, wide: bool):
+    def __init__(self, address: int, wide: bool, kinds: Optional[str] = None):
         self.fn = ctypes.CFUNCTYPE(ctypes.c_longlong if wide else ctypes.c_int)(address)
+        self.kinds = kinds
 
     def __call__(self, *args):
+        kinds = self.kinds
+        if kinds is None:
+            kinds = ["f" if isinstance(a, float) else "p" if a is None or isinstance(a, torch.Tensor) else "i" for a in args]
+        elif len(kinds) != len(args):
+            raise TypeError(f"this launcher takes {len(kinds)} arguments, not {len(args)}")
         given = []
-        for a in args:
-            if isinstance(a, float):
+        for n, (kind, a) in enumerate(zip(kinds, args)):
+            if kind == "f":
                 given.append(ctypes.c_float(a))
-            elif a is None:
-                given.append(ctypes.c_void_p(0))
+            elif isinstance(a, int):
+                given.append(ctypes.c_longlong(a))
+            elif kind == "i":
+                given.append(ctypes.c_longlong(operator.index(a)))  # (refuses floats and None)
             elif isinstance(a, torch.Tensor):
                 given.append(ctypes.c_void_p(a.data_ptr()))
+            elif a is None:
+                given.append(ctypes.c_void_p(0))
             else:
-                given.append(ctypes.c_longlong(a))
+                raise TypeError(f"argument {n + 1} of a launcher is a tensor, an address or None, not {type(a).__name__}")
         return self.fn(*given)
 
 
@@ -92,16 +106,41 @@ else:
     empty, columns, launcher = python_empty, python_columns, PythonLauncher
 
 
+_RETURNS = {"int": False, "long long": True}
+
+
+def launcher_kinds(source: str) -> Dict[str, Tuple[bool, str]]:
+    """The launchers that a source exports: whether each returns 64 bits, and the kinds of its arguments as `PythonLauncher` takes them."""
+    found = {}
+    for returns, name, declared in re.findall(r"^RL_API\s+([\w ]+?)\s+(rl_\w+)\(([^)]*)\)", source, re.M):
+        kinds = ""
+        for argument in filter(None, (a.strip() for a in declared.split(","))):
+            kind = " ".join(w for w in argument.split()[:-1] if w != "const")
+            if "*" in argument or kind == "cudaStream_t":
+                kinds += "p"
+            elif kind in ("int", "long long", "unsigned", "unsigned int"):
+                kinds += "i"
+            elif kind == "float":
+                kinds += "f"
+            else:
+                raise KernelError(f"{name}: no way to pass '{argument}'")
+        found[name] = (_RETURNS[returns], kinds)
+    return found
+
+
 class Library:
     """A kernel library's launchers as attributes, made when first asked for."""
 
-    _WIDE = ("rl_delta_chunked_scratch",)  # (what returns long long; everything else returns int)
-
     def __init__(self, name: str):
         self._cdll = build.load(name)
+        with open(os.path.join(build.CSRC_DIR, name + ".cu")) as f:
+            self._kinds = launcher_kinds(f.read())
 
     def __getattr__(self, name: str):
-        fn = launcher(ctypes.cast(getattr(self._cdll, name), ctypes.c_void_p).value, name in self._WIDE)
+        if name not in self._kinds:
+            raise AttributeError(name)
+        wide, kinds = self._kinds[name]
+        fn = launcher(ctypes.cast(getattr(self._cdll, name), ctypes.c_void_p).value, wide, kinds)
         setattr(self, name, fn)
         return fn
 

@@ -107,3 +107,62 @@ def test_the_native_side_is_what_launches():
         assert host._module.stream() == host.python_stream() == torch.cuda.current_stream().cuda_stream
     with pytest.raises(torch.OutOfMemoryError):
         host._module.empty(x, torch.float32, 1 << 45)
+
+
+def _exported():
+    import os
+
+    kinds = {}
+    for name in build.source_names():
+        with open(os.path.join(build.CSRC_DIR, name + ".cu")) as f:
+            kinds.update(host.launcher_kinds(f.read()))
+    return kinds
+
+
+def test_arguments_of_another_kind_or_number_are_refused(library):
+    """What ctypes refused stays refused: a float, None or a tensor of floats where a whole number goes moved every argument behind it."""
+    native, makers = launchers()
+    at = lambda name: ctypes.cast(getattr(library, name), ctypes.c_void_p).value  # noqa: E731
+    t = torch.zeros(8)
+    for make in makers:
+        few = make(at("few"), False, "pif")
+        assert few(t, torch.tensor(5), 2) == -5 and library.last()[:3] == [0.0, 5.0, 2.0]  # (whole numbers and floats of every sort, as ctypes took them)
+        assert few(t.data_ptr(), True, torch.tensor(0.5)) == -1 and library.last()[:3] == [0.0, 1.0, 0.5]
+        for wrong in ((t, 5.0, 2.0), (t, None, 2.0), (t, t, 2.0), (t, torch.tensor(1.0), 2.0), (t, 1, None), (t, 1, "x"), (t, 1, t), (1.0, 1, 1.0), ("x", 1, 1.0), (t, 1), (t, 1, 1.0, 1), ()):
+            with pytest.raises((TypeError, RuntimeError, ValueError) if any(a is t for a in wrong[1:]) else TypeError):
+                few(*wrong)
+        with pytest.raises(TypeError):
+            make(at("none"), False, "")(1)
+
+
+def test_a_library_knows_what_its_launchers_take():
+    if not shutil.which("nvcc"):
+        pytest.skip("no CUDA compiler")
+    takes = host.library("grouped_gemm").rl_grouped_gemm_takes
+    assert takes(64, 8, 8) == 1
+    for wrong in ((64.0, 8, 8), (64, None, 8), (64, 8), (64, 8, 8, 0)):
+        with pytest.raises(TypeError):
+            takes(*wrong)
+
+
+def test_every_call_gives_a_launcher_as_many_arguments_as_it_takes():
+    import ast
+    import inspect
+
+    from rusty_llama_b200.kernels import ops
+
+    kinds, stars, seen = _exported(), {"_wt": 2, "_act": 2, "_bias_args": 2}, 0
+    for call in ast.walk(ast.parse(inspect.getsource(ops))):
+        if not (isinstance(call, ast.Call) and isinstance(call.func, ast.Attribute) and call.func.attr in kinds):
+            continue
+        n = 0
+        for a in call.args:
+            if not isinstance(a, ast.Starred):
+                n += 1
+            elif isinstance(a.value, ast.GeneratorExp):
+                n += 3  # the three numbers of a pair of maps
+            else:
+                n += stars[a.value.func.id]
+        assert n == len(kinds[call.func.attr][1]), call.func.attr
+        seen += 1
+    assert seen > 50
