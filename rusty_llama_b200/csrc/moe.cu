@@ -500,7 +500,8 @@ RL_API int rl_moe_gemm(const void* x, int ldx, int dtype, const int* order, int 
 // ---------------------------------------------------------------- weighted sum of a token's experts
 // out[t, :] = sum_j weights[t, j] * y[place[t * top + j], :]  (+ gate[t] * shared[t, :]); y is float32.  A negative place takes
 // x[t, :], the experts' input (of type TS, like `shared`), in the place of y.  The rows of `always` further matrices (see the plan) are
-// y[T top + j T + t, :] and count gate[t] (1 without a gate) each.
+// y[T top + j T + t, :]: their sum is a shared expert's result, and like the one that comes as `shared` from products of its own it is
+// rounded to bfloat16 before it counts gate[t] (1 without a gate) times, so that a token's result does not depend on which way it went.
 template <typename TS, typename TO>
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
                                    int top, const TS* __restrict__ shared, const float* __restrict__ gate, TO* __restrict__ out, int d,
@@ -515,7 +516,11 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
       v += weights[(size_t)t * top + j] * (p >= 0 ? y[(size_t)p * d + i] : x != nullptr ? to_f32(x[(size_t)t * ldx + i]) : 0.f);
     }
     if (shared) v += (gate ? gate[t] : 1.f) * to_f32(shared[(size_t)t * d + i]);
-    for (int j = 0; j < always; ++j) v += (gate ? gate[t] : 1.f) * y[((size_t)gridDim.x * (top + j) + t) * d + i];
+    if (always > 0) {
+      float s = 0.f;
+      for (int j = 0; j < always; ++j) s += y[((size_t)gridDim.x * (top + j) + t) * d + i];
+      v += (gate ? gate[t] : 1.f) * to_f32(__float2bfloat16_rn(s));
+    }
     out[(size_t)t * d + i] = from_f32<TO>(v);
   }
 }
@@ -531,7 +536,7 @@ moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ plac
   pdl_wait();
   const int t = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (i >= d) return;
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  float v[4] = {0.f, 0.f, 0.f, 0.f}, own[4] = {0.f, 0.f, 0.f, 0.f};  // own: of the matrices that take every token
   const int all = top + always;
   for (int j0 = 0; j0 < all; j0 += COMBINE_AHEAD) {
     int p[COMBINE_AHEAD];
@@ -541,7 +546,7 @@ moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ plac
       const int j = j0 + u;
       const bool in = j < top;
       p[u] = in ? __ldcg(place + (size_t)t * top + j) : j < all ? (int)gridDim.x * j + t : -1;
-      w[u] = in ? __ldcg(weights + (size_t)t * top + j) : j < all && gate ? __ldcg(gate + t) : 1.f;
+      w[u] = in ? __ldcg(weights + (size_t)t * top + j) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u) {
@@ -551,16 +556,26 @@ moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ plac
     }
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u)
-      if (j0 + u < all)
+      if (j0 + u < top) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] += w[u] * f[u][e];
-  }
-  if (shared) {
-    float s[4];
-    load4_g<TS>(shared + (size_t)t * d + i, s);
-    const float g = gate ? __ldcg(gate + t) : 1.f;
+      } else if (j0 + u < all) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] += g * s[e];
+        for (int e = 0; e < 4; ++e) own[e] += f[u][e];
+      }
+  }
+  if (shared || always > 0) {
+    const float g = gate ? __ldcg(gate + t) : 1.f;
+    if (shared) {
+      float s[4];
+      load4_g<TS>(shared + (size_t)t * d + i, s);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] += g * s[e];
+    }
+    if (always > 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] += g * to_f32(__float2bfloat16_rn(own[e]));
+    }
   }
   store4<TO>(out + (size_t)t * d + i, v);
 }

@@ -1484,7 +1484,7 @@ def moe_combine(
 ) -> torch.Tensor:
     """out[t] = sum_j weights[t, j] * y[place[t, j]] (+ gate[t] * shared[t]); y float32 [T (top + always), d].  Where place is negative the
     term is weights[t, j] * x[t] (x [T, d], the experts' input: a choice that hands the input on).  always: the rows of that many
-    matrices that take every token stand behind the pairs' (`moe_plan`) and are added like `shared`."""
+    matrices that take every token stand behind the pairs' (`moe_plan`); their sum, rounded to bfloat16, is added like `shared`."""
     _cuda(y, "moe_combine y", torch.float32)
     _cuda(weights, "moe_combine weights", torch.float32)
     _cuda(place, "moe_combine place", torch.int32)

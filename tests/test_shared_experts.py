@@ -111,3 +111,44 @@ def test_part(T, shared_ff, gated):
         if rows.numel():
             want.index_add_(0, rows, mlp(xf[rows], f"e{e}.") * score[rows, place, None])
     assert float((got - want).norm() / want.norm()) <= 8e-3
+
+
+@pytest.mark.parametrize("d", [128, 136])
+@pytest.mark.parametrize("shared_ff, gated", [(64, False), (192, True)])
+def test_a_shared_experts_way_does_not_show(d, shared_ff, gated, monkeypatch):
+    """The same tokens with the shared expert's rows in the experts' products and in products of their own.  Both round its result to
+    bfloat16; their 32-bit sums differ by some 2^-22, which puts one number in 2^13 on the other side of a rounding, 2^-8 off: 5e-5 in
+    all, twice that allowed.  (Unrounded on one of the ways it is 1e-3.)"""
+    from rusty_llama_b200.parts import FEED_FORWARDS, Runtime
+    from rusty_llama_b200.spec import PartSpec
+
+    part = FEED_FORWARDS.build(PartSpec("routed_experts", {"hidden_size": d, "n_experts": 6, "top": 2, "expert_ff": 64, "bias": False, "renormalize": True,
+                                                           "shared_ff": shared_ff, "shared_gate": gated}), Runtime.create(DEV, torch.bfloat16))
+    g = torch.Generator().manual_seed(shared_ff + d)
+    w = {}
+    for name, info in part.param_infos().items():
+        t = (torch.randn(info.shape, generator=g) * info.shape[-1] ** -0.5).to(torch.bfloat16)
+        w[name] = (t.float() if info.kind == "scalars" else t).to(DEV)
+    part.load(w)
+    x = torch.randn(150, d, generator=g).to(torch.bfloat16).to(DEV)
+    assert part.always and part._joins(150)
+    joined = part.forward(x, None).double()
+    monkeypatch.setattr(part, "_joins", lambda T: False)
+    apart = part.forward(x, None).double()
+    assert float((joined - apart).norm() / apart.norm()) <= 1e-4
+
+
+@pytest.mark.parametrize("d", [6, 8])  # (rows of whole fours have a kernel of their own)
+@pytest.mark.parametrize("always, gated", [(1, True), (3, False), (9, True)])
+def test_sum_of_the_matrices_that_take_every_token(d, always, gated):
+    T, top = 5, 2
+    g = torch.Generator().manual_seed(d + always)
+    y = torch.randn(T * (top + always), d, generator=g)
+    place = torch.randperm(T * top, generator=g).to(torch.int32)
+    weights, gate = torch.rand(T, top, generator=g), torch.rand(T, generator=g)
+    got = ops.moe_combine(y.to(DEV), place.to(DEV), weights.to(DEV), None, gate.to(DEV) if gated else None, always=always).cpu()
+    own = torch.zeros(T, d)
+    for j in range(always):
+        own += y[T * (top + j) : T * (top + j + 1)]
+    want = (weights.double()[:, :, None] * y.double()[place.long()].view(T, top, d)).sum(1) + own.to(torch.bfloat16).double() * (gate.double()[:, None] if gated else 1.0)
+    assert float((got.double() - want).abs().max()) <= 4 * 2.0**-24 * 8  # (four roundings of numbers below eight)
