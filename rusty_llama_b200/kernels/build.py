@@ -149,6 +149,13 @@ def build(name: str, verbose: bool = True) -> str:
 HOST_CALLS = "_rl_host_calls"
 
 
+def _host_flags() -> List[str]:
+    import torch
+
+    return ["-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-ltorch_python", "-ltorch_cpu",
+            "-lc10", "-lc10_cuda"]
+
+
 def _host_command(out: str) -> List[str]:
     import sysconfig
 
@@ -156,56 +163,63 @@ def _host_command(out: str) -> List[str]:
 
     root = os.path.dirname(torch.__file__)
     cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
-    flags = ["-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    where = ["-L" + os.path.join(root, "lib")]
     for inc in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"], cuda):
-        flags += ["-isystem", inc]
-    libs = ["-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    return [shutil.which("g++") or "c++"] + flags + ["-o", out, os.path.join(CSRC_DIR, "host_calls.cpp")] + libs
+        where += ["-isystem", inc]
+    return [shutil.which("g++") or "c++", "-o", out, os.path.join(CSRC_DIR, "host_calls.cpp")] + where + _host_flags()
 
 
 def _host_fingerprint() -> str:
     import torch
 
     with open(os.path.join(CSRC_DIR, "host_calls.cpp"), "rb") as f:
-        return hashlib.sha256(f.read() + f"{sys.version}|{torch.__version__}".encode()).hexdigest()
+        return hashlib.sha256(f.read() + f"{sys.version}|{torch.__version__}|{' '.join(_host_flags())}".encode()).hexdigest()
 
 
 def build_host_calls(verbose: bool = True) -> str:
-    """Compile `csrc/host_calls.cpp` against this Python and this PyTorch if that has not been done; returns the path."""
+    """Compile `csrc/host_calls.cpp` against this Python and this PyTorch if that has not been done; returns the path.  One process of
+    those that share the folder compiles, the others wait for it."""
+    import fcntl
+
     out = os.path.join(_build_dir(), HOST_CALLS + ".so")
     want = _host_fingerprint()
-    if _host_is_built(out, want):
-        return out
-    if verbose:
-        _say("compiling host_calls.cpp ...")
-    tmp = f"{out}.{os.getpid()}.tmp"
-    proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if proc.returncode != 0:
-        if os.path.exists(tmp):
-            os.remove(tmp)
-        raise KernelError(f"compiling host_calls.cpp failed (exit {proc.returncode}):\n{proc.stdout}")
-    os.replace(tmp, out)
-    with open(out + ".sha256", "w") as f:
-        f.write(want)
+    with open(out + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if _is_stamped(out, ".sha256", want):
+            return out
+        if verbose:
+            _say("compiling host_calls.cpp ...")
+        tmp = f"{out}.{os.getpid()}.tmp"
+        proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if proc.returncode != 0:
+            if os.path.exists(tmp):
+                os.remove(tmp)
+            with open(out + ".failed", "w") as f:
+                f.write(want)
+            raise KernelError(f"compiling host_calls.cpp failed (exit {proc.returncode}):\n{proc.stdout}")
+        os.replace(tmp, out)
+        with open(out + ".sha256", "w") as f:
+            f.write(want)
     return out
 
 
-def _host_is_built(out: str, want: str) -> bool:
+def _is_stamped(out: str, stamp: str, want: str) -> bool:
     try:
-        with open(out + ".sha256") as f:
-            return os.path.isfile(out) and f.read().strip() == want
+        with open(out + stamp) as f:
+            return f.read().strip() == want and (stamp == ".failed" or os.path.isfile(out))
     except OSError:
         return False
 
 
 def load_host_calls(may_build: bool):
-    """The module of `csrc/host_calls.cpp`; None where it is not built and may not be."""
+    """The module of `csrc/host_calls.cpp`; None where it is not built and may not be, or did not compile here before (`build_all` tries again)."""
     import importlib.machinery
     import importlib.util
 
     out = os.path.join(_build_dir(), HOST_CALLS + ".so")
-    if not _host_is_built(out, _host_fingerprint()):
-        if not may_build:
+    want = _host_fingerprint()
+    if not _is_stamped(out, ".sha256", want):
+        if not may_build or _is_stamped(out, ".failed", want):
             return None
         build_host_calls()
     loader = importlib.machinery.ExtensionFileLoader(HOST_CALLS, out)

@@ -2,7 +2,8 @@
 
 `csrc/host_calls.cpp` does this natively (an `add_rmsnorm` with the tensor of its result: 6.2 us instead of 10.9, of which the driver has 3; a
 sublayer of nine kernels: 92 us a pass instead of 165, which is the host's time); the classes and functions below are the same in Python,
-used where that module cannot be built (no Python or PyTorch headers) and where there is no GPU to launch on.  Results and errors are the same.
+used until a library is first asked for, where that module cannot be built (no Python or PyTorch headers) and where there is no GPU to launch on.
+Results and errors are the same.
 """
 
 from __future__ import annotations
@@ -11,7 +12,8 @@ import ctypes
 import operator
 import os
 import re
-from typing import Dict, Optional, Tuple
+import threading
+from typing import Dict, List, Optional, Tuple
 
 import torch
 
@@ -87,23 +89,48 @@ def python_columns(t: torch.Tensor, first: int, end: int) -> torch.Tensor:
     return t[:, first:end]
 
 
-def _native():
-    """The native module, or None.  It is built here if there is a GPU whose launches would gain from it; never for shape-only runs."""
-    try:
-        return build.load_host_calls(torch.cuda.is_available())
-    except Exception as e:  # whatever is missing on this machine: the Python side does the same
-        build._say(f"host_calls.cpp is not used: {str(e).strip().splitlines()[-1][:200] if str(e).strip() else type(e).__name__}")
-        return None
+cuda, rows, odd, stream = python_cuda, python_rows, python_odd, python_stream
+empty, columns, launcher = python_empty, python_columns, PythonLauncher
+
+_lock = threading.Lock()
+_bound: List[Tuple[dict, Dict[str, str]]] = []
 
 
-_module = _native()
-if _module is not None:
-    _module.set_error(KernelError)
-    cuda, rows, odd, stream = _module.cuda, _module.rows, _module.odd, _module.stream
-    empty, columns, launcher = _module.empty, _module.columns, _module.launcher
-else:
-    cuda, rows, odd, stream = python_cuda, python_rows, python_odd, python_stream
-    empty, columns, launcher = python_empty, python_columns, PythonLauncher
+def bind(namespace: dict, **names: str) -> None:
+    """Puts this module's functions into another's namespace, under names of its own, and puts the native ones there once they are loaded."""
+    with _lock:
+        _bound.append((namespace, names))
+        namespace.update((own, globals()[name]) for own, name in names.items())
+
+
+def _find_native() -> None:
+    """Takes the native module up, from the first library on: importing this package touches neither CUDA nor a compiler.  It is built
+    where a process that uses a GPU finds it missing; a run of shapes alone stays with Python."""
+    with _lock:
+        if "_module" in globals():
+            return
+        try:
+            module = build.load_host_calls(torch.cuda.is_initialized())
+            if module is None and not torch.cuda.is_initialized():
+                return  # (asked again by the next library)
+        except Exception as e:  # whatever is missing on this machine: the Python side does the same
+            build._say(f"host_calls.cpp is not used: {str(e).strip().splitlines()[-1][:200] if str(e).strip() else type(e).__name__}")
+            module = None
+        globals()["_module"] = module
+        if module is None:
+            return
+        module.set_error(KernelError)
+        for name in ("cuda", "rows", "odd", "stream", "empty", "columns", "launcher"):
+            globals()[name] = getattr(module, name)
+        for namespace, names in _bound:
+            namespace.update((own, globals()[name]) for own, name in names.items())
+
+
+def __getattr__(name: str):
+    if name == "_module":  # the native module, or None
+        _find_native()
+        return globals().get("_module")
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 _RETURNS = {"int": False, "long long": True}
@@ -132,6 +159,7 @@ class Library:
     """A kernel library's launchers as attributes, made when first asked for."""
 
     def __init__(self, name: str):
+        _find_native()
         self._cdll = build.load(name)
         with open(os.path.join(build.CSRC_DIR, name + ".cu")) as f:
             self._kinds = launcher_kinds(f.read())

@@ -19,7 +19,9 @@ import torch
 from ..errors import KernelError
 from . import ops
 from .device import sm_count
-from .host import odd as _odd  # whether the operands' rows cannot be moved in 16-byte pieces
+from .host import bind
+
+bind(globals(), _odd="odd")  # whether the operands' rows cannot be moved in 16-byte pieces
 
 _library_gemm = False
 

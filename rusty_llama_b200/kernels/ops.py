@@ -18,8 +18,9 @@ import torch
 from ..errors import KernelError
 from . import build
 from .device import sm_count
-from .host import columns, library  # noqa: F401  (columns is for the parts)
-from .host import cuda as _cuda, empty as _empty, rows as _rows, stream as _stream
+from .host import bind, library
+
+bind(globals(), columns="columns", _cuda="cuda", _empty="empty", _rows="rows", _stream="stream")  # (columns is for the parts)
 
 PAGE_SIZE = 64  # tokens per cache page; the attention kernels' key tile
 

@@ -166,3 +166,55 @@ def test_every_call_gives_a_launcher_as_many_arguments_as_it_takes():
         assert n == len(kinds[call.func.attr][1]), call.func.attr
         seen += 1
     assert seen > 50
+
+
+def test_importing_touches_neither_cuda_nor_a_compiler():
+    import os
+    import sys
+
+    code = """
+import subprocess, torch
+def never(*a, **k): raise AssertionError("called by the import")
+torch.cuda.is_available = torch.cuda.device_count = torch.cuda.init = torch._C._cuda_getDeviceCount = subprocess.run = subprocess.Popen = never
+import rusty_llama_b200
+from rusty_llama_b200.kernels import host, linear, ops
+assert "_module" not in vars(host) and ops._cuda is host.python_cuda and linear._odd is host.python_odd
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], cwd=root, check=True)
+
+
+def test_functions_are_native_from_the_first_library_on():
+    if not shutil.which("nvcc"):
+        pytest.skip("no CUDA compiler")
+    from rusty_llama_b200.kernels import linear, ops
+
+    build.build_host_calls()
+    host.library("grouped_gemm")
+    assert host._module is not None and ops._cuda is host._module.cuda and ops._empty is host.empty and linear._odd is host._module.odd
+
+
+def test_one_process_builds_and_a_failure_is_remembered(tmp_path, monkeypatch):
+    import os
+    import threading
+
+    monkeypatch.setattr(build, "_build_dir_cached", str(tmp_path))
+    runs = tmp_path / "runs"
+    tool = tmp_path / "compiler"
+    tool.write_text(f"#!/bin/sh\necho run >> {runs}\nsleep 0.3\n[ -e {tmp_path}/works ] && echo built > $1\n")
+    tool.chmod(0o755)
+    monkeypatch.setattr(build, "_host_command", lambda out: [str(tool), out])
+    with pytest.raises(KernelError):
+        build.load_host_calls(True)
+    assert build.load_host_calls(True) is None and build.load_host_calls(False) is None and len(runs.read_text().split()) == 1
+    (tmp_path / "works").write_text("")
+    several = [threading.Thread(target=build.build_host_calls) for _ in range(4)]
+    for t in several:
+        t.start()
+    for t in several:
+        t.join()
+    assert len(runs.read_text().split()) == 2 and os.path.isfile(tmp_path / (build.HOST_CALLS + ".so"))
+    flags = build._host_flags()
+    before = build._host_fingerprint()
+    monkeypatch.setattr(build, "_host_flags", lambda: flags + ["-O1"])
+    assert build._host_fingerprint() != before
