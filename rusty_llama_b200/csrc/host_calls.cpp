@@ -10,6 +10,7 @@
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <exception>
@@ -22,27 +23,19 @@ static PyObject* kernel_error = nullptr;  // errors.KernelError
 
 static PyObject* refuse(PyObject* what, const char* rest) { return PyErr_Format(kernel_error, "%S: %s", what, rest); }
 
-// A C++ exception (a tensor without storage, no memory) as a Python one
+// A C++ exception (a tensor without storage, no memory, a range that is not there) as the Python one that PyTorch makes of it
 #define HC_TRY try {
-#define HC_CATCH                                       \
-  }                                                    \
-  catch (const c10::OutOfMemoryError& e) {             \
-    raise_out_of_memory(e.what_without_backtrace());   \
-    return nullptr;                                    \
-  }                                                    \
-  catch (const std::exception& e) {                    \
-    PyErr_SetString(PyExc_RuntimeError, e.what());     \
-    return nullptr;                                    \
+#define HC_CATCH                                                      \
+  }                                                                   \
+  catch (...) {                                                       \
+    torch::translate_exception_to_python(std::current_exception());   \
+    return nullptr;                                                   \
   }
 
-static void raise_out_of_memory(const char* text) {
-  PyObject* torch = PyImport_ImportModule("torch");
-  PyObject* kind = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
-  PyErr_Clear();
-  PyErr_SetString(kind ? kind : PyExc_RuntimeError, text);
-  Py_XDECREF(kind);
-  Py_XDECREF(torch);
-}
+struct Unlocked {  // without the interpreter's lock, which an exception takes again on its way out
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
 
 // ---------------------------------------------------------------- launchers
 // An exported launcher takes pointers, int, long long, unsigned, float and the stream, and returns int (or long long).  Both calling
@@ -64,6 +57,8 @@ struct Launcher {
   char kinds[HC_INTS + HC_FLOATS];  // of each: 'p' a pointer, 'i' a whole number, 'f' a float
 };
 
+static PyObject* too_many() { return PyErr_Format(PyExc_TypeError, "a launcher takes %d floats and %d integers and tensors at most", HC_FLOATS, HC_INTS); }
+
 static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* kwnames) {
   const Launcher* l = reinterpret_cast<Launcher*>(self);
   const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
@@ -77,13 +72,13 @@ static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nar
     PyObject* a = args[k];
     const char kind = l->n >= 0 ? l->kinds[k] : PyFloat_Check(a) ? 'f' : a == Py_None || THPVariable_Check(a) ? 'p' : 'i';
     if (kind == 'f') {
-      if (nf == HC_FLOATS) return PyErr_Format(PyExc_TypeError, "a launcher takes %d floats at most", HC_FLOATS);
+      if (nf == HC_FLOATS) return too_many();
       const double x = PyFloat_AsDouble(a);
       if (x == -1.0 && PyErr_Occurred()) return nullptr;
       f[nf++] = (float)x;
       continue;
     }
-    if (ni == HC_INTS) return PyErr_Format(PyExc_TypeError, "a launcher takes %d integers and tensors at most", HC_INTS);
+    if (ni == HC_INTS) return too_many();
     if (PyLong_Check(a)) {  // (a pointer's, too: an address)
       i[ni] = (L)PyLong_AsUnsignedLongLongMask(a);
       if (i[ni] == -1 && PyErr_Occurred()) return nullptr;
@@ -100,11 +95,12 @@ static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nar
     }
   }
   L r;
-  Py_BEGIN_ALLOW_THREADS
-  r = l->fn(i[0], i[1], i[2], i[3], i[4], i[5], i[6], i[7], i[8], i[9], i[10], i[11], i[12], i[13], i[14], i[15], i[16], i[17], i[18], i[19], i[20], i[21],
-            i[22], i[23], i[24], i[25], i[26], i[27], i[28], i[29], i[30], i[31], i[32], i[33], i[34], i[35], i[36], i[37], i[38], i[39], i[40], i[41], i[42],
-            i[43], i[44], i[45], i[46], i[47], i[48], i[49], i[50], i[51], i[52], i[53], i[54], i[55], f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
-  Py_END_ALLOW_THREADS
+  {
+    Unlocked here;
+    r = l->fn(i[0], i[1], i[2], i[3], i[4], i[5], i[6], i[7], i[8], i[9], i[10], i[11], i[12], i[13], i[14], i[15], i[16], i[17], i[18], i[19], i[20], i[21],
+              i[22], i[23], i[24], i[25], i[26], i[27], i[28], i[29], i[30], i[31], i[32], i[33], i[34], i[35], i[36], i[37], i[38], i[39], i[40], i[41], i[42],
+              i[43], i[44], i[45], i[46], i[47], i[48], i[49], i[50], i[51], i[52], i[53], i[54], i[55], f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
+  }
   return PyLong_FromLongLong(l->wide ? r : (L)(int)r);
   HC_CATCH
 }
@@ -123,8 +119,7 @@ static PyObject* make_launcher(PyObject*, PyObject* args) {
     if (kinds[n] == 'f') ++floats;
     else if (kinds[n] != 'p' && kinds[n] != 'i') return PyErr_Format(PyExc_ValueError, "unknown kind of argument in '%s'", kinds);
   }
-  if (floats > HC_FLOATS || n - floats > HC_INTS)
-    return PyErr_Format(PyExc_TypeError, "a launcher takes %d floats and %d integers and tensors at most", HC_FLOATS, HC_INTS);
+  if (floats > HC_FLOATS || n - floats > HC_INTS) return too_many();
   Launcher* l = PyObject_New(Launcher, &launcher_type);
   if (!l) return nullptr;
   l->call = launcher_call;
@@ -212,14 +207,10 @@ static PyObject* make_empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Device device = THPVariable_Unpack(args[0]).device();
   const at::ScalarType type = reinterpret_cast<THPDtype*>(args[1])->scalar_type;
   at::Tensor out;
-  Py_BEGIN_ALLOW_THREADS
-  try {
+  {
+    Unlocked here;
     out = at::empty(at::IntArrayRef(sizes, n - 2), at::TensorOptions().dtype(type).device(device));
-  } catch (...) {
-    PyEval_RestoreThread(_save);
-    throw;
   }
-  Py_END_ALLOW_THREADS
   return THPVariable_Wrap(out);
   HC_CATCH
 }

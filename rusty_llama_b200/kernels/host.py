@@ -21,11 +21,17 @@ from ..errors import KernelError
 from . import build
 
 
+_MOST_FLOATS, _MOST_INTS = 8, 56
+_TOO_MANY = f"a launcher takes {_MOST_FLOATS} floats and {_MOST_INTS} integers and tensors at most"
+
+
 class PythonLauncher:
     """A launcher called with tensors, numbers and None as they are.  kinds: of every argument 'p' (a pointer: a tensor, an address or
     None), 'i' (a whole number) or 'f' (a float); calls are checked against it.  Without kinds each argument goes by its own type."""
 
     def __init__(self, address: int, wide: bool, kinds: Optional[str] = None):
+        if kinds is not None and (kinds.count("f") > _MOST_FLOATS or len(kinds) - kinds.count("f") > _MOST_INTS):
+            raise TypeError(_TOO_MANY)
         self.fn = ctypes.CFUNCTYPE(ctypes.c_longlong if wide else ctypes.c_int)(address)
         self.kinds = kinds
 
@@ -35,6 +41,8 @@ class PythonLauncher:
             kinds = ["f" if isinstance(a, float) else "p" if a is None or isinstance(a, torch.Tensor) else "i" for a in args]
         elif len(kinds) != len(args):
             raise TypeError(f"this launcher takes {len(kinds)} arguments, not {len(args)}")
+        if kinds is not self.kinds and (sum(k == "f" for k in kinds) > _MOST_FLOATS or sum(k != "f" for k in kinds) > _MOST_INTS):
+            raise TypeError(_TOO_MANY)
         given = []
         for n, (kind, a) in enumerate(zip(kinds, args)):
             if kind == "f":
@@ -57,6 +65,8 @@ def python_cuda(t: torch.Tensor, what: str, dtype=None, contiguous=True) -> torc
         raise KernelError(f"{what}: not a tensor")
     if not t.is_cuda:
         raise KernelError(f"{what}: tensor is on {t.device}, the kernels run on CUDA only")
+    if dtype is not None and not isinstance(dtype, torch.dtype):
+        raise TypeError("cuda: dtype is not a torch.dtype")
     if dtype is not None and t.dtype != dtype:
         raise KernelError(f"{what}: dtype {t.dtype}, expected {dtype}")
     if contiguous and not t.is_contiguous():
@@ -66,6 +76,8 @@ def python_cuda(t: torch.Tensor, what: str, dtype=None, contiguous=True) -> torc
 
 def python_rows(t: torch.Tensor, what: str) -> int:
     """Row stride of a 2-D tensor whose rows are dense."""
+    if not isinstance(t, torch.Tensor):
+        raise TypeError("rows(tensor, what)")
     if t.dim() != 2 or t.stride(1) != 1:
         raise KernelError(f"{what}: expected a 2-D tensor with dense rows")
     return t.stride(0)
@@ -73,6 +85,10 @@ def python_rows(t: torch.Tensor, what: str) -> int:
 
 def python_odd(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether rows of the two cannot be moved in 16-byte pieces (eight 16-bit numbers)."""
+    if not (isinstance(x, torch.Tensor) and isinstance(w, torch.Tensor)):
+        raise TypeError("odd(x, w)")
+    if x.dim() != 2 or w.dim() < 1:
+        raise IndexError("odd: rows expected")
     return bool(x.shape[1] % 8 or x.stride(0) % 8 or w.stride(0) % 8 or x.data_ptr() % 16 or w.data_ptr() % 16)
 
 
@@ -82,11 +98,15 @@ def python_stream() -> int:
 
 
 def python_empty(like: torch.Tensor, dtype, *sizes: int) -> torch.Tensor:
+    if not (isinstance(like, torch.Tensor) and isinstance(dtype, torch.dtype) and 1 <= len(sizes) <= 4):
+        raise TypeError("empty(like, dtype, one to four sizes)")
     return torch.empty(sizes, dtype=dtype, device=like.device)
 
 
 def python_columns(t: torch.Tensor, first: int, end: int) -> torch.Tensor:
-    return t[:, first:end]
+    if not isinstance(t, torch.Tensor):
+        raise TypeError("columns(tensor, first, end)")
+    return t.narrow(1, first, end - first)  # (what is not there is refused, not left out)
 
 
 cuda, rows, odd, stream = python_cuda, python_rows, python_odd, python_stream

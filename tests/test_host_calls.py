@@ -218,3 +218,29 @@ def test_one_process_builds_and_a_failure_is_remembered(tmp_path, monkeypatch):
     before = build._host_fingerprint()
     monkeypatch.setattr(build, "_host_flags", lambda: flags + ["-O1"])
     assert build._host_fingerprint() != before
+
+
+def test_refusals_agree_with_python(library):
+    """What one side refuses the other does too, with the same kind of error and, where it is the library's own, the same words."""
+    native, (make, python_make) = launchers()
+    at = ctypes.cast(library.none, ctypes.c_void_p).value
+    t, i = torch.zeros(4, 6), torch.zeros(())
+    pairs = [
+        (make(at, False), python_make(at, False), [tuple([1.0] * 9), tuple([1] * 57)]),
+        (lambda k: make(at, False, k), lambda k: python_make(at, False, k), ["f" * 9, "i" * 57]),
+        (make(at, False, "pif"), python_make(at, False, "pif"), [(t, 1), (1.5, 1, 1.0), (t, 1.5, 1.0), (t, 1, "x")]),
+        (native.rows, host.python_rows, [(3, "r"), (t[0], "r"), (t.t(), "r")]),
+        (native.odd, host.python_odd, [(t[0], t), (t.view(2, 2, 6), t), (t, i), (3, t), (t, 3)]),
+        (native.empty, host.python_empty, [(t, torch.float32), (t, torch.float32, 1, 1, 1, 1, 1), (t, 3, 1), (3, torch.float32, 1), (t, torch.float32, -1)]),
+        (native.columns, host.python_columns, [(t, 2, 9), (t, 7, 8), (t, 4, 2), (t[0], 0, 1), (3, 0, 1)]),
+        (native.cuda, host.python_cuda, [(3, "a"), (t, "a")]),
+    ]
+    for one, other, calls in pairs:
+        for args in calls:
+            seen = []
+            for f in (one, other):
+                with pytest.raises(Exception) as e:
+                    f(*(args if isinstance(args, tuple) else (args,)))
+                words = str(e.value)
+                seen.append((e.type, words if e.type is KernelError or "launcher" in words else ""))
+            assert seen[0] == seen[1], (args, seen)
