@@ -102,6 +102,7 @@ gemm_fma_kernel(const TA* __restrict__ x, int ldx, const TA* __restrict__ w, int
 #define GEMV_SUB 32       // k of a chunk that a stage of the ring holds: 128 bytes of an item, whose 16-byte pieces lie swizzled by the item
 #define GEMV_XCHUNK (KCHUNK + 4)      // the rows of x, per chunk: eight chunks' same places meet all banks
 #define GEMV_MAX_ITEMS 2048           // items of a block, whose sums wait in shared memory
+#define GEMV_FEW 8                    // features that make up for what a block reads of x
 #define GEMV_STAGE_BYTES (GEMV_THREADS * GEMV_SUB * 4)
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
@@ -346,38 +347,61 @@ static size_t gemv_f32_smem(int stages, int mb, int nch, int R) {
   return (size_t)stages * GEMV_STAGE_BYTES + (size_t)mb * nch * (GEMV_XCHUNK + R) * sizeof(float);
 }
 
+// How the few rows of a product are streamed: mb rows of x a block (0: not at all), R features a block, the ring's stages.
+struct GemvPlan {
+  int mb, R, stages;
+  size_t smem;
+};
+static GemvPlan gemv_f32_plan(int M, int N, int K, int sms) {
+  const int nch = (K + KCHUNK - 1) / KCHUNK;
+  const size_t half = 112 * 1024, third = 74 * 1024, whole = 224 * 1024;
+  // features whose sums a block has room for beside a ring of three stages and its rows of x
+  auto room = [&](int mb, size_t limit) {
+    const long long sums = ((long long)limit - 3 * GEMV_STAGE_BYTES) / (4LL * mb * nch) - GEMV_XCHUNK;
+    return (int)(nch <= GEMV_MAX_ITEMS && sums > GEMV_MAX_ITEMS / nch ? GEMV_MAX_ITEMS / nch : sums);
+  };
+  // features a block: as many as make one wave of per_sm blocks an SM, or where a block has no room for those, of as few equal waves as it takes
+  auto features = [&](int per_sm, int most) {
+    const int R = (N + per_sm * sms - 1) / (per_sm * sms), waves = (R + most - 1) / most;
+    return (R + waves - 1) / waves;
+  };
+  auto walk = [&](int per_sm, int R) {  // passes of 128 pairs on the busiest SM
+    const long long waves = ((N + R - 1) / R + (long long)per_sm * sms - 1) / (per_sm * sms);
+    return waves * per_sm * ((R * nch + GEMV_THREADS - 1) / GEMV_THREADS);
+  };
+  // As many rows of x a block as there are, up to four, while two blocks of a few features fit an SM: blocks of fewer rows read all weights
+  // again.  Else one row, and at last one block an SM (up to 338 chunks: K of 43264).
+  const int wave = (N + 2 * sms - 1) / (2 * sms), few = wave < GEMV_FEW ? wave : GEMV_FEW;
+  int mb = M == 1 ? 1 : M == 2 ? 2 : 4;
+  while (mb > 1 && room(mb, half) < few) mb /= 2;
+  const bool two = room(mb, half) >= few;
+  const size_t limit = two ? half : whole;
+  const int most = room(mb, limit), most3 = two ? room(mb, third) : 0;
+  if (most < 1) return {0, 0, 0, 0};
+  int R = features(two ? 2 : 1, most), stages = gemv_f32_smem(4, mb, nch, R) > limit ? 3 : 4;
+  // three blocks an SM where that is less to walk through (2560 x 2048 with 2 rows: 9 features of 16 chunks are 144 pairs, two passes of 128; 6
+  // are one: 7.9 and 6.0 us)
+  if (most3 >= 1 && walk(3, features(3, most3)) < walk(2, R)) R = features(3, most3), stages = 3;
+  return {mb, R, stages, gemv_f32_smem(stages, mb, nch, R)};
+}
+// Rows of x that a block takes beside the weights, or 0 where the product goes by tiles (operands in 16-byte pieces).
+RL_API int rl_gemm_f32_streams(int M, int N, int K, int sms) { return M > 0 && M <= GEMV_ROWS && N > 0 && K > 0 && sms > 0 ? gemv_f32_plan(M, N, K, sms).mb : 0; }
+
 RL_API int rl_gemm_f32(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int M, int N, int K, int sms,
                        cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) RL_REFUSE(1, "gemm_f32: M=%d N=%d K=%d on %d SMs", M, N, K, sms);
   if (ldx < K || ldw < K || ldo < N) RL_REFUSE(2, "gemm_f32: leading sizes %d/%d/%d too small", ldx, ldw, ldo);
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-  const int nch = (K + KCHUNK - 1) / KCHUNK;
-  if (M <= GEMV_ROWS && vec && nch <= GEMV_MAX_ITEMS) {
-    // features a block: as many as make one wave of two blocks an SM, or of three where that is less to walk through (2560 x 2048 with 2 rows: 9
-    // features of 16 chunks are 144 pairs, two passes of 128; 6 are one: 7.9 and 6.0 us) and three fit
-    auto features = [&](int per_sm) {
-      const int R = (N + per_sm * sms - 1) / (per_sm * sms);
-      return R < GEMV_MAX_ITEMS / nch ? R : GEMV_MAX_ITEMS / nch;
-    };
-    auto passes = [&](int R) { return (R * nch + GEMV_THREADS - 1) / GEMV_THREADS; };
-    const int R2 = features(2), R3 = features(3);
-    // as many rows of x a block as there are, up to four, while two blocks fit an SM; else one row (up to 338 chunks: K of 43264)
-    const size_t half = 112 * 1024, third = 74 * 1024;
-    int mb = M == 1 ? 1 : M == 2 ? 2 : 4;
-    while (mb > 1 && gemv_f32_smem(3, mb, nch, R2) > half) mb /= 2;
-    const bool three = 3 * passes(R3) < 2 * passes(R2) && gemv_f32_smem(3, mb, nch, R3) <= third;
-    const int R = three ? R3 : R2, stages = three || gemv_f32_smem(4, mb, nch, R) > half ? 3 : 4;
-    const size_t smem = gemv_f32_smem(stages, mb, nch, R);
-    if (smem <= 224 * 1024) {
-#define RL_GEMV(MB, STAGES) return launch_gemv_f32<MB, STAGES>(x, ldx, w, ldw, out, ldo, M, N, K, R, smem, stream)
-      if (mb == 1 && stages == 4) RL_GEMV(1, 4);
-      if (mb == 1) RL_GEMV(1, 3);
-      if (mb == 2 && stages == 4) RL_GEMV(2, 4);
-      if (mb == 2) RL_GEMV(2, 3);
-      if (stages == 4) RL_GEMV(4, 4);
-      RL_GEMV(4, 3);
+  const GemvPlan p = M <= GEMV_ROWS && vec ? gemv_f32_plan(M, N, K, sms) : GemvPlan{};
+  if (p.mb > 0) {
+#define RL_GEMV(MB, STAGES) return launch_gemv_f32<MB, STAGES>(x, ldx, w, ldw, out, ldo, M, N, K, p.R, p.smem, stream)
+    if (p.mb == 1 && p.stages == 4) RL_GEMV(1, 4);
+    if (p.mb == 1) RL_GEMV(1, 3);
+    if (p.mb == 2 && p.stages == 4) RL_GEMV(2, 4);
+    if (p.mb == 2) RL_GEMV(2, 3);
+    if (p.stages == 4) RL_GEMV(4, 4);
+    RL_GEMV(4, 3);
 #undef RL_GEMV
-    }
   }
   // the tile with the least work on the busiest SM: its blocks there, times the tile's outputs, times what an output costs with
   // that many outputs a thread (shared-memory reads per FMA)

@@ -43,10 +43,10 @@ def test_product_in_every_form(ops, M, N, K):
 
 
 def test_product_of_a_very_long_k(ops):
-    """The longest rows of the few-row kernel (327 chunks of 128 and one row of a block's shared memory) and ones too long for it, which go to
+    """The longest rows of the few-row kernel (338 chunks of 128 and one row of a block's shared memory) and ones too long for it, which go to
     the tile kernel however few they are: the same bits as among many rows."""
     g = torch.Generator().manual_seed(5)
-    for K in (20000, 41856, 41860, 44000, 70000):
+    for K in (20000, 41856, 41860, 43264, 43268, 70000):
         x, w = torch.randn(12, K, generator=g), torch.randn(9, K, generator=g)
         xd, wd = x.to(DEV), w.to(DEV)
         many = ops.gemm_f32(xd, wd)
@@ -55,11 +55,12 @@ def test_product_of_a_very_long_k(ops):
             assert torch.equal(ops.gemm_f32(xd[:rows], wd), many[:rows])
 
 
-@pytest.mark.parametrize("N, K", [(2560, 2048), (2553, 1924), (11264, 2048), (40001, 2048), (2048, 5632), (2047, 14336)])
+@pytest.mark.parametrize("N, K", [(2560, 2048), (2553, 1924), (11264, 2048), (40001, 2048), (2048, 5632), (2047, 14336), (16384, 3072), (9001, 3712),
+                                  (1500, 41856), (1000, 43264)])
 @pytest.mark.parametrize("M", [1, 2, 4, 5, 8])
 def test_few_rows_of_large_matrices(ops, M, N, K):
-    """Three blocks an SM and two, one pass and many, the most sums a block holds, the last block's fewer features: the same bits as among
-    many rows."""
+    """Three blocks an SM, two and one, one pass and many, one wave of blocks and several, the most sums a block holds, the last block's fewer
+    features: the same bits as among many rows."""
     g = torch.Generator(device=DEV).manual_seed(M * 7919 + N + K)
     x, w = torch.randn(40, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
     assert torch.equal(ops.gemm_f32(x[:M], w), ops.gemm_f32(x, w)[:M])
