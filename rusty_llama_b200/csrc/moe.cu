@@ -121,17 +121,18 @@ moe_router_choose_kernel(const float* __restrict__ logits, int parts, const floa
   float gate_z = 0.f;
 #pragma unroll
   for (int i = 0; i < EACH; ++i) z[i] = 0.f;
-  for (int p0 = 0; p0 < parts; p0 += 4) {  // four partial sums asked for at once
-    float v[4][EACH], gv[4];
+  constexpr int AHEAD = EACH <= 16 ? 4 : 1;  // partial sums asked for at once (four of 48 experts a lane would not fit its registers)
+  for (int p0 = 0; p0 < parts; p0 += AHEAD) {
+    float v[AHEAD][EACH], gv[AHEAD];
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
+    for (int p = 0; p < AHEAD; ++p) {
       const bool in = p0 + p < parts;
 #pragma unroll
       for (int i = 0; i < EACH; ++i) v[p][i] = in && lane + 32 * i < E ? __ldcg(lg + (p0 + p) * part + lane + 32 * i) : 0.f;
       gv[p] = in && rows > E ? __ldcg(lg + (p0 + p) * part + E) : 0.f;
     }
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
+    for (int p = 0; p < AHEAD; ++p) {
 #pragma unroll
       for (int i = 0; i < EACH; ++i) z[i] = p0 + p ? z[i] + v[p][i] : v[p][i];
       gate_z = p0 + p ? gate_z + gv[p] : gv[p];
@@ -208,6 +209,8 @@ static int launch_choose(const float* logits, int parts, const float* bias, int 
   else if (E <= 128) RL_CHOOSE(4);
   else if (E <= 256) RL_CHOOSE(8);
   else if (E <= 512) RL_CHOOSE(16);
+  else if (E <= 768) RL_CHOOSE(24);
+  else if (E <= 1024) RL_CHOOSE(32);
   else RL_CHOOSE(48);
 #undef RL_CHOOSE
   return 0;

@@ -41,7 +41,7 @@ def test_plan(T, top, E, always, rows):
     assert not steps or max(steps) - min(steps) <= 1
 
 
-@pytest.mark.parametrize("E, top", [(1, 1), (31, 3), (32, 32), (33, 2), (64, 6), (65, 33), (128, 8), (200, 4), (256, 40), (512, 9), (600, 5), (1536, 2)])
+@pytest.mark.parametrize("E, top", [(1, 1), (31, 3), (32, 32), (33, 2), (64, 6), (65, 33), (128, 8), (200, 4), (256, 40), (512, 9), (600, 5), (1000, 7), (1536, 2)])
 @pytest.mark.parametrize("parts, gated, logistic, renorm", [(1, False, False, True), (3, True, True, False), (8, True, False, True)])
 def test_choice_from_partial_sums(E, top, parts, gated, logistic, renorm):
     """Scores are one exponential and one division off the oracle's: 1e-5 (the sum over E experts rounds 11 times at most); choices differ
