@@ -39,7 +39,9 @@ __global__ void embed_gather_kernel(const int* __restrict__ tokens, const TW* __
 
 // The same for the many rows of a prompt step: a thread takes up to PIECES pieces of eight numbers, all asked for before the first is stored, so
 // that an SM has twice the bytes on their way (2048 rows of 4096: 13 us instead of 15, of 2048: 7.0 instead of 8.4; memory's work is 8 and 4).
+// Rows of two whole rounds of the block gain nothing: 2048 of 8192 31 us instead of 29 (of 5120 22 instead of 25).
 #define EMBED_ROWS_MIN 64
+#define EMBED_ROWS_MAX_WIDTH 6144
 #define EMBED_THREADS 128
 template <int PIECES>
 __global__ void __launch_bounds__(EMBED_THREADS)
@@ -79,7 +81,7 @@ RL_API int rl_embed_gather(const int* tokens, const void* table, int table_dtype
                            int d, float scale, cudaStream_t stream) {
   if (n_tokens <= 0 || d <= 0) RL_REFUSE(1, "embed_gather: n_tokens=%d d=%d", n_tokens, d);
   const int th = row_threads(d);
-  if (table_dtype == RL_BF16 && d % 8 == 0 && n_tokens >= EMBED_ROWS_MIN && (((uintptr_t)table | (uintptr_t)out) & 15) == 0)
+  if (table_dtype == RL_BF16 && d % 8 == 0 && n_tokens >= EMBED_ROWS_MIN && d <= EMBED_ROWS_MAX_WIDTH && (((uintptr_t)table | (uintptr_t)out) & 15) == 0)
     RL_LAUNCH_CHECK(rl_launch(embed_gather_rows_kernel<4>, n_tokens, EMBED_THREADS, 0, stream, tokens, (const bf16*)table, out, d, scale));
   else if (table_dtype == RL_BF16 && d % 4 == 0)
     RL_LAUNCH_CHECK(rl_launch(embed_gather_kernel<bf16, true>, n_tokens, th, 0, stream, tokens, (const bf16*)table, out, d, scale));

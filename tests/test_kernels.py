@@ -134,6 +134,19 @@ def test_embed_gather(ops, dtype, d):
     assert torch.equal(out.cpu(), table[toks.long()].float())
 
 
+@pytest.mark.parametrize("T, d", [(63, 5120), (64, 8), (64, 4096), (65, 4104), (64, 5120), (70, 6144), (66, 6152), (130, 8200)])
+def test_embed_gather_of_many_rows(ops, T, d):
+    """The rows of prompt steps: 4096 numbers a round of the block, so whole rounds, a piece of a second one and one that only some threads have,
+    and wider rows and fewer, which another kernel takes."""
+    g = torch.Generator().manual_seed(T + d)
+    table = torch.randn(200, d, generator=g).to(torch.bfloat16)
+    table[3, d - 1], table[5, 0], table[5, d // 2] = float("nan"), float("inf"), float("-inf")
+    toks = torch.randint(0, 200, (T,), generator=g, dtype=torch.int32)
+    toks[:4] = torch.tensor([3, 199, 0, 5])
+    out = ops.embed_gather(toks.to(DEV), table.to(DEV), scale=0.375)
+    assert torch.equal(out.cpu().nan_to_num(7.0), (table[toks.long()].float() * 0.375).nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("d, parts", [(200, 0), (72, 1), (4104, 3), (201, 2)])
