@@ -95,12 +95,25 @@ struct Groups {
   const bf16* gate;    // SIGMOID
   long long ldg, gh;
   int N, K;
+  int matrices;        // matrices of w
+  int always;          // and how many more of other places: the plan's groups of higher numbers have theirs in map_s
+  int piece_first;     // whose dimensions go by their strides: [feature][piece][k] instead of [piece][feature][k]
   float act_alpha, act_limit;
+};
+
+// Matrices that take every token (a shared expert in pieces of the others' size), where they lie: feature n of the j-th at w + j * piece +
+// n * row, K numbers.  So rows of gate and up that alternate and columns of one wide matrix serve as they are, and no copy beside the
+// others is held.
+struct Always {
+  const bf16 *w, *w2;
+  long long row, piece;
+  int n;
 };
 
 template <typename TO, int EPI, int NT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
+                       const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_s2,
                        const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
                        const Groups g, int* __restrict__ status, int test_role, uint32_t test_ns) {
   using SH = Shape<NT>;
@@ -176,7 +189,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         int e, r0, rows;
         group(unit, e, r0, rows);
         if (rows <= 0) continue;
-        const int w_row = e * g.N + (unit % blocks_n) * UNIT_N;
+        const bool own = e < g.matrices || g.always == 0;
+        const int piece = e - g.matrices, w_row = (own ? e * g.N : 0) + (unit % blocks_n) * UNIT_N;
         const int w_row2 = EPI == GATED ? w_row : w_row + FEATURES / 2;
         for (int kb = 0; kb < n_k; ++kb, ++it) {
           if (it >= STAGES && !mbar_wait_role(&empty_bar[s], parity, ctl, 61)) {
@@ -186,8 +200,13 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             break;
           }
           mbar_expect_tx_s(full0 + 8 * s, A_BYTES);
-          tma_load_2d_s(dst, &map_w, full0 + 8 * s, kb * BK, w_row);
-          tma_load_2d_s(dst + A_BYTES / 2, &map_w2, full0 + 8 * s, kb * BK, w_row2);
+          if (own) {
+            tma_load_2d_s(dst, &map_w, full0 + 8 * s, kb * BK, w_row);
+            tma_load_2d_s(dst + A_BYTES / 2, &map_w2, full0 + 8 * s, kb * BK, w_row2);
+          } else {
+            tma_load_3d_s(dst, &map_s, full0 + 8 * s, kb * BK, g.piece_first ? piece : w_row, g.piece_first ? w_row : piece);
+            tma_load_3d_s(dst + A_BYTES / 2, &map_s2, full0 + 8 * s, kb * BK, g.piece_first ? piece : w_row2, g.piece_first ? w_row2 : piece);
+          }
           dst += SH::STAGE_BYTES;
           if (++s == STAGES) {
             s = 0;
@@ -416,14 +435,34 @@ static int make_rows_map(CUtensorMap* map, const Groups& g, int box_rows) {
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
 }
 
+// Boxes of 64 k x FEATURES / 2 features of a piece, the dimension of the smaller stride first.  0 on success.
+static int make_always_map(CUtensorMap* map, const bf16* w, const Always& a, int N, int K) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return 1;
+  const int at_n = a.piece < a.row ? 2 : 1, at_piece = 3 - at_n;
+  cuuint64_t dims[3] = {(cuuint64_t)K}, strides[2];
+  cuuint32_t box[3] = {BK}, estr[3] = {1, 1, 1};
+  dims[at_n] = (cuuint64_t)N, strides[at_n - 1] = (cuuint64_t)a.row * 2, box[at_n] = FEATURES / 2;
+  dims[at_piece] = (cuuint64_t)a.n, strides[at_piece - 1] = (cuuint64_t)a.piece * 2, box[at_piece] = 1;
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
+}
+
 template <typename TO, int EPI, int NT>
-static int launch_grouped(const void* w, const void* w2, int matrices, void* out, const Groups& g, long long max_groups, int* status,
+static int launch_grouped(const void* w, const void* w2, int matrices, void* out, Groups g, const Always& always, long long max_groups, int* status,
                           int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
   using SH = Shape<NT>;
-  CUtensorMap map_w, map_w2, map_x;
+  CUtensorMap map_w, map_w2, map_s, map_s2, map_x;
   const int rows = matrices * g.N;
+  g.matrices = matrices;
+  g.always = always.n;
+  g.piece_first = always.piece < always.row;
   if (make_matrix_map(&map_w, w, rows, g.K, g.K, FEATURES / 2) || make_matrix_map(&map_w2, EPI == GATED ? w2 : w, rows, g.K, g.K, FEATURES / 2))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices to TMA");
+  map_s = map_w;
+  map_s2 = map_w2;
+  if (always.n > 0 && (make_always_map(&map_s, always.w, always, g.N, g.K) || make_always_map(&map_s2, EPI == GATED ? always.w2 : always.w, always, g.N, g.K)))
+    RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices that take every token to TMA");
   if (g.order != nullptr ? make_matrix_map(&map_x, g.x, g.x_rows, g.K, (int)g.ldx, 1) : make_rows_map(&map_x, g, SH::BOX_ROWS))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the rows to TMA");
   auto kern = grouped_gemm_tc_kernel<TO, EPI, NT>;
@@ -434,7 +473,7 @@ static int launch_grouped(const void* w, const void* w2, int matrices, void* out
   const int unit_n = EPI == GATED ? FEATURES / 2 : FEATURES;
   const long long units = max_groups * ((g.N + unit_n - 1) / unit_n);
   if (units > 0x7fffffffLL) RL_REFUSE(11, "grouped_gemm_tc: too many units of work");
-  RL_LAUNCH_CHECK(rl_launch(kern, dim3((unsigned)(units < sms ? units : sms)), NUM_THREADS, SH::SMEM_BYTES, stream, map_w, map_w2, map_x, (TO*)out, g,
+  RL_LAUNCH_CHECK(rl_launch(kern, dim3((unsigned)(units < sms ? units : sms)), NUM_THREADS, SH::SMEM_BYTES, stream, map_w, map_w2, map_s, map_s2, map_x, (TO*)out, g,
                             status, wait_test_role, (uint32_t)wait_test_ns));
   return 0;
 }
@@ -481,14 +520,18 @@ RL_API int rl_moe_gather_rows(const void* x, int ldx, int x_rows, const int* ord
   return 0;
 }
 
-// tile_rows: the height of the plan's row tiles, 32, 128 or 256.  n_experts: matrices in w (and w2).
+// tile_rows: the height of the plan's row tiles, 32, 128 or 256.  n_experts: matrices in w (and w2).  always: how many more the plan has, which
+// take every token: feature n of the j-th at ws (ws2) + j * ws_piece + n * ws_row.
 RL_API int rl_moe_gemm_tc(const void* x, int ldx, int x_rows, const int* order, int gather_div, const void* w, const void* w2, void* out, int out_dtype,
                           int ldo, const int* tiles, int max_tiles, int tile_rows, int n_experts, int N, int K, float act_alpha, float act_limit,
-                          int* status, int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
+                          const void* ws, const void* ws2, long long ws_row, long long ws_piece, int always, int* status, int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
   if (max_tiles <= 0 || N <= 0 || K <= 0 || gather_div <= 0 || n_experts <= 0 || x_rows <= 0)
     RL_REFUSE(1, "moe_gemm_tc: tiles=%d experts=%d N=%d K=%d div=%d", max_tiles, n_experts, N, K, gather_div);
   if (status == nullptr || tiles == nullptr) RL_REFUSE(2, "moe_gemm_tc: no status word or no plan");
   if (int rc = refuse_operands("moe_gemm_tc", x, ldx, 0, w, w2, n_experts, N, K)) return rc;
+  if (always < 0 || (always > 0 && (ws == nullptr || (ws2 == nullptr) != (w2 == nullptr) || ws_row < K || ws_piece <= 0 || ws_row % 8 || ws_piece % 8 || (((uintptr_t)ws | (uintptr_t)ws2) & 15))))
+    RL_REFUSE(12, "moe_gemm_tc: %d matrices that take every token, rows %lld and pieces %lld apart", always, ws_row, ws_piece);
+  const Always more = {(const bf16*)ws, (const bf16*)ws2, ws_row, ws_piece, always};
   Groups g = {};
   g.x = (const bf16*)x;
   g.ldx = ldx;
@@ -501,7 +544,7 @@ RL_API int rl_moe_gemm_tc(const void* x, int ldx, int x_rows, const int* order, 
   g.K = K;
   g.act_alpha = act_alpha;
   g.act_limit = act_limit;
-#define RL_GROUPED(TO, EPI, NT) return launch_grouped<TO, EPI, NT>(w, w2, n_experts, out, g, max_tiles, status, wait_test_role, wait_test_ns, stream)
+#define RL_GROUPED(TO, EPI, NT) return launch_grouped<TO, EPI, NT>(w, w2, n_experts, out, g, more, max_tiles, status, wait_test_role, wait_test_ns, stream)
 #define RL_GROUPED_ROWS(TO, EPI)               \
   do {                                         \
     if (tile_rows == 32) RL_GROUPED(TO, EPI, 32);   \
@@ -542,6 +585,6 @@ RL_API int rl_head_linear_tc(const void* x, int ldx, int xh, const void* w, void
   g.held = held;
   g.seq_rows = seq_rows;
   const long long groups = (long long)H * (held != nullptr ? M / seq_rows * ((seq_rows + 255) / 256) : (M + 255) / 256);
-  if (gate != nullptr) return launch_grouped<bf16, SIGMOID, 256>(w, nullptr, H, out, g, groups, status, wait_test_role, wait_test_ns, stream);
-  return launch_grouped<bf16, PLAIN, 256>(w, nullptr, H, out, g, groups, status, wait_test_role, wait_test_ns, stream);
+  if (gate != nullptr) return launch_grouped<bf16, SIGMOID, 256>(w, nullptr, H, out, g, Always{}, groups, status, wait_test_role, wait_test_ns, stream);
+  return launch_grouped<bf16, PLAIN, 256>(w, nullptr, H, out, g, Always{}, groups, status, wait_test_role, wait_test_ns, stream);
 }

@@ -1435,13 +1435,16 @@ def moe_plan(ids: torch.Tensor, n_experts: int, tile_rows: int = 0, always: int 
 def moe_gemm(
     x: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, max_tiles: int, n_rows: int, order: Optional[torch.Tensor] = None,
     gather_div: int = 1, w2: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None, tile_rows: int = 0, act=None,
+    always: Optional[torch.Tensor] = None, always2: Optional[torch.Tensor] = None,
 ) -> torch.Tensor:
     """out[r] = w[expert of r] . x[row of r] for the n_rows rows of a plan's layout; w: [E, N, K].
 
     order given: row r reads x[order[r] // gather_div], else x[r].  w2 given: out = silu(w x) * (w2 x), or with act = (alpha, limit)
     g s(alpha g) (u + 1), g = min(w x, limit), u = clamp(w2 x, -limit, limit).  Without w2, act "relu2": out = relu(w x)^2.
     tile_rows: the height of the plan's tiles; bfloat16 operands whose rows can be moved in 16-byte pieces go to the
-    tensor cores if it is one of MOE_MMA_TILE_ROWS, everything else to the plain kernel (which wants its own height)."""
+    tensor cores if it is one of MOE_MMA_TILE_ROWS, everything else to the plain kernel (which wants its own height).
+    always (always2 beside w2): [n, N, K], the matrices of a plan of so many that take every token; rows and matrices any multiple of 8 apart
+    (a view of weights that lie in another order).  The tensor-core product only."""
     _cuda(x, "moe_gemm x", contiguous=False)
     _cuda(w, "moe_gemm w", x.dtype)
     if not (w.dim() == 3 and w.shape[2] == x.shape[1]):
@@ -1450,6 +1453,15 @@ def moe_gemm(
     if w2 is not None:
         _cuda(w2, "moe_gemm w2", x.dtype)
         _need(tuple(w2.shape) == (E, N, K), "moe_gemm: w2 does not match w")
+    more, ws_row, ws_piece = 0, 0, 0
+    if always is not None:
+        _cuda(always, "moe_gemm always", x.dtype, contiguous=False)
+        if not (always.dim() == 3 and tuple(always.shape[1:]) == (N, K) and always.stride(2) == 1 and (always2 is None) == (w2 is None)):
+            raise KernelError(f"moe_gemm: always {tuple(always.shape)} does not match w {tuple(w.shape)}")
+        more, (ws_piece, ws_row, _) = always.shape[0], always.stride()
+        if always2 is not None:
+            _cuda(always2, "moe_gemm always2", x.dtype, contiguous=False)
+            _need(always2.shape == always.shape and always2.stride() == always.stride(), "moe_gemm: always2 does not lie as always does")
     out_dtype = out_dtype or x.dtype
     out = _empty(x, out_dtype, n_rows, N)
     tile_rows = tile_rows or moe_tile_rows()
@@ -1457,19 +1469,20 @@ def moe_gemm(
     alpha, limit = _act(act)
     if x.dtype == torch.bfloat16 and tile_rows in MOE_MMA_TILE_ROWS and grouped_gemm_takes(K, x.stride(0), 0) and (x.data_ptr() | w.data_ptr()) % 16 == 0:
         lib = library("grouped_gemm_tc")
-        if order is not None and n_rows >= MOE_GATHER_ROWS_PER_EXPERT * E:
+        if order is not None and n_rows >= MOE_GATHER_ROWS_PER_EXPERT * (E + more):
             rows = _empty(x, x.dtype, n_rows, K)
             rc = lib.rl_moe_gather_rows(x, x.stride(0), x.shape[0], order, gather_div, rows, n_rows, K, _stream())
             _check(lib, rc, "moe_gather_rows")
             x, order = rows, None
         rc = lib.rl_moe_gemm_tc(
             x, x.stride(0), x.shape[0], order, gather_div, w, w2, out, _dt(out, "moe_gemm out"), N,
-            tiles, max_tiles, tile_rows, E, N, K, alpha, limit, _tc_status_word(x.device), *_wt(), _stream(),
+            tiles, max_tiles, tile_rows, E, N, K, alpha, limit, always, always2, ws_row, ws_piece, more, _tc_status_word(x.device), *_wt(), _stream(),
         )
         _check(lib, rc, "moe_gemm_tc")
         return out
     if tile_rows != moe_tile_rows():
         raise KernelError(f"moe_gemm: the plain kernel wants tiles of {moe_tile_rows()} rows, the plan has {tile_rows}")
+    _need(always is None, "moe_gemm: the plain kernel has no matrices that take every token")
     lib = library("moe")
     rc = lib.rl_moe_gemm(
         x, _rows(x, "moe_gemm x"), _dt(x, "moe_gemm"), order, gather_div, w, w2, out,

@@ -130,14 +130,6 @@ class RoutedExperts(FeedForward):
             exact = self.rt.dtype == torch.bfloat16 and self.d % 8 == 0 and torch.equal(narrow.to(torch.float32), self.w_router)
             self.w_router16 = narrow if exact else None
         self.bias = tensors[self.prefix + self.names["bias"]].contiguous() if self.has_bias else None
-        # A shared expert of a multiple of the others' size is that many experts more that take every token: for steps that `_joins` names
-        # its matrices stand behind the others', too.
-        self.always = 0
-        if self.shared_ff and self.shared_ff % self.ff == 0 and self.rt.dtype == torch.bfloat16 and self.d % 8 == 0 and self.ff % 8 == 0:
-            n = self.always = self.shared_ff // self.ff
-            self.w_gate = torch.cat([self.w_gate, tensors[self._shared("gate")].view(n, self.ff, self.d)])
-            self.w_up = torch.cat([self.w_up, tensors[self._shared("up")].view(n, self.ff, self.d)])
-            self.w_down = torch.cat([self.w_down, tensors[self._shared("down")].view(self.d, n, self.ff).transpose(0, 1)])
         if self.shared_ff:
             gate, up = tensors[self._shared("gate")], tensors[self._shared("up")]
             self.shared_fused = self.rt.dtype == torch.bfloat16
@@ -146,6 +138,15 @@ class RoutedExperts(FeedForward):
             else:
                 self.ws_gate_up = torch.cat([gate, up], dim=0).contiguous()
             self.ws_down = tensors[self._shared("down")].contiguous()
+        # A shared expert of a multiple of the others' size is that many experts more that take every token, in steps that `_joins` names: views
+        # of its matrices, gate and up of alternating rows, down of neighbouring columns.
+        self.always = 0
+        if (self.shared_ff and self.shared_ff % self.ff == 0 and self.rt.dtype == torch.bfloat16 and self.d % 8 == 0 and self.ff % 8 == 0
+                and self.ws_down.data_ptr() % 16 == 0):
+            n = self.always = self.shared_ff // self.ff
+            both = self.ws_gate_up.view(n, self.ff, 2, self.d)
+            self.always_gate, self.always_up = both[:, :, 0], both[:, :, 1]
+            self.always_down = self.ws_down.view(self.d, n, self.ff).transpose(0, 1)
 
     def forward(self, xn: torch.Tensor, step) -> torch.Tensor:
         T = xn.shape[0]
@@ -166,10 +167,11 @@ class RoutedExperts(FeedForward):
         order, place, tiles, max_tiles = ops.moe_plan(ids, self.E, tile_rows, always)
         n_rows = T * (self.top + always)
         if self.gated:
-            h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, n_rows, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act)
+            more = dict(always=self.always_gate, always2=self.always_up) if always else {}
+            h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, n_rows, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act, **more)
         else:
             h = ops.moe_gemm(xn, self.w_up, tiles, max_tiles, n_rows, order=order, gather_div=self.top, tile_rows=tile_rows, act="relu2")
-        y = ops.moe_gemm(h, self.w_down, tiles, max_tiles, n_rows, out_dtype=torch.float32, tile_rows=tile_rows)
+        y = ops.moe_gemm(h, self.w_down, tiles, max_tiles, n_rows, out_dtype=torch.float32, tile_rows=tile_rows, always=self.always_down if always else None)
         shared = None
         if self.shared_ff and not always:
             if self.shared_fused:

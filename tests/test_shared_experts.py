@@ -113,18 +113,18 @@ def test_part(T, shared_ff, gated):
     assert float((got - want).norm() / want.norm()) <= 8e-3
 
 
-@pytest.mark.parametrize("d", [128, 136])
-@pytest.mark.parametrize("shared_ff, gated", [(64, False), (192, True)])
-def test_a_shared_experts_way_does_not_show(d, shared_ff, gated, monkeypatch):
+@pytest.mark.parametrize("d, ff", [(128, 64), (136, 64), (64, 200), (328, 72)])  # (whole tiles of features and slices of k, and parts of them)
+@pytest.mark.parametrize("pieces, gated", [(1, False), (3, True)])
+def test_a_shared_experts_way_does_not_show(d, ff, pieces, gated, monkeypatch):
     """The same tokens with the shared expert's rows in the experts' products and in products of their own.  Both round its result to
     bfloat16; their 32-bit sums differ by some 2^-22, which puts one number in 2^13 on the other side of a rounding, 2^-8 off: 5e-5 in
     all, twice that allowed.  (Unrounded on one of the ways it is 1e-3.)"""
     from rusty_llama_b200.parts import FEED_FORWARDS, Runtime
     from rusty_llama_b200.spec import PartSpec
 
-    part = FEED_FORWARDS.build(PartSpec("routed_experts", {"hidden_size": d, "n_experts": 6, "top": 2, "expert_ff": 64, "bias": False, "renormalize": True,
-                                                           "shared_ff": shared_ff, "shared_gate": gated}), Runtime.create(DEV, torch.bfloat16))
-    g = torch.Generator().manual_seed(shared_ff + d)
+    part = FEED_FORWARDS.build(PartSpec("routed_experts", {"hidden_size": d, "n_experts": 6, "top": 2, "expert_ff": ff, "bias": False, "renormalize": True,
+                                                           "shared_ff": pieces * ff, "shared_gate": gated}), Runtime.create(DEV, torch.bfloat16))
+    g = torch.Generator().manual_seed(pieces + d)
     w = {}
     for name, info in part.param_infos().items():
         t = (torch.randn(info.shape, generator=g) * info.shape[-1] ** -0.5).to(torch.bfloat16)
