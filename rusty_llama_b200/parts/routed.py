@@ -185,10 +185,13 @@ class RoutedExperts(FeedForward):
 
     def _joins(self, T: int) -> bool:
         """Whether a shared expert's rows go through the experts' two products: where both stream weights, which two launches less and one tail
-        instead of three help (a part alone, us: 64 experts of 1408 x 2048 and two more, 64 tokens 222 instead of 245, 16 tokens 173 instead of
-        198; 32 of 2048 x 4096 and one, 96 tokens 312 instead of 332, 8 tokens 202 instead of 209).  One token has too few tiles for that (64 and 92
-        instead of 59 and 80), and many tokens' products of one matrix are dense ones, where the prompt product is the faster kernel (1400 and
-        2048 tokens: level)."""
+        instead of three help.  A part alone, us, joined and apart, from 8 tokens to the border's 64 rows an expert:
+            tokens                                     8          64         256         512     682
+            16 experts of 1024 x 1024, 2 a token     53  63     60  80     68  85      80  90
+            64 of 1408 x 2048, 6, a shared one of 2 144 150    235 255    252 267     265 277  277 290
+            32 of 2048 x 4096, 4                    217 232    324 331    351 355     378 380
+        One token has too few tiles for that (64 and 92 instead of 59 and 80), and many tokens' products of one matrix are dense ones, where the
+        prompt product is the faster kernel (1024 tokens at the last sizes 450 and 438)."""
         return T >= 8 and T * self.top <= 64 * self.E
 
     def _logits(self, xn: torch.Tensor) -> torch.Tensor:
