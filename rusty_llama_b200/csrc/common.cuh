@@ -97,16 +97,17 @@ __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
-// x / d for d >= 1, infinities and NaN as the division's and the last digit too (but for quotients below the normal numbers): the hardware's
-// reciprocal, of a quarter of d so that it is a normal number, a product and one correction by the remainder (Newton's step for the
-// quotient).  The division itself branches where a quotient might be out of range, and a branch in each of a thread's many logistic functions
-// keeps them from overlapping: x / (1 + exp(-x)) takes a warp alone 104 clocks with it and 39 so, an SM's 16 warps 32 and 21 each.
+// x / d for d >= 1, infinities and NaN as the division's: the hardware's reciprocal, of a quarter of d so that it is a normal number, a
+// product and one correction by the remainder (Newton's step for the quotient).  A normal quotient is at most one unit in its last place
+// from the division's: 30 of 1.2e10 random pairs were, and no 1 / d of all d in nine of the exponents.  The division itself branches
+// where a quotient might be out of range, and a branch in each of a thread's many logistic functions keeps them from overlapping:
+// x / (1 + exp(-x)) takes a warp alone 104 clocks with it and 39 so, an SM's 16 warps 32 and 21 each.
 __device__ __forceinline__ float divide_by_1up(float x, float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d * 0.25f));
   r *= 0.25f;
   const float near = x * r, q = fmaf(-fmaf(d, near, -x), r, near);
-  return d < 3e38f && fabsf(x) < 3e38f ? q : near;  // (the remainder of an infinity is no number)
+  return d <= 3.402823466e38f && fabsf(x) < 3e38f ? q : near;  // (the remainder of an infinity is no number)
 }
 __device__ __forceinline__ float logistic_no_branch(float x) { return divide_by_1up(1.0f, 1.0f + expf(-x)); }
 
