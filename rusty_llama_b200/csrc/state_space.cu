@@ -504,42 +504,21 @@ scalar_chunk_out_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, 
 #pragma unroll
         for (int e = 0; e < 4; ++e) inter[4 * part + j][e] = t4 < 2 ? both[2 * j][e] : both[2 * j + 1][e];
     }
-  } else {
-  for (int pass = 0; pass < 2; ++pass) {
+  } else {  // (rows that are no whole fours)
+    for (int pass = 0; pass < 2; ++pass) {
       __syncthreads();  // the keys and values (or the first half) are no longer read
-      if ((vdim & 3) == 0) {  // four numbers a load, four loads in flight
-  #pragma unroll 4
-        for (int idx = tid; idx < HDK * (HDV / 4); idx += 128) {
-          const int r = idx / (HDV / 4), cc = 4 * (idx - r * (HDV / 4));
-          float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (r < dim && cc < vdim) t = __ldcg(reinterpret_cast<const float4*>(sp + (size_t)r * vdim + cc));
-          const float f[4] = {t.x, t.y, t.z, t.w};
-          bf16 o[4];
-  #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            bf16 hi, lo;
-            sc_split(f[e], hi, lo);
-            o[e] = pass == 0 ? hi : lo;
-          }
-          uint2 raw;
-          raw.x = sc_pack(o[0], o[1]);
-          raw.y = sc_pack(o[2], o[3]);
-          *reinterpret_cast<uint2*>(st_s + r * VS + cc) = raw;
-        }
-      } else {
-        for (int idx = tid; idx < HDK * HDV; idx += 128) {
-          const int r = idx / HDV, cc = idx - r * HDV;
-          bf16 hi = __float2bfloat16_rn(0.f), lo = hi;
-          if (r < dim && cc < vdim) sc_split(__ldcg(sp + (size_t)r * vdim + cc), hi, lo);
-          st_s[r * VS + cc] = pass == 0 ? hi : lo;
-        }
+      for (int idx = tid; idx < HDK * HDV; idx += 128) {
+        const int r = idx / HDV, cc = idx - r * HDV;
+        bf16 hi = __float2bfloat16_rn(0.f), lo = hi;
+        if (r < dim && cc < vdim) sc_split(__ldcg(sp + (size_t)r * vdim + cc), hi, lo);
+        st_s[r * VS + cc] = pass == 0 ? hi : lo;
       }
       __syncthreads();
-  #pragma unroll
+#pragma unroll
       for (int kk = 0; kk < HDK / 16; ++kk) {
         uint32_t a[4];
         sc_ldmatrix_x4(a, qa + kk * 16);
-  #pragma unroll
+#pragma unroll
         for (int dp = 0; dp < HDV / 16; ++dp) {
           uint32_t b[4];
           sc_ldmatrix_x4_trans(b, st_s + (size_t)(kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * VS + dp * 16 + 8 * (lane >> 4));
