@@ -186,3 +186,30 @@ def test_a_step_without_room_for_the_rows_works_on_the_latents():
     assert part._expands(step, torch.empty(1, 8, device=DEV, dtype=torch.bfloat16), None)
     scratch = 2 * (held + n) * (16 * 320 + 512)
     assert torch.equal(with_memory_left(scratch - (8 << 20), run), want)
+
+
+@pytest.mark.parametrize("vdim", [8, 64, 72, 128])
+def test_output_gates_of_every_size(vdim):
+    """The gate beside whole row blocks, short ones and one of a single row: logistic functions of large gates, of infinite ones and of what is no
+    number, which stays in its place.  Against the same without a gate, whose result is rounded too: 2^-8 of it at most, twice."""
+    from rusty_llama_b200.kernels import ops
+
+    lens, H, rows = [128, 33, 129, 1], 2, 192
+    T, dim = sum(lens), 64
+    g = torch.Generator().manual_seed(vdim)
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    kv = torch.randn(rows * len(lens), H, dim + vdim, generator=g).to(torch.bfloat16).to(DEV)
+    q = torch.randn(T, H * dim, generator=g).to(torch.bfloat16).to(DEV)
+    gate = torch.randn(T, H * vdim + 8, generator=g) * 4
+    for value in (float("inf"), float("-inf"), float("nan"), 100.0, -100.0, -80.0):
+        gate.view(-1)[torch.randperm(gate.numel(), generator=g)[:40]] = value
+    gate[starts[2] - 1, 0], gate[T - 1, vdim - 1] = float("nan"), float("-inf")
+    gate = gate.to(torch.bfloat16).to(DEV)[:, : H * vdim]
+    args = (q, kv, rows, i32(starts), i32([0] * len(lens)), max(lens), vdim, 0, dim ** -0.5)
+    plain, got = ops.flash_expanded(*args).double(), ops.flash_expanded(*args, gate=gate).double()
+    want = plain * torch.sigmoid(gate.double())
+    assert torch.equal(got.isnan(), want.isnan())
+    assert bool(((got - want).abs() <= want.abs() * (2.0 ** -7 * 1.01) + 1e-38)[~want.isnan()].all())
