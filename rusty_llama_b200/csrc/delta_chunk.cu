@@ -620,7 +620,6 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const bf16* __restrict__ K,
   float* s_s = reinterpret_cast<float*>(p_s + 3 * SPL_TRI_BYTES);  // [DP][LS]
   float* u_s = s_s;                                           // [64][LU]
   __shared__ double L[DC];
-  __shared__ __align__(16) float ss[DC * 8];
   pdl_trigger();
   pdl_wait();
   const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z % n_seqs, col0 = blockIdx.z / n_seqs * 128, kh = h / (H / G), tid = threadIdx.x;
@@ -726,7 +725,7 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const bf16* __restrict__ K,
       }
     }
   }
-  spl_finish(acc, ss, n, t0, h, vdim, col0, out, out_stride, norm);
+  spl_finish(acc, reinterpret_cast<float*>(dc_smem), n, t0, h, vdim, col0, out, out_stride, norm);
 }
 
 // ---------------------------------------------------------------- host side
@@ -790,7 +789,8 @@ RL_API int rl_delta_chunked(const float* qn, const float* kn, const void* v, int
   if (v_stride < H * vdim || out_stride < H * vdim) RL_REFUSE(5, "delta_chunked: rows of %d and %d for %d values", v_stride, out_stride, H * vdim);
   if (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)state | (uintptr_t)scratch) & 15) RL_REFUSE(6, "delta_chunked: operands must be 16-byte aligned");
   if (!norm_w && (out_stride % 4 || ((uintptr_t)out & 15))) RL_REFUSE(6, "delta_chunked: the result's rows must be 16-byte aligned");
-  if (norm_w && (vdim > 128 || out_stride % 2 || ((uintptr_t)out & 3) || gate_stride % 2 || ((uintptr_t)gate & 3) || ((uintptr_t)norm_w & 7)))
+  // (rows of whole fours: a step with sequences of a few tokens has the norm made by head_norm_gate, four columns a lane, and the bits are the same)
+  if (norm_w && (vdim > 128 || out_stride % 4 || ((uintptr_t)out & 7) || gate_stride % 4 || ((uintptr_t)gate & 7) || ((uintptr_t)norm_w & 7)))
     return RL_NOT_FUSED;
   const SplNorm norm{norm_w, eps, (const bf16*)gate, gate_stride, gate_act, out_scale};
   if (dim <= 64)

@@ -161,7 +161,7 @@ __device__ __forceinline__ float gm_sum8(float (&s)[8], int lane) {
 // columns, so that the state, split as it is read, is split once.  Scores and queries are kept as their three parts and come by ldmatrix;
 // the queries' parts take the place of the sums and the scores, the state's halves (eight columns of every warp) that of q and k.
 // With a norm the heads' norm and gate are applied before the result leaves (the sums of squares meet in shared memory): a pass over
-// 32-bit rows less than head_norm_gate behind it, whose arithmetic this is.
+// 32-bit rows less than head_norm_gate behind it, with the same bits.
 // Bound: of a block's 42000 cycles (two share the SM, in step) the loads take 7000, the scores 15000 (exponentials and splits: issue slots)
 // and the outputs 16000, which is what the tensor cores' legacy instruction takes there (4320 a block, 3072 of them the queries against the
 // state).  With operands split by every warp that reads them, from 32-bit tiles of 64 columns, it was 65 us instead of 58.
@@ -201,7 +201,7 @@ gated_mma_out_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, con
   unsigned char* p_s = gm_smem + L::X + L::SUMS;                   // [3][10 tiles]: the scores' parts
   bf16* qp_s = reinterpret_cast<bf16*>(gm_smem + L::X);            // [3][GC][LP]: the decayed queries' parts, later
   bf16* v_s = reinterpret_cast<bf16*>(gm_smem + L::X + L::MIDDLE); // [GC][LV]
-  __shared__ __align__(16) float2 tot[D::PARTS][D::PAIRS];         // later the sums of squares [8][GC]
+  __shared__ __align__(16) float2 tot[D::PARTS][D::PAIRS];
   pdl_trigger();
   pdl_wait();
   const int s = blockIdx.x / H, h = blockIdx.x % H, c = blockIdx.y, qh = h / (H / QH);
@@ -394,7 +394,7 @@ gated_mma_out_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, con
       }
     }
   }
-  spl_finish(acc, reinterpret_cast<float*>(&tot[0][0]), n, t0, h, vdim, 0, out, out_stride, norm);
+  spl_finish(acc, reinterpret_cast<float*>(gm_smem), n, t0, h, vdim, 0, out, out_stride, norm);
 }
 
 // Sizes and addresses that these kernels take: rows in whole 16-byte pieces, keys and values up to 128.  (That the state's, the scratch's and the

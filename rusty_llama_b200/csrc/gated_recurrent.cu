@@ -1009,7 +1009,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ x, int x_stride,
 #pragma unroll
     for (int j = 0; j < V; ++j) {
       vals[e][j] *= inv_den;
-      ss += vals[e][j] * vals[e][j];
+      ss = fmaf(vals[e][j], vals[e][j], ss);  // (spl_finish has the same sums in the same order)
     }
   }
   const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)n + eps);

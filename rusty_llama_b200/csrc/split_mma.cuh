@@ -149,7 +149,9 @@ __device__ __forceinline__ void spl_rows_a(SplA& a, const float* at, int ld) {
 
 // The end of a chunk of 64 tokens and a head of up to 128 values: warp w of eight has the sums of columns 16 w + 8 half + 2 t (and one on) of
 // tokens 32 mm + 16 m + g and + 8 as acc[half][mm][m][0].  Without `w` they leave as float32 rows; with it they go through the head's
-// norm and gate (what head_norm_gate does) and leave as bfloat16.  ss: 64 x 8 floats of shared memory.
+// norm and gate and leave as bfloat16, with the arithmetic of head_norm_gate in the order that it has for rows of whole fours (a lane has four
+// neighbouring columns, whose squares are a chain, and the lanes' sums meet pairwise from the farthest apart): a row has the same bits
+// whichever of the two makes it.  ss: 64 x 32 floats of shared memory that nobody uses any more once all threads are here.
 #define RL_NOT_FUSED (-20)  // what a launcher answers, before it launches anything, where it cannot take the norm along
 struct SplNorm {
   const float* w;  // [vdim]
@@ -178,20 +180,25 @@ __device__ __forceinline__ void spl_finish(const float (&acc)[2][2][2][1][4], fl
     }
     return;
   }
+  __syncthreads();
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float v2 = 0.f;
+    for (int e = 0; e < 2; ++e)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const float(&y)[4] = acc[half][m >> 1][m & 1][0];
-        v2 += y[2 * e] * y[2 * e] + y[2 * e + 1] * y[2 * e + 1];
+        const float first = fmaf(y[2 * e + 1], y[2 * e + 1], __fmul_rn(y[2 * e], y[2 * e]));  // the even lanes': their four's first two
+        const float before = __shfl_xor_sync(0xffffffffu, first, 1);
+        const float four = fmaf(y[2 * e + 1], y[2 * e + 1], fmaf(y[2 * e], y[2 * e], before));
+        if (t & 1) ss[((2 * half + (t >> 1)) * 8 + warp) * 64 + 16 * m + 8 * e + g] = four;
       }
-      v2 += __shfl_xor_sync(0xffffffffu, v2, 1);
-      v2 += __shfl_xor_sync(0xffffffffu, v2, 2);
-      if (t == 0) ss[(16 * m + 8 * e + g) * 8 + warp] = v2;
-    }
+  __syncthreads();
+  {
+    float* at = ss + (threadIdx.x >> 6) * 8 * 64 + (threadIdx.x & 63);  // one of a row's four places in its 16 columns, of all warps
+    const float s0 = at[0] + at[4 * 64], s1 = at[64] + at[5 * 64], s2 = at[2 * 64] + at[6 * 64], s3 = at[3 * 64] + at[7 * 64];
+    at[0] = (s0 + s2) + (s1 + s3);
+  }
   __syncthreads();
   float2 w[2];
 #pragma unroll
@@ -205,8 +212,8 @@ __device__ __forceinline__ void spl_finish(const float (&acc)[2][2][2][1][4], fl
     for (int e = 0; e < 2; ++e) {
       const int i = 16 * m + 8 * e + g;
       if (i >= n) continue;
-      const float4 s0 = *reinterpret_cast<const float4*>(ss + i * 8), s1 = *reinterpret_cast<const float4*>(ss + i * 8 + 4);
-      const float inv = 1.0f / sqrtf((((s0.x + s0.y) + (s0.z + s0.w)) + ((s1.x + s1.y) + (s1.z + s1.w))) / (float)vdim + norm.eps);
+      const float sum = (ss[i] + ss[16 * 64 + i]) + (ss[8 * 64 + i] + ss[24 * 64 + i]);
+      const float inv = 1.0f / sqrtf(sum / (float)vdim + norm.eps);
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int col = 16 * warp + 8 * half + 2 * t;

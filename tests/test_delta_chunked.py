@@ -308,3 +308,68 @@ def test_the_norm_taken_along(dim, vdim):
     assert got.dtype == torch.bfloat16 and float(((got.float() - want.float()).abs() / (want.float().abs() + 1e-3)).max()) <= 2.0 ** -7
     assert float((got != want).float().mean()) <= 0.01
     assert run((w, 1e-5, gate, ops.GATE_SILU, 0.5, torch.empty(T, H * vdim + 1, dtype=torch.bfloat16, device=DEV)[:, 1:])) is None
+
+
+def _layer(seed=0):
+    from rusty_llama_b200.parts import MIXERS, Runtime
+    from rusty_llama_b200.spec import PartSpec
+
+    part = MIXERS.build(PartSpec("gated_delta", {"hidden_size": 64, "num_heads": 4, "num_qk_heads": 2, "dim": 32, "vdim": 48, "taps": 4, "eps": 1e-5}), Runtime.create(DEV, torch.bfloat16))
+    g = torch.Generator().manual_seed(seed)
+    w = {}
+    for name, info in part.param_infos().items():
+        t = torch.randn(info.shape, generator=g) * (0.2 if len(info.shape) > 1 else 0.5) + (1.0 if name == "norm" else 0.0)
+        w[name] = (t if info.kind == "scalars" else t.to(torch.bfloat16)).to(DEV)
+    part.load(w)
+    return part
+
+
+def _rows(part, lens, xs):
+    """The layer's rows, before the output projection, of sequences that share one step, and the records' states behind it."""
+    from rusty_llama_b200.cache import Cache
+
+    from test_parts import ctx_for
+
+    cache = Cache([(0, part.cache_need())], 64 * 16, len(lens), torch.bfloat16, DEV)
+    slots = [cache.open_sequence() for _ in lens]
+    step, tables = ctx_for(cache, slots, [0] * len(lens), lens)
+    view = cache.view(0, tables)
+    a, _ = part.forward_unprojected(torch.cat(xs), step, view)
+    return list(a.split(lens)), [view[0].state[s].clone() for s in slots]
+
+
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (36, 72), (64, 20), (100, 4)])
+def test_the_norm_taken_along_has_the_same_bits(dim, vdim):
+    from rusty_llama_b200.kernels import ops
+
+    lens, H, G = [130, 40], 2, 1
+    q, k, v, beta, logd = inputs(lens, H, G, dim, vdim, 12, "usual")
+    T, g = sum(lens), torch.Generator().manual_seed(3)
+    rows = torch.randn(T, H * vdim + 4, generator=g).to(torch.bfloat16).to(DEV)
+    w = torch.randn(vdim, generator=g).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    scratch = torch.empty(ops.delta_chunked_scratch_floats(T, 2, H, dim, vdim), device=DEV)
+
+    def run(norm):
+        return ops.delta_chunked(q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV), v.reshape(T, -1).to(DEV), beta.to(DEV), logd.to(DEV),
+                                 torch.zeros(2, H, dim, vdim, device=DEV), i32([0, 1]), i32([0, 130, 170]), H, G, dim, vdim, 130, scratch, norm=norm)
+
+    plain = run(None)
+    for gate in (None, rows[:, 4:]):
+        for act in (ops.GATE_NONE, ops.GATE_SIGMOID, ops.GATE_SILU):
+            assert torch.equal(run((w, 1e-5, gate, act, 0.3, None)), ops.head_norm_gate(plain, H, vdim, w, 1e-5, gate, act, torch.bfloat16, out_scale=0.3))
+
+
+def test_a_prompts_bits_do_not_depend_on_its_company():
+    """A prompt alone, whose norm is in the last of the chunks' kernels, and beside sequences of few tokens, where it is a kernel of its own; and those
+    few tokens, which keep to the kernels of single tokens and come out as they do beside another prompt."""
+    part = _layer()
+    g = torch.Generator().manual_seed(1)
+    x = {n: torch.randn(n, 64, generator=g).to(torch.bfloat16).to(DEV) for n in (100, 5, 31, 200, 1)}
+    (want,), (want_S,) = _rows(part, [100], [x[100]])
+    (_, few), (_, few_S) = _rows(part, [200, 5], [x[200], x[5]])
+    for lens in ([100, 5], [5, 100], [31, 100, 1, 5], [200, 5, 100], [100, 200]):
+        got, got_S = _rows(part, lens, [x[n] for n in lens])
+        assert torch.equal(got[lens.index(100)], want) and torch.equal(got_S[lens.index(100)], want_S), lens
+        if 5 in lens:
+            assert torch.equal(got[lens.index(5)], few) and torch.equal(got_S[lens.index(5)], few_S), lens
