@@ -25,9 +25,13 @@ RL_DEFINE_ERROR_TEXT()
 
 #define DC 64  // tokens per chunk
 
-// Chunks are numbered over the whole call: those of sequence s start at seq_start[s] / 64 + s (room for every sequence's last, partly
-// filled one).
-__device__ __forceinline__ int dc_first_chunk(int start, int s) { return start / DC + s; }
+// The chunks that one go of the three steps works on, and their places in the scratch.  All of them at once (count 0): those of sequence s
+// start at seq_start[s] / 64 + s (room for every sequence's last, partly filled one).  Where the scratch is smaller, `count` of every sequence at
+// a time, from its chunk `first` on: the state goes from one go to the next in the sequences' records, the same 32 bits as in registers.
+struct DcWindow {
+  int first, count;
+};
+__device__ __forceinline__ int dc_chunk(const DcWindow& w, int start, int s, int c) { return w.count ? s * w.count + c - w.first : start / DC + s + c; }
 
 // Running sums of 64 log decays (zero past the chunk's last token) by one warp, two to a lane.  In 64 bits: what is used of them are
 // differences, and those of fast decays are small beside the sums.  A log decay may be minus infinity, whose differences are no numbers:
@@ -237,7 +241,7 @@ template <int DP>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_solve_kernel(const float* __restrict__ kn, const bf16* __restrict__ v, int v_stride, int v_wide, const float* __restrict__ beta,
                          const float* __restrict__ log_decay, const int* __restrict__ seq_start, bf16* __restrict__ W, bf16* __restrict__ K,
-                         float* __restrict__ U, float* __restrict__ tails, int H, int G, int dim, int vdim, int min_len) {
+                         float* __restrict__ U, float* __restrict__ tails, int H, int G, int dim, int vdim, int min_len, DcWindow win) {
   extern __shared__ __align__(16) unsigned char dc_smem[];
   constexpr int LA = DcSolve<DP>::LA, LV = DcSolve<DP>::LV;
   bf16* k_s = reinterpret_cast<bf16*>(dc_smem);                             // the keys' parts, then W's
@@ -250,7 +254,7 @@ delta_chunk_solve_kernel(const float* __restrict__ kn, const bf16* __restrict__ 
   __shared__ int good;  // tokens before the first whose numbers are none
   pdl_trigger();
   pdl_wait();
-  const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z, kh = h / (H / G), tid = threadIdx.x;
+  const int c = win.first + blockIdx.x, h = blockIdx.y, s = blockIdx.z, kh = h / (H / G), tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int start = __ldcg(seq_start + s), end = __ldcg(seq_start + s + 1), t0 = start + c * DC;
   const int n = min(DC, end - t0);
@@ -292,7 +296,7 @@ delta_chunk_solve_kernel(const float* __restrict__ kn, const bf16* __restrict__ 
   }
   __syncthreads();
   const int ok = good;
-  const size_t chunk = dc_first_chunk(start, s) + c, slot = chunk * H + h;
+  const size_t chunk = dc_chunk(win, start, s, c), slot = chunk * H + h;
   if (h % (H / G) == 0) {  // the keys' parts, once for the heads that share them
     uint4* to = reinterpret_cast<uint4*>(K + (chunk * G + kh) * 3 * DC * DP);
 #pragma unroll 4
@@ -453,7 +457,7 @@ template <int DP, int COLS>
 __global__ void __launch_bounds__(256)
 delta_chunk_walk_kernel(const bf16* __restrict__ K, const float* __restrict__ tails, float* __restrict__ state, const int* __restrict__ slot_ids,
                         const int* __restrict__ seq_start, const bf16* __restrict__ W, float* __restrict__ U, float* __restrict__ states, int H,
-                        int G, int dim, int vdim, int min_len) {
+                        int G, int dim, int vdim, int min_len, DcWindow win) {
   static_assert(DP == 128 || COLS == 32, "four warps to 16 rows each would share 16 columns");
   extern __shared__ __align__(16) unsigned char dc_smem[];
   using D = DcWalk<DP, COLS>;
@@ -469,16 +473,16 @@ delta_chunk_walk_kernel(const bf16* __restrict__ K, const float* __restrict__ ta
   pdl_wait();
   const int col0 = blockIdx.x * COLS, h = blockIdx.y, s = blockIdx.z, kh = h / (H / G);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int start = __ldcg(seq_start + s), len = __ldcg(seq_start + s + 1) - start, n_chunks = (len + DC - 1) / DC;
-  if (n_chunks <= 0 || len < min_len) return;
-  const int chunk0 = dc_first_chunk(start, s);
+  const int start = __ldcg(seq_start + s), len = __ldcg(seq_start + s + 1) - start;
+  const int n_chunks = win.count ? min((len + DC - 1) / DC, win.first + win.count) : (len + DC - 1) / DC;
+  if (n_chunks <= win.first || len < min_len) return;
   auto load_w = [&](int c) {
-    const size_t slot = (size_t)(chunk0 + c) * H + h;
+    const size_t slot = (size_t)dc_chunk(win, start, s, c) * H + h;
     dc_load_parts<DP>(w_s, W + slot * 3 * DC * DP);
     if (tid < DC / 4 + 1) spl_cp16(&tail[c & 1][4 * tid], tails + slot * (DC + 4) + 4 * tid, true);
     spl_cp_commit();
   };
-  load_w(0);
+  load_w(win.first);
   // this lane's rows r0 + g and + 8 and its columns of the state; of W S: tokens m0 + g and + 8
   const int r0 = 16 * (warp % ROW_WARPS), sc = warp / ROW_WARPS * NB * 8, m0 = 16 * (warp & 3), uc = (warp >> 2) * NA * 8;
   float* record = state + ((size_t)__ldcg(slot_ids + s) * H + h) * dim * vdim + col0;
@@ -493,8 +497,8 @@ delta_chunk_walk_kernel(const bf16* __restrict__ K, const float* __restrict__ ta
       S[0][i][2 * e] = v.x, S[0][i][2 * e + 1] = v.y;
     }
   }
-  for (int c = 0; c < n_chunks; ++c) {
-    const size_t slot = (size_t)(chunk0 + c) * H + h;
+  for (int c = win.first; c < n_chunks; ++c) {
+    const size_t chunk = dc_chunk(win, start, s, c), slot = chunk * H + h;
     // the chunk's X at this lane's places, asked for early
     float2 x[NA][2];
     float* u_at = U + (slot * DC + m0 + g) * vdim + col0 + uc + 2 * t;
@@ -522,7 +526,7 @@ delta_chunk_walk_kernel(const bf16* __restrict__ K, const float* __restrict__ ta
     }
     spl_cp_wait<0>();
     __syncthreads();  // W and the state's parts are there; the keys are used up
-    dc_load_parts<DP>(k_s, K + ((size_t)(chunk0 + c) * G + kh) * 3 * DC * DP);
+    dc_load_parts<DP>(k_s, K + (chunk * G + kh) * 3 * DC * DP);
     spl_cp_commit();
     float acc[1][NA][4] = {};
 #pragma unroll 2
@@ -610,7 +614,7 @@ template <int DP>
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_out_kernel(const float* __restrict__ qn, const bf16* __restrict__ K, const float* __restrict__ log_decay,
                        const int* __restrict__ seq_start, const float* __restrict__ U, const float* __restrict__ states, void* __restrict__ out,
-                       int out_stride, int H, int G, int dim, int vdim, int n_seqs, int min_len, SplNorm norm) {
+                       int out_stride, int H, int G, int dim, int vdim, int n_seqs, int min_len, DcWindow win, SplNorm norm) {
   extern __shared__ __align__(16) unsigned char dc_smem[];
   using D = DcOut<DP>;
   constexpr int LU = D::LU, LS = D::LS;
@@ -622,12 +626,12 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const bf16* __restrict__ K,
   __shared__ double L[DC];
   pdl_trigger();
   pdl_wait();
-  const int c = blockIdx.x, h = blockIdx.y, s = blockIdx.z % n_seqs, col0 = blockIdx.z / n_seqs * 128, kh = h / (H / G), tid = threadIdx.x;
+  const int c = win.first + blockIdx.x, h = blockIdx.y, s = blockIdx.z % n_seqs, col0 = blockIdx.z / n_seqs * 128, kh = h / (H / G), tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int start = __ldcg(seq_start + s), end = __ldcg(seq_start + s + 1), t0 = start + c * DC;
   const int n = min(DC, end - t0);
   if (n <= 0 || end - start < min_len) return;
-  const size_t chunk = dc_first_chunk(start, s) + c, slot = chunk * H + h;
+  const size_t chunk = dc_chunk(win, start, s, c), slot = chunk * H + h;
   {
     DcRows<DP> rows;
     rows.load(qn + ((size_t)t0 * G + kh) * dim, (size_t)G * dim, n, dim);
@@ -733,26 +737,35 @@ delta_chunk_out_kernel(const float* __restrict__ qn, const bf16* __restrict__ K,
 RL_API int rl_delta_chunked_takes(int dim, int vdim) { return dim > 0 && vdim > 0 && dim <= 128 && dim % 4 == 0 && vdim % 4 == 0; }
 
 // Floats of scratch for n_tokens tokens of n_seqs sequences: W's parts, the keys' parts, U, the states and the tails.
+static long long chunk_floats(int H, int dim, int vdim) {
+  return H * (2 * (3 * DC / 2) * (dim <= 64 ? 64LL : 128LL) + (long long)DC * vdim + (long long)dim * vdim + DC + 4);
+}
 RL_API long long rl_delta_chunked_scratch(int n_tokens, int n_seqs, int H, int dim, int vdim) {
-  const long long chunks = n_tokens / DC + n_seqs + 1, row = dim <= 64 ? 64 : 128;
-  return chunks * H * (2 * (3 * DC / 2) * row + (long long)DC * vdim + (long long)dim * vdim + DC + 4);
+  return ((long long)n_tokens / DC + n_seqs + 1) * chunk_floats(H, dim, vdim);
+}
+// How many chunks of every sequence a scratch of so many floats has room for at a time; 0: for all of them, -1: for none.
+RL_API int rl_delta_chunked_window(long long scratch_floats, int n_tokens, int n_seqs, int H, int dim, int vdim) {
+  if (n_seqs <= 0 || H <= 0 || dim <= 0 || vdim <= 0) return -1;
+  if (scratch_floats >= rl_delta_chunked_scratch(n_tokens, n_seqs, H, dim, vdim)) return 0;
+  const long long fit = scratch_floats / (n_seqs * chunk_floats(H, dim, vdim));
+  return fit < 1 ? -1 : (int)(fit < 0x1000000 ? fit : 0x1000000);
 }
 
 // qn, kn: float32 [T, G dim] (unit vectors, the queries times their constant); v: bfloat16 rows of >= H vdim; beta, log_decay: float32
 // [T, H]; state: float32 [slots, H, dim, vdim]; out: float32 [T, >= H vdim], or with norm_w (the heads' norm weights [vdim], up to 128
 // values) bfloat16 rows that have been through what head_norm_gate does.  Sequences of fewer than min_len tokens (and their rows of out) are
-// left alone.
+// left alone.  window: 0, or how many chunks of every sequence to take at a time.
 template <int DP>
 static int launch_delta_chunked(const float* qn, const float* kn, const bf16* v, int v_stride, const float* beta, const float* log_decay,
                                 float* state, const int* slot_ids, const int* seq_start, void* out, int out_stride, int n_tokens, int n_seqs,
-                                int max_q_len, int H, int G, int dim, int vdim, int min_len, float* scratch, const SplNorm& norm, cudaStream_t stream) {
-  const long long chunks = n_tokens / DC + n_seqs + 1;
+                                int max_q_len, int H, int G, int dim, int vdim, int min_len, float* scratch, int window, const SplNorm& norm, cudaStream_t stream) {
+  const long long chunks = window ? (long long)window * n_seqs : n_tokens / DC + n_seqs + 1;
   bf16* W = reinterpret_cast<bf16*>(scratch);
   bf16* K = W + chunks * H * 3 * DC * DP;
   float* U = reinterpret_cast<float*>(K + chunks * H * 3 * DC * DP);
   float* states = U + chunks * H * DC * vdim;
   float* tails = states + chunks * H * dim * vdim;  // [chunk][head][64 + 4]
-  const int groups = (vdim + 127) / 128, n_chunks = (max_q_len + DC - 1) / DC;
+  const int groups = (vdim + 127) / 128, all_chunks = (max_q_len + DC - 1) / DC, n_chunks = window && window < all_chunks ? window : all_chunks;
   if ((long long)groups * n_seqs > 65535) RL_REFUSE(4, "delta_chunked: %d sequences of %d values exceed the grid", n_seqs, vdim);
   const dim3 per_chunk(n_chunks, H, n_seqs), per_group(n_chunks, H, n_seqs * groups);
   const int v_wide = vdim % 8 == 0 && v_stride % 8 == 0 && ((uintptr_t)v & 15) == 0;
@@ -769,18 +782,21 @@ static int launch_delta_chunked(const float* qn, const float* kn, const bf16* v,
       cudaFuncSetAttribute(delta_chunk_out_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3) != cudaSuccess)
     RL_REFUSE(7, "delta_chunked: cannot get %d, %d or %d bytes of shared memory", s1, s2, s3);
   const dim3 per_tile((vdim + cols - 1) / cols, H, n_seqs);
-  RL_LAUNCH_CHECK(rl_launch<false>(delta_chunk_solve_kernel<DP>, per_chunk, 256, s1, stream, kn, v, v_stride, v_wide, beta, log_decay, seq_start, W, K, U,
-                                   tails, H, G, dim, vdim, min_len));
-  RL_LAUNCH_CHECK(rl_launch(walk, per_tile, 256, s2, stream, (const bf16*)K, (const float*)tails, state, slot_ids, seq_start, (const bf16*)W, U, states,
-                            H, G, dim, vdim, min_len));
-  RL_LAUNCH_CHECK(rl_launch(delta_chunk_out_kernel<DP>, per_group, 256, s3, stream, qn, (const bf16*)K, log_decay, seq_start, (const float*)U,
-                            (const float*)states, out, out_stride, H, G, dim, vdim, n_seqs, min_len, norm));
+  for (int first = 0; first < all_chunks; first += n_chunks) {
+    const DcWindow win = {first, window};
+    RL_LAUNCH_CHECK(rl_launch<false>(delta_chunk_solve_kernel<DP>, per_chunk, 256, s1, stream, kn, v, v_stride, v_wide, beta, log_decay, seq_start, W, K, U,
+                                     tails, H, G, dim, vdim, min_len, win));
+    RL_LAUNCH_CHECK(rl_launch(walk, per_tile, 256, s2, stream, (const bf16*)K, (const float*)tails, state, slot_ids, seq_start, (const bf16*)W, U, states,
+                              H, G, dim, vdim, min_len, win));
+    RL_LAUNCH_CHECK(rl_launch(delta_chunk_out_kernel<DP>, per_group, 256, s3, stream, qn, (const bf16*)K, log_decay, seq_start, (const float*)U,
+                              (const float*)states, out, out_stride, H, G, dim, vdim, n_seqs, min_len, win, norm));
+  }
   return 0;
 }
 
 RL_API int rl_delta_chunked(const float* qn, const float* kn, const void* v, int v_stride, const float* beta, const float* log_decay, float* state,
                             const int* slot_ids, const int* seq_start, void* out, int out_stride, int n_tokens, int n_seqs, int max_q_len, int H,
-                            int G, int dim, int vdim, int min_len, float* scratch, const float* norm_w, float eps, const void* gate, int gate_stride,
+                            int G, int dim, int vdim, int min_len, float* scratch, long long scratch_floats, const float* norm_w, float eps, const void* gate, int gate_stride,
                             int gate_act, float out_scale, cudaStream_t stream) {
   if (n_tokens <= 0 || n_seqs <= 0 || max_q_len <= 0 || H <= 0 || G <= 0) RL_REFUSE(1, "delta_chunked: T=%d S=%d max_q=%d H=%d G=%d", n_tokens, n_seqs, max_q_len, H, G);
   if (!rl_delta_chunked_takes(dim, vdim)) RL_REFUSE(2, "delta_chunked: sizes %d / %d (multiples of 4, keys up to 128)", dim, vdim);
@@ -792,10 +808,12 @@ RL_API int rl_delta_chunked(const float* qn, const float* kn, const void* v, int
   // (rows of whole fours: a step with sequences of a few tokens has the norm made by head_norm_gate, four columns a lane, and the bits are the same)
   if (norm_w && (vdim > 128 || out_stride % 4 || ((uintptr_t)out & 7) || gate_stride % 4 || ((uintptr_t)gate & 7) || ((uintptr_t)norm_w & 7)))
     return RL_NOT_FUSED;
+  const int window = rl_delta_chunked_window(scratch_floats, n_tokens, n_seqs, H, dim, vdim);
+  if (window < 0) RL_REFUSE(8, "delta_chunked: %lld floats of scratch hold no chunk of %d sequences", scratch_floats, n_seqs);
   const SplNorm norm{norm_w, eps, (const bf16*)gate, gate_stride, gate_act, out_scale};
   if (dim <= 64)
     return launch_delta_chunked<64>(qn, kn, (const bf16*)v, v_stride, beta, log_decay, state, slot_ids, seq_start, out, out_stride, n_tokens, n_seqs,
-                                    max_q_len, H, G, dim, vdim, min_len, scratch, norm, stream);
+                                    max_q_len, H, G, dim, vdim, min_len, scratch, window, norm, stream);
   return launch_delta_chunked<128>(qn, kn, (const bf16*)v, v_stride, beta, log_decay, state, slot_ids, seq_start, out, out_stride, n_tokens, n_seqs,
-                                   max_q_len, H, G, dim, vdim, min_len, scratch, norm, stream);
+                                   max_q_len, H, G, dim, vdim, min_len, scratch, window, norm, stream);
 }

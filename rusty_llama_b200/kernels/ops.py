@@ -2324,14 +2324,29 @@ def delta_chunked_scratch_floats(n_tokens: int, n_seqs: int, num_heads: int, dim
     return int(lib.rl_delta_chunked_scratch(n_tokens, n_seqs, num_heads, dim, vdim))
 
 
+DELTA_CHUNK = 64
+
+
+def delta_chunked_less_scratch_floats(n_tokens: int, n_seqs: int, num_heads: int, dim: int, vdim: int) -> int:
+    """What the chunks' matrices would take as 32-bit numbers instead of the parts they are split into, a third to half less: with so much
+    scratch `delta_chunked` has the chunks in two or three goes."""
+    return (n_tokens // DELTA_CHUNK + n_seqs + 1) * num_heads * (DELTA_CHUNK * (dim + vdim) + dim * vdim + DELTA_CHUNK + 4)
+
+
+def delta_chunked_window(scratch_floats: int, n_tokens: int, n_seqs: int, num_heads: int, dim: int, vdim: int) -> int:
+    """How many chunks of every sequence `delta_chunked` takes at a time with so much scratch (0: all of them, -1: it is too little)."""
+    return int(library("delta_chunk").rl_delta_chunked_window(scratch_floats, n_tokens, n_seqs, num_heads, dim, vdim))
+
+
 def delta_chunked(
     qn: torch.Tensor, kn: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, log_decay: torch.Tensor, state: torch.Tensor, slot_ids: torch.Tensor,
     seq_start: torch.Tensor, num_heads: int, num_qk_heads: int, dim: int, vdim: int, max_q_len: int, scratch: torch.Tensor, min_len: int = 1,
     norm=None,
 ) -> Optional[torch.Tensor]:
     """`delta_rule` chunk by chunk, for prompts of bfloat16 runs: the same result within 32-bit rounding.  log_decay: float32 [T, H], the
-    logarithms of the decays; v: bfloat16 rows; scratch: float32, `delta_chunked_scratch_floats` numbers.  Sequences of fewer than min_len
-    tokens are left alone, and their rows of the result undefined.
+    logarithms of the decays; v: bfloat16 rows; scratch: float32, `delta_chunked_scratch_floats` numbers, or fewer: the chunks then come in
+    several goes, with the same bits, as long as there is room for one of every sequence (`delta_chunked_window`).  Sequences of fewer than
+    min_len tokens are left alone, and their rows of the result undefined.
 
     norm: None, or (weight [vdim], eps, gate, gate_act, out_scale, out) as `head_norm_gate` takes them (out may be None): returns what
     `head_norm_gate` would make of the result, in bfloat16, in the same kernels; None where they cannot (nothing is launched)."""
@@ -2350,7 +2365,8 @@ def delta_chunked(
     S = slot_ids.numel()
     _need(seq_start.numel() == S + 1, "delta_chunked: seq_start must hold one more entry than there are sequences")
     _cuda(scratch, "delta_chunked scratch", torch.float32)
-    _need(scratch.numel() >= delta_chunked_scratch_floats(T, S, H, dim, vdim), "delta_chunked: scratch too small")
+    window = delta_chunked_window(scratch.numel(), T, S, H, dim, vdim)
+    _need(window >= 0, "delta_chunked: scratch too small")
     weight, eps, gate, gs, gate_act, out_scale, out = _norm_args(norm, "delta_chunked", T, H, vdim)
     if norm is not None and weight is None:
         return None
@@ -2359,12 +2375,13 @@ def delta_chunked(
     lib = library("delta_chunk")
     rc = lib.rl_delta_chunked(
         qn, kn, v, _rows(v, "delta_chunked v"), beta, log_decay, state, slot_ids, seq_start, out, out.stride(0),
-        T, S, max_q_len, H, G, dim, vdim, min_len, scratch, weight, float(eps),
+        T, S, max_q_len, H, G, dim, vdim, min_len, scratch, scratch.numel(), weight, float(eps),
         gate, gs, gate_act, float(out_scale), _stream(),
     )
     if rc == _NOT_FUSED:
         return None
-    _check(lib, rc, "delta_chunked", kernels=3)
+    chunks = (max_q_len + DELTA_CHUNK - 1) // DELTA_CHUNK
+    _check(lib, rc, "delta_chunked", kernels=3 * ((chunks + window - 1) // window if window else 1))
     return out
 
 

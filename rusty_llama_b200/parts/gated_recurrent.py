@@ -28,7 +28,7 @@ from .base import MIXERS, Mixer, ParamInfo, StateNeed, scratch_for_call
 # that brings fewer does
 _CHUNKED_MIN_TOKENS = 32
 # the most scratch that the delta rule's chunks may take (3 GB: 30000 tokens of 32 heads of 128 x 128 a step); beyond it, and where the
-# device has less, token by token
+# device has less than two thirds of what they need, token by token
 _CHUNKED_MAX_FLOATS = 3 << 28
 
 
@@ -326,6 +326,9 @@ class GatedDeltaRule(Mixer):
             floats = ops.delta_chunked_scratch_floats(step.n_tokens, step.n_seqs, H, self.dim, self.vdim)
             if floats <= _CHUNKED_MAX_FLOATS:
                 scratch = scratch_for_call(floats, torch.float32, xn.device)
+                less = ops.delta_chunked_less_scratch_floats(step.n_tokens, step.n_seqs, H, self.dim, self.vdim)
+                if scratch is None and ops.delta_chunked_window(less, step.n_tokens, step.n_seqs, H, self.dim, self.vdim) > 0:
+                    scratch = scratch_for_call(less, torch.float32, xn.device)  # (the chunks come in several goes)
         chunked = scratch is not None
         qn, kn, kq, beta, decay, *log = ops.delta_prep(ops.columns(conv, 0, 2 * self.qd), ba, self.a_log, self.dt_bias, self.G, H, self.dim, self.unit_eps,
                                                        self.q_scale, log_decay=chunked)

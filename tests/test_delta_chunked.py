@@ -373,3 +373,62 @@ def test_a_prompts_bits_do_not_depend_on_its_company():
         assert torch.equal(got[lens.index(100)], want) and torch.equal(got_S[lens.index(100)], want_S), lens
         if 5 in lens:
             assert torch.equal(got[lens.index(5)], few) and torch.equal(got_S[lens.index(5)], few_S), lens
+
+
+@pytest.mark.parametrize("lens, H, G, dim, vdim", [([200, 64, 1, 63], 4, 2, 128, 128), ([400], 2, 1, 100, 132), ([33, 300], 3, 3, 64, 20)])
+def test_chunks_in_several_goes(lens, H, G, dim, vdim):
+    """With room for one, two or three chunks of every sequence at a time: the same bits, results and states, and the same sequences left alone."""
+    from rusty_llama_b200.errors import KernelError
+    from rusty_llama_b200.kernels import ops
+
+    q, k, v, beta, logd = inputs(lens, H, G, dim, vdim, 21, "usual")
+    T, S = sum(lens), len(lens)
+    starts = [sum(lens[:i]) for i in range(S + 1)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    first = torch.randn(S, H, dim, vdim, generator=torch.Generator().manual_seed(4)).to(DEV)
+    gate, w = torch.randn(T, H * vdim, device=DEV).to(torch.bfloat16), torch.randn(vdim, device=DEV)
+    full = ops.delta_chunked_scratch_floats(T, S, H, dim, vdim)
+    a_chunk = full // (T // 64 + S + 1) * S
+
+    def run(floats, norm, min_len):
+        state, out = first.clone(), torch.zeros(T, H * vdim, dtype=torch.bfloat16, device=DEV)
+        got = ops.delta_chunked(q.reshape(T, -1).to(DEV), k.reshape(T, -1).to(DEV), v.reshape(T, -1).to(DEV), beta.to(DEV), logd.to(DEV), state, i32(list(range(S))),
+                                i32(starts), H, G, dim, vdim, max(lens), torch.full((floats,), float("nan"), device=DEV), min_len,
+                                norm=(w, 1e-5, gate, ops.GATE_SILU, 1.0, out) if norm else None)
+        return got, state
+
+    for norm, min_len in ((False, 1), (vdim <= 128, 64)):
+        want, want_S = run(full, norm, min_len)
+        for chunks in (1, 2, 3):
+            assert ops.delta_chunked_window(chunks * a_chunk, T, S, H, dim, vdim) == (chunks if chunks * a_chunk < full else 0)
+            got, got_S = run(chunks * a_chunk, norm, min_len)
+            for i, n in enumerate(lens):
+                if n >= min_len:
+                    assert torch.equal(got[starts[i] : starts[i + 1]], want[starts[i] : starts[i + 1]])
+                elif norm:
+                    assert not bool(got[starts[i] : starts[i + 1]].any())
+            assert torch.equal(got_S, want_S)
+    with pytest.raises(KernelError):
+        run(a_chunk - 1, False, 1)
+
+
+def test_a_step_with_little_memory_left_still_goes_by_chunks(monkeypatch):
+    """Where the device has no room for the whole scratch, what the matrices take unsplit does, with the same bits; with less it is token by token."""
+    import rusty_llama_b200.parts.gated_recurrent as module
+    from rusty_llama_b200.kernels import ops
+
+    part, before = _layer(), ops.delta_chunked
+    x = torch.randn(700, 64, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).to(DEV)
+    (want,), (want_S,) = _rows(part, [700], [x])
+    full, less, called = ops.delta_chunked_scratch_floats(700, 1, 4, 32, 48), ops.delta_chunked_less_scratch_floats(700, 1, 4, 32, 48), []
+    assert 3 * less < 2 * full
+    monkeypatch.setattr(ops, "delta_chunked", lambda *a, **k: called.append(a[13].numel()) or before(*a, **k))
+    for room, takes in ((full, full), (full - 1, less), (less, less), (less - 1, None)):
+        called.clear()
+        monkeypatch.setattr(module, "scratch_for_call", lambda n, dtype, device: torch.empty(n, dtype=dtype, device=device) if n <= room else None)
+        (got,), (got_S,) = _rows(part, [700], [x])
+        assert called == ([takes] if takes else [])
+        if takes:
+            assert torch.equal(got, want) and torch.equal(got_S, want_S)
+        else:
+            assert float((got_S - want_S).norm() / want_S.norm()) <= 1e-5
