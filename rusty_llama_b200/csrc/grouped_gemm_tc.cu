@@ -102,7 +102,7 @@ struct Groups {
 };
 
 // Matrices that take every token (a shared expert in pieces of the others' size), where they lie: feature n of the j-th at w + j * piece +
-// n * row, K numbers.  So rows of gate and up that alternate and columns of one wide matrix serve as they are, and no copy beside the
+// n * row, K numbers (the others' are described to TMA in the same way).  So rows of gate and up that alternate and columns of one wide matrix serve as they are, and no copy beside the
 // others is held.
 struct Always {
   const bf16 *w, *w2;
@@ -190,8 +190,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         group(unit, e, r0, rows);
         if (rows <= 0) continue;
         const bool own = e < g.matrices || g.always == 0;
-        const int piece = e - g.matrices, w_row = (own ? e * g.N : 0) + (unit % blocks_n) * UNIT_N;
-        const int w_row2 = EPI == GATED ? w_row : w_row + FEATURES / 2;
+        const CUtensorMap *from = own ? &map_w : &map_s, *from2 = own ? &map_w2 : &map_s2;
+        const int matrix = own ? e : e - g.matrices, row = (unit % blocks_n) * UNIT_N, row2 = EPI == GATED ? row : row + FEATURES / 2;
+        const bool matrix_first = !own && g.piece_first;
+        const int y = matrix_first ? matrix : row, z = matrix_first ? row : matrix, y2 = matrix_first ? matrix : row2, z2 = matrix_first ? row2 : matrix;
         for (int kb = 0; kb < n_k; ++kb, ++it) {
           if (it >= STAGES && !mbar_wait_role(&empty_bar[s], parity, ctl, 61)) {
             give_up_code(status, 61);
@@ -200,13 +202,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             break;
           }
           mbar_expect_tx_s(full0 + 8 * s, A_BYTES);
-          if (own) {
-            tma_load_2d_s(dst, &map_w, full0 + 8 * s, kb * BK, w_row);
-            tma_load_2d_s(dst + A_BYTES / 2, &map_w2, full0 + 8 * s, kb * BK, w_row2);
-          } else {
-            tma_load_3d_s(dst, &map_s, full0 + 8 * s, kb * BK, g.piece_first ? piece : w_row, g.piece_first ? w_row : piece);
-            tma_load_3d_s(dst + A_BYTES / 2, &map_s2, full0 + 8 * s, kb * BK, g.piece_first ? piece : w_row2, g.piece_first ? w_row2 : piece);
-          }
+          tma_load_3d_s(dst, from, full0 + 8 * s, kb * BK, y, z);
+          tma_load_3d_s(dst + A_BYTES / 2, from2, full0 + 8 * s, kb * BK, y2, z2);
           dst += SH::STAGE_BYTES;
           if (++s == STAGES) {
             s = 0;
@@ -435,8 +432,8 @@ static int make_rows_map(CUtensorMap* map, const Groups& g, int box_rows) {
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
 }
 
-// Boxes of 64 k x FEATURES / 2 features of a piece, the dimension of the smaller stride first.  0 on success.
-static int make_always_map(CUtensorMap* map, const bf16* w, const Always& a, int N, int K) {
+// Boxes of 64 k x FEATURES / 2 features of a matrix, the dimension of the smaller stride first.  0 on success.
+static int make_weights_map(CUtensorMap* map, const void* w, const Always& a, int N, int K) {
   EncodeTiledFn enc = encode_tiled();
   if (!enc) return 1;
   const int at_n = a.piece < a.row ? 2 : 1, at_piece = 3 - at_n;
@@ -444,7 +441,7 @@ static int make_always_map(CUtensorMap* map, const bf16* w, const Always& a, int
   cuuint32_t box[3] = {BK}, estr[3] = {1, 1, 1};
   dims[at_n] = (cuuint64_t)N, strides[at_n - 1] = (cuuint64_t)a.row * 2, box[at_n] = FEATURES / 2;
   dims[at_piece] = (cuuint64_t)a.n, strides[at_piece - 1] = (cuuint64_t)a.piece * 2, box[at_piece] = 1;
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
 }
 
@@ -453,15 +450,15 @@ static int launch_grouped(const void* w, const void* w2, int matrices, void* out
                           int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
   using SH = Shape<NT>;
   CUtensorMap map_w, map_w2, map_s, map_s2, map_x;
-  const int rows = matrices * g.N;
   g.matrices = matrices;
   g.always = always.n;
   g.piece_first = always.piece < always.row;
-  if (make_matrix_map(&map_w, w, rows, g.K, g.K, FEATURES / 2) || make_matrix_map(&map_w2, EPI == GATED ? w2 : w, rows, g.K, g.K, FEATURES / 2))
+  const Always dense = {nullptr, nullptr, g.K, (long long)g.N * g.K, matrices};
+  if (make_weights_map(&map_w, w, dense, g.N, g.K) || make_weights_map(&map_w2, EPI == GATED ? w2 : w, dense, g.N, g.K))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices to TMA");
   map_s = map_w;
   map_s2 = map_w2;
-  if (always.n > 0 && (make_always_map(&map_s, always.w, always, g.N, g.K) || make_always_map(&map_s2, EPI == GATED ? always.w2 : always.w, always, g.N, g.K)))
+  if (always.n > 0 && (make_weights_map(&map_s, always.w, always, g.N, g.K) || make_weights_map(&map_s2, EPI == GATED ? always.w2 : always.w, always, g.N, g.K)))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices that take every token to TMA");
   if (g.order != nullptr ? make_matrix_map(&map_x, g.x, g.x_rows, g.K, (int)g.ldx, 1) : make_rows_map(&map_x, g, SH::BOX_ROWS))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the rows to TMA");
