@@ -268,6 +268,7 @@ __device__ __forceinline__ int plan_before(int p, int few, int all) {  // the le
   return (int)(((long long)p * few + all - 1) / all);
 }
 
+template <bool MANY>  // pairs, eight or more a thread, whose ids are 16-byte aligned
 __global__ void __launch_bounds__(PLAN_THREADS)
 moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* __restrict__ order, int* __restrict__ place,
                 int* __restrict__ tiles, int tile_rows, int always, int top) {
@@ -279,23 +280,19 @@ moe_plan_kernel(const int* __restrict__ ids, int n, int E, int* __restrict__ ord
   for (int i = tid; i < E; i += PLAN_THREADS) cnt[i] = 0;
   if (tid < 3) sums[tid] = 0;
   __syncthreads();
-  // A thread has neighbouring pairs, of many of them whole fours, which it reads 16 bytes at a time; eight asked for at once: one after the other the
-  // trips to L2 were most of the kernel (and number by number they still were 15 us for 2048 tokens of 6, 13 and now).
+  // A thread has neighbouring pairs, eight of which are asked for at once (one after the other the trips to L2 were most of the kernel), of MANY by 16
+  // bytes: 2048 tokens of 6 12.1 us instead of 14.3.
   int per = (n + PLAN_THREADS - 1) / PLAN_THREADS;
-  const bool fours = per >= 4 && ((uintptr_t)ids & 15) == 0;
-  if (fours) per = (per + 3) & ~3;
+  if (MANY) per = (per + 7) & ~7;
   const int lo = min(n, tid * per), hi = min(n, lo + per);
   auto load = [&](int i0, int (&id)[8], int none) {
-#pragma unroll
-    for (int u = 0; u < 8; u += 4) {
-      if (fours && i0 + u + 3 < hi) {
-        const int4 v = __ldcg(reinterpret_cast<const int4*>(ids + i0 + u));
-        id[u] = v.x, id[u + 1] = v.y, id[u + 2] = v.z, id[u + 3] = v.w;
-      } else {
-#pragma unroll
-        for (int e = u; e < u + 4; ++e) id[e] = i0 + e < hi ? __ldcg(ids + i0 + e) : none;
-      }
+    if (MANY && i0 + 7 < hi) {
+      const int4 v = __ldcg(reinterpret_cast<const int4*>(ids + i0)), w = __ldcg(reinterpret_cast<const int4*>(ids + i0 + 4));
+      id[0] = v.x, id[1] = v.y, id[2] = v.z, id[3] = v.w, id[4] = w.x, id[5] = w.y, id[6] = w.z, id[7] = w.w;
+      return;
     }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) id[u] = i0 + u < hi ? __ldcg(ids + i0 + u) : none;
   };
   int mine = 0;
   for (int i0 = lo; i0 < hi; i0 += 8) {
@@ -407,7 +404,8 @@ RL_API int rl_moe_plan(const int* ids, int n, int E, int* order, int* place, int
   if (n <= 0 || E <= 0 || tile_rows <= 0 || always < 0 || top <= 0 || n % top) RL_REFUSE(1, "moe_plan: n=%d E=%d tile_rows=%d always=%d top=%d", n, E, tile_rows, always, top);
   const size_t smem = (size_t)E * sizeof(int);
   if (smem > 40 * 1024) RL_REFUSE(2, "moe_plan: %d experts exceed the kernel's shared memory", E);
-  RL_LAUNCH_CHECK(rl_launch(moe_plan_kernel, E + always, PLAN_THREADS, smem, stream, ids, n, E, order, place, tiles, tile_rows, always, top));
+  const bool many = n > 7 * PLAN_THREADS && ((uintptr_t)ids & 15) == 0;
+  RL_LAUNCH_CHECK(rl_launch(many ? moe_plan_kernel<true> : moe_plan_kernel<false>, E + always, PLAN_THREADS, smem, stream, ids, n, E, order, place, tiles, tile_rows, always, top));
   return 0;
 }
 
