@@ -541,8 +541,10 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
 }
 
 // The same sums, four neighbouring columns a thread and everything a thread needs of eight choices in flight at once.
+// With rows of matrices that take every token (OWN) the first of those are asked for before the choices': where they are is known.
 #define COMBINE_AHEAD 8
-template <typename TS, typename TO>
+#define COMBINE_OWN 2
+template <typename TS, typename TO, bool OWN>
 __global__ void __launch_bounds__(256)
 moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights, int top,
                        const TS* __restrict__ shared, const float* __restrict__ gate, TO* __restrict__ out, int d,
@@ -551,35 +553,39 @@ moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ plac
   pdl_wait();
   const int t = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (i >= d) return;
-  float v[4] = {0.f, 0.f, 0.f, 0.f}, own[4] = {0.f, 0.f, 0.f, 0.f};  // own: of the matrices that take every token
-  const int all = top + always;
-  for (int j0 = 0; j0 < all; j0 += COMBINE_AHEAD) {
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  float ahead[COMBINE_OWN][4];
+  const float* own_row = y + ((size_t)gridDim.x * top + t) * d + i;
+  const size_t own_step = (size_t)gridDim.x * d;
+  if constexpr (OWN) {
+#pragma unroll
+    for (int j = 0; j < COMBINE_OWN; ++j) {
+      ahead[j][0] = ahead[j][1] = ahead[j][2] = ahead[j][3] = 0.f;
+      if (j < always) load4_g<float>(own_row + j * own_step, ahead[j]);
+    }
+  }
+  for (int j0 = 0; j0 < top; j0 += COMBINE_AHEAD) {
     int p[COMBINE_AHEAD];
     float w[COMBINE_AHEAD], f[COMBINE_AHEAD][4];
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u) {
-      const int j = j0 + u;
-      const bool in = j < top;
-      p[u] = in ? __ldcg(place + (size_t)t * top + j) : j < all ? (int)gridDim.x * j + t : -1;
-      w[u] = in ? __ldcg(weights + (size_t)t * top + j) : 0.f;
+      const bool in = j0 + u < top;
+      p[u] = in ? __ldcg(place + (size_t)t * top + j0 + u) : -1;
+      w[u] = in ? __ldcg(weights + (size_t)t * top + j0 + u) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u) {
-      if (j0 + u >= all || (p[u] < 0 && x == nullptr)) f[u][0] = f[u][1] = f[u][2] = f[u][3] = 0.f;
+      if (j0 + u >= top || (p[u] < 0 && x == nullptr)) f[u][0] = f[u][1] = f[u][2] = f[u][3] = 0.f;
       else if (p[u] >= 0) load4_g<float>(y + (size_t)p[u] * d + i, f[u]);
       else load4_g<TS>(x + (size_t)t * ldx + i, f[u]);
     }
 #pragma unroll
     for (int u = 0; u < COMBINE_AHEAD; ++u)
-      if (j0 + u < top) {
+      if (j0 + u < top)
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] += w[u] * f[u][e];
-      } else if (j0 + u < all) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) own[e] += f[u][e];
-      }
   }
-  if (shared || always > 0) {
+  if (shared || OWN) {
     const float g = gate ? __ldcg(gate + t) : 1.f;
     if (shared) {
       float s[4];
@@ -587,7 +593,18 @@ moe_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ plac
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[e] += g * s[e];
     }
-    if (always > 0) {
+    if constexpr (OWN) {
+      float own[4] = {ahead[0][0], ahead[0][1], ahead[0][2], ahead[0][3]};
+#pragma unroll
+      for (int j = 1; j < COMBINE_OWN; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) own[e] += ahead[j][e];
+      for (int j = COMBINE_OWN; j < always; ++j) {
+        float f[4];
+        load4_g<float>(own_row + j * own_step, f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) own[e] += f[e];
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[e] += g * to_f32(__float2bfloat16_rn(own[e]));
     }
@@ -607,7 +624,7 @@ RL_API int rl_moe_combine(const float* y, const int* place, const float* weights
   dim3 grid(n_tokens, (d / 4 + 255) / 256);
 #define RL_MC(TS, TO)                                                                                                          \
   if (vec)                                                                                                                     \
-    RL_LAUNCH_CHECK(rl_launch(moe_combine_vec_kernel<TS, TO>, grid, 256, 0, stream, y, place, weights, top, (const TS*)shared, gate, \
+    RL_LAUNCH_CHECK(rl_launch(always > 0 ? moe_combine_vec_kernel<TS, TO, true> : moe_combine_vec_kernel<TS, TO, false>, grid, 256, 0, stream, y, place, weights, top, (const TS*)shared, gate, \
                               (TO*)out, d, (const TS*)x, ldx, always));                                                        \
   else                                                                                                                         \
   RL_LAUNCH_CHECK(rl_launch<false>(moe_combine_kernel<TS, TO>, n_tokens, 256, 0, stream, y, place, weights, top, (const TS*)shared, \
