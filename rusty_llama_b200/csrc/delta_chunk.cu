@@ -17,8 +17,8 @@
 //
 // All operands are 32-bit (but for the values) and go to the tensor cores as three bfloat16 numbers each, which loses no digits against
 // FMAs (split_mma.cuh).  Token by token every token is one chain of dependent steps per column; here only (2) is serial, with 64 tokens a
-// step.  Sequences of 1029, 700 and 319 tokens, 16 heads of 128 x 128: 53, 80 and 59 us (with the heads' norm); by FMAs fed from shared
-// memory 62, 106 and 72 (and 17 for the norm), token by token 444.
+// step.  Sequences of 1029, 700 and 319 tokens, 16 heads of 128 x 128: 53, 80 and 58 us (78 with the heads' norm and gate); by FMAs fed from shared
+// memory 62, 106 and 72 (and 17 for norm and gate), token by token 444.
 #include "split_mma.cuh"
 
 RL_DEFINE_ERROR_TEXT()

@@ -2,7 +2,8 @@
 // normaliser column: the 32-bit factors go in as three bfloat16 numbers each (split_mma.cuh), so nothing is lost against the FMA kernels.
 // Included by gated_recurrent.cu, whose header has the formulas.
 //
-// (1): 22 us where the FMA kernel takes 53, (3): 58 us where it takes 117, for 2048 tokens and 16 heads of 128 x 128.
+// (1): 22 us where the FMA kernel takes 53, (3): 58 us where it takes 117, for 2048 tokens and 16 heads of 128 x 128.  The heads' norm and gate in
+// (3) are 4 and 15 us more (the gate's rows, four bytes a lane), which is what head_norm_gate takes for them and the rows' way there and back.
 #pragma once
 #include "split_mma.cuh"
 

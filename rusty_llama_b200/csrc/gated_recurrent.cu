@@ -923,7 +923,7 @@ RL_API int rl_gated_attn_chunked(const void* q, const void* k, const void* v, in
   dim3 grid((unsigned)sh, max_chunks, col_tiles), grid2((unsigned)sh, (elems / scan_elems + 255) / 256), grid3((unsigned)sh, max_chunks);
   if (norm_w && (out_stride % 2 || ((uintptr_t)result & 3) || gate_stride % 2 || ((uintptr_t)gate & 3) || ((uintptr_t)norm_w & 7))) return RL_NOT_FUSED;
   // A decay per channel on bfloat16 rows in 16-byte pieces goes to the tensor cores (gated_chunk_mma.cuh): 2048 tokens, 16 heads of
-  // 128 x 128: 97 instead of 185 us for the three steps.  One decay per head comes with a normaliser column, whose odd rows do not fit.
+  // 128 x 128: 98 instead of 185 us for the three steps (117 with the heads' norm and gate, 202 with both behind them).  One decay per head comes with a normaliser column, whose odd rows do not fit.
   if (dtype == RL_BF16 && per_channel && !in_scale && !ext && (wide & GC_WIDE_STATE) && gated_mma_takes(q, k, v, in_stride, log_decay, dim, vdim)) {
 #define RL_GM(DP)                                                                                                                     \
   do {                                                                                                                                \
