@@ -84,7 +84,7 @@ def test_scores_that_are_no_numbers_choose_each_expert_once():
 @pytest.mark.parametrize("shared_ff, gated", [(64, False), (192, True), (96, True)])
 def test_part(T, shared_ff, gated):
     """All of a shared expert's forms (of the experts' size, of a multiple of it, of another size) against the plain sum in 32 bits: the
-    hidden rows are rounded to bfloat16 (2^-9 of each, at random), and so is a shared expert's result that goes its own way."""
+    hidden rows are rounded to bfloat16 (2^-9 of each, at random), and so is a shared expert's result."""
     from rusty_llama_b200.parts import FEED_FORWARDS, Runtime
     from rusty_llama_b200.spec import PartSpec
 
