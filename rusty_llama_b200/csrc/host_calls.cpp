@@ -178,6 +178,21 @@ static PyObject* check_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HC_CATCH
 }
 
+// matrices(t, other, what) -> (matrices, rows, columns, row stride, matrix stride) of a 3-D tensor whose rows are dense; other: None or a tensor
+// that has to lie in the same way
+static PyObject* check_matrices(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3 || !THPVariable_Check(args[0]) || !(args[1] == Py_None || THPVariable_Check(args[1]))) return PyErr_Format(PyExc_TypeError, "matrices(tensor, tensor or None, what)");
+  HC_TRY
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  if (x.dim() != 3 || x.stride(2) != 1) return refuse(args[2], "expected a 3-D tensor with dense rows");
+  if (args[1] != Py_None) {
+    const at::Tensor& y = THPVariable_Unpack(args[1]);
+    if (y.sizes() != x.sizes() || y.strides() != x.strides()) return refuse(args[2], "two tensors that do not lie in the same way");
+  }
+  return Py_BuildValue("(LLLLL)", (L)x.size(0), (L)x.size(1), (L)x.size(2), (L)x.stride(1), (L)x.stride(0));
+  HC_CATCH
+}
+
 // odd(x, w) -> whether rows of the two cannot be moved in 16-byte pieces: eight 16-bit numbers
 static PyObject* check_odd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != 2 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) return PyErr_Format(PyExc_TypeError, "odd(x, w)");
@@ -236,6 +251,7 @@ static PyMethodDef methods[] = {
     {"launcher", make_launcher, METH_VARARGS, nullptr},
     {"cuda", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check_cuda)), METH_FASTCALL | METH_KEYWORDS, nullptr},
     {"rows", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check_rows)), METH_FASTCALL, nullptr},
+    {"matrices", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check_matrices)), METH_FASTCALL, nullptr},
     {"odd", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(check_odd)), METH_FASTCALL, nullptr},
     {"stream", current_stream, METH_NOARGS, nullptr},
     {"empty", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(make_empty)), METH_FASTCALL, nullptr},

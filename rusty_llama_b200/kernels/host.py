@@ -83,6 +83,17 @@ def python_rows(t: torch.Tensor, what: str) -> int:
     return t.stride(0)
 
 
+def python_matrices(t: torch.Tensor, other: Optional[torch.Tensor], what: str) -> Tuple[int, int, int, int, int]:
+    """(matrices, rows, columns, row stride, matrix stride) of a 3-D tensor whose rows are dense; other: None or one that has to lie in the same way."""
+    if not isinstance(t, torch.Tensor) or not (other is None or isinstance(other, torch.Tensor)):
+        raise TypeError("matrices(tensor, tensor or None, what)")
+    if t.dim() != 3 or t.stride(2) != 1:
+        raise KernelError(f"{what}: expected a 3-D tensor with dense rows")
+    if other is not None and (other.shape != t.shape or other.stride() != t.stride()):
+        raise KernelError(f"{what}: two tensors that do not lie in the same way")
+    return (*t.shape, t.stride(1), t.stride(0))
+
+
 def python_odd(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether rows of the two cannot be moved in 16-byte pieces (eight 16-bit numbers)."""
     if not (isinstance(x, torch.Tensor) and isinstance(w, torch.Tensor)):
@@ -109,7 +120,7 @@ def python_columns(t: torch.Tensor, first: int, end: int) -> torch.Tensor:
     return t.narrow(1, first, end - first)  # (what is not there is refused, not left out)
 
 
-cuda, rows, odd, stream = python_cuda, python_rows, python_odd, python_stream
+cuda, rows, matrices, odd, stream = python_cuda, python_rows, python_matrices, python_odd, python_stream
 empty, columns, launcher = python_empty, python_columns, PythonLauncher
 
 _lock = threading.Lock()
@@ -140,7 +151,7 @@ def _find_native() -> None:
         if module is None:
             return
         module.set_error(KernelError)
-        for name in ("cuda", "rows", "odd", "stream", "empty", "columns", "launcher"):
+        for name in ("cuda", "rows", "matrices", "odd", "stream", "empty", "columns", "launcher"):
             globals()[name] = getattr(module, name)
         for namespace, names in _bound:
             namespace.update((own, globals()[name]) for own, name in names.items())

@@ -20,7 +20,7 @@ from . import build
 from .device import sm_count
 from .host import bind, library
 
-bind(globals(), columns="columns", _cuda="cuda", _empty="empty", _rows="rows", _stream="stream")  # (columns is for the parts)
+bind(globals(), columns="columns", _cuda="cuda", _empty="empty", _matrices="matrices", _rows="rows", _stream="stream")  # (columns is for the parts)
 
 PAGE_SIZE = 64  # tokens per cache page; the attention kernels' key tile
 
@@ -1455,13 +1455,12 @@ def moe_gemm(
         _need(tuple(w2.shape) == (E, N, K), "moe_gemm: w2 does not match w")
     more, ws_row, ws_piece = 0, 0, 0
     if always is not None:
-        _cuda(always, "moe_gemm always", x.dtype, contiguous=False)
-        if not (always.dim() == 3 and tuple(always.shape[1:]) == (N, K) and always.stride(2) == 1 and (always2 is None) == (w2 is None)):
-            raise KernelError(f"moe_gemm: always {tuple(always.shape)} does not match w {tuple(w.shape)}")
-        more, (ws_piece, ws_row, _) = always.shape[0], always.stride()
+        _cuda(always, "moe_gemm always", x.dtype, False)
         if always2 is not None:
-            _cuda(always2, "moe_gemm always2", x.dtype, contiguous=False)
-            _need(always2.shape == always.shape and always2.stride() == always.stride(), "moe_gemm: always2 does not lie as always does")
+            _cuda(always2, "moe_gemm always2", x.dtype, False)
+        more, rows, columns, ws_row, ws_piece = _matrices(always, always2, "moe_gemm always")
+        if rows != N or columns != K or (always2 is None) != (w2 is None):
+            raise KernelError(f"moe_gemm: always {tuple(always.shape)} does not match w {tuple(w.shape)}")
     out_dtype = out_dtype or x.dtype
     out = _empty(x, out_dtype, n_rows, N)
     tile_rows = tile_rows or moe_tile_rows()

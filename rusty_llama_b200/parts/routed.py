@@ -167,8 +167,9 @@ class RoutedExperts(FeedForward):
         order, place, tiles, max_tiles = ops.moe_plan(ids, self.E, tile_rows, always)
         n_rows = T * (self.top + always)
         if self.gated:
-            more = dict(always=self.always_gate, always2=self.always_up) if always else {}
-            h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, n_rows, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act, **more)
+            own, own2 = (self.always_gate, self.always_up) if always else (None, None)
+            h = ops.moe_gemm(xn, self.w_gate, tiles, max_tiles, n_rows, order=order, gather_div=self.top, w2=self.w_up, tile_rows=tile_rows, act=self.act,
+                             always=own, always2=own2)
         else:
             h = ops.moe_gemm(xn, self.w_up, tiles, max_tiles, n_rows, order=order, gather_div=self.top, tile_rows=tile_rows, act="relu2")
         y = ops.moe_gemm(h, self.w_down, tiles, max_tiles, n_rows, out_dtype=torch.float32, tile_rows=tile_rows, always=self.always_down if always else None)

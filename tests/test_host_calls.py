@@ -81,6 +81,10 @@ def test_checks_and_views_agree_with_python():
     for x in (t, t[:, 2:4], t.t(), t[0]):
         assert outcome(native.rows, x, "r") == outcome(host.python_rows, x, "r")
     assert torch.equal(native.columns(t, 1, 4), host.python_columns(t, 1, 4)) and native.columns(t, 1, 4).stride() == (6, 1)
+    m = torch.zeros(3, 4, 2, 8)[:, :, 1]
+    for x, y in ((m, None), (m, torch.zeros(3, 4, 2, 8)[:, :, 0]), (torch.zeros(8, 3, 4).transpose(0, 1), None)):
+        assert native.matrices(x, y, "m") == host.python_matrices(x, y, "m")
+    assert native.matrices(m, None, "m") == (3, 4, 8, 16, 64)
     e = native.empty(t, torch.bfloat16, 3, 5)
     assert e.dtype == torch.bfloat16 and tuple(e.shape) == (3, 5) and e.device == t.device
     w = torch.zeros(64, 64, dtype=torch.bfloat16)
@@ -224,12 +228,13 @@ def test_refusals_agree_with_python(library):
     """What one side refuses the other does too, with the same kind of error and, where it is the library's own, the same words."""
     native, (make, python_make) = launchers()
     at = ctypes.cast(library.none, ctypes.c_void_p).value
-    t, i = torch.zeros(4, 6), torch.zeros(())
+    t, i, m = torch.zeros(4, 6), torch.zeros(()), torch.zeros(2, 2, 8)
     pairs = [
         (make(at, False), python_make(at, False), [tuple([1.0] * 9), tuple([1] * 57)]),
         (lambda k: make(at, False, k), lambda k: python_make(at, False, k), ["f" * 9, "i" * 57]),
         (make(at, False, "pif"), python_make(at, False, "pif"), [(t, 1), (1.5, 1, 1.0), (t, 1.5, 1.0), (t, 1, "x")]),
         (native.rows, host.python_rows, [(3, "r"), (t[0], "r"), (t.t(), "r")]),
+        (native.matrices, host.python_matrices, [(t, None, "m"), (m.transpose(1, 2), None, "m"), (m, m[:1], "m"), (m, m.transpose(0, 1), "m"), (3, m, "m"), (m, 3, "m")]),
         (native.odd, host.python_odd, [(t[0], t), (t.view(2, 2, 6), t), (t, i), (3, t), (t, 3)]),
         (native.empty, host.python_empty, [(t, torch.float32), (t, torch.float32, 1, 1, 1, 1, 1), (t, 3, 1), (3, torch.float32, 1), (t, torch.float32, -1)]),
         (native.columns, host.python_columns, [(t, 2, 9), (t, 7, 8), (t, 4, 2), (t[0], 0, 1), (3, 0, 1)]),
