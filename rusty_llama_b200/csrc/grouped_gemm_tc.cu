@@ -96,8 +96,8 @@ struct Groups {
   long long ldg, gh;
   int N, K;
   int matrices;        // matrices of w
-  int always;          // and how many more of other places: the plan's groups of higher numbers have theirs in map_s
-  int piece_first;     // whose dimensions go by their strides: [feature][piece][k] instead of [piece][feature][k]
+  int piece_first;     // the dimensions of those beside them go by their strides: [feature][piece][k] instead of [piece][feature][k]
+  int shift;           // where in a row of theirs the second half of a tile begins: behind the first matrix's K numbers, or 0
   float act_alpha, act_limit;
 };
 
@@ -110,11 +110,19 @@ struct Always {
   int n;
 };
 
-template <typename TO, int EPI, int NT>
+// How TMA finds the weights: the matrices of w (and w2), and with MORE those that take every token, the plan's groups of higher numbers.
+template <bool MORE>
+struct WeightMaps {
+  CUtensorMap w, w2;
+};
+template <>
+struct WeightMaps<true> {
+  CUtensorMap w, w2, s, s2;
+};
+
+template <typename TO, int EPI, int NT, bool MORE>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
-                       const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_s2,
-                       const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
+grouped_gemm_tc_kernel(const __grid_constant__ WeightMaps<MORE> maps, const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
                        const Groups g, int* __restrict__ status, int test_role, uint32_t test_ns) {
   using SH = Shape<NT>;
   constexpr int STAGES = SH::STAGES, UNIT_N = EPI == GATED ? FEATURES / 2 : FEATURES;
@@ -189,11 +197,18 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         int e, r0, rows;
         group(unit, e, r0, rows);
         if (rows <= 0) continue;
-        const bool own = e < g.matrices || g.always == 0;
-        const CUtensorMap *from = own ? &map_w : &map_s, *from2 = own ? &map_w2 : &map_s2;
-        const int matrix = own ? e : e - g.matrices, row = (unit % blocks_n) * UNIT_N, row2 = EPI == GATED ? row : row + FEATURES / 2;
-        const bool matrix_first = !own && g.piece_first;
-        const int y = matrix_first ? matrix : row, z = matrix_first ? row : matrix, y2 = matrix_first ? matrix : row2, z2 = matrix_first ? row2 : matrix;
+        const CUtensorMap *from = &maps.w, *from2 = &maps.w2;
+        const int row = (unit % blocks_n) * UNIT_N, row2 = EPI == GATED ? row : row + FEATURES / 2;
+        int y = row, z = e, y2 = row2, z2 = e, shift = 0;
+        if constexpr (MORE) {
+          if (e >= g.matrices) {
+            const int piece = e - g.matrices;
+            from = &maps.s, from2 = &maps.s2;
+            y = g.piece_first ? piece : row, z = g.piece_first ? row : piece;
+            y2 = g.piece_first ? piece : row2, z2 = g.piece_first ? row2 : piece;
+            shift = g.shift;
+          }
+        }
         for (int kb = 0; kb < n_k; ++kb, ++it) {
           if (it >= STAGES && !mbar_wait_role(&empty_bar[s], parity, ctl, 61)) {
             give_up_code(status, 61);
@@ -203,7 +218,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           }
           mbar_expect_tx_s(full0 + 8 * s, A_BYTES);
           tma_load_3d_s(dst, from, full0 + 8 * s, kb * BK, y, z);
-          tma_load_3d_s(dst + A_BYTES / 2, from2, full0 + 8 * s, kb * BK, y2, z2);
+          tma_load_3d_s(dst + A_BYTES / 2, from2, full0 + 8 * s, kb * BK + shift, y2, z2);
           dst += SH::STAGE_BYTES;
           if (++s == STAGES) {
             s = 0;
@@ -445,24 +460,32 @@ static int make_weights_map(CUtensorMap* map, const void* w, const Always& a, in
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : 2;
 }
 
-template <typename TO, int EPI, int NT>
+template <typename TO, int EPI, int NT, bool MORE = false>
 static int launch_grouped(const void* w, const void* w2, int matrices, void* out, Groups g, const Always& always, long long max_groups, int* status,
                           int wait_test_role, unsigned int wait_test_ns, cudaStream_t stream) {
   using SH = Shape<NT>;
-  CUtensorMap map_w, map_w2, map_s, map_s2, map_x;
+  WeightMaps<MORE> maps;
+  CUtensorMap map_x;
   g.matrices = matrices;
-  g.always = always.n;
-  g.piece_first = always.piece < always.row;
   const Always dense = {nullptr, nullptr, g.K, (long long)g.N * g.K, matrices};
-  if (make_weights_map(&map_w, w, dense, g.N, g.K) || make_weights_map(&map_w2, EPI == GATED ? w2 : w, dense, g.N, g.K))
+  maps.w2 = {};
+  if (make_weights_map(&maps.w, w, dense, g.N, g.K) || (EPI == GATED && make_weights_map(&maps.w2, w2, dense, g.N, g.K)))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices to TMA");
-  map_s = map_w;
-  map_s2 = map_w2;
-  if (always.n > 0 && (make_weights_map(&map_s, always.w, always, g.N, g.K) || make_weights_map(&map_s2, EPI == GATED ? always.w2 : always.w, always, g.N, g.K)))
-    RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices that take every token to TMA");
+  if (EPI != GATED) maps.w2 = maps.w;
+  if constexpr (MORE) {
+    // Rows of gate and up that alternate are one row of both behind each other, which one description serves (it takes the host 0.4 us); where k
+    // is no multiple of a slice the first one's last slice would run into the second.
+    g.piece_first = always.piece < always.row;
+    const bool both = EPI == GATED && always.w2 == always.w + g.K && always.row >= 2LL * g.K && g.K % BK == 0;
+    g.shift = both ? g.K : 0;
+    if (make_weights_map(&maps.s, always.w, always, g.N, both ? 2 * g.K : g.K) ||
+        (EPI == GATED && !both && make_weights_map(&maps.s2, always.w2, always, g.N, g.K)))
+      RL_REFUSE(9, "grouped_gemm_tc: cannot describe the matrices that take every token to TMA");
+    if (EPI != GATED || both) maps.s2 = maps.s;
+  }
   if (g.order != nullptr ? make_matrix_map(&map_x, g.x, g.x_rows, g.K, (int)g.ldx, 1) : make_rows_map(&map_x, g, SH::BOX_ROWS))
     RL_REFUSE(9, "grouped_gemm_tc: cannot describe the rows to TMA");
-  auto kern = grouped_gemm_tc_kernel<TO, EPI, NT>;
+  auto kern = grouped_gemm_tc_kernel<TO, EPI, NT, MORE>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::SMEM_BYTES) != cudaSuccess)
     RL_REFUSE(5, "grouped_gemm_tc: cannot get %d bytes of shared memory", SH::SMEM_BYTES);
   const int sms = rl_sm_count();
@@ -470,7 +493,7 @@ static int launch_grouped(const void* w, const void* w2, int matrices, void* out
   const int unit_n = EPI == GATED ? FEATURES / 2 : FEATURES;
   const long long units = max_groups * ((g.N + unit_n - 1) / unit_n);
   if (units > 0x7fffffffLL) RL_REFUSE(11, "grouped_gemm_tc: too many units of work");
-  RL_LAUNCH_CHECK(rl_launch(kern, dim3((unsigned)(units < sms ? units : sms)), NUM_THREADS, SH::SMEM_BYTES, stream, map_w, map_w2, map_s, map_s2, map_x, (TO*)out, g,
+  RL_LAUNCH_CHECK(rl_launch(kern, dim3((unsigned)(units < sms ? units : sms)), NUM_THREADS, SH::SMEM_BYTES, stream, maps, map_x, (TO*)out, g,
                             status, wait_test_role, (uint32_t)wait_test_ns));
   return 0;
 }
@@ -541,7 +564,9 @@ RL_API int rl_moe_gemm_tc(const void* x, int ldx, int x_rows, const int* order, 
   g.K = K;
   g.act_alpha = act_alpha;
   g.act_limit = act_limit;
-#define RL_GROUPED(TO, EPI, NT) return launch_grouped<TO, EPI, NT>(w, w2, n_experts, out, g, more, max_tiles, status, wait_test_role, wait_test_ns, stream)
+#define RL_GROUPED(TO, EPI, NT)                                                                                                              \
+  return always > 0 ? launch_grouped<TO, EPI, NT, true>(w, w2, n_experts, out, g, more, max_tiles, status, wait_test_role, wait_test_ns, stream) \
+                    : launch_grouped<TO, EPI, NT>(w, w2, n_experts, out, g, more, max_tiles, status, wait_test_role, wait_test_ns, stream)
 #define RL_GROUPED_ROWS(TO, EPI)               \
   do {                                         \
     if (tile_rows == 32) RL_GROUPED(TO, EPI, 32);   \
