@@ -102,8 +102,8 @@ struct Groups {
 };
 
 // Matrices that take every token (a shared expert in pieces of the others' size), where they lie: feature n of the j-th at w + j * piece +
-// n * row, K numbers (the others' are described to TMA in the same way).  So rows of gate and up that alternate and columns of one wide matrix serve as they are, and no copy beside the
-// others is held.
+// n * row, K numbers (the others' are described to TMA in the same way).  So rows of gate and up that alternate and columns of one wide
+// matrix serve as they are, and no copy beside the others is held.
 struct Always {
   const bf16 *w, *w2;
   long long row, piece;

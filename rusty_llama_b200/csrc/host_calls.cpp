@@ -73,7 +73,7 @@ static PyObject* launcher_call(PyObject* self, PyObject* const* args, size_t nar
     const char kind = l->n >= 0 ? l->kinds[k] : PyFloat_Check(a) ? 'f' : a == Py_None || THPVariable_Check(a) ? 'p' : 'i';
     if (kind == 'f') {
       if (nf == HC_FLOATS) return too_many();
-      const double x = PyFloat_AsDouble(a);
+      const double x = PyFloat_CheckExact(a) ? PyFloat_AS_DOUBLE(a) : PyFloat_AsDouble(a);
       if (x == -1.0 && PyErr_Occurred()) return nullptr;
       f[nf++] = (float)x;
       continue;
@@ -178,16 +178,18 @@ static PyObject* check_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HC_CATCH
 }
 
-// matrices(t, other, what) -> (matrices, rows, columns, row stride, matrix stride) of a 3-D tensor whose rows are dense; other: None or a tensor
-// that has to lie in the same way
+// matrices(t, other, like, what) -> (matrices, rows, columns, row stride, matrix stride) of a 3-D tensor of like's type and device whose rows are
+// dense; other: None or a tensor that has to lie in the same way
 static PyObject* check_matrices(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 3 || !THPVariable_Check(args[0]) || !(args[1] == Py_None || THPVariable_Check(args[1]))) return PyErr_Format(PyExc_TypeError, "matrices(tensor, tensor or None, what)");
+  if (n != 4 || !THPVariable_Check(args[0]) || !(args[1] == Py_None || THPVariable_Check(args[1])) || !THPVariable_Check(args[2]))
+    return PyErr_Format(PyExc_TypeError, "matrices(tensor, tensor or None, tensor, what)");
   HC_TRY
-  const at::Tensor& x = THPVariable_Unpack(args[0]);
-  if (x.dim() != 3 || x.stride(2) != 1) return refuse(args[2], "expected a 3-D tensor with dense rows");
+  const at::Tensor &x = THPVariable_Unpack(args[0]), &like = THPVariable_Unpack(args[2]);
+  if (x.dim() != 3 || x.stride(2) != 1 || x.scalar_type() != like.scalar_type() || x.device() != like.device())
+    return refuse(args[3], "expected a 3-D tensor with dense rows beside the others");
   if (args[1] != Py_None) {
     const at::Tensor& y = THPVariable_Unpack(args[1]);
-    if (y.sizes() != x.sizes() || y.strides() != x.strides()) return refuse(args[2], "two tensors that do not lie in the same way");
+    if (y.sizes() != x.sizes() || y.strides() != x.strides() || y.scalar_type() != x.scalar_type() || y.device() != x.device()) return refuse(args[3], "two tensors that do not lie in the same way");
   }
   return Py_BuildValue("(LLLLL)", (L)x.size(0), (L)x.size(1), (L)x.size(2), (L)x.stride(1), (L)x.stride(0));
   HC_CATCH

@@ -69,11 +69,16 @@ def _build_dir() -> str:
         return _build_dir_cached
 
 
-def _find_build_dir() -> str:
+def _build_dir_candidates() -> List[str]:
     override = os.environ.get("RUSTY_LLAMA_BUILD_DIR")
     cands = [override] if override else []
     cands.append(os.path.join(CSRC_DIR, "_build"))
     cands.append(os.path.join(tempfile.gettempdir(), f"rusty_llama_b200_build_{os.getuid()}"))
+    return cands
+
+
+def _find_build_dir() -> str:
+    cands = _build_dir_candidates()
     for d in cands:
         try:
             os.makedirs(d, exist_ok=True)
@@ -211,17 +216,31 @@ def _is_stamped(out: str, stamp: str, want: str) -> bool:
         return False
 
 
+def built_host_calls():
+    """The module of `csrc/host_calls.cpp` if it is built and current in the folder that a build would use, else None.  Reads files only."""
+    want = _host_fingerprint()
+    for d in _build_dir_candidates() if _build_dir_cached is None else [_build_dir_cached]:
+        if os.path.isdir(d) and os.access(d, os.W_OK):
+            out = os.path.join(d, HOST_CALLS + ".so")
+            return _load_module(out) if _is_stamped(out, ".sha256", want) else None
+    return None
+
+
 def load_host_calls(may_build: bool):
     """The module of `csrc/host_calls.cpp`; None where it is not built and may not be, or did not compile here before (`build_all` tries again)."""
-    import importlib.machinery
-    import importlib.util
-
     out = os.path.join(_build_dir(), HOST_CALLS + ".so")
     want = _host_fingerprint()
     if not _is_stamped(out, ".sha256", want):
         if not may_build or _is_stamped(out, ".failed", want):
             return None
         build_host_calls()
+    return _load_module(out)
+
+
+def _load_module(out: str):
+    import importlib.machinery
+    import importlib.util
+
     loader = importlib.machinery.ExtensionFileLoader(HOST_CALLS, out)
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader(HOST_CALLS, loader))
     loader.exec_module(module)

@@ -2,7 +2,7 @@
 
 `csrc/host_calls.cpp` does this natively (an `add_rmsnorm` with the tensor of its result: 6.2 us instead of 10.9, of which the driver has 3; a
 sublayer of nine kernels: 92 us a pass instead of 165, which is the host's time); the classes and functions below are the same in Python,
-used until a library is first asked for, where that module cannot be built (no Python or PyTorch headers) and where there is no GPU to launch on.
+used until a library is first asked for if that module is not built yet, where it cannot be built (no Python or PyTorch headers) and where there is no GPU to launch on.
 Results and errors are the same.
 """
 
@@ -83,13 +83,14 @@ def python_rows(t: torch.Tensor, what: str) -> int:
     return t.stride(0)
 
 
-def python_matrices(t: torch.Tensor, other: Optional[torch.Tensor], what: str) -> Tuple[int, int, int, int, int]:
-    """(matrices, rows, columns, row stride, matrix stride) of a 3-D tensor whose rows are dense; other: None or one that has to lie in the same way."""
-    if not isinstance(t, torch.Tensor) or not (other is None or isinstance(other, torch.Tensor)):
-        raise TypeError("matrices(tensor, tensor or None, what)")
-    if t.dim() != 3 or t.stride(2) != 1:
-        raise KernelError(f"{what}: expected a 3-D tensor with dense rows")
-    if other is not None and (other.shape != t.shape or other.stride() != t.stride()):
+def python_matrices(t: torch.Tensor, other: Optional[torch.Tensor], like: torch.Tensor, what: str) -> Tuple[int, int, int, int, int]:
+    """(matrices, rows, columns, row stride, matrix stride) of a 3-D tensor of like's type and device whose rows are dense; other: None or one
+    that has to lie in the same way."""
+    if not (isinstance(t, torch.Tensor) and isinstance(like, torch.Tensor) and (other is None or isinstance(other, torch.Tensor))):
+        raise TypeError("matrices(tensor, tensor or None, tensor, what)")
+    if t.dim() != 3 or t.stride(2) != 1 or t.dtype != like.dtype or t.device != like.device:
+        raise KernelError(f"{what}: expected a 3-D tensor with dense rows beside the others")
+    if other is not None and (other.shape != t.shape or other.stride() != t.stride() or other.dtype != t.dtype or other.device != t.device):
         raise KernelError(f"{what}: two tensors that do not lie in the same way")
     return (*t.shape, t.stride(1), t.stride(0))
 
@@ -134,15 +135,16 @@ def bind(namespace: dict, **names: str) -> None:
         namespace.update((own, globals()[name]) for own, name in names.items())
 
 
-def _find_native() -> None:
-    """Takes the native module up, from the first library on: importing this package touches neither CUDA nor a compiler.  It is built
-    where a process that uses a GPU finds it missing; a run of shapes alone stays with Python."""
+def _find_native(importing: bool = False) -> None:
+    """Takes the native module up: at import where it is built, which touches neither CUDA nor a compiler (functions that change under code that
+    has run already cost its calls 1 to 3 us a sublayer), else with the first library.  It is built where a process that uses a GPU finds it
+    missing; a run of shapes alone stays with Python."""
     with _lock:
         if "_module" in globals():
             return
         try:
-            module = build.load_host_calls(torch.cuda.is_initialized())
-            if module is None and not torch.cuda.is_initialized():
+            module = build.built_host_calls() if importing else build.load_host_calls(torch.cuda.is_initialized())
+            if module is None and (importing or not torch.cuda.is_initialized()):
                 return  # (asked again by the next library)
         except Exception as e:  # whatever is missing on this machine: the Python side does the same
             build._say(f"host_calls.cpp is not used: {str(e).strip().splitlines()[-1][:200] if str(e).strip() else type(e).__name__}")
@@ -155,6 +157,9 @@ def _find_native() -> None:
             globals()[name] = getattr(module, name)
         for namespace, names in _bound:
             namespace.update((own, globals()[name]) for own, name in names.items())
+
+
+_find_native(importing=True)
 
 
 def __getattr__(name: str):

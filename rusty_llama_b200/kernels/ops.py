@@ -1455,10 +1455,7 @@ def moe_gemm(
         _need(tuple(w2.shape) == (E, N, K), "moe_gemm: w2 does not match w")
     more, ws_row, ws_piece = 0, 0, 0
     if always is not None:
-        _cuda(always, "moe_gemm always", x.dtype, False)
-        if always2 is not None:
-            _cuda(always2, "moe_gemm always2", x.dtype, False)
-        more, rows, columns, ws_row, ws_piece = _matrices(always, always2, "moe_gemm always")
+        more, rows, columns, ws_row, ws_piece = _matrices(always, always2, w, "moe_gemm always")
         if rows != N or columns != K or (always2 is None) != (w2 is None):
             raise KernelError(f"moe_gemm: always {tuple(always.shape)} does not match w {tuple(w.shape)}")
     out_dtype = out_dtype or x.dtype

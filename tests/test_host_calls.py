@@ -83,8 +83,8 @@ def test_checks_and_views_agree_with_python():
     assert torch.equal(native.columns(t, 1, 4), host.python_columns(t, 1, 4)) and native.columns(t, 1, 4).stride() == (6, 1)
     m = torch.zeros(3, 4, 2, 8)[:, :, 1]
     for x, y in ((m, None), (m, torch.zeros(3, 4, 2, 8)[:, :, 0]), (torch.zeros(8, 3, 4).transpose(0, 1), None)):
-        assert native.matrices(x, y, "m") == host.python_matrices(x, y, "m")
-    assert native.matrices(m, None, "m") == (3, 4, 8, 16, 64)
+        assert native.matrices(x, y, m, "m") == host.python_matrices(x, y, m, "m")
+    assert native.matrices(m, None, m, "m") == (3, 4, 8, 16, 64)
     e = native.empty(t, torch.bfloat16, 3, 5)
     assert e.dtype == torch.bfloat16 and tuple(e.shape) == (3, 5) and e.device == t.device
     w = torch.zeros(64, 64, dtype=torch.bfloat16)
@@ -172,20 +172,27 @@ def test_every_call_gives_a_launcher_as_many_arguments_as_it_takes():
     assert seen > 50
 
 
-def test_importing_touches_neither_cuda_nor_a_compiler():
+def test_importing_touches_neither_cuda_nor_a_compiler(tmp_path):
     import os
     import sys
 
     code = """
-import subprocess, torch
+import os, subprocess, sys, torch
 def never(*a, **k): raise AssertionError("called by the import")
 torch.cuda.is_available = torch.cuda.device_count = torch.cuda.init = torch._C._cuda_getDeviceCount = subprocess.run = subprocess.Popen = never
 import rusty_llama_b200
 from rusty_llama_b200.kernels import host, linear, ops
-assert "_module" not in vars(host) and ops._cuda is host.python_cuda and linear._odd is host.python_odd
+assert (ops._cuda, linear._odd) == ((host.python_cuda, host.python_odd) if "_module" not in vars(host) else (host._module.cuda, host._module.odd))
+assert ("_module" in vars(host)) == sys.argv[1].startswith("built")
 """
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    subprocess.run([sys.executable, "-c", code], cwd=root, check=True)
+    build.build_host_calls()
+    subprocess.run([sys.executable, "-c", code, "built"], cwd=root, check=True)
+    # where it is not built, in a folder of its own: Python until the first library
+    empty = tmp_path / "empty"
+    empty.mkdir()
+    subprocess.run([sys.executable, "-c", code, "missing"], cwd=root, check=True, env=dict(os.environ, RUSTY_LLAMA_BUILD_DIR=str(empty)))
+    assert not list(empty.iterdir())
 
 
 def test_functions_are_native_from_the_first_library_on():
@@ -234,7 +241,8 @@ def test_refusals_agree_with_python(library):
         (lambda k: make(at, False, k), lambda k: python_make(at, False, k), ["f" * 9, "i" * 57]),
         (make(at, False, "pif"), python_make(at, False, "pif"), [(t, 1), (1.5, 1, 1.0), (t, 1.5, 1.0), (t, 1, "x")]),
         (native.rows, host.python_rows, [(3, "r"), (t[0], "r"), (t.t(), "r")]),
-        (native.matrices, host.python_matrices, [(t, None, "m"), (m.transpose(1, 2), None, "m"), (m, m[:1], "m"), (m, m.transpose(0, 1), "m"), (3, m, "m"), (m, 3, "m")]),
+        (native.matrices, host.python_matrices, [(t, None, m, "m"), (m.transpose(1, 2), None, m, "m"), (m, m[:1], m, "m"), (m, m.view(2, 8, 2).transpose(1, 2), m, "m"), (3, m, m, "m"),
+                                                    (m, 3, m, "m"), (m, m, 3, "m"), (m, None, m.double(), "m"), (m, m.double(), m, "m")]),
         (native.odd, host.python_odd, [(t[0], t), (t.view(2, 2, 6), t), (t, i), (3, t), (t, 3)]),
         (native.empty, host.python_empty, [(t, torch.float32), (t, torch.float32, 1, 1, 1, 1, 1), (t, 3, 1), (3, torch.float32, 1), (t, torch.float32, -1)]),
         (native.columns, host.python_columns, [(t, 2, 9), (t, 7, 8), (t, 4, 2), (t[0], 0, 1), (3, 0, 1)]),
